@@ -242,7 +242,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
     __syncwarp();
   } else if (warp == SOFTMAX_WARPS + 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_S = make_idesc(BQ, BKV, 0);
       constexpr uint32_t IDESC_O = make_idesc(BQ, DH, 1);
       // S of tile t into buffer t % 2: needs its keys, and the buffer given back by the threads that

@@ -202,7 +202,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   [[maybe_unused]] int share_row = 0, share_group0 = 0, share_nn = 0;    // worked out before the main loop ends: divisions off the critical path
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       // The weight does not depend on the kernels before this one: its first
       // stages start streaming at once; the rows X wait for the predecessor.
@@ -242,7 +242,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __syncwarp();
     if (DELIVERIES) cluster_wait();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int i = 0; i < num_kb && ok; ++i) {
         const int s = i % STAGES;

@@ -361,7 +361,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   pdl_trigger();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // A cursor walks this CTA's tiles and their K blocks; no division or modulo per K block
       // (one thread issues every copy, and its arithmetic set the pace of the whole pipeline).
       const int total_it = my_tiles * my_kb;
@@ -419,7 +419,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int s = 0;
       uint32_t full_parity = 0;
@@ -718,7 +718,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   pdl_trigger();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int total_it = my_tiles * num_kb;
       struct Cursor { int tile, kx, m0, n0, kb; };
       auto place = [&](Cursor& c) {
@@ -765,7 +765,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       bool ok = true;
       int s = 0;
       uint32_t full_parity = 0;
