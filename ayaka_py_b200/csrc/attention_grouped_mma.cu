@@ -50,7 +50,6 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
   __nv_bfloat16* tiles = Qs + qrows * LDK;                              // NBUF buffers: keys [KT][LDK], values [KT][LDV]
   const int TILE = KT * (LDK + LDV);
   unsigned char* okflag = reinterpret_cast<unsigned char*>(tiles + NBUF * TILE);   // [NBUF][KT]: the key lies on a page
-  pdl_trigger();
   pdl_wait();
   const int QH = a.QH, DK = a.DK, DV = a.DV;
   const int NG = max(a.KH, a.VH), hpg = QH / NG;

@@ -36,7 +36,7 @@ gemm_simt_kernel(TO* C, const TA* __restrict__ A, const TW* __restrict__ W,
                  int M, int N, int K, int act) {
   __shared__ float As[BK][BM + 4];
   __shared__ float Ws[BK][BN + 4];
-  pdl_trigger();
+  if (gridDim.x * gridDim.y <= AYK_FEW_BLOCKS) pdl_trigger();
   pdl_wait();
   const int tid = threadIdx.x;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
@@ -98,10 +98,10 @@ int launch(void* C, const void* A, const void* W, const float* bias, const float
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   bool vec = (K % 4 == 0) && ((uintptr_t)A % 16 == 0) && ((uintptr_t)W % 16 == 0);
   if (vec)
-    ayk_launch(gemm_simt_kernel<TA, TW, TO, true>, grid, dim3(256), 0, stream, (TO*)C, (const TA*)A, (const TW*)W, bias,
+    ayk_launch_as(grid.x * grid.y <= AYK_FEW_BLOCKS, gemm_simt_kernel<TA, TW, TO, true>, grid, dim3(256), 0, stream, (TO*)C, (const TA*)A, (const TW*)W, bias,
                residual, M, N, K, act);
   else
-    ayk_launch(gemm_simt_kernel<TA, TW, TO, false>, grid, dim3(256), 0, stream, (TO*)C, (const TA*)A, (const TW*)W, bias,
+    ayk_launch_as(grid.x * grid.y <= AYK_FEW_BLOCKS, gemm_simt_kernel<TA, TW, TO, false>, grid, dim3(256), 0, stream, (TO*)C, (const TA*)A, (const TW*)W, bias,
                residual, M, N, K, act);
   return ayk_check_launch("ayk_gemm_simt");
 }

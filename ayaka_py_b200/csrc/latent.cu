@@ -214,7 +214,6 @@ head_matvec_kernel(O* __restrict__ out, long long out_row, int out_head, const f
                    int a_head, const W* __restrict__ w, const float* __restrict__ gate, long long gate_row, int gate_head, int gate_col, int T, int N,
                    int K) {
   extern __shared__ __align__(16) float rows[];          // [T][K]
-  pdl_trigger();
   const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = blockIdx.y * MV_WARPS + warp;
   // the weight row does not depend on the kernel before: its first piece is asked for ahead of the wait

@@ -63,7 +63,6 @@ latent_attention_mma_kernel(float* __restrict__ out, float* __restrict__ partial
                             const int* __restrict__ req_pos0, int num_req, int H, int HG, int BR, int rank, int rot,
                             int page_size, float scale_log2, int window, int parts, int part_keys) {
   constexpr int AQ = 16 * WM;
-  pdl_trigger();
   // the last tiles of a request see the most keys: they start first (blocks are handed out in order)
   int tile = gridDim.x - 1 - blockIdx.x, req = -1, q0 = 0, q_len = 0;
   for (int r = 0; r < num_req; ++r) {
@@ -372,7 +371,6 @@ head_matmul_mma_kernel(O* __restrict__ out, long long out_row, int out_head, con
   __shared__ __align__(16) __nv_bfloat16 As[PM * PLD];
   __shared__ __align__(16) __nv_bfloat16 Al[PM * PLD];       // what rounding to bfloat16 left over
   __shared__ __align__(16) __nv_bfloat16 Ws[PN * PLD];
-  pdl_trigger();
   const int h = blockIdx.y, t0 = blockIdx.x * PM, n0 = blockIdx.z * PN;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const __nv_bfloat16* wh = w + (size_t)h * N * K;

@@ -199,7 +199,6 @@ mlstm_chunk_kernel(float* __restrict__ raw, float* __restrict__ nm, float* __res
   float* den = wv + CT;                    // [CT]
   float* nq0 = den + CT;                   // [CT] n_0 . q_t (unscaled)
   float* carry = nq0 + CT;                 // [2] g_C and b_C
-  pdl_trigger();
   const int c0 = blockIdx.x * COLS, h = blockIdx.y, r = blockIdx.z, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   constexpr int SUB = 32 / COLS;                     // groups of COLS lanes in a warp
@@ -504,10 +503,10 @@ AYK_EXPORT int ayk_mlstm(void* out, float* state, const float* proj, long long s
     chunk_configured[narrow].here() = true;
   }
   if (narrow)
-    ayk_launch(mlstm_chunk_kernel<CHUNK_TOKENS, 16>, dim3((DV + 15) / 16, H, num_req), dim3(CTHREADS), smem, stream, raw, nm,
+    ayk_launch_after(mlstm_chunk_kernel<CHUNK_TOKENS, 16>, dim3((DV + 15) / 16, H, num_req), dim3(CTHREADS), smem, stream, raw, nm,
                state, proj, stride, req_q_start, req_slot, H, D, DV, cap);
   else
-    ayk_launch(mlstm_chunk_kernel<CHUNK_TOKENS, 32>, dim3((DV + 31) / 32, H, num_req), dim3(CTHREADS), smem, stream, raw, nm,
+    ayk_launch_after(mlstm_chunk_kernel<CHUNK_TOKENS, 32>, dim3((DV + 31) / 32, H, num_req), dim3(CTHREADS), smem, stream, raw, nm,
                state, proj, stride, req_q_start, req_slot, H, D, DV, cap);
   if (out_dtype == AYK_DTYPE_F32)
     ayk_launch(mlstm_finish_kernel<float>, dim3(T, H), dim3(128), 0, stream, (float*)out, state, (const float*)raw, (const float*)nm,

@@ -504,7 +504,6 @@ moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* __restrict__ a, long l
                 const __nv_bfloat16* __restrict__ w, const int* __restrict__ ids, int top, int gather, int N, int N_w,
                 int Kd, float limit, float slope, float plus, int act, const float* __restrict__ early) {
   extern __shared__ __align__(16) float xs[];          // [Kd]
-  pdl_trigger();
   pdl_wait();
   const int pair = blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
