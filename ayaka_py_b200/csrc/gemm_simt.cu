@@ -4,24 +4,171 @@
 // F.linear (layers/linear/methods.py:73-76); the activation formulas are those
 // of kernel/triton/activation.py:145-154, applied in 32-bit in the epilogue.
 //
-// Tile 64x64x16, 256 threads, 4x4 outputs per thread; products are accumulated
-// in ascending k in one float per output, so a row's result does not depend on
-// which other rows are in the batch.
+// float32 operands: gemm_f32_kernel below.  bfloat16 operands (K no multiple of 8): gemm_simt_kernel, tile
+// 64x64x16, 256 threads, 4x4 outputs per thread, products accumulated in ascending k in one float per output.
+// In both a row's result does not depend on which other rows are in the batch.
 #include "common.cuh"
 
 namespace {
 
 constexpr int BM = 64, BN = 64, BK = 16;
 
-template <typename T>
-__device__ __forceinline__ void load4(const T* p, float (&v)[4]);
-template <>
-__device__ __forceinline__ void load4<float>(const float* p, float (&v)[4]) {
-  float4 x = *reinterpret_cast<const float4*>(p);
-  v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+// ---------------------------------------------------------------- float32 --
+// A tile of TM x 64 outputs; the block's 256 threads are four groups of 64, and of every slab of 32 k each group takes
+// its own eight, so that a tile keeps eight warps busy whatever its height: a group's thread holds TM / 8 x 8 sums and
+// reads, for four k at a time, TM / 8 + 8 float4 from shared memory for 32 * (TM / 8) products.  Slabs arrive by
+// cp.async, three ahead.  At the end the four groups' sums meet in shared memory and are added in one order,
+// (0 + 1) + (2 + 3), the same for every TM: the height is chosen by the row count, a row's result is not.
+//
+// Bound by the FP32 pipes (128 FMA a clock and multiprocessor) and, per tile, by how many multiprocessors have one.  The
+// height is the one whose fullest multiprocessor has the least to do (f32_rows).  Measured for 377 rows, alone and cold
+// (us; before: 64-row tiles, slabs of 16 without copies ahead, 4 x 4 sums a thread): N 2304 K 768 71 -> 57, N 768 K 768
+// 56 -> 29, N 3072 K 768 74 -> 66, N 768 K 3072 207 -> 90; a GPT-2 small layer of 1 row 293 -> 139, of 130 rows 428 -> 286.
+constexpr int FN = 64, FK = 32, FLD = FK + 4, FSTAGES = 4, FGROUPS = 4;      // rows of 36 floats: eight neighbours' 16-byte pieces lie on different banks
+constexpr int f32_stage_floats(int tm) { return (tm + FN) * FLD; }
+constexpr size_t f32_smem(int tm) {
+  const size_t ring = (size_t)FSTAGES * f32_stage_floats(tm), sums = (size_t)FGROUPS * tm * FN;
+  return (ring > sums ? ring : sums) * sizeof(float);
 }
-template <>
-__device__ __forceinline__ void load4<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[4]) {
+
+__device__ __forceinline__ void f32_copy16(float* dst, const float* src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void f32_copy4(float* dst, const float* src, bool on) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 4 : 0) : "memory");
+}
+
+template <int TM, bool VEC>
+__global__ void __launch_bounds__(256, 2)
+gemm_f32_kernel(float* C, const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                const float* residual,               // C and residual may be one buffer (the residual stream in place)
+                int M, int N, int K, int act) {
+  constexpr int RM = TM / 8;
+  extern __shared__ __align__(16) float f32_tiles[];
+  if (gridDim.x * gridDim.y <= AYK_FEW_BLOCKS) pdl_trigger();
+  const int tid = threadIdx.x, group = tid >> 6, tn = tid & 7, tm = (tid >> 3) & 7;
+  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * FN;
+  const int slabs = (K + FK - 1) / FK;
+  // one slab into buffer b; rows past the matrices' ends and k past K are zeros
+  auto fetch = [&](int slab, int b) {
+    float* to = f32_tiles + b * f32_stage_floats(TM);
+    constexpr int PER_ROW = VEC ? FK / 4 : FK, WIDTH = VEC ? 4 : 1;
+    for (int i = tid; i < (TM + FN) * PER_ROW; i += 256) {
+      const int row = i / PER_ROW, c = (i % PER_ROW) * WIDTH, k = slab * FK + c;
+      const bool of_a = row < TM;
+      const int at = of_a ? m0 + row : n0 + row - TM;
+      const bool on = at < (of_a ? M : N) && k < K;
+      const float* src = on ? (of_a ? A : W) + (size_t)at * K + k : A;
+      if (VEC) f32_copy16(to + row * FLD + c, src, on);
+      else f32_copy4(to + row * FLD + c, src, on);
+    }
+  };
+  float acc[RM][8];
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  pdl_wait();
+#pragma unroll
+  for (int st = 0; st < FSTAGES - 1; ++st) {
+    if (st < slabs) fetch(st, st);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int slab = 0; slab < slabs; ++slab) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
+    __syncthreads();                                 // this slab is there for everybody; the one before has been read
+    if (slab + FSTAGES - 1 < slabs) fetch(slab + FSTAGES - 1, (slab + FSTAGES - 1) % FSTAGES);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* as = f32_tiles + (slab % FSTAGES) * f32_stage_floats(TM) + tm * FLD + group * 8;
+    const float* ws = f32_tiles + (slab % FSTAGES) * f32_stage_floats(TM) + (TM + tn) * FLD + group * 8;
+#pragma unroll
+    for (int k = 0; k < 8; k += 4) {
+      float4 a[RM];
+#pragma unroll
+      for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * 8 * FLD + k);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 w = *reinterpret_cast<const float4*>(ws + j * 8 * FLD + k);
+#pragma unroll
+        for (int i = 0; i < RM; ++i) {
+          acc[i][j] = fmaf(a[i].x, w.x, acc[i][j]);
+          acc[i][j] = fmaf(a[i].y, w.y, acc[i][j]);
+          acc[i][j] = fmaf(a[i].z, w.z, acc[i][j]);
+          acc[i][j] = fmaf(a[i].w, w.w, acc[i][j]);
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();                                   // the ring is free for the sums
+  float* mine = f32_tiles + group * TM * FN;
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mine[(tm + 8 * i) * FN + tn + 8 * j] = acc[i][j];
+  __syncthreads();
+  const int col = tid & (FN - 1), n = n0 + col;
+  if (n >= N) return;
+  const float b = bias ? bias[n] : 0.f;
+#pragma unroll
+  for (int r = tid / FN; r < TM; r += 256 / FN) {
+    const int m = m0 + r;
+    if (m >= M) break;
+    const float* at = f32_tiles + r * FN + col;
+    float v = ((at[0] + at[TM * FN]) + (at[2 * TM * FN] + at[3 * TM * FN])) + b;
+    v = apply_activation(v, act);
+    if (residual) v += residual[(size_t)m * N + n];
+    C[(size_t)m * N + n] = v;
+  }
+}
+
+// Rows per tile: the least work on the fullest multiprocessor, a multiprocessor taking whole tiles one after the other
+// (two at a time do not make it faster: the pipes are the bound).  Lower tiles read more of shared memory per product and
+// pay the same for a slab's barrier, which is what the factors say.
+int f32_rows(int M, int N, int sms) {
+  const int heights[4] = {64, 32, 16, 8};
+  const double factor[4] = {1.0, 1.2, 1.6, 2.6};
+  int best = 64;
+  double least = -1.0;
+  for (int i = 0; i < 4; ++i) {
+    const long tiles = (long)((M + heights[i] - 1) / heights[i]) * ((N + FN - 1) / FN);
+    const double work = (double)((tiles + sms - 1) / sms) * heights[i] * factor[i];
+    if (least < 0 || work < least) { least = work; best = heights[i]; }
+  }
+  return best;
+}
+
+template <int TM, bool VEC>
+int launch_f32(float* C, const float* A, const float* W, const float* bias, const float* residual, int M, int N, int K, int act,
+               cudaStream_t stream) {
+  static AykPerDevice configured;
+  bool& done = configured.here();
+  if (!done) {
+    cudaError_t err = cudaFuncSetAttribute(gemm_f32_kernel<TM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f32_smem(TM));
+    if (err != cudaSuccess) return ayk_fail("ayk_gemm_simt: shared memory %zu: %s", f32_smem(TM), cudaGetErrorString(err));
+    done = true;
+  }
+  dim3 grid((N + FN - 1) / FN, (M + TM - 1) / TM);
+  AYK_REQUIRE(grid.y <= 65535, "ayk_gemm_simt: M = %d exceeds %d rows", M, 65535 * TM);
+  ayk_launch_as(grid.x * grid.y <= AYK_FEW_BLOCKS, gemm_f32_kernel<TM, VEC>, grid, dim3(256), f32_smem(TM), stream, C, A, W, bias, residual,
+                M, N, K, act);
+  return ayk_check_launch("ayk_gemm_simt");
+}
+
+template <bool VEC>
+int launch_f32_rows(float* C, const float* A, const float* W, const float* bias, const float* residual, int M, int N, int K, int act,
+                    cudaStream_t stream) {
+  switch (f32_rows(M, N, ayk_sm_count())) {
+    case 64: return launch_f32<64, VEC>(C, A, W, bias, residual, M, N, K, act, stream);
+    case 32: return launch_f32<32, VEC>(C, A, W, bias, residual, M, N, K, act, stream);
+    case 16: return launch_f32<16, VEC>(C, A, W, bias, residual, M, N, K, act, stream);
+    default: return launch_f32<8, VEC>(C, A, W, bias, residual, M, N, K, act, stream);
+  }
+}
+
+// --------------------------------------------------------------- bfloat16 --
+
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
   uint2 x = *reinterpret_cast<const uint2*>(p);
   __nv_bfloat162 a = *reinterpret_cast<__nv_bfloat162*>(&x.x);
   __nv_bfloat162 b = *reinterpret_cast<__nv_bfloat162*>(&x.y);
@@ -48,8 +195,8 @@ gemm_simt_kernel(TO* C, const TA* __restrict__ A, const TW* __restrict__ W,
     float a[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
     const int gm = m0 + lr, gn = n0 + lr, gk = k0 + lk;
     if (VEC) {
-      if (gm < M && gk < K) load4<TA>(A + (size_t)gm * K + gk, a);
-      if (gn < N && gk < K) load4<TW>(W + (size_t)gn * K + gk, w);
+      if (gm < M && gk < K) load4(A + (size_t)gm * K + gk, a);
+      if (gn < N && gk < K) load4(W + (size_t)gn * K + gk, w);
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -116,8 +263,11 @@ AYK_EXPORT int ayk_gemm_simt(void* C, const void* A, const void* W, const float*
   if (M == 0 || N == 0) return 0;
   AYK_REQUIRE(K >= 1, "ayk_gemm_simt: K must be positive");
   AYK_REQUIRE((M + BM - 1) / BM <= 65535, "ayk_gemm_simt: M = %d exceeds %d rows", M, 65535 * BM);
-  if (in_dtype == AYK_DTYPE_F32 && out_dtype == AYK_DTYPE_F32)
-    return launch<float, float, float>(C, A, W, bias, residual, M, N, K, act, stream);
+  if (in_dtype == AYK_DTYPE_F32 && out_dtype == AYK_DTYPE_F32) {
+    const bool vec = K % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+    return vec ? launch_f32_rows<true>((float*)C, (const float*)A, (const float*)W, bias, residual, M, N, K, act, stream)
+               : launch_f32_rows<false>((float*)C, (const float*)A, (const float*)W, bias, residual, M, N, K, act, stream);
+  }
   if (in_dtype == AYK_DTYPE_BF16 && out_dtype == AYK_DTYPE_F32)
     return launch<__nv_bfloat16, __nv_bfloat16, float>(C, A, W, bias, residual, M, N, K, act, stream);
   if (in_dtype == AYK_DTYPE_BF16 && out_dtype == AYK_DTYPE_BF16)

@@ -142,6 +142,22 @@ ATTENTION_CASES = [
 ]
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 64, 4), (8, 65, 31), (9, 768, 768), (40, 2304, 100), (377, 768, 96), (700, 2304, 33)])
+def test_gemm_simt_float32_tiles(M, N, K):
+    """Every tile height with ragged edges, within the rounding of the four groups' sums (a product and an addition per
+    term and two more additions, each off by at most 2^-24), and a row the same bits whatever tile it is in."""
+    from ayaka_py_b200 import ops
+    rs = np.random.RandomState(3)
+    a, w = rs.randn(M, K).astype(np.float32), rs.randn(N, K).astype(np.float32)
+    A, W = dev(a), dev(w)
+    out = ops.gemm_simt(A, W)
+    want = a.astype(np.float64) @ w.astype(np.float64).T
+    bound = (K / 4 + 12) * 2.0 ** -24 * (np.abs(a).astype(np.float64) @ np.abs(w).astype(np.float64).T)
+    assert (np.abs(out.cpu().numpy() - want) <= bound).all()
+    last = ops.gemm_simt(A[M - 1:].contiguous(), W)
+    assert torch.equal(last, out[M - 1:])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("case", ATTENTION_CASES)
 def test_append_then_attention(dtype, case):
