@@ -173,6 +173,20 @@ def test_append_then_attention(dtype, case):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("lens_q,lens_ctx,Dh,window", [([63, 1, 66], [1, 127, 62], 64, None), ([65], [64], 65, 33), ([8, 25], [120, 0], 128, 64),
+                                                       ([31, 2], [1, 63], 129, None), ([33], [31], 192, 32), ([2, 9], [95, 0], 193, None)])
+def test_attention_simt_tile_edges(dtype, lens_q, lens_ctx, Dh, window):
+    """Edges of the row tiles (8 rows a warp, 32 a block), of the key tiles (64, or 32 for heads beyond 128) and of the
+    runs of 64 head-dim columns."""
+    from ayaka_py_b200 import ops
+    x, plain = paged_case(np.random.RandomState(12), lens_q, lens_ctx, 2, 1, Dh, 16, dtype)
+    ops.kv_append(x["kc"], x["vc"], x["k"], x["v"], x["row_req"], x["pos"], x["table"])
+    out = ops.attention_simt(x["q"], x["kc"], x["vc"], x["table"], x["q_start"], x["pos0"], sum(lens_q), 2, 0.7 / np.sqrt(Dh),
+                             window).float().cpu().numpy()
+    assert np.abs(out - plain(0.7 / np.sqrt(Dh), window)).max() < tol(dtype)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("qpos,kpos", [(299, 0), (299, 15), (299, 16), (255, 127), (256, 128)])
 def test_far_key_stands_out(dtype, qpos, kpos):
     """One query's score for one far key (at a page's edge) is made large, so
