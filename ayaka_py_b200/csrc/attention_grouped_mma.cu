@@ -40,7 +40,10 @@ __device__ __forceinline__ void cp_async_16(void* dst, const void* src, bool val
 
 // DVT: the value width rounded up to 32, 64 or 128 (O's registers); KT: keys per tile; DKP: the key
 // width rounded up to a multiple of 16 (the padding is zeros in shared memory).
-template <int DVT, int KT>
+// SPLIT: a step of single rows whose heads of a group fit one warp's 16 rows.  The four warps then share the rows and
+// each takes a quarter of every tile's keys, with a running softmax and sums of its own that meet at the end; with the
+// rows dealt out instead one warp did all products (64 keys of 128 numbers: 128 mma.sync, 1.7 us) and three looked on.
+template <int DVT, int KT, bool SPLIT>
 __global__ void __launch_bounds__(128, DVT > 64 && KT == 64 ? 2 : 3)
 grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int qrows) {
   const int LDK = DKP + 8;
@@ -77,6 +80,8 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
   const int k_last = a.part_keys > 0 ? min(last_pos, k_first + a.part_keys - 1) : last_pos;
   if (k_first > last_pos) return;                   // the merge does not read parts beyond the context
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+  constexpr int KW = SPLIT ? KT / 4 : KT;               // keys of a tile that a warp takes
+  const int wrow = SPLIT ? 0 : warp * 16, wkey = SPLIT ? warp * KW : 0;      // its first row, its first key of a tile
   const int* my_table = a.table + (size_t)req * a.table_stride;
   const int page_mask = (1 << page_shift) - 1;
   const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(a.q);
@@ -141,7 +146,7 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
   float slope2[2];
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
-    const int m = warp * 16 + gid + half * 8;
+    const int m = wrow + gid + half * 8;
     const int tok = m / hpg;
     qpos[half] = m < rows ? pos0 + tok : -1;                       // a dead row sees nothing
     cstart[half] = (a.chunk > 0 && m < rows) ? (pos0 + tok) / a.chunk * a.chunk : 0;      // first key of the row's own chunk
@@ -154,16 +159,16 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
 #pragma unroll
     for (int c = 0; c < 4; ++c) o[nt][c] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};     // l: this thread's share of the row's denominator
-  if (a.sinks && part == 0) {                          // the sink counts once per row: in the first part, one of the row's four threads
+  if (a.sinks && part == 0 && (!SPLIT || warp == 0)) {                          // the sink counts once per row: in the first part, one of the row's four threads
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      const int m = warp * 16 + gid + half * 8;
+      const int m = wrow + gid + half * 8;
       if (m >= rows) continue;
       m_run[half] = a.sinks[g * hpg + m % hpg] * LOG2E;
       l_run[half] = tig == 0 ? 1.f : 0.f;
     }
   }
-  const uint32_t q_addr = (uint32_t)__cvta_generic_to_shared(Qs + (warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDK + (lane >> 4) * 8);
+  const uint32_t q_addr = (uint32_t)__cvta_generic_to_shared(Qs + (wrow + (lane & 7) + ((lane >> 3) & 1) * 8) * LDK + (lane >> 4) * 8);
   const int ksteps = DKP / 16;
 
   int buf = 0;
@@ -177,22 +182,22 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
     __syncthreads();
     const __nv_bfloat16* Ks = tiles + buf * TILE;
     const __nv_bfloat16* Vs = Ks + KT * LDK;
-    if (warp * 16 < rows) {                            // a warp without live rows only helps with the loads
-      // S = Q K^T: KT / 8 tiles of 8 keys
-      float sc[KT / 8][4];
+    if (wrow < rows) {                                 // a warp without live rows only helps with the loads
+      // S = Q K^T: KW / 8 tiles of 8 keys
+      float sc[KW / 8][4];
 #pragma unroll
-      for (int nt = 0; nt < KT / 8; ++nt)
+      for (int nt = 0; nt < KW / 8; ++nt)
 #pragma unroll
         for (int c = 0; c < 4; ++c) sc[nt][c] = 0.f;
       // key fragments four 8x8 matrices at a time: (keys 0-7 | 8-15 of a pair of tiles) x (dimensions 0-7 | 8-15)
-      const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(Ks + ((lane >> 4) * 8 + (lane & 7)) * LDK + ((lane >> 3) & 1) * 8);
+      const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(Ks + (wkey + (lane >> 4) * 8 + (lane & 7)) * LDK + ((lane >> 3) & 1) * 8);
 #pragma unroll 2
       for (int ks = 0; ks < ksteps; ++ks) {
         uint32_t qf[4];
         asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                      : "=r"(qf[0]), "=r"(qf[1]), "=r"(qf[2]), "=r"(qf[3]) : "r"(q_addr + ks * 32));
 #pragma unroll
-        for (int np = 0; np < KT / 16; ++np) {
+        for (int np = 0; np < KW / 16; ++np) {
           uint32_t b0, b1, b2, b3;
           asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                        : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(k_addr + (uint32_t)(np * 16 * LDK + ks * 16) * 2u));
@@ -200,16 +205,16 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
           mma_bf16(sc[2 * np + 1], qf, b2, b3);
         }
       }
-      // scores in base 2, masked; fragment element c of tile nt: row gid + 8 (c / 2), key k0 + 8 nt + 2 tig + (c & 1)
+      // scores in base 2, masked; fragment element c of tile nt: row gid + 8 (c / 2), key k0 + wkey + 8 nt + 2 tig + (c & 1)
       const bool inside = k0 + KT - 1 <= min(pos0, k_last) && (a.window <= 0 || last_pos - k0 < a.window) &&
                           (a.chunk <= 0 || k0 >= last_pos / a.chunk * a.chunk);   // dead rows are never written
-      const unsigned char* ok = okflag + buf * KT + tig * 2;
+      const unsigned char* ok = okflag + buf * KT + wkey + tig * 2;
       float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-      for (int nt = 0; nt < KT / 8; ++nt)
+      for (int nt = 0; nt < KW / 8; ++nt)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const int key = k0 + nt * 8 + tig * 2 + (c & 1), i = qpos[c >> 1];
+          const int key = k0 + wkey + nt * 8 + tig * 2 + (c & 1), i = qpos[c >> 1];
           float s = fmaf(-slope2[c >> 1], (float)(i - key), sc[nt][c] * scale2);
           if (!inside) {
             const bool seen = key <= min(i, k_last) && (a.window <= 0 || i - key < a.window || key < a.keep_first) &&
@@ -232,7 +237,7 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
       }
       float sum[2] = {0.f, 0.f};
 #pragma unroll
-      for (int nt = 0; nt < KT / 8; ++nt)
+      for (int nt = 0; nt < KW / 8; ++nt)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const float p = fast_exp2(sc[nt][c] - mx[c >> 1]);
@@ -248,7 +253,7 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
       }
       // O += P V: the 32-bit weights enter the product rounded to bfloat16, as the values they multiply are
 #pragma unroll
-      for (int ks = 0; ks < KT / 16; ++ks) {
+      for (int ks = 0; ks < KW / 16; ++ks) {
         uint32_t pf[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
@@ -257,7 +262,7 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
         for (int np = 0; np < DVT / 16; ++np) {
           // two value tiles (16 columns) at a time: four 8x8 matrices, transposed on the way in
           uint32_t b0, b1, b2, b3;
-          const __nv_bfloat16* at = Vs + (ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDV + np * 16 + (lane >> 4) * 8;
+          const __nv_bfloat16* at = Vs + (wkey + ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDV + np * 16 + (lane >> 4) * 8;
           const uint32_t addr = (uint32_t)__cvta_generic_to_shared(at);
           asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                        : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(addr));
@@ -272,12 +277,69 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
     k2 = k3;
   }
 
+  if constexpr (SPLIT) {
+    // the warps' maxima, sums and O of the (up to 16) rows meet in the tiles' shared memory, in warp order
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    constexpr int LDO = DVT + 4;
+    float* So = reinterpret_cast<float*>(tiles);        // [4 warps][16 rows][LDO]
+    float2* Sml = reinterpret_cast<float2*>(So + 4 * 16 * LDO);      // [4 warps][16 rows]
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      float l = l_run[half];
+      l += __shfl_xor_sync(0xffffffffu, l, 1);
+      l += __shfl_xor_sync(0xffffffffu, l, 2);
+      const int r = gid + half * 8;
+      if (tig == 0) Sml[warp * 16 + r] = make_float2(m_run[half], l);
+#pragma unroll
+      for (int nt = 0; nt < DVT / 8; ++nt)
+        *reinterpret_cast<float2*>(So + (warp * 16 + r) * LDO + nt * 8 + tig * 2) = make_float2(o[nt][half * 2], o[nt][half * 2 + 1]);
+    }
+    __syncthreads();
+    const int D4 = DV / 4;                              // DV is a multiple of 8
+    for (int i = tid; i < rows * D4; i += 128) {
+      const int r = i / D4, col = (i - r * D4) * 4;
+      float m = -INFINITY, l = 0.f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) m = fmaxf(m, Sml[w * 16 + r].x);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const float2 ml = Sml[w * 16 + r];
+        const float f = m > -INFINITY ? fast_exp2(ml.x - m) : 0.f;
+        const float4 x = *reinterpret_cast<const float4*>(So + (w * 16 + r) * LDO + col);
+        l = fmaf(ml.y, f, l);
+        v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
+      }
+      const int head = g * hpg + r;                     // one row a request: the rows are its heads of this group
+      const size_t head_at = (size_t)row0 * QH + head;
+      if (a.partial_o) {
+        *reinterpret_cast<float4*>(a.partial_o + ((size_t)part * a.total_rows * QH + head_at) * DV + col) = v;
+        if (col == 0) {
+          float* pml = a.partial_ml + ((size_t)part * a.total_rows * QH + head_at) * 2;
+          pml[0] = m * LN2;                             // the merge works in base e
+          pml[1] = l;
+        }
+      } else {
+        const float inv = l > 0.f ? 1.0f / l : 0.f;
+        v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+        if (a.gate) {
+          const float* gate = a.gate + (size_t)row0 * a.gate_stride + (size_t)head * DV + col;
+          v.x = __fdividef(v.x, 1.0f + __expf(-gate[0])); v.y = __fdividef(v.y, 1.0f + __expf(-gate[1]));
+          v.z = __fdividef(v.z, 1.0f + __expf(-gate[2])); v.w = __fdividef(v.w, 1.0f + __expf(-gate[3]));
+        }
+        uint2 packed = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(a.out) + head_at * DV + col) = packed;
+      }
+    }
+    return;
+  }
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     float l = l_run[half];
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
-    const int m = warp * 16 + gid + half * 8;
+    const int m = wrow + gid + half * 8;
     if (m >= rows) continue;
     const int tok = m / hpg, head = g * hpg + (m - tok * hpg);
     const size_t head_at = (size_t)(row0 + tok) * QH + head;
@@ -320,18 +382,18 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
   }
 }
 
-template <int DVT, int KT>
+template <int DVT, int KT, bool SPLIT>
 int launch(const GroupedArgs& a, int page_shift, int tq, int DKP, int qrows, size_t smem, dim3 grid, cudaStream_t stream) {
   static AykPerDevice granted;
   static size_t most = 0;
   if (!granted.here() || smem > most) {
-    cudaError_t e = cudaFuncSetAttribute(grouped_attention_mma_kernel<DVT, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(grouped_attention_mma_kernel<DVT, KT, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(227 * 1024));
     if (e != cudaSuccess) return ayk_fail("ayk_grouped_attention: shared memory %zu: %s", smem, cudaGetErrorString(e));
     granted.here() = true;
     most = 227 * 1024;
   }
-  ayk_launch(grouped_attention_mma_kernel<DVT, KT>, grid, dim3(128), smem, stream, a, page_shift, tq, DKP, qrows);
+  ayk_launch(grouped_attention_mma_kernel<DVT, KT, SPLIT>, grid, dim3(128), smem, stream, a, page_shift, tq, DKP, qrows);
   return ayk_check_launch("ayk_grouped_attention (tensor cores)");
 }
 
@@ -364,8 +426,14 @@ int ayk_grouped_attention_mma(const GroupedArgs& a, cudaStream_t stream) {
   const size_t smem = smem_bytes(DKP, DVT, KT, qrows);
   if (smem > 227 * 1024) return 1;
   dim3 grid(single ? a.total_rows : a.total_rows / tq + a.num_req, NG, a.parts);
+  // 64 keys a tile split 16 to a warp (the sums' meeting place, 4 x 16 rows of DVT + 4 floats and their maxima, fits the three tiles)
+  const bool split = single && KT == 64 && qrows == 16;
 #define AYK_GROUPED(V, K) \
-  if (DVT == V && KT == K) return launch<V, K>(a, page_shift, tq, DKP, qrows, smem, grid, stream);
+  if (DVT == V && KT == K && !split) return launch<V, K, false>(a, page_shift, tq, DKP, qrows, smem, grid, stream);
+#define AYK_GROUPED_SPLIT(V) \
+  if (DVT == V && split) return launch<V, 64, true>(a, page_shift, tq, DKP, qrows, smem, grid, stream);
+  AYK_GROUPED_SPLIT(32) AYK_GROUPED_SPLIT(64) AYK_GROUPED_SPLIT(128)
+#undef AYK_GROUPED_SPLIT
   AYK_GROUPED(32, 64) AYK_GROUPED(64, 64) AYK_GROUPED(128, 64) AYK_GROUPED(32, 32) AYK_GROUPED(64, 32) AYK_GROUPED(128, 32)
 #undef AYK_GROUPED
   return 1;

@@ -442,6 +442,39 @@ def test_attention_on_the_tensor_cores_against_the_fp32_pipes(step, QH, KH, VH, 
     cache.rollback(res)
 
 
+@pytest.mark.parametrize("QH,KH,DV,window,sinks", [(32, 8, 128, None, True), (8, 8, 64, None, False), (128, 8, 32, 300, True),
+                                                   (24, 2, 96, None, True), (8, 8, 128, None, False)])
+def test_single_rows_whose_keys_the_warps_share(QH, KH, DV, window, sinks):
+    """Contexts that end at the edges of the warps' 16 keys, of the 64-key tiles and of partitions of 64 to 256 keys
+    (which grow with requests times groups), sinks, and a context short enough not to be cut."""
+    from ayaka_py_b200 import ops
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts.base import KVNeed
+    torch.manual_seed(QH + DV)
+    DK = 64
+    need = KVNeed(kv_heads=KH, head_dim=DK, window=window, value_heads=KH, value_dim=DV)
+    for positions, before in ((1024, [0, 1, 15, 16, 62, 63, 64, 127, 128, 255, 256, 511, 1000]), (64, [0, 15, 16, 63])):
+        cache, runner = context_for([CacheGroupSpec("g", need, 1)], "bfloat16", max_requests=len(before), page_size=16, pages=260,
+                                    positions=positions)
+        kpages, vpages = cache.kv_layer(0, 0)
+        kpages.copy_(torch.randn(kpages.shape, device="cuda") * 0.7)
+        vpages.copy_(torch.randn(vpages.shape, device="cuda"))
+        for i, n in enumerate(before):
+            slot = cache.open(i)
+            if n:
+                cache.commit(cache.reserve([(slot, 0, n)]))
+        ctx, res = step_of(cache, runner, {i: 1 for i in range(len(before))})
+        q = (torch.randn(ctx.num_rows, QH * DK, device="cuda") * 0.4).to(torch.bfloat16)
+        gate = torch.randn(ctx.num_rows, QH * DV, device="cuda")
+        kw = dict(heads=QH, key_heads=KH, key_dim=DK, scale=0.8, window=window, gate=gate,
+                  sinks=torch.randn(QH, device="cuda") if sinks else None)
+        got = ops.grouped_attention(q, kpages, vpages, ctx.tables[0], ctx, tensor_cores=True, **kw).float()
+        want = ops.grouped_attention(q, kpages, vpages, ctx.tables[0], ctx, tensor_cores=False, **kw).float()
+        assert torch.isfinite(got).all()
+        assert float((got - want).abs().max()) < 1.5e-2 * float(want.abs().max())
+        cache.rollback(res)
+
+
 def test_lambda_and_the_scaling_after_the_difference():
     """The layer's factor from its four vectors, and values the given sizes would hide: diff 0 and a
     second map that weighs more than the first."""
