@@ -12,9 +12,9 @@
 // compute dtype.  z_q, z_k, v, z_i, z_f and the gate are columns of one projection row:
 // [q (H D) | k (H D) | v (H DV) | z_i (H) | z_f (H) | gate (H DV)].  Everything here is 32-bit.
 //
-// Two forms.  mlstm_walk_kernel takes the tokens one by one, a block per (request, head): the step of a
+// Three forms.  mlstm_walk_kernel takes the tokens one by one, a block per (request, head): the step of a
 // request that brings one token reads and writes its state once, and the head's norm and gate are applied
-// in the same kernel.  mlstm_chunk_kernel takes CT tokens at a time (prompt portions).  Inside a chunk, with
+// in the same kernel.  mlstm_chunk_kernel takes CT tokens at a time (prompt portions; long ones: mlstm_long_*, below).  Inside a chunk, with
 // b_t = sum_(r<=t) f_r, a_s = i_s - b_s and g_t = max(m_0, max_(s<=t) a_s), the recurrence of m unrolls to
 // m_t = b_t + g_t, and
 //   S_t^T q_t = e^(m_0 - g_t) S_0^T q_t + sum_(s<=t) e^(a_s - g_t) (k_s . q_t) v_s
@@ -430,6 +430,398 @@ mlstm_finish_kernel(C* __restrict__ out, float* __restrict__ state, const float*
   }
 }
 
+// ---------------------------------------------------------- long portions --
+// The chunked form above walks a portion's chunks one after the other, and a block's chain of 16 tokens (5.6 us) sets
+// the time whatever the width.  For long portions the chunks of LC tokens go side by side, in three kernels:
+//   mlstm_long_sum    a chunk's own share of the memory, against its own maximum G = max_s a_s:
+//                     dS = sum_s e^(a_s - G) k_s v_s^T, dn likewise; G and B = b_C beside them
+//   mlstm_long_scan   per cell of the memory, over the chunks: leaves every chunk's S_0, n_0, m_0 in the place of its dS
+//                     (S' = e^(m - m') S + e^(G - m') dS with m' = max(m, G), then m = B + m'), and files the last into the state
+//   mlstm_long_out    a chunk's outputs from its S_0, n_0, m_0 (formulas above), with the head's norm and gate applied
+// All three are float32; the products are register tiles fed with float4 from shared memory (8 x 8 sums a thread in the
+// first, 4 x 4 and 4 x 8 in the last), bound by the FP32 pipes and shared memory; the memories' round trips
+// (4 x 64 KB a chunk and head of 128 x 128) stay in the L2 for portions of a few thousand tokens.
+// Measured for the layer at 16 heads of 128 x 128 (us; before: the chunked form): 1,024 and 777 tokens 471 -> 261; at 8 heads
+// 2 x 1,024 tokens 461 -> 131, 2 x 200 113 -> 70, 2 x 17 (the chunked form) 64.  The line lies at one whole chunk: 64 tokens.
+constexpr int LC = 64, LMAX = 128, LLD = LMAX + 4, LTHREADS = 256;
+
+__device__ __forceinline__ void cp_async_16(float* dst, const float* src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+
+// Which chunk of which request is chunk `ci` of the step?  false: there is none.
+__device__ __forceinline__ bool find_chunk(int ci, const int* __restrict__ req_q_start, int num_req, int& r, int& row0, int& L, int& c) {
+  for (r = 0; r < num_req; ++r) {
+    const int first = req_q_start[r], len = req_q_start[r + 1] - first, n = (len + LC - 1) / LC;
+    if (ci < n) {
+      c = ci;
+      row0 = first + ci * LC;
+      L = min(LC, len - ci * LC);
+      return true;
+    }
+    ci -= n;
+  }
+  return false;
+}
+
+// Lane l of one warp: tokens 2 l and 2 l + 1 of a chunk.  a = i - b with b the sum of f from the chunk's start on (minus
+// infinity past its end), the prefix maximum of a, b itself; returns G and B in every lane.
+__device__ __forceinline__ void chunk_gates(const float* proj, long long stride, int row0, int L, int icol, int fcol, float cap, int lane,
+                                            float (&a)[2], float (&top)[2], float (&b)[2], float& G, float& B) {
+  float f[2], i[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int t = 2 * lane + e;
+    i[e] = -INFINITY;
+    f[e] = 0.f;
+    if (t < L) {
+      const float* row = proj + (size_t)(row0 + t) * stride;
+      i[e] = cap * tanhf(row[icol] / cap);
+      f[e] = log_sigmoid(cap * tanhf(row[fcol] / cap));
+    }
+  }
+  float sum = f[0] + f[1];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float up = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= o) sum += up;
+  }
+  b[1] = sum;
+  b[0] = sum - f[1];
+  a[0] = i[0] - b[0];
+  a[1] = i[1] - b[1];
+  float m = fmaxf(a[0], a[1]);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float up = __shfl_up_sync(0xffffffffu, m, o);
+    if (lane >= o) m = fmaxf(m, up);
+  }
+  const float before = __shfl_up_sync(0xffffffffu, m, 1);
+  top[0] = lane > 0 ? fmaxf(before, a[0]) : a[0];
+  top[1] = m;
+  G = __shfl_sync(0xffffffffu, m, 31);
+  B = __shfl_sync(0xffffffffu, sum, 31);
+}
+
+struct LongScratch {
+  float* S;        // [chunks][H][D * DV]
+  float* n;        // [chunks][H][D]
+  float* gb;       // [chunks][H][2]: G, B
+  float* m;        // [chunks][H]: m_0
+  float* m_end;    // [requests][H]
+};
+__host__ __device__ inline long long long_chunks(int T, int num_req) { return (long long)T / LC + num_req; }
+__host__ __device__ inline LongScratch long_scratch(float* base, long long chunks, int H, int D, int DV) {
+  LongScratch x;
+  x.S = base;
+  x.n = x.S + chunks * H * D * DV;
+  x.gb = x.n + chunks * H * D;
+  x.m = x.gb + chunks * H * 2;
+  x.m_end = x.m + chunks * H;
+  return x;
+}
+
+constexpr size_t LONG_SUM_SMEM = (size_t)(2 * LC * LLD + LC) * sizeof(float);
+__global__ void __launch_bounds__(LTHREADS, 2)
+mlstm_long_sum_kernel(LongScratch x, const float* __restrict__ proj, long long stride, const int* __restrict__ req_q_start, int num_req,
+                      int H, int D, int DV, float cap) {
+  extern __shared__ __align__(16) float sm[];
+  float* Ks = sm;                      // [LC][LLD], each row times its token's weight
+  float* Vs = Ks + LC * LLD;           // [LC][LLD]
+  float* w = Vs + LC * LLD;            // [LC]
+  const int h = blockIdx.y, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const MlstmCols col(H, D, DV);
+  int r, row0, L, c;
+  pdl_wait();
+  if (!find_chunk(blockIdx.x, req_q_start, num_req, r, row0, L, c)) return;
+  for (int i = tid; i < LC * (LMAX / 4); i += LTHREADS) {
+    const int t = i / (LMAX / 4), d = (i % (LMAX / 4)) * 4;
+    const float* row = proj + (size_t)(row0 + min(t, L - 1)) * stride;
+    cp_async_16(Ks + t * LLD + d, row + col.k + h * D + (d < D ? d : 0), t < L && d < D);
+    cp_async_16(Vs + t * LLD + d, row + col.v + h * DV + (d < DV ? d : 0), t < L && d < DV);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  if (tid < 32) {
+    float a[2], top[2], b[2], G, B;
+    chunk_gates(proj, stride, row0, L, col.i + h, col.f + h, cap, tid, a, top, b, G, B);
+    w[2 * tid] = expf(a[0] - G);
+    w[2 * tid + 1] = expf(a[1] - G);
+    if (tid == 0) *reinterpret_cast<float2*>(x.gb + ((size_t)blockIdx.x * H + h) * 2) = make_float2(G, B);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  for (int i = tid; i < LC * (LMAX / 4); i += LTHREADS) {
+    const int t = i / (LMAX / 4);
+    float4* at = reinterpret_cast<float4*>(Ks + t * LLD + (i % (LMAX / 4)) * 4);
+    float4 v = *at;
+    v.x *= w[t]; v.y *= w[t]; v.z *= w[t]; v.w *= w[t];
+    *at = v;
+  }
+  __syncthreads();
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
+  for (int s = 0; s < L; ++s) {
+    float k[8], v[8];
+    *reinterpret_cast<float4*>(k) = *reinterpret_cast<const float4*>(Ks + s * LLD + ty * 4);
+    *reinterpret_cast<float4*>(k + 4) = *reinterpret_cast<const float4*>(Ks + s * LLD + 64 + ty * 4);
+    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(Vs + s * LLD + tx * 4);
+    *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(Vs + s * LLD + 64 + tx * 4);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(k[i], v[j], acc[i][j]);
+  }
+  float* S = x.S + ((size_t)blockIdx.x * H + h) * D * DV;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int d = (i >> 2) * 64 + ty * 4 + (i & 3);
+    if (d >= D) continue;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int v = half * 64 + tx * 4;
+      if (v < DV) *reinterpret_cast<float4*>(S + (size_t)d * DV + v) = *reinterpret_cast<float4*>(&acc[i][half * 4]);
+    }
+  }
+  if (tid < D) {
+    float sum = 0.f;
+    for (int s = 0; s < L; ++s) sum += Ks[s * LLD + tid];
+    x.n[((size_t)blockIdx.x * H + h) * D + tid] = sum;
+  }
+}
+
+// A thread owns four neighbouring cells of S (or of n) of one head and walks the request's chunks; eight chunks' loads
+// are on their way together.
+__global__ void __launch_bounds__(256)
+mlstm_long_scan_kernel(LongScratch x, float* __restrict__ state, const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int H,
+                       int D, int DV) {
+  const int h = blockIdx.y, r = blockIdx.z;
+  pdl_wait();
+  int first = 0;
+  for (int i = 0; i < r; ++i) first += (req_q_start[i + 1] - req_q_start[i] + LC - 1) / LC;
+  const int chunks = (req_q_start[r + 1] - req_q_start[r] + LC - 1) / LC;
+  if (chunks == 0) return;
+  const size_t head_floats = (size_t)D * DV + D + HEAD_EXTRA;
+  float* S = state + ((size_t)req_slot[r] * H + h) * head_floats;
+  const int cells = D * DV / 4, at = blockIdx.x * 256 + threadIdx.x;
+  const bool of_s = at < cells;
+  if (!of_s && at - cells >= D / 4) return;
+  float m = S[(size_t)D * DV + D];                 // read by every block of the head, filed by mlstm_long_out
+  float4* own = reinterpret_cast<float4*>(of_s ? S + 4 * (size_t)at : S + (size_t)D * DV + 4 * (at - cells));
+  const size_t step = (size_t)H * (of_s ? D * DV : D);
+  float* d0 = (of_s ? x.S + ((size_t)first * H + h) * D * DV + 4 * (size_t)at : x.n + ((size_t)first * H + h) * D + 4 * (at - cells));
+  const float* gb = x.gb + ((size_t)first * H + h) * 2;
+  float4 cur = *own;
+  for (int c0 = 0; c0 < chunks; c0 += 8) {
+    float4 d[8];
+    float2 g[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (c0 + u < chunks) {
+        d[u] = *reinterpret_cast<const float4*>(d0 + (c0 + u) * step);
+        g[u] = *reinterpret_cast<const float2*>(gb + (size_t)(c0 + u) * H * 2);
+      }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (c0 + u < chunks) {
+        *reinterpret_cast<float4*>(d0 + (c0 + u) * step) = cur;
+        if (at == 0) x.m[(size_t)(first + c0 + u) * H + h] = m;
+        const float top = fmaxf(m, g[u].x), keep = expf(m - top), add = expf(g[u].x - top);
+        cur.x = fmaf(add, d[u].x, keep * cur.x);
+        cur.y = fmaf(add, d[u].y, keep * cur.y);
+        cur.z = fmaf(add, d[u].z, keep * cur.z);
+        cur.w = fmaf(add, d[u].w, keep * cur.w);
+        m = g[u].y + top;
+      }
+  }
+  *own = cur;
+  if (at == 0) x.m_end[(size_t)r * H + h] = m;
+}
+
+constexpr int LPD = LC + 4;
+constexpr size_t LONG_OUT_SMEM = (size_t)(2 * LC * LLD + LMAX * LMAX + LMAX + LC * LPD + 5 * LC + LMAX) * sizeof(float);
+template <typename C>
+__global__ void __launch_bounds__(LTHREADS, 1)
+mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ state, const float* __restrict__ proj, long long stride,
+                      const float* __restrict__ norm_w, const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int num_req,
+                      int H, int D, int DV, float cap, float eps) {
+  extern __shared__ __align__(16) float sm[];
+  float* Qs = sm;                      // [LC][LLD]
+  float* KV = Qs + LC * LLD;           // [LC][LLD]: k, then v
+  float* Ss = KV + LC * LLD;           // [D][DV], and a row's worth behind it that is read and not used
+  float* Ps = Ss + LMAX * LMAX + LMAX; // [LC][LPD]
+  float* av = Ps + LC * LPD;           // [LC] a_s
+  float* gv = av + LC;                 // [LC] g_t
+  float* eg = gv + LC;                 // [LC] e^(m_0 - g_t) times the query's factor
+  float* em = eg + LC;                 // [LC] e^(-m_t)
+  float* den = em + LC;                // [LC]
+  float* ns = den + LC;                // [LMAX]
+  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, tx = tid & 15, ty = tid >> 4;
+  const MlstmCols col(H, D, DV);
+  const float qscale = rsqrtf((float)D);
+  int r, row0, L, c;
+  pdl_wait();
+  if (!find_chunk(blockIdx.x, req_q_start, num_req, r, row0, L, c)) return;
+  const size_t at = (size_t)blockIdx.x * H + h;
+  auto rows_in = [&](float* dst, int first_col, int width) {
+    for (int i = tid; i < LC * (LMAX / 4); i += LTHREADS) {
+      const int t = i / (LMAX / 4), d = (i % (LMAX / 4)) * 4;
+      cp_async_16(dst + t * LLD + d, proj + (size_t)(row0 + min(t, L - 1)) * stride + first_col + (d < width ? d : 0), t < L && d < width);
+    }
+  };
+  rows_in(Qs, col.q + h * D, D);
+  rows_in(KV, col.k + h * D, D);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int i = tid; i < D * DV / 4; i += LTHREADS) cp_async_16(Ss + 4 * i, x.S + at * D * DV + 4 * i, true);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  if (warp == 0) {
+    float a[2], top[2], b[2], G, B;
+    chunk_gates(proj, stride, row0, L, col.i + h, col.f + h, cap, tid, a, top, b, G, B);
+    const float m0 = x.m[at];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = 2 * tid + e;
+      const float g = fmaxf(m0, top[e]);
+      av[t] = a[e];
+      gv[t] = g;
+      eg[t] = expf(m0 - g) * qscale;
+      em[t] = expf(-(b[e] + g));
+    }
+  } else {
+    for (int d = tid - 32; d < D; d += LTHREADS - 32) ns[d] = x.n[at * D + d];
+  }
+  if (c == 0 && tid == 32) state[((size_t)req_slot[r] * H + h) * ((size_t)D * DV + D + HEAD_EXTRA) + (size_t)D * DV + D] = x.m_end[(size_t)r * H + h];
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncthreads();
+
+  const bool live = warp * 8 < L;      // this warp's tokens 8 warp ... + 7; thread: tokens 4 ty + i
+  const float* qrow = Qs + ty * 4 * LLD;
+  if (live) {
+    // the pairs' weights (k_s . q_t) e^(a_s - g_t), s = tx + 16 j, and the denominators
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 2
+    for (int d = 0; d < D; d += 4) {
+      float4 q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(qrow + i * LLD + d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (16 * j > 8 * warp + 7) continue;            // later than every token of the warp
+        const float4 k = *reinterpret_cast<const float4*>(KV + (tx + 16 * j) * LLD + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          s[i][j] = fmaf(q[i].x, k.x, s[i][j]);
+          s[i][j] = fmaf(q[i].y, k.y, s[i][j]);
+          s[i][j] = fmaf(q[i].z, k.z, s[i][j]);
+          s[i][j] = fmaf(q[i].w, k.w, s[i][j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = ty * 4 + i;
+      float sum = 0.f, nq = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = tx + 16 * j;
+        const float p = key <= t ? s[i][j] * qscale * expf(av[key] - gv[t]) : 0.f;
+        Ps[t * LPD + key] = p;
+        sum += p;
+      }
+      for (int d = tx * 4; d < D; d += 64) {
+        const float4 n4 = *reinterpret_cast<const float4*>(ns + d), q4 = *reinterpret_cast<const float4*>(qrow + i * LLD + d);
+        nq = fmaf(n4.x, q4.x, nq); nq = fmaf(n4.y, q4.y, nq); nq = fmaf(n4.z, q4.z, nq); nq = fmaf(n4.w, q4.w, nq);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        nq += __shfl_xor_sync(0xffffffffu, nq, o);
+      }
+      if (tx == 0) den[t] = fmaxf(fabsf(fmaf(eg[t], nq, sum)), em[t]) + 1e-6f;
+    }
+  }
+  __syncthreads();                     // every read of k is done
+  rows_in(KV, col.v + h * DV, DV);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncthreads();                     // S is there
+  float o[4][8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[i][j] = 0.f;
+  if (live) {
+#pragma unroll 2
+    for (int d = 0; d < D; d += 4) {
+      float4 q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(qrow + i * LLD + d);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 lo = *reinterpret_cast<const float4*>(Ss + (d + u) * DV + tx * 4), hi = *reinterpret_cast<const float4*>(Ss + (d + u) * DV + 64 + tx * 4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float qv = u == 0 ? q[i].x : (u == 1 ? q[i].y : (u == 2 ? q[i].z : q[i].w));
+          o[i][0] = fmaf(qv, lo.x, o[i][0]); o[i][1] = fmaf(qv, lo.y, o[i][1]); o[i][2] = fmaf(qv, lo.z, o[i][2]); o[i][3] = fmaf(qv, lo.w, o[i][3]);
+          o[i][4] = fmaf(qv, hi.x, o[i][4]); o[i][5] = fmaf(qv, hi.y, o[i][5]); o[i][6] = fmaf(qv, hi.z, o[i][6]); o[i][7] = fmaf(qv, hi.w, o[i][7]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[i][j] *= eg[ty * 4 + i];
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();                     // v is there
+  if (!live) return;
+#pragma unroll 2
+  for (int s = 0; s < 8 * warp + 8; s += 4) {
+    float4 p[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (ty * 4 + i) * LPD + s);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float4 lo = *reinterpret_cast<const float4*>(KV + (s + u) * LLD + tx * 4), hi = *reinterpret_cast<const float4*>(KV + (s + u) * LLD + 64 + tx * 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float pv = u == 0 ? p[i].x : (u == 1 ? p[i].y : (u == 2 ? p[i].z : p[i].w));
+        o[i][0] = fmaf(pv, lo.x, o[i][0]); o[i][1] = fmaf(pv, lo.y, o[i][1]); o[i][2] = fmaf(pv, lo.z, o[i][2]); o[i][3] = fmaf(pv, lo.w, o[i][3]);
+        o[i][4] = fmaf(pv, hi.x, o[i][4]); o[i][5] = fmaf(pv, hi.y, o[i][5]); o[i][6] = fmaf(pv, hi.z, o[i][6]); o[i][7] = fmaf(pv, hi.w, o[i][7]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = ty * 4 + i;
+    const float d = den[t];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      o[i][j] /= d;
+      if ((j >> 2) * 64 + tx * 4 < DV) ss = fmaf(o[i][j], o[i][j], ss);
+    }
+#pragma unroll
+    for (int m = 8; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+    const float inv = 1.0f / sqrtf(ss / (float)DV + eps);
+    if (t >= L) continue;
+    const float* gate = proj + (size_t)(row0 + t) * stride + col.g + h * DV;
+    C* dst = out + (size_t)(row0 + t) * H * DV + h * DV;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int v = (j >> 2) * 64 + tx * 4 + (j & 3);
+      if (v < DV) dst[v] = from_float<C>(o[i][j] * inv * norm_w[h * DV + v] / (1.0f + expf(-gate[v])));
+    }
+  }
+}
+
 constexpr int CHUNK_TOKENS = 16;
 
 size_t chunk_smem(int D) { return chunk_floats(D, CHUNK_TOKENS, 32) * sizeof(float); }
@@ -515,4 +907,45 @@ AYK_EXPORT int ayk_mlstm(void* out, float* state, const float* proj, long long s
     ayk_launch(mlstm_finish_kernel<__nv_bfloat16>, dim3(T, H), dim3(128), 0, stream, (__nv_bfloat16*)out, state, (const float*)raw,
                (const float*)nm, proj, stride, norm_w, row_req, req_q_start, req_slot, H, D, DV, eps);
   return ayk_check_launch("ayk_mlstm");
+}
+
+// The form for long portions (see mlstm_long_sum_kernel): heads of up to 128 x 128 in whole 16-byte pieces.
+AYK_EXPORT int ayk_mlstm_long_takes(int H, int D, int DV, long long stride, const void* proj) {
+  return D >= 4 && DV >= 4 && D <= LMAX && DV <= LMAX && D % 4 == 0 && DV % 4 == 0 && stride % 4 == 0 && (uintptr_t)proj % 16 == 0;
+}
+AYK_EXPORT long long ayk_mlstm_long_scratch_floats(int T, int num_req, int H, int D, int DV) {
+  return long_chunks(T, num_req) * H * ((long long)D * DV + D + 3) + (long long)num_req * H;
+}
+// As ayk_mlstm with the scratch of ayk_mlstm_long_scratch_floats (16-byte aligned); three launches.
+AYK_EXPORT int ayk_mlstm_long(void* out, float* state, const float* proj, long long stride, const float* norm_w, const int* req_q_start,
+                              const int* req_slot, int num_req, int T, int H, int D, int DV, float cap, float eps, float* scratch,
+                              int out_dtype, cudaStream_t stream) {
+  if (T == 0 || num_req == 0) return 0;
+  AYK_REQUIRE(ayk_mlstm_long_takes(H, D, DV, stride, proj) && (uintptr_t)state % 16 == 0 && (uintptr_t)scratch % 16 == 0,
+              "ayk_mlstm_long: %d heads of %d x %d, or the operands' alignment, are not taken", H, D, DV);
+  AYK_REQUIRE(cap > 0.f, "ayk_mlstm: the gates' cap must be positive");
+  AYK_REQUIRE(out_dtype == AYK_DTYPE_F32 || out_dtype == AYK_DTYPE_BF16, "ayk_mlstm: unknown dtype %d", out_dtype);
+  const long long chunks = long_chunks(T, num_req);
+  AYK_REQUIRE(H <= 65535 && num_req <= 65535 && chunks < (1ll << 31), "ayk_mlstm: %d heads, %d requests", H, num_req);
+  static AykPerDevice configured;
+  bool& done = configured.here();
+  if (!done) {
+    cudaError_t e = cudaFuncSetAttribute(mlstm_long_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LONG_SUM_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(mlstm_long_out_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LONG_OUT_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(mlstm_long_out_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LONG_OUT_SMEM);
+    if (e != cudaSuccess) return ayk_fail("ayk_mlstm: shared memory: %s", cudaGetErrorString(e));
+    done = true;
+  }
+  const LongScratch x = long_scratch(scratch, chunks, H, D, DV);
+  ayk_launch_after(mlstm_long_sum_kernel, dim3((unsigned)chunks, H), dim3(LTHREADS), LONG_SUM_SMEM, stream, x, proj, stride, req_q_start,
+                   num_req, H, D, DV, cap);
+  ayk_launch(mlstm_long_scan_kernel, dim3((D * DV / 4 + D / 4 + 255) / 256, H, num_req), dim3(256), 0, stream, x, state, req_q_start,
+             req_slot, H, D, DV);
+  if (out_dtype == AYK_DTYPE_F32)
+    ayk_launch(mlstm_long_out_kernel<float>, dim3((unsigned)chunks, H), dim3(LTHREADS), LONG_OUT_SMEM, stream, (float*)out, x, state, proj,
+               stride, norm_w, req_q_start, req_slot, num_req, H, D, DV, cap, eps);
+  else
+    ayk_launch(mlstm_long_out_kernel<__nv_bfloat16>, dim3((unsigned)chunks, H), dim3(LTHREADS), LONG_OUT_SMEM, stream, (__nv_bfloat16*)out, x,
+               state, proj, stride, norm_w, req_q_start, req_slot, num_req, H, D, DV, cap, eps);
+  return ayk_check_launch("ayk_mlstm_long");
 }

@@ -593,6 +593,9 @@ def mlstm_head_floats(dim: int, vdim: int) -> int:
     return dim * vdim + dim + 4
 
 
+MLSTM_LONG = 64          # rows of one request from which on its chunks go side by side
+
+
 def mlstm(proj: torch.Tensor, state: torch.Tensor, norm_weight: torch.Tensor, ctx, heads: int, dim: int, vdim: int,
           cap: float, eps: float, out_dtype: torch.dtype, chunked: bool | None = None, slice_cols: int = 0) -> torch.Tensor:
     """The mLSTM recurrence over the step's rows, request by request, from and into ``state`` [slots, heads,
@@ -600,7 +603,8 @@ def mlstm(proj: torch.Tensor, state: torch.Tensor, norm_weight: torch.Tensor, ct
     rows [q | k | v | z_i (heads) | z_f (heads) | gate (heads * vdim)]; returns [T, heads * vdim] in
     ``out_dtype``.  ``chunked``: the kernel that takes 16 tokens at a time (default: whenever a request brings
     more than one row, or the values are wider than the token-by-token kernel's 256 numbers, and the head size
-    fits it); ``slice_cols``: value columns per block of that kernel, 16 or 32 (0: 32, or 16 where blocks of 32
+    fits it; from ``MLSTM_LONG`` rows of one request on, heads of up to 128 x 128 have their chunks of 64 tokens side by
+    side); ``slice_cols``: value columns per block of that kernel, 16 or 32 (0: 32, or 16 where blocks of 32
     would leave most SMs idle)."""
     lib = _ready()
     lib.ayk_mlstm_slice_cols(ctypes.c_int(slice_cols))
@@ -617,7 +621,20 @@ def mlstm(proj: torch.Tensor, state: torch.Tensor, norm_weight: torch.Tensor, ct
         raise KernelError(f"mlstm: the chunked kernel does not take heads of {dim} numbers")
     if not chunked and vdim > 256:
         raise KernelError(f"mlstm: heads of {dim} x {vdim} fit neither kernel (values over 256 need keys under about 750)")
+    global launches
     scratch = None
+    if (chunked and slice_cols == 0 and ctx.max_q_len >= MLSTM_LONG and state.data_ptr() % 16 == 0 and
+            lib.ayk_mlstm_long_takes(ctypes.c_int(heads), ctypes.c_int(dim), ctypes.c_int(vdim), ctypes.c_longlong(proj.stride(0)), _ptr(proj))):
+        lib.ayk_mlstm_long_scratch_floats.restype = ctypes.c_longlong
+        floats = int(lib.ayk_mlstm_long_scratch_floats(ctypes.c_int(T), ctypes.c_int(ctx.num_requests), ctypes.c_int(heads),
+                                                       ctypes.c_int(dim), ctypes.c_int(vdim)))
+        scratch = torch.empty((floats,), dtype=torch.float32, device=proj.device)
+        _launch(lib.ayk_mlstm_long(_ptr(out), _ptr(state), _ptr(proj), ctypes.c_longlong(proj.stride(0)), _ptr(norm_weight),
+                                   _ptr(ctx.req_q_start), _ptr(ctx.req_slot), ctypes.c_int(ctx.num_requests), ctypes.c_int(T),
+                                   ctypes.c_int(heads), ctypes.c_int(dim), ctypes.c_int(vdim), ctypes.c_float(cap), ctypes.c_float(eps),
+                                   _ptr(scratch), ctypes.c_int(_tag(out_dtype)), _stream()))
+        launches += 2
+        return out
     if chunked:
         lib.ayk_mlstm_scratch_floats.restype = ctypes.c_longlong
         floats = int(lib.ayk_mlstm_scratch_floats(ctypes.c_int(T), ctypes.c_int(ctx.num_requests), ctypes.c_int(heads),
@@ -628,7 +645,6 @@ def mlstm(proj: torch.Tensor, state: torch.Tensor, norm_weight: torch.Tensor, ct
                           ctypes.c_int(T), ctypes.c_int(heads), ctypes.c_int(dim), ctypes.c_int(vdim), ctypes.c_float(cap),
                           ctypes.c_float(eps), _ptr(scratch), ctypes.c_int(_tag(out_dtype)), _stream()))
     if chunked:
-        global launches
         launches += 1
     return out
 

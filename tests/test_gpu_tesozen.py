@@ -412,6 +412,36 @@ def test_mlstm_with_strong_gates_and_long_memory(f_bias, i_bias, i_gain):
         assert np.abs(out[k + 1] - out[5]).max() < 2e-4 * max(1.0, np.abs(out[5]).max())
 
 
+@pytest.mark.parametrize("H,D,Dv", [(3, 128, 128), (2, 64, 128), (1, 12, 20), (2, 128, 36)])
+def test_mlstm_chunks_side_by_side(H, D, Dv):
+    """The form for long portions against the token-by-token kernel: portions that end at the edges of the 64-token
+    chunks, beside requests of one row and of few, on top of a state; rows, memories and maxima in 32-bit."""
+    from ayaka_py_b200 import ops
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts import StateNeed
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    width = -(-(2 * H * D + 2 * H * Dv + 2 * H) // 4) * 4
+    w = torch.rand(H * Dv, generator=gen, device="cuda") + 0.5
+    spec = CacheGroupSpec("g", StateNeed((H, ops.mlstm_head_floats(D, Dv)), torch.float32), 1)
+    cache, runner = context_for([spec], "float32", max_requests=4, page_size=8, pages=8)
+    state = cache.state_layer(0, 0)
+    for plan in ({0: 64, 1: 65, 2: 1}, {0: 129, 2: 63}, {1: 200, 0: 1, 3: 2}):
+        ctx, res = step_of(cache, runner, plan)
+        proj = torch.randn(ctx.num_rows, width, generator=gen, device="cuda")
+        proj[:, 2 * H * D + H * Dv + H:2 * H * D + H * Dv + 2 * H] += 2.0          # forget gates near one
+        before = state.clone()
+        walk = ops.mlstm(proj, state, w, ctx, H, D, Dv, 10.0, 1e-5, torch.float32, chunked=False)
+        walked = state.clone()
+        state.copy_(before)
+        out = ops.mlstm(proj, state, w, ctx, H, D, Dv, 10.0, 1e-5, torch.float32)
+        assert float((out - walk).abs().max()) < 1e-4 * float(walk.abs().max())
+        used = [cache.slot_of[i] for i in plan]
+        assert float((state - walked)[used].abs().max()) < 1e-4 * max(1.0, float(walked[used].abs().max()))
+        rest = [i for i in range(state.shape[0]) if i not in used]
+        assert torch.equal(state[rest], before[rest])
+        cache.commit(res)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,D,Dv,rank", [(3, 12, 10, 20), (2, 32, 16, 40), (4, 64, 64, 128), (1, 16, 48, 8), (8, 64, 48, 96), (2, 24, 256, 36)])
 def test_latent_attention_without_rotation_alone(dtype, H, D, Dv, rank):
