@@ -150,7 +150,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   volatile uint32_t* tmem_slot_ptr = (volatile uint32_t*)(generic_base + (tmem_slot - base));
   volatile float* pair_slot = (volatile float*)(generic_base + (pair_at - base));    // [128]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     mbar_init(k_full0, 1); mbar_init(k_full0 + 8, 1);
@@ -171,7 +171,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot_ptr;
+  const uint32_t tmem_base = uniform(*tmem_slot_ptr);
   // Only now may the next kernel be scheduled: a dependent CTA that landed on this SM before the
   // allocation above could take tensor-memory columns that this CTA then waits for without bound,
   // while the dependent waits for this kernel.  (Kernels that can share an SM must ask for 512

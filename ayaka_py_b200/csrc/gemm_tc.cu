@@ -161,7 +161,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const float* red_ptr = (const float*)(smem_raw + (red - raw));
 
   if (threadIdx.x == 0) mark(args, 0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * BLOCK_N, t0 = blockIdx.y * BT;
   const int total_kb = (args.K + BLOCK_K - 1) / BLOCK_K;
   const int kb_begin = CLUSTER ? (int)blockIdx.z * args.kb_base + min((int)blockIdx.z, args.kb_rem)
@@ -191,7 +191,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   __syncthreads();
   if (DELIVERIES) cluster_arrive();       // matched by cluster_wait() in every role below
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot_ptr;
+  const uint32_t tmem_base = uniform(*tmem_slot_ptr);
   if (threadIdx.x == 0) mark(args, 1);
   pdl_trigger();     // the next kernel may be scheduled; it waits for this one before it touches its data
 

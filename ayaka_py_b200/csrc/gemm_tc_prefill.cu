@@ -324,7 +324,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   auto res_full = [&](int half, int buf) { return bars + 8u * (2 * MAX_STAGES + 5 + 2 * half + buf); };
   volatile uint32_t* tmem_slot_ptr = (volatile uint32_t*)(smem_raw + (tmem_slot - raw));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   const int total_tiles = args.m_tiles * args.n_tiles;
   const int num_kb = (args.K + BLOCK_K - 1) / BLOCK_K;
   // Whole tiles go round the CTAs; with a split along K a CTA has one tile and one part of its K blocks.
@@ -357,7 +357,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot_ptr;
+  const uint32_t tmem_base = uniform(*tmem_slot_ptr);
   pdl_trigger();
 
   if (warp == 0) {
@@ -691,7 +691,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   const uint32_t tmem_slot = bars + 8u * (2 * MAX_STAGES + 4);
   volatile uint32_t* tmem_slot_ptr = (volatile uint32_t*)(smem_raw + (tmem_slot - raw));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_number(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();                          // 0 issues the MMAs
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int total_tiles = args.m_tiles * args.n_tiles;           // m_tiles counts 256-row tiles here
@@ -714,7 +714,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   __syncthreads();
   cluster_sync_all();   // the partner's barriers exist before anything signals them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot_ptr;
+  const uint32_t tmem_base = uniform(*tmem_slot_ptr);
   pdl_trigger();
 
   if (warp == 0) {

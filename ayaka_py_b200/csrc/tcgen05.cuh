@@ -14,11 +14,12 @@ constexpr uint32_t WAIT_LIMIT = 1u << 24;      // polls of a barrier before a ke
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// One lane of a converged warp, the same one each time.  The threads that issue copies and MMAs are chosen with
-// elect.sync and not with `lane == 0`: the compiler then knows that one thread runs what follows.  A thread that issues
-// four MMAs and a commit per K block sets the pace of short tiles; measured with nothing else changed (products over
-// weights in turn, us): 576 x 3840 x 1280 13.2 -> 11.1, 2048 x 1600 x 6400 with a residual 42.9 -> 39.8,
-// 8192 x 8192 x 4096 457 -> 443, 8 x 6400 x 1600 5.95 -> 5.67, 8 x 1600 x 1600 3.91 -> 3.70.
+// The thread that issues MMAs sets the pace of short tiles, and it is fast only when the compiler can keep what it hands
+// to the tensor core (descriptors, the accumulator's address, barriers) in the warp's uniform registers.  Three things tell
+// it so: the issuing lane is chosen with elect.sync, the warp's number and the tensor-memory base that came through shared
+// memory go through a shuffle (`uniform`).  Measured clocks per tcgen05.mma of 128 x N x 16 in a bare chain: 75 for N = 32,
+// 64 and 128 before, 40, 48 and 64 now, which is what their operands take to leave shared memory (128 bytes a clock); 128
+// for N = 256 either way.
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;
   asm volatile(
@@ -28,6 +29,9 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(one));
   return one != 0;
 }
+
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }      // whole warps only
+__device__ __forceinline__ int warp_number() { return (int)uniform(threadIdx.x >> 5); }
 
 // ---------------------------------------------------------------- mbarriers --
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
