@@ -14,10 +14,8 @@
 // (grid.z) whose partial results (maximum, sum, unnormalised O) a second kernel merges.  With a window a block visits
 // the tiles from its first row's window on, and a row's partitions are counted from the one that holds its first key.
 //
-// tcgen05 is not used here: O for 128 pairs x 512 columns would fill tensor memory alone, and
-// the score tile's K extent (rank + rot up to 576) wants operands staged in more shared memory
-// than one SM has beside it; the warp-level form keeps O in registers and works for every latent
-// size that is a multiple of 8.
+// Prompt portions whose latent and rotated part are whole runs of 64 numbers take the tcgen05 form (latent_tc.cu); this one
+// keeps O in registers and works for every latent size that is a multiple of 8, and for a few rows.
 #include <math.h>
 
 #include "common.cuh"

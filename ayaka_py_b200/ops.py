@@ -517,9 +517,9 @@ def latent_attention(query: torch.Tensor, latent_pages: torch.Tensor, rope_pages
     """Causal attention of the step's rows over cached (latent, rotated key part) pairs shared by
     all heads: query [T, H, rank + rot] float32; returns sum_j p_j latent_j as float32 [T, H, rank].  ``window``: a
     row sees its own position and the window - 1 before it.
-    bfloat16 pages whose rows are whole 16-byte pieces go through the tensor-core kernel (a decode
-    step's context cut into partitions and merged); 32-bit pages and other sizes through the
-    kernel on the FP32 pipes."""
+    bfloat16 pages whose rows are whole 16-byte pieces go through the tensor-core kernels (tcgen05 for prompt portions
+    whose latent and rotated part are whole runs of 64 numbers; else mma.sync, a decode step's context cut into
+    partitions and merged); 32-bit pages and other sizes through the kernel on the FP32 pipes."""
     lib = _ready()
     T, H, Dk = query.shape
     rank, rot = latent_pages.shape[-1], rope_pages.shape[-1]
@@ -531,6 +531,14 @@ def latent_attention(query: torch.Tensor, latent_pages: torch.Tensor, rope_pages
         tensor_cores = takes
     elif tensor_cores and not takes:
         raise KernelError(f"latent_attention: the tensor-core kernel does not take {latent_pages.dtype} pages of {rank} + {rot}")
+    if tensor_cores and ctx.max_q_len > 1 and lib.ayk_latent_attention_tc_takes(
+            ctypes.c_int(rank), ctypes.c_int(rot), ctypes.c_int(latent_pages.shape[1]), _ptr(query), _ptr(latent_pages), _ptr(rope_pages)):
+        _launch(lib.ayk_latent_attention_tc(_ptr(out), _ptr(query), _ptr(latent_pages), _ptr(rope_pages), ctypes.c_int(latent_pages.shape[0]),
+                                            _ptr(_i32(table, "table")), ctypes.c_int(table.stride(0)), _ptr(ctx.req_q_start),
+                                            _ptr(ctx.req_pos0), ctypes.c_int(ctx.num_requests), ctypes.c_int(T), ctypes.c_int(H),
+                                            ctypes.c_int(rank), ctypes.c_int(rot), ctypes.c_int(latent_pages.shape[1]),
+                                            ctypes.c_float(scale), ctypes.c_int(window or 0), _stream()))
+        return out
     if tensor_cores:
         parts, part_keys, partial = 1, 0, None
         if ctx.max_q_len == 1:
@@ -1596,10 +1604,10 @@ MIXED_DECODE_MIN = 1     # single-token requests in a mixed step from which they
 
 def tc_error() -> int:
     """0, or the code of the bounded wait that ran out in a tensor-core kernel
-    (1-4: matrix product, 11-17: attention)."""
+    (1-4: matrix product, 11-17: attention, 51-58: latent attention)."""
     lib = library()
     return (int(lib.ayk_gemm_tc_error()) or int(lib.ayk_attention_tc_error())
-            or int(lib.ayk_gemm_tc_prefill_error()))
+            or int(lib.ayk_gemm_tc_prefill_error()) or int(lib.ayk_latent_tc_error()))
 
 
 def attention(q, kcache, vcache, table, ctx, num_heads: int, scale: float,

@@ -451,6 +451,42 @@ def test_tensor_core_latent_attention_against_the_32_bit_pipes(H, rank, rot, P):
         cache.commit(res)
 
 
+@pytest.mark.parametrize("H,rank,rot,P,window", [(16, 512, 64, 16, None), (8, 512, 0, 8, 40), (5, 384, 64, 64, 33), (40, 256, 64, 32, 1),
+                                                 (130, 64, 0, 16, None), (1, 128, 128, 8, 100)])
+def test_latent_attention_on_tcgen05_tile_edges(H, rank, rot, P, window):
+    """Portions that start and end at the edges of the 32-key tiles and of the pairs' tiles, windows that begin inside a
+    tile, one and two halves of the latent, with and without foreign chunks, more heads than a tile has pairs; stale
+    values that are no numbers lie behind the last row."""
+    from ayaka_py_b200 import ops
+    cache, runner, lat, rope = kv_context(H, rank, rot, P, None)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    # a wait that runs out would leave its code for the tests after this one: the word is as it was
+    before = ops.tc_error()
+    for plan in ({0: 32, 1: 31, 2: 33}, {0: 1, 1: 2, 2: 95}, {0: 200, 1: 1, 2: 3}):
+        ctx, res = step_of(cache, runner, plan)
+        for i, n in plan.items():
+            slot = cache.slot_of[i]
+            end = int(cache.length[slot]) + n
+            if end % P:                                # the rest of the last page
+                page = int(cache.table_rows(0, [slot])[0][end // P])
+                lat[page, end % P:] = float("nan")
+                rope[page, end % P:] = float("nan")
+        q = torch.randn(ctx.num_rows, H, rank + rot, generator=gen, device="cuda") * 0.5
+        a = ops.latent_attention(q, lat, rope, ctx.tables[0], ctx, 0.2, tensor_cores=False, window=window)
+        b = ops.latent_attention(q, lat, rope, ctx.tables[0], ctx, 0.2, tensor_cores=True, window=window)
+        assert ops.tc_error() == before
+        assert not torch.isnan(b).any()
+        assert float((a - b).abs().max()) < 0.01 * float(a.abs().max()) + 1e-3, plan
+        for i, n in plan.items():                      # the next portion's rows are numbers again
+            slot = cache.slot_of[i]
+            end = int(cache.length[slot]) + n
+            if end % P:
+                page = int(cache.table_rows(0, [slot])[0][end // P])
+                lat[page, end % P:] = torch.randn(lat[page, end % P:].shape, generator=gen, device="cuda").to(lat.dtype)
+                rope[page, end % P:] = torch.randn(rope[page, end % P:].shape, generator=gen, device="cuda").to(rope.dtype)
+        cache.commit(res)
+
+
 @pytest.mark.parametrize("H,N,K", [(3, 24, 40), (16, 512, 128), (2, 70, 264), (5, 8, 96)])
 def test_per_head_products_on_both_pipes(H, N, K):
     from ayaka_py_b200 import ops
