@@ -499,7 +499,10 @@ def head_matmul(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate: torch
     if lib.ayk_head_matvec_takes(_ptr(a), ctypes.c_longlong(a.stride(0)), ctypes.c_int(a.stride(1)), _ptr(w), ctypes.c_int(T),
                                  ctypes.c_int(K)):
         _launch(lib.ayk_head_matvec(*common, ctypes.c_int(_tag(w.dtype)), ctypes.c_int(_tag(out.dtype)), _stream()))
-    # bfloat16 weights: the tensor cores, the float32 operand in two bfloat16 parts; else the FP32 pipes
+    # bfloat16 weights: the tensor cores, the float32 operand in two bfloat16 parts (tcgen05 from 64 rows on); else the FP32 pipes
+    elif w.dtype == torch.bfloat16 and lib.ayk_head_matmul_tc_takes(_ptr(a), ctypes.c_longlong(a.stride(0)), ctypes.c_int(a.stride(1)), _ptr(w),
+                                                                  ctypes.c_int(T), ctypes.c_int(H), ctypes.c_int(N), ctypes.c_int(K)):
+        _launch(lib.ayk_head_matmul_tc(*common, ctypes.c_int(_tag(out.dtype)), _stream()))
     elif w.dtype == torch.bfloat16 and lib.ayk_head_matmul_mma_takes(_ptr(a), ctypes.c_longlong(a.stride(0)),
                                                                    ctypes.c_int(a.stride(1)), ctypes.c_int(K)):
         _launch(lib.ayk_head_matmul_mma(*common, ctypes.c_int(_tag(out.dtype)), _stream()))
@@ -1604,10 +1607,10 @@ MIXED_DECODE_MIN = 1     # single-token requests in a mixed step from which they
 
 def tc_error() -> int:
     """0, or the code of the bounded wait that ran out in a tensor-core kernel
-    (1-4: matrix product, 11-17: attention, 51-58: latent attention)."""
+    (1-4: matrix product, 11-17: attention, 51-58: latent attention, 61-68: per-head products)."""
     lib = library()
     return (int(lib.ayk_gemm_tc_error()) or int(lib.ayk_attention_tc_error())
-            or int(lib.ayk_gemm_tc_prefill_error()) or int(lib.ayk_latent_tc_error()))
+            or int(lib.ayk_gemm_tc_prefill_error()) or int(lib.ayk_latent_tc_error()) or int(lib.ayk_head_tc_error()))
 
 
 def attention(q, kcache, vcache, table, ctx, num_heads: int, scale: float,

@@ -487,6 +487,29 @@ def test_latent_attention_on_tcgen05_tile_edges(H, rank, rot, P, window):
         cache.commit(res)
 
 
+@pytest.mark.parametrize("T,H,N,K,wide_gate", [(64, 2, 128, 64, None), (127, 3, 129, 72, True), (129, 1, 512, 128, False), (300, 2, 8, 520, True),
+                                               (128, 5, 136, 512, None)])
+def test_per_head_products_on_tcgen05(T, H, N, K, wide_gate):
+    """Edges of the 128 x 128 tiles and of the 64-wide chunks of K, both gates, strided operands and results: the operand
+    keeps 16 bits of mantissa (2^-17 a term at most), the sums are 32-bit."""
+    from ayaka_py_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    before = ops.tc_error()
+    a = torch.randn(T, H, K + 8, generator=gen, device="cuda")[:, :, 4:K + 4]
+    w = (torch.randn(H, N, K, generator=gen, device="cuda") / K ** 0.5).to(torch.bfloat16)
+    gate = None if wide_gate is None else torch.randn(T, H * N if wide_gate else H, generator=gen, device="cuda")
+    want = torch.einsum("thk,hnk->thn", a.double(), w.double())
+    bound = torch.einsum("thk,hnk->thn", a.double().abs(), w.double().abs()) * (2.0 ** -17 + K * 2.0 ** -24) + 1e-6
+    if gate is not None:
+        want = want * torch.sigmoid(gate.double()).view(T, H, -1)
+    for out_dtype in (torch.float32, torch.bfloat16):
+        out = torch.zeros(T, H, N + 1, dtype=out_dtype, device="cuda")[:, :, :N]
+        ops.head_matmul(a, w, out, gate=gate)
+        slack = bound if out_dtype == torch.float32 else bound + want.abs() * 2.0 ** -8
+        assert ((out.double() - want).abs() <= slack).all()
+    assert ops.tc_error() == before
+
+
 @pytest.mark.parametrize("H,N,K", [(3, 24, 40), (16, 512, 128), (2, 70, 264), (5, 8, 96)])
 def test_per_head_products_on_both_pipes(H, N, K):
     from ayaka_py_b200 import ops
