@@ -438,8 +438,8 @@ mlstm_finish_kernel(C* __restrict__ out, float* __restrict__ state, const float*
 //   mlstm_long_scan   per cell of the memory, over the chunks: leaves every chunk's S_0, n_0, m_0 in the place of its dS
 //                     (S' = e^(m - m') S + e^(G - m') dS with m' = max(m, G), then m = B + m'), and files the last into the state
 //   mlstm_long_out    a chunk's outputs from its S_0, n_0, m_0 (formulas above), with the head's norm and gate applied
-// All three are float32; the products are register tiles fed with float4 from shared memory (8 x 8 sums a thread in the
-// first, 4 x 4 and 4 x 8 in the last), bound by the FP32 pipes and shared memory; the memories' round trips
+// All three are float32; the products are register tiles fed with float4 from shared memory (8 x 8 sums a thread,
+// 8 x 4 for the pairs' weights), bound by the FP32 pipes and shared memory; the memories' round trips
 // (4 x 64 KB a chunk and head of 128 x 128) stay in the L2 for portions of a few thousand tokens.
 // Measured for the layer at 16 heads of 128 x 128 (us; before: the chunked form): 1,024 and 777 tokens 471 -> 261; at 8 heads
 // 2 x 1,024 tokens 461 -> 131, 2 x 200 113 -> 70, 2 x 17 (the chunked form) 64.  The line lies at one whole chunk: 64 tokens.
@@ -641,19 +641,22 @@ mlstm_long_scan_kernel(LongScratch x, float* __restrict__ state, const int* __re
   if (at == 0) x.m_end[(size_t)r * H + h] = m;
 }
 
-constexpr int LPD = LC + 4;
-constexpr size_t LONG_OUT_SMEM = (size_t)(2 * LC * LLD + LMAX * LMAX + LMAX + LC * LPD + 5 * LC + LMAX) * sizeof(float);
+// A block of 256 threads, two to a multiprocessor: a thread owns tokens 4 ty ... + 3 and columns 4 tx ... + 3 and 64 + 4 tx
+// ... + 3 (32 sums; 12 float4 from shared memory for 128 products).  Shared memory, 100 KB: the queries, whose place P takes
+// at the end; k, then v; one half of S (64 of its rows), then the other.
+constexpr int LPD = LC + 4, OTHREADS = 256, SHALF = 64, RT = LC * 16 / OTHREADS, WT = 2 * RT;      // tokens of a thread, of a warp
+constexpr size_t LONG_OUT_SMEM = (size_t)(LC * LMAX + LC * LLD + SHALF * LMAX + LMAX + 5 * LC + LMAX) * sizeof(float);
+static_assert(LC * LPD <= LC * LMAX, "P fits the queries' place");
 template <typename C>
-__global__ void __launch_bounds__(LTHREADS, 1)
+__global__ void __launch_bounds__(OTHREADS, 2)
 mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ state, const float* __restrict__ proj, long long stride,
                       const float* __restrict__ norm_w, const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int num_req,
                       int H, int D, int DV, float cap, float eps) {
   extern __shared__ __align__(16) float sm[];
-  float* Qs = sm;                      // [LC][LLD]
-  float* KV = Qs + LC * LLD;           // [LC][LLD]: k, then v
-  float* Ss = KV + LC * LLD;           // [D][DV], and a row's worth behind it that is read and not used
-  float* Ps = Ss + LMAX * LMAX + LMAX; // [LC][LPD]
-  float* av = Ps + LC * LPD;           // [LC] a_s
+  float* Qs = sm;                      // [LC][LMAX]; at the end P [LC][LPD]
+  float* KV = Qs + LC * LMAX;          // [LC][LLD]: k, then v
+  float* Ss = KV + LC * LLD;           // [SHALF][DV], and a row's worth behind it that is read and not used
+  float* av = Ss + SHALF * LMAX + LMAX;       // [LC] a_s
   float* gv = av + LC;                 // [LC] g_t
   float* eg = gv + LC;                 // [LC] e^(m_0 - g_t) times the query's factor
   float* em = eg + LC;                 // [LC] e^(-m_t)
@@ -666,16 +669,19 @@ mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ st
   pdl_wait();
   if (!find_chunk(blockIdx.x, req_q_start, num_req, r, row0, L, c)) return;
   const size_t at = (size_t)blockIdx.x * H + h;
-  auto rows_in = [&](float* dst, int first_col, int width) {
-    for (int i = tid; i < LC * (LMAX / 4); i += LTHREADS) {
-      const int t = i / (LMAX / 4), d = (i % (LMAX / 4)) * 4;
-      cp_async_16(dst + t * LLD + d, proj + (size_t)(row0 + min(t, L - 1)) * stride + first_col + (d < width ? d : 0), t < L && d < width);
-    }
+  auto rows_in = [&](float* dst, int ld, int first_col, int width) {
+    const int d = (tid & 31) * 4;
+    for (int t = warp; t < LC; t += OTHREADS / 32)
+      cp_async_16(dst + t * ld + d, proj + (size_t)(row0 + min(t, L - 1)) * stride + first_col + (d < width ? d : 0), t < L && d < width);
   };
-  rows_in(Qs, col.q + h * D, D);
-  rows_in(KV, col.k + h * D, D);
+  auto memory_in = [&](int first) {    // rows first ... of S
+    const int n = min(SHALF, D - first) * DV / 4;
+    for (int i = tid; i < n; i += OTHREADS) cp_async_16(Ss + 4 * i, x.S + at * D * DV + (size_t)first * DV + 4 * i, true);
+  };
+  rows_in(Qs, LMAX, col.q + h * D, D);
+  memory_in(0);
   asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int i = tid; i < D * DV / 4; i += LTHREADS) cp_async_16(Ss + 4 * i, x.S + at * D * DV + 4 * i, true);
+  rows_in(KV, LLD, col.k + h * D, D);
   asm volatile("cp.async.commit_group;" ::: "memory");
   if (warp == 0) {
     float a[2], top[2], b[2], G, B;
@@ -691,32 +697,61 @@ mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ st
       em[t] = expf(-(b[e] + g));
     }
   } else {
-    for (int d = tid - 32; d < D; d += LTHREADS - 32) ns[d] = x.n[at * D + d];
+    for (int d = tid - 32; d < D; d += OTHREADS - 32) ns[d] = x.n[at * D + d];
   }
   if (c == 0 && tid == 32) state[((size_t)req_slot[r] * H + h) * ((size_t)D * DV + D + HEAD_EXTRA) + (size_t)D * DV + D] = x.m_end[(size_t)r * H + h];
-  asm volatile("cp.async.wait_group 1;" ::: "memory");
-  __syncthreads();
 
-  const bool live = warp * 8 < L;      // this warp's tokens 8 warp ... + 7; thread: tokens 4 ty + i
-  const float* qrow = Qs + ty * 4 * LLD;
-  if (live) {
-    // the pairs' weights (k_s . q_t) e^(a_s - g_t), s = tx + 16 j, and the denominators
-    float s[4][4];
+  const int t_first = ty * RT;         // this thread's first token; its warp's tokens are WT warp ... + WT - 1
+  const bool live = warp * WT < L;
+  const float* qrow = Qs + t_first * LMAX;
+  float o[RT][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[i][j] = 0.f;
+  // o += q S over rows first ... of S
+  auto remember = [&](int first) {
+    const int n = min(SHALF, D - first);
+    for (int d = 0; d < n; d += 4) {
+      float4 q[RT];
+#pragma unroll
+      for (int i = 0; i < RT; ++i) q[i] = *reinterpret_cast<const float4*>(qrow + i * LMAX + first + d);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 lo = *reinterpret_cast<const float4*>(Ss + (d + u) * DV + tx * 4), hi = *reinterpret_cast<const float4*>(Ss + (d + u) * DV + 64 + tx * 4);
+#pragma unroll
+        for (int i = 0; i < RT; ++i) {
+          const float qv = u == 0 ? q[i].x : (u == 1 ? q[i].y : (u == 2 ? q[i].z : q[i].w));
+          o[i][0] = fmaf(qv, lo.x, o[i][0]); o[i][1] = fmaf(qv, lo.y, o[i][1]); o[i][2] = fmaf(qv, lo.z, o[i][2]); o[i][3] = fmaf(qv, lo.w, o[i][3]);
+          o[i][4] = fmaf(qv, hi.x, o[i][4]); o[i][5] = fmaf(qv, hi.y, o[i][5]); o[i][6] = fmaf(qv, hi.z, o[i][6]); o[i][7] = fmaf(qv, hi.w, o[i][7]);
+        }
+      }
+    }
+  };
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncthreads();                     // the queries and the first half of S
+  if (live) remember(0);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();                     // k is there, every read of the first half is done
+  if (D > SHALF) memory_in(SHALF);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  // the pairs' weights (k_s . q_t) e^(a_s - g_t), s = tx + 16 j, and the denominators
+  float s[RT][4];
+  if (live) {
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 2
     for (int d = 0; d < D; d += 4) {
-      float4 q[4];
+      float4 q[RT];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(qrow + i * LLD + d);
+      for (int i = 0; i < RT; ++i) q[i] = *reinterpret_cast<const float4*>(qrow + i * LMAX + d);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (16 * j > 8 * warp + 7) continue;            // later than every token of the warp
+        if (16 * j > WT * warp + WT - 1) continue;                          // later than every token of the warp
         const float4 k = *reinterpret_cast<const float4*>(KV + (tx + 16 * j) * LLD + d);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < RT; ++i) {
           s[i][j] = fmaf(q[i].x, k.x, s[i][j]);
           s[i][j] = fmaf(q[i].y, k.y, s[i][j]);
           s[i][j] = fmaf(q[i].z, k.z, s[i][j]);
@@ -725,87 +760,77 @@ mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ st
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = ty * 4 + i;
+    for (int i = 0; i < RT; ++i) {
+      const int t = t_first + i;
       float sum = 0.f, nq = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int key = tx + 16 * j;
-        const float p = key <= t ? s[i][j] * qscale * expf(av[key] - gv[t]) : 0.f;
-        Ps[t * LPD + key] = p;
-        sum += p;
+        s[i][j] = key <= t ? s[i][j] * qscale * expf(av[key] - gv[t]) : 0.f;
+        sum += s[i][j];
       }
       for (int d = tx * 4; d < D; d += 64) {
-        const float4 n4 = *reinterpret_cast<const float4*>(ns + d), q4 = *reinterpret_cast<const float4*>(qrow + i * LLD + d);
+        const float4 n4 = *reinterpret_cast<const float4*>(ns + d), q4 = *reinterpret_cast<const float4*>(qrow + i * LMAX + d);
         nq = fmaf(n4.x, q4.x, nq); nq = fmaf(n4.y, q4.y, nq); nq = fmaf(n4.z, q4.z, nq); nq = fmaf(n4.w, q4.w, nq);
       }
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        nq += __shfl_xor_sync(0xffffffffu, nq, o);
+      for (int m = 8; m > 0; m >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, m);
+        nq += __shfl_xor_sync(0xffffffffu, nq, m);
       }
       if (tx == 0) den[t] = fmaxf(fabsf(fmaf(eg[t], nq, sum)), em[t]) + 1e-6f;
     }
   }
   __syncthreads();                     // every read of k is done
-  rows_in(KV, col.v + h * DV, DV);
+  rows_in(KV, LLD, col.v + h * DV, DV);
   asm volatile("cp.async.commit_group;" ::: "memory");
   asm volatile("cp.async.wait_group 1;" ::: "memory");
-  __syncthreads();                     // S is there
-  float o[4][8];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) o[i][j] = 0.f;
+  __syncthreads();                     // the second half of S
   if (live) {
-#pragma unroll 2
-    for (int d = 0; d < D; d += 4) {
-      float4 q[4];
+    if (D > SHALF) remember(SHALF);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(qrow + i * LLD + d);
+    for (int i = 0; i < RT; ++i)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float4 lo = *reinterpret_cast<const float4*>(Ss + (d + u) * DV + tx * 4), hi = *reinterpret_cast<const float4*>(Ss + (d + u) * DV + 64 + tx * 4);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float qv = u == 0 ? q[i].x : (u == 1 ? q[i].y : (u == 2 ? q[i].z : q[i].w));
-          o[i][0] = fmaf(qv, lo.x, o[i][0]); o[i][1] = fmaf(qv, lo.y, o[i][1]); o[i][2] = fmaf(qv, lo.z, o[i][2]); o[i][3] = fmaf(qv, lo.w, o[i][3]);
-          o[i][4] = fmaf(qv, hi.x, o[i][4]); o[i][5] = fmaf(qv, hi.y, o[i][5]); o[i][6] = fmaf(qv, hi.z, o[i][6]); o[i][7] = fmaf(qv, hi.w, o[i][7]);
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[i][j] *= eg[ty * 4 + i];
+      for (int j = 0; j < 8; ++j) o[i][j] *= eg[t_first + i];
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();                     // v is there
+  __syncthreads();                     // v is there, every read of the queries is done
   if (!live) return;
-#pragma unroll 2
-  for (int s = 0; s < 8 * warp + 8; s += 4) {
-    float4 p[4];
+  float* P = Qs + t_first * LPD;       // a warp reads the weights of its own tokens only
 #pragma unroll
-    for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (ty * 4 + i) * LPD + s);
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) P[i * LPD + tx + 16 * j] = s[i][j];
+  __syncwarp();
+  for (int k = 0; k < WT * warp + WT; k += 4) {
+    float4 p[RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i) p[i] = *reinterpret_cast<const float4*>(P + i * LPD + k);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const float4 lo = *reinterpret_cast<const float4*>(KV + (s + u) * LLD + tx * 4), hi = *reinterpret_cast<const float4*>(KV + (s + u) * LLD + 64 + tx * 4);
+      const float4 lo = *reinterpret_cast<const float4*>(KV + (k + u) * LLD + tx * 4), hi = *reinterpret_cast<const float4*>(KV + (k + u) * LLD + 64 + tx * 4);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < RT; ++i) {
         const float pv = u == 0 ? p[i].x : (u == 1 ? p[i].y : (u == 2 ? p[i].z : p[i].w));
         o[i][0] = fmaf(pv, lo.x, o[i][0]); o[i][1] = fmaf(pv, lo.y, o[i][1]); o[i][2] = fmaf(pv, lo.z, o[i][2]); o[i][3] = fmaf(pv, lo.w, o[i][3]);
         o[i][4] = fmaf(pv, hi.x, o[i][4]); o[i][5] = fmaf(pv, hi.y, o[i][5]); o[i][6] = fmaf(pv, hi.z, o[i][6]); o[i][7] = fmaf(pv, hi.w, o[i][7]);
       }
     }
   }
+  float w[8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = ty * 4 + i;
-    const float d = den[t];
+  for (int j = 0; j < 8; ++j) {
+    const int v = (j >> 2) * 64 + tx * 4 + (j & 3);
+    w[j] = v < DV ? norm_w[h * DV + v] : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < RT; ++i) {
+    const int t = t_first + i;
+    const float below = den[t];
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      o[i][j] /= d;
+      o[i][j] /= below;
       if ((j >> 2) * 64 + tx * 4 < DV) ss = fmaf(o[i][j], o[i][j], ss);
     }
 #pragma unroll
@@ -814,10 +839,16 @@ mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ st
     if (t >= L) continue;
     const float* gate = proj + (size_t)(row0 + t) * stride + col.g + h * DV;
     C* dst = out + (size_t)(row0 + t) * H * DV + h * DV;
+    float g[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int v = (j >> 2) * 64 + tx * 4 + (j & 3);
-      if (v < DV) dst[v] = from_float<C>(o[i][j] * inv * norm_w[h * DV + v] / (1.0f + expf(-gate[v])));
+      g[j] = v < DV ? __ldg(gate + v) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int v = (j >> 2) * 64 + tx * 4 + (j & 3);
+      if (v < DV) dst[v] = from_float<C>(o[i][j] * inv * w[j] / (1.0f + expf(-g[j])));
     }
   }
 }
@@ -942,10 +973,10 @@ AYK_EXPORT int ayk_mlstm_long(void* out, float* state, const float* proj, long l
   ayk_launch(mlstm_long_scan_kernel, dim3((D * DV / 4 + D / 4 + 255) / 256, H, num_req), dim3(256), 0, stream, x, state, req_q_start,
              req_slot, H, D, DV);
   if (out_dtype == AYK_DTYPE_F32)
-    ayk_launch(mlstm_long_out_kernel<float>, dim3((unsigned)chunks, H), dim3(LTHREADS), LONG_OUT_SMEM, stream, (float*)out, x, state, proj,
+    ayk_launch(mlstm_long_out_kernel<float>, dim3((unsigned)chunks, H), dim3(OTHREADS), LONG_OUT_SMEM, stream, (float*)out, x, state, proj,
                stride, norm_w, req_q_start, req_slot, num_req, H, D, DV, cap, eps);
   else
-    ayk_launch(mlstm_long_out_kernel<__nv_bfloat16>, dim3((unsigned)chunks, H), dim3(LTHREADS), LONG_OUT_SMEM, stream, (__nv_bfloat16*)out, x,
+    ayk_launch(mlstm_long_out_kernel<__nv_bfloat16>, dim3((unsigned)chunks, H), dim3(OTHREADS), LONG_OUT_SMEM, stream, (__nv_bfloat16*)out, x,
                state, proj, stride, norm_w, req_q_start, req_slot, num_req, H, D, DV, cap, eps);
   return ayk_check_launch("ayk_mlstm_long");
 }
