@@ -20,12 +20,13 @@
 // Warps 0..3: softmax, a TMEM lane (pair) per thread, and the output; warp 4: TMA producer (a box per lane); warp 5: MMA
 // issue and TMEM allocation.  All warps convert the queries first.  Every mbarrier wait is bounded; one that runs out
 // records a code and the CTA winds down.
-// Measured, 1,024 + 777 rows of 16 heads, latent 512 + 64, no window: the layer 452 -> 356 us (mma.sync before: 286 us of it).  A tile takes
-// 4,200 clocks, a third of it more than its MMAs need; staging the queries 12,600, writing O 8,000.
+// Measured, 1,024 + 777 rows of 16 heads, latent 512 + 64, no window: the layer 452 -> 356 us (mma.sync before: 286 us of it), and with
+// the chunk counts as constants (straight lines of MMAs) 288 -> 272, this kernel then 167.
 #include <cuda.h>
 #include <math.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -79,6 +80,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// FOREIGN, OWN: chunks of either kind, constants for the usual sizes (the products are then straight lines of MMAs); 0, 0: by
+// the arguments.
+template <int FOREIGN, int OWN>
 __global__ void __launch_bounds__(THREADS, 1)
 latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_constant__ CUtensorMap map_rope, const LatentArgs args) {
   // Tiles of the requests' last rows see the most keys: they start first (blocks are handed out in order).
@@ -101,7 +105,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
   const int k_begin = (int)uniform(args.window > 0 ? max(0, pos0 - args.window + 1) / NK * NK : 0);
   const int num_tiles = (last_pos - k_begin) / NK + 1;
   const int* my_table = args.table + (size_t)req * args.table_stride;
-  const int lat_chunks = rank / 64, chunks = Dk / 64, own = args.own, foreign = chunks - own;
+  const int own = OWN ? OWN : args.own, chunks = OWN ? OWN + FOREIGN : Dk / 64, foreign = chunks - own, lat_chunks = rank / 64;
   const int own_first = half * own;                    // chunk numbers: latent first, then the rotated part
   // the i-th foreign chunk's number
   auto foreign_chunk = [&](int i) { return i < own_first ? i : i + own; };
@@ -155,8 +159,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
           const int piece = lane + 32 * j;
           x[u][j][0] = x[u][j][1] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (exists && piece < pieces) {
-            x[u][j][0] = __ldg(src + 2 * piece);
-            x[u][j][1] = __ldg(src + 2 * piece + 1);
+            x[u][j][0] = src[2 * piece];               // (not __ldg: it must not move ahead of the wait above)
+            x[u][j][1] = src[2 * piece + 1];
           }
         }
       }
@@ -238,7 +242,8 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
       return __all_sync(0xffffffffu, fine);
     };
     const bool late = foreign < 4;                     // few foreign chunks: P C waits behind all of the next tile's S
-    auto scores = [&](int t, bool owned) -> bool {
+    auto scores = [&](int t, auto which) -> bool {
+      constexpr bool owned = decltype(which)::value;
       const int b = t & 1, n = owned ? own : foreign;
       if (n == 0) return true;
       if (!wait((owned ? own_full : foreign_full) + 8 * b, (uint32_t)(t >> 1) & 1u, 53)) return false;
@@ -259,6 +264,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
       __syncwarp();
       tc_fence_after();
       if (elect_one()) {
+#pragma unroll
         for (int c = 0; c < n; ++c) {
           const int number = owned ? own_first + c : foreign_chunk(c);
           const uint64_t da = make_desc(q_tile + (uint32_t)number * Q_CHUNK), db = make_desc(from + (uint32_t)c * K_CHUNK);
@@ -281,6 +287,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
 #pragma unroll
         for (int k = 0; k < NK / 16; ++k) {
           const uint64_t da = make_desc_64(p_tile) + (uint64_t)(2 * k);
+#pragma unroll
           for (int c = 0; c < own; ++c)
             umma(tmem + 64u * c, da, make_desc(from + (uint32_t)c * K_CHUNK + (uint32_t)k * 2048u), IDESC_O, (t > 0 || k > 0) ? 1u : 0u);
         }
@@ -290,12 +297,14 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
       __syncwarp();
       return true;
     };
-    bool ok = scores(0, false) && scores(0, true);
+    const std::false_type not_own;
+    const std::true_type its_own;
+    bool ok = scores(0, not_own) && scores(0, its_own);
     for (int t = 0; t < num_tiles && ok; ++t) {
       const bool more = t + 1 < num_tiles;
-      if (more) ok = scores(t + 1, false) && (!late || scores(t + 1, true));
+      if (more) ok = scores(t + 1, not_own) && (!late || scores(t + 1, its_own));
       if (ok) ok = weigh(t);
-      if (ok && more && !late) ok = scores(t + 1, true);
+      if (ok && more && !late) ok = scores(t + 1, its_own);
     }
   } else {
     // ---- softmax: TMEM lane = pair
@@ -459,7 +468,9 @@ int setup() {
     if (err != cudaSuccess) return ayk_fail("ayk_latent_attention_tc: cudaHostGetDevicePointer: %s", cudaGetErrorString(err));
   }
   if (!g_configured.here()) {
-    cudaError_t err = cudaFuncSetAttribute(latent_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(MAX_CHUNKS));
+    cudaError_t err = cudaFuncSetAttribute(latent_tc_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(MAX_CHUNKS));
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(latent_tc_kernel<5, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(9));
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(latent_tc_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(8));
     if (err != cudaSuccess) return ayk_fail("ayk_latent_attention_tc: shared memory %zu: %s", smem_bytes(MAX_CHUNKS), cudaGetErrorString(err));
     g_configured.here() = true;
   }
@@ -516,6 +527,9 @@ AYK_EXPORT int ayk_latent_attention_tc(float* out, const float* query, const voi
   AYK_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "ayk_latent_attention_tc: %d rows, %d requests, %d heads", total_rows, num_req, H);
   LatentArgs args{out, query, table, req_q_start, req_pos0, g_error_dev, table_stride, num_req, H, HG, BR, rank, rot, shift, window,
                   rank / 64 / halves, scale * 1.4426950408889634f};
-  ayk_launch(latent_tc_kernel, grid, dim3(THREADS), smem_bytes((rank + rot) / 64), stream, ml, mr, args);
+  const size_t smem = smem_bytes((rank + rot) / 64);
+  if (rank == 512 && rot == 64) ayk_launch(latent_tc_kernel<5, 4>, grid, dim3(THREADS), smem, stream, ml, mr, args);
+  else if (rank == 512 && rot == 0) ayk_launch(latent_tc_kernel<4, 4>, grid, dim3(THREADS), smem, stream, ml, mr, args);
+  else ayk_launch(latent_tc_kernel<0, 0>, grid, dim3(THREADS), smem, stream, ml, mr, args);
   return ayk_check_launch("ayk_latent_attention_tc");
 }

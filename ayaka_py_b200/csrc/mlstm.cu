@@ -523,7 +523,7 @@ __host__ __device__ inline LongScratch long_scratch(float* base, long long chunk
 
 constexpr size_t LONG_SUM_SMEM = (size_t)(2 * LC * LLD + LC) * sizeof(float);
 __global__ void __launch_bounds__(LTHREADS, 2)
-mlstm_long_sum_kernel(LongScratch x, const float* __restrict__ proj, long long stride, const int* __restrict__ req_q_start, int num_req,
+mlstm_long_sum_kernel(LongScratch x, const float* proj, long long stride, const int* __restrict__ req_q_start, int num_req,
                       int H, int D, int DV, float cap) {
   extern __shared__ __align__(16) float sm[];
   float* Ks = sm;                      // [LC][LLD], each row times its token's weight
@@ -649,7 +649,7 @@ constexpr size_t LONG_OUT_SMEM = (size_t)(LC * LMAX + LC * LLD + SHALF * LMAX + 
 static_assert(LC * LPD <= LC * LMAX, "P fits the queries' place");
 template <typename C>
 __global__ void __launch_bounds__(OTHREADS, 2)
-mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ state, const float* __restrict__ proj, long long stride,
+mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ state, const float* proj, long long stride,
                       const float* __restrict__ norm_w, const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int num_req,
                       int H, int D, int DV, float cap, float eps) {
   extern __shared__ __align__(16) float sm[];
@@ -843,7 +843,7 @@ mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ st
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int v = (j >> 2) * 64 + tx * 4 + (j & 3);
-      g[j] = v < DV ? __ldg(gate + v) : 0.f;
+      g[j] = v < DV ? gate[v] : 0.f;
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
