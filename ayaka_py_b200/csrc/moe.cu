@@ -481,10 +481,14 @@ moe_gemm_mma_kernel(O* __restrict__ out, const __nv_bfloat16* __restrict__ a, lo
 // --------------------------------------------- few pairs: matrix times vector --
 // A step of single tokens has a handful of (token, choice) pairs, most on experts of their own: each pair
 // then streams its expert's matrix once, and the product is bound by that stream.  A block takes one pair and
-// 64 output features; the pair's activation row waits in shared memory as float32; a warp takes 8 features, two
-// at a time, its lanes striding along K in 16-byte pieces of the weight rows (with the activation, both the gate
-// row and the up row of a feature).  No sorting: pair p reads row p / top (gather) or p, and writes row p.
-constexpr int GV_COLS = 64;
+// 64 output features (32 with the activation); the pair's activation row waits in shared memory as float32; a warp takes 8 (4)
+// features, two at a time, its lanes striding along K in 16-byte pieces of the weight rows (with the activation, both the gate
+// row and the up row of a feature), sixteen pieces asked for before the first is used; the first sixteen are on
+// their way while the activation row is laid out.  No sorting: pair p reads row p / top (gather) or p, and writes row p.
+// Measured, the routed layer of width 2,048 (us; before: 64 features a block, four pieces at a time): 1 row 65 -> 33, 3 rows
+// 92 -> 62, 8 rows 99 -> 96; of width 1,024 1 row 33 -> 25, 8 rows 44 -> 35.  The first product of the 8 rows 56 -> 37, the second
+// 20 -> 24.
+constexpr int gv_cols(bool glu) { return glu ? 32 : 64; }
 
 __device__ __forceinline__ float dot8(const uint4& w, const float4& x0, const float4& x1) {
   // a bfloat16 is the upper half of a float
@@ -499,15 +503,43 @@ __device__ __forceinline__ float dot8(const uint4& w, const float4& x0, const fl
 }
 
 template <typename O, bool GLU>
-__global__ void __launch_bounds__(256)
-moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* __restrict__ a, long long a_stride,
-                const __nv_bfloat16* __restrict__ w, const int* __restrict__ ids, int top, int gather, int N, int N_w,
-                int Kd, float limit, float slope, float plus, int act, const float* __restrict__ early) {
+__global__ void __launch_bounds__(256, 2)
+moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
+                const __nv_bfloat16* __restrict__ w, const int* ids, int top, int gather, int N, int N_w,
+                int Kd, float limit, float slope, float plus, int act, const float* early) {
+  // (what kernels before this one write has no __restrict__: a load that the compiler takes for constant may be moved ahead
+  // of the wait below)
+  constexpr int STREAMS = GLU ? 4 : 2, STEPS = 16 / STREAMS, PER_WARP = gv_cols(GLU) / 8;
   extern __shared__ __align__(16) float xs[];          // [Kd]
   pdl_wait();
   const int pair = blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const __nv_bfloat16* arow = a + (size_t)(gather ? pair / top : pair) * a_stride;
+  const __nv_bfloat16* we = w + (size_t)ids[pair] * N_w * Kd;
+  const int first = (blockIdx.y * 8 + warp) * PER_WARP;
+  // the rows of two neighbouring features from n0 on (of their up halves too); past the last feature the last one's again
+  const __nv_bfloat16* rows[STREAMS];
+  auto rows_of = [&](int n0) {
+    const int m0 = min(n0, N - 1), m1 = min(n0 + 1, N - 1);
+    rows[0] = we + (size_t)m0 * Kd;
+    rows[1] = we + (size_t)m1 * Kd;
+    if (GLU) {
+      rows[2] = rows[0] + (size_t)N * Kd;
+      rows[3] = rows[1] + (size_t)N * Kd;
+    }
+  };
+  uint4 piece[STREAMS][STEPS];
+  auto ask = [&](int k) {                              // this lane's pieces at k, k + 256, ...
+#pragma unroll
+    for (int i = 0; i < STEPS; ++i)
+#pragma unroll
+      for (int st = 0; st < STREAMS; ++st) {
+        piece[st][i] = make_uint4(0u, 0u, 0u, 0u);
+        if (k + 256 * i < Kd) piece[st][i] = __ldg(reinterpret_cast<const uint4*>(rows[st] + k + 256 * i));
+      }
+  };
+  rows_of(first);
+  ask(lane * 8);
   for (int i = tid; i < Kd / 8; i += 256) {
     const uint4 v = *reinterpret_cast<const uint4*>(arow + i * 8);
     float4 lo, hi;
@@ -520,32 +552,35 @@ moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* __restrict__ a, long l
   }
   __syncthreads();
   const float factor = early ? early[pair] : 1.f;
-  const __nv_bfloat16* we = w + (size_t)ids[pair] * N_w * Kd;
-  const int first = blockIdx.y * GV_COLS + warp * 8;
 #pragma unroll 1
-  for (int j = 0; j < 8; j += 2) {
+  for (int j = 0; j < PER_WARP; j += 2) {
     const int n0 = first + j, n1 = n0 + 1;               // warp-uniform
     if (n0 >= N) break;
-    const bool two = n1 < N;
-    float g0 = 0.f, g1 = 0.f, u0 = 0.f, u1 = 0.f;
-    const __nv_bfloat16* r0 = we + (size_t)n0 * Kd;
-    const __nv_bfloat16* r1 = we + (size_t)(two ? n1 : n0) * Kd;
-    for (int k = lane * 8; k < Kd; k += 256) {
-      const float4 x0 = *reinterpret_cast<const float4*>(xs + k), x1 = *reinterpret_cast<const float4*>(xs + k + 4);
-      const uint4 wa = *reinterpret_cast<const uint4*>(r0 + k), wb = *reinterpret_cast<const uint4*>(r1 + k);
-      if (GLU) {
-        const uint4 wc = *reinterpret_cast<const uint4*>(r0 + (size_t)N * Kd + k), wd = *reinterpret_cast<const uint4*>(r1 + (size_t)N * Kd + k);
-        u0 += dot8(wc, x0, x1);
-        u1 += dot8(wd, x0, x1);
-      }
-      g0 += dot8(wa, x0, x1);
-      g1 += dot8(wb, x0, x1);
+    if (j > 0) {
+      rows_of(n0);
+      ask(lane * 8);
     }
-    g0 = factor * warp_sum(g0); g1 = factor * warp_sum(g1);
-    if (GLU) { u0 = factor * warp_sum(u0); u1 = factor * warp_sum(u1); }
+    float sum[STREAMS];
+#pragma unroll
+    for (int st = 0; st < STREAMS; ++st) sum[st] = 0.f;
+    for (int k = lane * 8; k < Kd; k += 256 * STEPS) {
+      if (k != lane * 8) ask(k);
+#pragma unroll
+      for (int i = 0; i < STEPS; ++i) {
+        const int at = k + 256 * i;
+        if (at < Kd) {
+          const float4 x0 = *reinterpret_cast<const float4*>(xs + at), x1 = *reinterpret_cast<const float4*>(xs + at + 4);
+#pragma unroll
+          for (int st = 0; st < STREAMS; ++st) sum[st] += dot8(piece[st][i], x0, x1);
+        }
+      }
+    }
+#pragma unroll
+    for (int st = 0; st < STREAMS; ++st) sum[st] = factor * warp_sum(sum[st]);
     if (lane == 0) {
-      out[(size_t)pair * N + n0] = from_float<O>(GLU ? glu_limited(g0, u0, limit, slope, plus) : apply_activation(g0, act));
-      if (two) out[(size_t)pair * N + n1] = from_float<O>(GLU ? glu_limited(g1, u1, limit, slope, plus) : apply_activation(g1, act));
+      out[(size_t)pair * N + n0] = from_float<O>(GLU ? glu_limited(sum[0], sum[STREAMS - 2], limit, slope, plus) : apply_activation(sum[0], act));
+      if (n1 < N)
+        out[(size_t)pair * N + n1] = from_float<O>(GLU ? glu_limited(sum[1], sum[STREAMS - 1], limit, slope, plus) : apply_activation(sum[1], act));
     }
   }
 }
@@ -612,21 +647,54 @@ glu_limited_vec_kernel(O* __restrict__ out, const I* __restrict__ in, long long 
 
 // shared[t, :] = sum_k weights[t, k] * picked[row of pair t * top + k, :] + sigmoid(mix[t]) * shared[t, :], the
 // chosen experts in the order of their choice; row_of_pair null: the pair's own number; weights null: 1.
+// A thread takes four columns (one where rows are no whole 16-byte pieces), grid (tokens, runs of 256 threads): a step of a
+// few rows spreads over as many blocks as it has columns for, and four choices' loads are on their way together.  Bound by
+// the rows' bytes.  Measured, width 2,048, two choices (us; before: a column a thread, one block to a token): 8 rows 11.7 -> 3.7, 2,048 rows 23.7 -> 14.1.
+template <int V>
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(float* __restrict__ shared, const float* __restrict__ picked, const int* __restrict__ row_of_pair,
-                   const float* __restrict__ weights, const float* __restrict__ mix, long long mix_stride, int top, int d) {
+moe_combine_kernel(float* shared, const float* picked, const int* row_of_pair, const float* weights, const float* mix, long long mix_stride,
+                   int top, int d) {
   pdl_trigger();
   pdl_wait();
-  const int t = blockIdx.x;
-  const float gate = mix ? sigmoidf(mix[(size_t)t * mix_stride]) : 1.0f;
-  for (int c = threadIdx.x; c < d; c += blockDim.x) {
-    float s = 0.f;
-    for (int k = 0; k < top; ++k) {
-      const size_t pair = (size_t)t * top + k;
-      s = fmaf(weights ? weights[pair] : 1.f, picked[(size_t)(row_of_pair ? row_of_pair[pair] : pair) * d + c], s);
-    }
-    shared[(size_t)t * d + c] = fmaf(gate, shared[(size_t)t * d + c], s);
+  const int t = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * V;
+  if (c >= d) return;
+  float own[V], s[V];
+  float* at = shared + (size_t)t * d + c;
+#pragma unroll
+  for (int i = 0; i < V; ++i) s[i] = 0.f;
+  if constexpr (V == 4) {
+    const float4 x = *reinterpret_cast<const float4*>(at);
+    own[0] = x.x; own[1] = x.y; own[2] = x.z; own[3] = x.w;
+  } else {
+    own[0] = at[0];
   }
+  const float gate = mix ? sigmoidf(mix[(size_t)t * mix_stride]) : 1.0f;
+  for (int k0 = 0; k0 < top; k0 += 4) {
+    float x[4][V], w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (k0 + u >= top) continue;
+      const size_t pair = (size_t)t * top + k0 + u;
+      const float* from = picked + (size_t)(row_of_pair ? row_of_pair[pair] : pair) * d + c;
+      w[u] = weights ? weights[pair] : 1.f;
+      if constexpr (V == 4) {
+        const float4 f = *reinterpret_cast<const float4*>(from);
+        x[u][0] = f.x; x[u][1] = f.y; x[u][2] = f.z; x[u][3] = f.w;
+      } else {
+        x[u][0] = from[0];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (k0 + u >= top) continue;
+#pragma unroll
+      for (int i = 0; i < V; ++i) s[i] = fmaf(w[u], x[u][i], s[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < V; ++i) s[i] = fmaf(gate, own[i], s[i]);
+  if constexpr (V == 4) *reinterpret_cast<float4*>(at) = make_float4(s[0], s[1], s[2], s[3]);
+  else at[0] = s[0];
 }
 
 }  // namespace
@@ -747,7 +815,11 @@ AYK_EXPORT int ayk_moe_plan_padded(int* row_of_pair, int* w_rows1, int* w_rows2,
 AYK_EXPORT int ayk_moe_combine(float* shared, const float* picked, const int* row_of_pair, const float* weights,
                                const float* mix, long long mix_stride, int T, int top, int d, cudaStream_t stream) {
   if (T == 0 || d == 0) return 0;
-  ayk_launch(moe_combine_kernel, dim3(T), dim3(256), 0, stream, shared, picked, row_of_pair, weights, mix, mix_stride, top, d);
+  const bool vec = d % 4 == 0 && ((uintptr_t)shared | (uintptr_t)picked) % 16 == 0;
+  dim3 grid(T, (d + (vec ? 1024 : 256) - 1) / (vec ? 1024 : 256));
+  AYK_REQUIRE(grid.y <= 65535, "ayk_moe_combine: rows of %d", d);
+  if (vec) ayk_launch(moe_combine_kernel<4>, grid, dim3(256), 0, stream, shared, picked, row_of_pair, weights, mix, mix_stride, top, d);
+  else ayk_launch(moe_combine_kernel<1>, grid, dim3(256), 0, stream, shared, picked, row_of_pair, weights, mix, mix_stride, top, d);
   return ayk_check_launch("ayk_moe_combine");
 }
 
@@ -762,7 +834,7 @@ AYK_EXPORT int ayk_moe_gemv(void* out, const void* a, long long a_stride, const 
                             cudaStream_t stream) {
   if (pairs == 0 || N == 0) return 0;
   AYK_REQUIRE(ayk_moe_gemv_takes(Kd, a_stride), "ayk_moe_gemv: rows of %d elements (stride %lld)", Kd, a_stride);
-  dim3 grid(pairs, (N + GV_COLS - 1) / GV_COLS);
+  dim3 grid(pairs, (N + gv_cols(glu) - 1) / gv_cols(glu));
   const size_t smem = (size_t)Kd * sizeof(float);
   if (glu)
     ayk_launch(moe_gemv_kernel<__nv_bfloat16, true>, grid, dim3(256), smem, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)a,
