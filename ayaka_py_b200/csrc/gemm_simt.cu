@@ -23,11 +23,14 @@ constexpr int BM = 64, BN = 64, BK = 16;
 // Bound by the FP32 pipes (128 FMA a clock and multiprocessor) and, per tile, by how many multiprocessors have one.  The
 // height is the one whose fullest multiprocessor has the least to do (f32_rows).  Measured for 377 rows, alone and cold
 // (us; before: 64-row tiles, slabs of 16 without copies ahead, 4 x 4 sums a thread): N 2304 K 768 71 -> 57, N 768 K 768
-// 56 -> 29, N 3072 K 768 74 -> 66, N 768 K 3072 207 -> 90; a GPT-2 small layer of 1 row 293 -> 139, of 130 rows 428 -> 286.
+// 56 -> 29, N 3072 K 768 74 -> 66, N 768 K 3072 207 -> 90; a GPT-2 small layer of 1 row 293 -> 139, of 130 rows 428 -> 286.  With the
+// copies' addresses worked out once and the groups' sums free of bank conflicts: the layer over 377 ragged rows 276 -> 236, over
+// 130 rows 197 -> 157.
 constexpr int FN = 64, FK = 32, FLD = FK + 4, FSTAGES = 4, FGROUPS = 4;      // rows of 36 floats: eight neighbours' 16-byte pieces lie on different banks
+constexpr int FSUM = FN + 8;             // floats per row of the groups' sums: a warp's four rows of eight lie on different banks
 constexpr int f32_stage_floats(int tm) { return (tm + FN) * FLD; }
 constexpr size_t f32_smem(int tm) {
-  const size_t ring = (size_t)FSTAGES * f32_stage_floats(tm), sums = (size_t)FGROUPS * tm * FN;
+  const size_t ring = (size_t)FSTAGES * f32_stage_floats(tm), sums = (size_t)FGROUPS * tm * FSUM;
   return (ring > sums ? ring : sums) * sizeof(float);
 }
 
@@ -49,18 +52,39 @@ gemm_f32_kernel(float* C, const float* __restrict__ A, const float* __restrict__
   const int tid = threadIdx.x, group = tid >> 6, tn = tid & 7, tm = (tid >> 3) & 7;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * FN;
   const int slabs = (K + FK - 1) / FK;
-  // one slab into buffer b; rows past the matrices' ends and k past K are zeros
-  auto fetch = [&](int slab, int b) {
-    float* to = f32_tiles + b * f32_stage_floats(TM);
-    constexpr int PER_ROW = VEC ? FK / 4 : FK, WIDTH = VEC ? 4 : 1;
-    for (int i = tid; i < (TM + FN) * PER_ROW; i += 256) {
-      const int row = i / PER_ROW, c = (i % PER_ROW) * WIDTH, k = slab * FK + c;
+  // One slab into buffer b; rows past the matrices' ends and k past K are zeros.  In 16-byte pieces a thread always brings
+  // the same piece of the same rows, whose addresses it works out once.
+  constexpr int COPIES = ((TM + FN) * (FK / 4) + 255) / 256;
+  const float* src[COPIES];
+  bool there[COPIES];
+  if (VEC) {
+#pragma unroll
+    for (int j = 0; j < COPIES; ++j) {
+      const int row = (tid >> 3) + 32 * j;
       const bool of_a = row < TM;
       const int at = of_a ? m0 + row : n0 + row - TM;
-      const bool on = at < (of_a ? M : N) && k < K;
-      const float* src = on ? (of_a ? A : W) + (size_t)at * K + k : A;
-      if (VEC) f32_copy16(to + row * FLD + c, src, on);
-      else f32_copy4(to + row * FLD + c, src, on);
+      there[j] = at < (of_a ? M : N);
+      src[j] = (there[j] ? (of_a ? A : W) + (size_t)at * K : A) + (tid & 7) * 4;
+    }
+  }
+  auto fetch = [&](int slab, int b) {
+    float* to = f32_tiles + b * f32_stage_floats(TM);
+    if (VEC) {
+      const int k = slab * FK + (tid & 7) * 4;
+#pragma unroll
+      for (int j = 0; j < COPIES; ++j) {
+        const int row = (tid >> 3) + 32 * j;
+        const bool on = there[j] && k < K;
+        if (row < TM + FN) f32_copy16(to + row * FLD + (tid & 7) * 4, on ? src[j] + slab * FK : A, on);
+      }
+    } else {
+      for (int i = tid; i < (TM + FN) * FK; i += 256) {
+        const int row = i / FK, c = i % FK, k = slab * FK + c;
+        const bool of_a = row < TM;
+        const int at = of_a ? m0 + row : n0 + row - TM;
+        const bool on = at < (of_a ? M : N) && k < K;
+        f32_copy4(to + row * FLD + c, on ? (of_a ? A : W) + (size_t)at * K + k : A, on);
+      }
     }
   };
   float acc[RM][8];
@@ -101,11 +125,11 @@ gemm_f32_kernel(float* C, const float* __restrict__ A, const float* __restrict__
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();                                   // the ring is free for the sums
-  float* mine = f32_tiles + group * TM * FN;
+  float* mine = f32_tiles + group * TM * FSUM;
 #pragma unroll
   for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) mine[(tm + 8 * i) * FN + tn + 8 * j] = acc[i][j];
+    for (int j = 0; j < 8; ++j) mine[(tm + 8 * i) * FSUM + tn + 8 * j] = acc[i][j];
   __syncthreads();
   const int col = tid & (FN - 1), n = n0 + col;
   if (n >= N) return;
@@ -114,8 +138,8 @@ gemm_f32_kernel(float* C, const float* __restrict__ A, const float* __restrict__
   for (int r = tid / FN; r < TM; r += 256 / FN) {
     const int m = m0 + r;
     if (m >= M) break;
-    const float* at = f32_tiles + r * FN + col;
-    float v = ((at[0] + at[TM * FN]) + (at[2 * TM * FN] + at[3 * TM * FN])) + b;
+    const float* at = f32_tiles + r * FSUM + col;
+    float v = ((at[0] + at[TM * FSUM]) + (at[2 * TM * FSUM] + at[3 * TM * FSUM])) + b;
     v = apply_activation(v, act);
     if (residual) v += residual[(size_t)m * N + n];
     C[(size_t)m * N + n] = v;
