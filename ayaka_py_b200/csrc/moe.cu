@@ -483,11 +483,11 @@ moe_gemm_mma_kernel(O* __restrict__ out, const __nv_bfloat16* __restrict__ a, lo
 // then streams its expert's matrix once, and the product is bound by that stream.  A block takes one pair and
 // 64 output features (32 with the activation); the pair's activation row waits in shared memory as float32; a warp takes 8 (4)
 // features, two at a time, its lanes striding along K in 16-byte pieces of the weight rows (with the activation, both the gate
-// row and the up row of a feature), sixteen pieces asked for before the first is used; the first sixteen are on
-// their way while the activation row is laid out.  No sorting: pair p reads row p / top (gather) or p, and writes row p.
+// row and the up row of a feature), sixteen pieces (eight without the activation, by twice as
+// many blocks) asked for before the first is used; the first are on their way while the activation row is laid out.  No sorting: pair p reads row p / top (gather) or p, and writes row p.
 // Measured, the routed layer of width 2,048 (us; before: 64 features a block, four pieces at a time): 1 row 65 -> 33, 3 rows
-// 92 -> 62, 8 rows 99 -> 96; of width 1,024 1 row 33 -> 25, 8 rows 44 -> 35.  The first product of the 8 rows 56 -> 37, the second
-// 20 -> 24.
+// 92 -> 62, 8 rows 99 -> 92; of width 1,024 1 row 33 -> 25, 8 rows 44 -> 34.  The first product of the 8 rows 56 -> 37; the second
+// 20 -> 24 with sixteen pieces, and the layer 89 -> 85 with eight and four blocks to a multiprocessor.
 constexpr int gv_cols(bool glu) { return glu ? 32 : 64; }
 
 __device__ __forceinline__ float dot8(const uint4& w, const float4& x0, const float4& x1) {
@@ -503,13 +503,13 @@ __device__ __forceinline__ float dot8(const uint4& w, const float4& x0, const fl
 }
 
 template <typename O, bool GLU>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, GLU ? 2 : 4)
 moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
                 const __nv_bfloat16* __restrict__ w, const int* ids, int top, int gather, int N, int N_w,
                 int Kd, float limit, float slope, float plus, int act, const float* early) {
   // (what kernels before this one write has no __restrict__: a load that the compiler takes for constant may be moved ahead
   // of the wait below)
-  constexpr int STREAMS = GLU ? 4 : 2, STEPS = 16 / STREAMS, PER_WARP = gv_cols(GLU) / 8;
+  constexpr int STREAMS = GLU ? 4 : 2, STEPS = 4, PER_WARP = gv_cols(GLU) / 8;
   extern __shared__ __align__(16) float xs[];          // [Kd]
   pdl_wait();
   const int pair = blockIdx.x;
