@@ -55,8 +55,8 @@ __device__ __forceinline__ float2 load_pair(const __nv_bfloat16* p) {
 
 template <typename T>
 __global__ void __launch_bounds__(WARPS * 32)
-decode_split_kernel(float* __restrict__ scratch, const T* __restrict__ q, int q_stride,
-                    const T* __restrict__ kcache, const T* __restrict__ vcache,
+decode_split_kernel(float* __restrict__ scratch, const T* q, int q_stride,
+                    const T* kcache, const T* vcache,
                     const int* __restrict__ table, int table_stride, const int* __restrict__ req_pos0,
                     int H, int Hkv, int Dh, int page_size, float scale, int window, int parts) {
   pdl_trigger();
@@ -218,11 +218,11 @@ template <int PPR> __device__ __forceinline__ int swizzled_piece(int row, int pi
 // and the kernel is bound by issue slots and latency, not by bandwidth.)
 template <int DH>
 __global__ void __launch_bounds__(WARPS * 32)
-decode_mma_kernel(float* __restrict__ scratch, const __nv_bfloat16* __restrict__ q, int q_stride,
-                  __nv_bfloat16* __restrict__ kcache, __nv_bfloat16* __restrict__ vcache,
+decode_mma_kernel(float* __restrict__ scratch, const __nv_bfloat16* q, int q_stride,
+                  __nv_bfloat16* kcache, __nv_bfloat16* vcache,
                   const int* __restrict__ table, int table_stride, const int* __restrict__ req_pos0,
                   int H, int Hkv, int group, int page_shift, float scale_log2, int window, int parts, int chunks, int rows,
-                  const __nv_bfloat16* __restrict__ knew, const __nv_bfloat16* __restrict__ vnew, int new_stride, int settled) {
+                  const __nv_bfloat16* knew, const __nv_bfloat16* vnew, int new_stride, int settled) {
   pdl_trigger();
   static_assert(WARPS * 32 == PART, "each warp owns 32 keys of the partition");
   constexpr int KS = DH / 16;                    // k steps of the first product
@@ -433,7 +433,7 @@ template <typename T> __device__ __forceinline__ float merge_exp(float x) {
 }
 
 template <typename T>
-__global__ void decode_merge_kernel(T* __restrict__ out, const float* __restrict__ scratch, int H, int Dh, int parts,
+__global__ void decode_merge_kernel(T* __restrict__ out, const float* scratch, int H, int Dh, int parts,
                                     const int* __restrict__ req_pos0, int window) {
   pdl_trigger();
   const int r = blockIdx.x, h = blockIdx.y;

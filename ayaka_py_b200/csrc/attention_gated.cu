@@ -23,7 +23,7 @@ constexpr int MAX_ROT_HALF = 128;
 
 template <typename C>
 __global__ void __launch_bounds__(512)
-qk_prepare_kernel(C* __restrict__ qout, C* __restrict__ kpages, C* __restrict__ vpages, const float* __restrict__ proj,
+qk_prepare_kernel(C* __restrict__ qout, C* __restrict__ kpages, C* __restrict__ vpages, const float* proj,
                   long long stride, const float* __restrict__ qw, const float* __restrict__ kw,
                   const float* __restrict__ freq, int rot_dims, const int* __restrict__ row_req,
                   const int* __restrict__ positions, const int* __restrict__ table, int table_stride, int page_size,
@@ -99,8 +99,8 @@ constexpr int MAX_D = 256;
 
 template <typename T>
 __global__ void __launch_bounds__(WARPS * 32)
-gated_attention_kernel(T* __restrict__ out, float* __restrict__ partial, const T* __restrict__ q,
-                       const T* __restrict__ kcache, const T* __restrict__ vcache, const int* __restrict__ table,
+gated_attention_kernel(T* __restrict__ out, float* __restrict__ partial, const T* q,
+                       const T* kcache, const T* vcache, const int* __restrict__ table,
                        int table_stride, const int* __restrict__ req_q_start, const int* __restrict__ req_pos0,
                        int num_req, int total_rows, int H, int Hkv, int D, int Dv, int page_size, float scale,
                        float cap, const float* __restrict__ head_bias, int part_keys) {
@@ -265,8 +265,8 @@ __device__ __forceinline__ void cp_async_16(void* dst, const void* src, bool val
 template <int D, int DV>
 __global__ void __launch_bounds__(128, 3)
 gated_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ partial,
-                           const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kcache,
-                           const __nv_bfloat16* __restrict__ vcache, const int* __restrict__ table, int table_stride,
+                           const __nv_bfloat16* q, const __nv_bfloat16* kcache,
+                           const __nv_bfloat16* vcache, const int* __restrict__ table, int table_stride,
                            const int* __restrict__ req_q_start, const int* __restrict__ req_pos0, int num_req,
                            int total_rows, int H, int Hkv, int page_shift, float scale, float cap,
                            const float* __restrict__ head_bias, int part_keys, int tq) {
@@ -444,7 +444,7 @@ gated_attention_mma_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ 
 // out[row] = sum over the parts that hold keys of the row's request, in order.
 template <typename T>
 __global__ void __launch_bounds__(256)
-gated_merge_kernel(T* __restrict__ out, const float* __restrict__ partial, const int* __restrict__ row_req,
+gated_merge_kernel(T* __restrict__ out, const float* partial, const int* __restrict__ row_req,
                    const int* __restrict__ positions, int total_rows, int width, int part_keys) {
   pdl_trigger();
   const int t = blockIdx.x;

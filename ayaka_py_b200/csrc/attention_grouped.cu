@@ -40,7 +40,7 @@ namespace {
 template <typename C>
 __global__ void __launch_bounds__(256)
 head_norm_prepare_kernel(C* __restrict__ qout, C* __restrict__ kpages, C* __restrict__ vpages,
-                         const float* __restrict__ proj, long long stride, const float* __restrict__ qw,
+                         const float* proj, long long stride, const float* __restrict__ qw,
                          const float* __restrict__ kw, const float* __restrict__ mix, const int* __restrict__ row_req,
                          const int* __restrict__ positions, const int* __restrict__ table, int table_stride,
                          int page_size, int H, int G, int D, int maps, int v_col0, int v_width, float eps, int writes) {
@@ -115,7 +115,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, float a, float b, flo
 template <typename C>
 __global__ void __launch_bounds__(256)
 head_norm_prepare_vec_kernel(C* __restrict__ qout, C* __restrict__ kpages, C* __restrict__ vpages,
-                             const float* __restrict__ proj, long long stride, const float* __restrict__ qw,
+                             const float* proj, long long stride, const float* __restrict__ qw,
                              const float* __restrict__ kw, const float* __restrict__ mix, const int* __restrict__ row_req,
                              const int* __restrict__ positions, const int* __restrict__ table, int table_stride,
                              int page_size, int H, int G, int D, int maps, int v_col0, int v_width, float eps, int writes) {
@@ -378,9 +378,9 @@ grouped_attention_kernel(GroupedArgs a) {
 //              number per head).
 template <typename C>
 __global__ void __launch_bounds__(64)
-grouped_finish_kernel(C* __restrict__ out, const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
+grouped_finish_kernel(C* __restrict__ out, const float* partial_o, const float* partial_ml,
                       const int* __restrict__ positions, int total_rows, int QH, int DV, int parts, int part_keys,
-                      int from_first, int window, int chunk, int maps, int hpg, const float* __restrict__ gate, long long gate_stride, float lambda,
+                      int from_first, int window, int chunk, int maps, int hpg, const float* gate, long long gate_stride, float lambda,
                       float post_scale, float eps) {
   __shared__ float other[MAX_DV];
   pdl_trigger();

@@ -364,8 +364,8 @@ grouped_attention_mma_kernel(GroupedArgs a, int page_shift, int tq, int DKP, int
       for (int nt = 0; nt < DVT / 8; ++nt) {
         const int col = nt * 8 + tig * 2;
         const bool on = gate != nullptr && col < DV;
-        gv[nt][0] = on ? __ldg(gate + col) : 0.f;
-        gv[nt][1] = on ? __ldg(gate + col + 1) : 0.f;
+        gv[nt][0] = on ? gate[col] : 0.f;
+        gv[nt][1] = on ? gate[col + 1] : 0.f;
       }
 #pragma unroll
       for (int nt = 0; nt < DVT / 8; ++nt) {

@@ -48,8 +48,8 @@ __device__ __forceinline__ void copy4(float* dst, const float* src) {
 // NC: head-dim columns in runs of 64.
 template <typename T, int NC>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_simt_kernel(T* __restrict__ out, const T* __restrict__ q, int q_stride,
-                      const T* __restrict__ kcache, const T* __restrict__ vcache,
+attention_simt_kernel(T* __restrict__ out, const T* q, int q_stride,
+                      const T* kcache, const T* vcache,
                       const int* __restrict__ table, int table_stride,
                       const int* __restrict__ req_q_start, const int* __restrict__ req_pos0,
                       int num_req, int H, int Hkv, int Dh, int page_size, float scale, int window) {

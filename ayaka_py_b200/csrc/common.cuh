@@ -94,6 +94,10 @@ __device__ __forceinline__ float apply_activation_tc(float x, int act) {
 // Programmatic dependent launch: a kernel launched with the attribute may start
 // while its predecessor in the stream still runs; it must not touch memory that
 // the predecessor writes (or write memory that it reads) before pdl_wait().
+// The compiler has to keep to that too.  Through a __restrict__ parameter (const or not), or with __ldg, it may take it
+// that nothing else writes the memory, and move a load ahead of the wait: so what kernels of the step write is read through
+// plain pointers in every kernel, and __restrict__ is for weights, for what the host uploads before the step, and for
+// results that the kernel only writes.  A function that is called behind the wait may have __restrict__ parameters.
 // pdl_trigger() lets the successor be scheduled; a block that never calls it does so by its end.
 // Without the attribute both are no-ops.
 //

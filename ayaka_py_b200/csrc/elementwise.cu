@@ -62,7 +62,7 @@ AYK_EXPORT int ayk_init(int device) {
 
 // ------------------------------------------------------------------- embed --
 template <typename W>
-__global__ void embed_kernel(float* __restrict__ out, const int* __restrict__ tok,
+__global__ void embed_kernel(float* __restrict__ out, const int* tok,
                              const int* __restrict__ pos, const W* __restrict__ wte,
                              const W* __restrict__ wpe, int d) {
   pdl_trigger();
@@ -107,7 +107,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 template <typename O>
-__global__ void layernorm_kernel(O* __restrict__ out, const float* __restrict__ x,
+__global__ void layernorm_kernel(O* __restrict__ out, const float* x,
                                  const float* __restrict__ gamma, const float* __restrict__ beta,
                                  const int* __restrict__ rows, int d, float eps) {
   extern __shared__ float row[];
@@ -156,7 +156,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float a, float b, float
 // variant took 10.2 us and was removed.
 template <typename O>
 __global__ void __launch_bounds__(128)
-layernorm_row_kernel(O* __restrict__ out, const float* __restrict__ x, const float* __restrict__ gamma,
+layernorm_row_kernel(O* __restrict__ out, const float* x, const float* __restrict__ gamma,
                      const float* __restrict__ beta, const int* __restrict__ rows, int d, float eps) {
   __shared__ float red[32];
   pdl_trigger();
@@ -231,7 +231,7 @@ AYK_EXPORT int ayk_layernorm(void* out, const float* x, const float* gamma, cons
 // --------------------------------------------------------------- kv append --
 template <typename T>
 __global__ void kv_append_kernel(T* __restrict__ kcache, T* __restrict__ vcache,
-                                 const T* __restrict__ k, const T* __restrict__ v, int row_stride,
+                                 const T* k, const T* v, int row_stride,
                                  const int* __restrict__ row_req, const int* __restrict__ pos,
                                  const int* __restrict__ table, int table_stride, int page_size,
                                  int width, int vec_ok) {
@@ -292,7 +292,7 @@ AYK_EXPORT int ayk_kv_append(void* kcache, void* vcache, const void* k, const vo
 // out[t, i] = act(z[t, i]) * z[t, n + i] for i < n: the two halves of a fused gate | up projection.
 template <typename I, typename O>
 __global__ void __launch_bounds__(256)
-gated_act_kernel(O* __restrict__ out, const I* __restrict__ z, long long z_stride, int n, int act, long long total) {
+gated_act_kernel(O* __restrict__ out, const I* z, long long z_stride, int n, int act, long long total) {
   pdl_trigger();
   pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -307,7 +307,7 @@ gated_act_kernel(O* __restrict__ out, const I* __restrict__ z, long long z_strid
 // bfloat16 results take the tanh form of GELU from the fast exponential (a few ulp in 32-bit before the rounding).
 template <typename O>
 __global__ void __launch_bounds__(256)
-gated_act_vec_kernel(O* __restrict__ out, const float* __restrict__ z, long long z_stride, int n, int act) {
+gated_act_vec_kernel(O* __restrict__ out, const float* z, long long z_stride, int n, int act) {
   pdl_trigger();
   pdl_wait();
   const int c = (blockIdx.y * 256 + threadIdx.x) * 4;
@@ -334,11 +334,14 @@ gated_act_vec_kernel(O* __restrict__ out, const float* __restrict__ z, long long
   }
 }
 
-__global__ void __launch_bounds__(256) add_rows_kernel(float* __restrict__ x, const float* __restrict__ y, long long total) {
-  pdl_trigger();
-  pdl_wait();
+__device__ __forceinline__ void add_rows(float* __restrict__ x, const float* __restrict__ y, long long total) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     x[i] += y[i];
+}
+__global__ void __launch_bounds__(256) add_rows_kernel(float* x, const float* y, long long total) {
+  pdl_trigger();
+  pdl_wait();
+  add_rows(x, y, total);
 }
 
 AYK_EXPORT int ayk_gated_act(void* out, const void* z, long long z_stride, int T, int n, int act, int in_dtype,

@@ -43,7 +43,7 @@ __device__ __forceinline__ void f32_copy4(float* dst, const float* src, bool on)
 
 template <int TM, bool VEC>
 __global__ void __launch_bounds__(256, 2)
-gemm_f32_kernel(float* C, const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+gemm_f32_kernel(float* C, const float* A, const float* __restrict__ W, const float* __restrict__ bias,
                 const float* residual,               // C and residual may be one buffer (the residual stream in place)
                 int M, int N, int K, int act) {
   constexpr int RM = TM / 8;
@@ -202,7 +202,7 @@ __device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&v)[4]) {
 
 template <typename TA, typename TW, typename TO, bool VEC>
 __global__ void __launch_bounds__(256)
-gemm_simt_kernel(TO* C, const TA* __restrict__ A, const TW* __restrict__ W,
+gemm_simt_kernel(TO* C, const TA* A, const TW* __restrict__ W,
                  const float* __restrict__ bias, const float* residual,      // C and residual may be one buffer (the residual stream in place)
                  int M, int N, int K, int act) {
   __shared__ float As[BK][BM + 4];

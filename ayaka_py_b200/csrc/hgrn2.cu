@@ -27,7 +27,7 @@ constexpr int WARPS = 4, COLS = 32, CHUNK = 16;
 
 template <int DP>      // state rows per thread: ceil(dim / 4) <= DP
 __global__ void __launch_bounds__(WARPS * 32)
-hgrn2_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ proj, int proj_stride,
+hgrn2_kernel(float* __restrict__ out, float* state, const float* proj, int proj_stride,
              const float* __restrict__ f_bias, const float* __restrict__ lower, const int* __restrict__ req_q_start,
              const int* __restrict__ req_slot, int H, int dim, int vdim) {
   extern __shared__ __align__(16) float smem[];
@@ -135,7 +135,7 @@ __device__ __forceinline__ bool find_chunk(const int* req_q_start, int num_req, 
 }
 
 __global__ void __launch_bounds__(128)
-hgrn2_chunk_prepare_kernel(float* __restrict__ scratch, const float* __restrict__ proj, int proj_stride,
+hgrn2_chunk_prepare_kernel(float* __restrict__ scratch, const float* proj, int proj_stride,
                            const float* __restrict__ f_bias, const float* __restrict__ lower,
                            const int* __restrict__ req_q_start, int num_req, int H, int dim) {
   extern __shared__ __align__(16) float smem[];
@@ -214,8 +214,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 template <int DP>
 __global__ void __launch_bounds__(SW * 32)
-hgrn2_chunk_scan_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ scratch,
-                        const float* __restrict__ proj, int proj_stride, const int* __restrict__ req_q_start,
+hgrn2_chunk_scan_kernel(float* __restrict__ out, float* state, const float* scratch,
+                        const float* proj, int proj_stride, const int* __restrict__ req_q_start,
                         const int* __restrict__ req_slot, int H, int dim, int vdim) {
   extern __shared__ __align__(16) float smem[];
   const size_t per_chunk = chunk_floats(dim);              // a multiple of 4 floats

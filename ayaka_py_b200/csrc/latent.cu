@@ -31,7 +31,7 @@ __device__ __forceinline__ void turn_pair(float& u, float& v, float angle, float
 // x[t, head * head_stride + offset + (0 .. dims)) turned in place; x rows lie x_stride apart.
 // ``halves``: dimension i is paired with i + dims/2 instead of neighbours (2i, 2i + 1).
 template <typename T>
-__global__ void rotary_kernel(T* __restrict__ x, long long x_stride, const int* __restrict__ positions,
+__global__ void rotary_kernel(T* x, long long x_stride, const int* __restrict__ positions,
                               const float* __restrict__ freq, float gain, int heads, int head_stride, int offset,
                               int dims, int halves) {
   pdl_trigger();
@@ -64,7 +64,7 @@ __global__ void rotary_kernel(T* __restrict__ x, long long x_stride, const int* 
 template <typename C, int VEC>
 __global__ void __launch_bounds__(128)
 latent_prepare_kernel(C* __restrict__ latent_pages, C* __restrict__ rope_pages, float* __restrict__ query,
-                      const float* __restrict__ proj, int proj_stride, const float* __restrict__ norm_w,
+                      const float* proj, int proj_stride, const float* __restrict__ norm_w,
                       const float* __restrict__ freq, float gain, int rot_dims, int halves, const int* __restrict__ row_req,
                       const int* __restrict__ positions, const int* __restrict__ table, int table_stride, int page_size,
                       int H, int dim, int rot, int rank, float eps, int writes) {
@@ -151,8 +151,8 @@ constexpr int HM_ROWS = 16, HM_COLS = 64, HM_K = 32;
 
 template <typename W, typename O>
 __global__ void __launch_bounds__(128)
-head_matmul_kernel(O* __restrict__ out, long long out_row, int out_head, const float* __restrict__ a, long long a_row,
-                   int a_head, const W* __restrict__ w, const float* __restrict__ gate, long long gate_row, int gate_head, int gate_col, int T, int N,
+head_matmul_kernel(O* __restrict__ out, long long out_row, int out_head, const float* a, long long a_row,
+                   int a_head, const W* __restrict__ w, const float* gate, long long gate_row, int gate_head, int gate_col, int T, int N,
                    int K) {
   __shared__ float As[HM_ROWS][HM_K + 1];
   __shared__ float Ws[HM_COLS][HM_K + 1];
@@ -210,8 +210,8 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
 
 template <typename W, typename O>
 __global__ void __launch_bounds__(MV_WARPS * 32)
-head_matvec_kernel(O* __restrict__ out, long long out_row, int out_head, const float* __restrict__ a, long long a_row,
-                   int a_head, const W* __restrict__ w, const float* __restrict__ gate, long long gate_row, int gate_head, int gate_col, int T, int N,
+head_matvec_kernel(O* __restrict__ out, long long out_row, int out_head, const float* a, long long a_row,
+                   int a_head, const W* __restrict__ w, const float* gate, long long gate_row, int gate_head, int gate_col, int T, int N,
                    int K) {
   extern __shared__ __align__(16) float rows[];          // [T][K]
   const int h = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -261,8 +261,8 @@ constexpr int AQ = 32, AKEYS = 32, AWARPS = 4, ARQ = AQ / AWARPS;
 
 template <typename C, int NC>
 __global__ void __launch_bounds__(AWARPS * 32)
-latent_attention_kernel(float* __restrict__ out, const float* __restrict__ query, const C* __restrict__ latent_pages,
-                        const C* __restrict__ rope_pages, const int* __restrict__ table, int table_stride,
+latent_attention_kernel(float* __restrict__ out, const float* query, const C* latent_pages,
+                        const C* rope_pages, const int* __restrict__ table, int table_stride,
                         const int* __restrict__ req_q_start, const int* __restrict__ req_pos0, int num_req, int H, int HG,
                         int BR, int rank, int rot, int page_size, float scale, int window) {
   pdl_trigger();

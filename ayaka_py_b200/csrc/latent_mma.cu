@@ -55,8 +55,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // partial: [pairs of the step = T * H][parts][2 + rank] floats (maximum in the log2 domain, sum, O).
 template <int RPW, int CG, int WM>
 __global__ void __launch_bounds__(32 * WM * CG)
-latent_attention_mma_kernel(float* __restrict__ out, float* __restrict__ partial, const float* __restrict__ query,
-                            const __nv_bfloat16* __restrict__ latent_pages, const __nv_bfloat16* __restrict__ rope_pages,
+latent_attention_mma_kernel(float* __restrict__ out, float* __restrict__ partial, const float* query,
+                            const __nv_bfloat16* latent_pages, const __nv_bfloat16* rope_pages,
                             const int* __restrict__ table, int table_stride, const int* __restrict__ req_q_start,
                             const int* __restrict__ req_pos0, int num_req, int H, int HG, int BR, int rank, int rot,
                             int page_size, float scale_log2, int window, int parts, int part_keys) {
@@ -317,7 +317,7 @@ latent_attention_mma_kernel(float* __restrict__ out, float* __restrict__ partial
 // sums are fetched side by side first, every warp reduces them for itself; then a thread adds up two columns at a time,
 // eight partitions' loads under way together.  A partition that saw nothing is skipped (its O was never written).
 constexpr int MERGE_PARTS = 1024;
-__global__ void __launch_bounds__(256) latent_merge_kernel(float* __restrict__ out, const float* __restrict__ partial, int rank, int parts) {
+__global__ void __launch_bounds__(256) latent_merge_kernel(float* __restrict__ out, const float* partial, int rank, int parts) {
   __shared__ float2 ml[MERGE_PARTS];
   pdl_trigger();
   pdl_wait();
@@ -363,8 +363,8 @@ constexpr int PM = 64, PN = 64, PK = 64, PLD = PK + 8;
 
 template <typename O>
 __global__ void __launch_bounds__(128)
-head_matmul_mma_kernel(O* __restrict__ out, long long out_row, int out_head, const float* __restrict__ a, long long a_row,
-                       int a_head, const __nv_bfloat16* __restrict__ w, const float* __restrict__ gate, long long gate_row, int gate_head, int gate_col,
+head_matmul_mma_kernel(O* __restrict__ out, long long out_row, int out_head, const float* a, long long a_row,
+                       int a_head, const __nv_bfloat16* __restrict__ w, const float* gate, long long gate_row, int gate_head, int gate_col,
                        int T, int N, int K) {
   __shared__ __align__(16) __nv_bfloat16 As[PM * PLD];
   __shared__ __align__(16) __nv_bfloat16 Al[PM * PLD];       // what rounding to bfloat16 left over

@@ -44,7 +44,7 @@ constexpr int WWARPS = 8, WCOLS = 32, WTOK = 16;
 
 template <int DP>          // rows of S per thread, at most
 __global__ void __launch_bounds__(WWARPS * 32, DP <= 16 ? 4 : 1)
-decay_walk_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ proj, long long stride,
+decay_walk_kernel(float* __restrict__ out, float* state, const float* proj, long long stride,
                   const float* __restrict__ powers, const int* __restrict__ req_q_start, const int* __restrict__ req_slot,
                   int H, int D, int DV, int settled) {
   extern __shared__ __align__(16) float sh[];
@@ -176,7 +176,7 @@ __host__ __device__ inline size_t decay_chunk_bytes(int D, int COLS) {
 // memory once per chunk for the product with q.
 template <int MT, int NT>
 __global__ void __launch_bounds__(CWARPS * 32)
-decay_chunk_kernel(float* __restrict__ out, float* __restrict__ state, const __nv_bfloat16* __restrict__ qkv, long long stride,
+decay_chunk_kernel(float* __restrict__ out, float* state, const __nv_bfloat16* qkv, long long stride,
                    const float* __restrict__ powers, const int* __restrict__ req_q_start, const int* __restrict__ req_slot,
                    int H, int D, int DV, int vec, int settled) {
   constexpr int CT = DECAY_CHUNK, COLS = NT * 8, LDV = COLS + 8, THREADS = CWARPS * 32;
@@ -457,7 +457,7 @@ __host__ __device__ inline size_t decay_sum_bytes(int D, int COLS) {
 // scratch [chunk][H][D][DV] = sum_s lambda^(L-1-s) k_s v_s^T.  Block (8 NT value columns, head, chunk), four warps.
 template <int MT, int NT>
 __global__ void __launch_bounds__(CWARPS * 32)
-decay_chunk_sum_kernel(float* __restrict__ scratch, const __nv_bfloat16* __restrict__ qkv, long long stride,
+decay_chunk_sum_kernel(float* __restrict__ scratch, const __nv_bfloat16* qkv, long long stride,
                        const float* __restrict__ powers, const int* __restrict__ req_q_start, int R, int H, int D, int DV, int vec) {
   constexpr int CT = DECAY_CHUNK, COLS = NT * 8, LDV = COLS + 8, THREADS = CWARPS * 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -545,7 +545,7 @@ decay_chunk_sum_kernel(float* __restrict__ scratch, const __nv_bfloat16* __restr
 // Per eight cells of S: the walk over a request's chunks.  Scratch gets every chunk's S_0 in the place of what the chunk
 // added, as two bfloat16 parts (eight roundings, then eight remainders: the 32 bytes of the eight cells); the state the last S.
 __global__ void __launch_bounds__(128)
-decay_chunk_scan_kernel(float* __restrict__ scratch, float* __restrict__ state, const float* __restrict__ powers,
+decay_chunk_scan_kernel(float* scratch, float* state, const float* __restrict__ powers,
                         const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int H, int cells) {
   constexpr int AHEAD = 8;
   pdl_trigger();
@@ -600,7 +600,7 @@ __host__ __device__ inline size_t decay_out_bytes(int D, int COLS) {
 // The outputs of one chunk from its S_0 (scratch).  Block (8 NT value columns, head, chunk), four warps of 16 tokens.
 template <int NT>
 __global__ void __launch_bounds__(CWARPS * 32)
-decay_chunk_out_kernel(float* __restrict__ out, const float* __restrict__ scratch, const __nv_bfloat16* __restrict__ qkv,
+decay_chunk_out_kernel(float* __restrict__ out, const float* scratch, const __nv_bfloat16* qkv,
                        long long stride, const float* __restrict__ powers, const int* __restrict__ req_q_start, int R, int H, int D,
                        int DV, int vec) {
   constexpr int CT = DECAY_CHUNK, COLS = NT * 8, LDV = COLS + 8, THREADS = CWARPS * 32;
@@ -744,7 +744,7 @@ int launch_side_by_side(float* out, float* state, float* scratch, const __nv_bfl
 // out[t, :] = raw[t, :] / rms(raw[t, :]) * w * sigmoid(gate[t, :]) over a row of n numbers (all heads together).
 template <typename C, int VEC>
 __global__ void __launch_bounds__(256)
-decay_finish_kernel(C* __restrict__ out, const float* __restrict__ raw, const float* __restrict__ gate, long long gate_stride,
+decay_finish_kernel(C* __restrict__ out, const float* raw, const float* gate, long long gate_stride,
                     const float* __restrict__ w, int n, float eps) {
   __shared__ float red[8];
   pdl_trigger();

@@ -60,7 +60,7 @@ constexpr int WALK_THREADS = 1024;
 
 template <typename C>
 __global__ void __launch_bounds__(WALK_THREADS)
-mlstm_walk_kernel(C* __restrict__ out, float* __restrict__ state, const float* __restrict__ proj, long long stride,
+mlstm_walk_kernel(C* __restrict__ out, float* state, const float* proj, long long stride,
                   const float* __restrict__ norm_w, const int* __restrict__ req_q_start, const int* __restrict__ req_slot,
                   int H, int D, int DV, float cap, float eps) {
   extern __shared__ float sh[];
@@ -179,7 +179,7 @@ __host__ __device__ inline size_t chunk_floats(int D, int CT, int COLS) {
 // two buffers while this chunk is worked on.  q stays unscaled in shared memory; D^-1/2 multiplies the sums.
 template <int CT, int COLS>
 __global__ void __launch_bounds__(CTHREADS)
-mlstm_chunk_kernel(float* __restrict__ raw, float* __restrict__ nm, float* __restrict__ state, const float* __restrict__ proj,
+mlstm_chunk_kernel(float* __restrict__ raw, float* __restrict__ nm, float* state, const float* proj,
                    long long stride, const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int H, int D,
                    int DV, float cap) {
   extern __shared__ __align__(16) float sh[];
@@ -403,8 +403,8 @@ mlstm_chunk_kernel(float* __restrict__ raw, float* __restrict__ nm, float* __res
 // request's first row also files the head's n and m from the scratch buffer into the state.
 template <typename C>
 __global__ void __launch_bounds__(128)
-mlstm_finish_kernel(C* __restrict__ out, float* __restrict__ state, const float* __restrict__ raw, const float* __restrict__ nm,
-                    const float* __restrict__ proj, long long stride, const float* __restrict__ norm_w,
+mlstm_finish_kernel(C* __restrict__ out, float* state, const float* raw, const float* nm,
+                    const float* proj, long long stride, const float* __restrict__ norm_w,
                     const int* __restrict__ row_req, const int* __restrict__ req_q_start, const int* __restrict__ req_slot,
                     int H, int D, int DV, float eps) {
   __shared__ float red[32];
@@ -596,7 +596,7 @@ mlstm_long_sum_kernel(LongScratch x, const float* proj, long long stride, const 
 // A thread owns four neighbouring cells of S (or of n) of one head and walks the request's chunks; eight chunks' loads
 // are on their way together.
 __global__ void __launch_bounds__(256)
-mlstm_long_scan_kernel(LongScratch x, float* __restrict__ state, const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int H,
+mlstm_long_scan_kernel(LongScratch x, float* state, const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int H,
                        int D, int DV) {
   const int h = blockIdx.y, r = blockIdx.z;
   pdl_wait();
@@ -649,7 +649,7 @@ constexpr size_t LONG_OUT_SMEM = (size_t)(LC * LMAX + LC * LLD + SHALF * LMAX + 
 static_assert(LC * LPD <= LC * LMAX, "P fits the queries' place");
 template <typename C>
 __global__ void __launch_bounds__(OTHREADS, 2)
-mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* __restrict__ state, const float* proj, long long stride,
+mlstm_long_out_kernel(C* __restrict__ out, LongScratch x, float* state, const float* proj, long long stride,
                       const float* __restrict__ norm_w, const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int num_req,
                       int H, int D, int DV, float cap, float eps) {
   extern __shared__ __align__(16) float sm[];

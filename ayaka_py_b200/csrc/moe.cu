@@ -42,7 +42,7 @@ constexpr int TILE_ROWS = 32;
 // ------------------------------------------------------------------- route --
 // A warp per token.
 __global__ void __launch_bounds__(128)
-moe_route_kernel(int* __restrict__ ids, float* __restrict__ weights, const float* __restrict__ logits, long long stride,
+moe_route_kernel(int* __restrict__ ids, float* __restrict__ weights, const float* logits, long long stride,
                  int T, int E, int top) {
   pdl_trigger();
   pdl_wait();
@@ -94,7 +94,7 @@ moe_route_kernel(int* __restrict__ ids, float* __restrict__ weights, const float
 // scores (the lower index wins a tie).
 template <bool SOFTMAX>
 __global__ void __launch_bounds__(128)
-moe_route_scored_kernel(int* __restrict__ ids, float* __restrict__ weights, const float* __restrict__ logits, long long stride,
+moe_route_scored_kernel(int* __restrict__ ids, float* __restrict__ weights, const float* logits, long long stride,
                         const float* __restrict__ correction, int T, int E, int top, int groups, int keep, int group_best,
                         int normalize, float factor) {
   pdl_trigger();
@@ -188,7 +188,7 @@ moe_route_scored_kernel(int* __restrict__ ids, float* __restrict__ weights, cons
 // One block.  tiles[0] = number of tiles; tile i: expert tiles[1 + 3 i], first sorted row
 // tiles[2 + 3 i], rows tiles[3 + 3 i].
 __global__ void __launch_bounds__(1024)
-moe_plan_kernel(int* __restrict__ sorted, int* __restrict__ tiles, const int* __restrict__ ids, int P, int E) {
+moe_plan_kernel(int* __restrict__ sorted, int* __restrict__ tiles, const int* ids, int P, int E) {
   extern __shared__ int sh[];
   int* count = sh;          // [E]
   int* start = sh + E;      // [E]
@@ -229,7 +229,7 @@ constexpr int PAD_ROWS = 128;
 
 __global__ void __launch_bounds__(1024)
 moe_plan_padded_kernel(int* __restrict__ row_of_pair, int* __restrict__ w_rows1, int* __restrict__ w_rows2,
-                       const int* __restrict__ ids, int P, int E, int n1, int n2, int max_tiles) {
+                       const int* ids, int P, int E, int n1, int n2, int max_tiles) {
   extern __shared__ int sh[];
   int* count = sh;          // [E]
   int* start = sh + E;      // [E]
@@ -261,8 +261,8 @@ moe_plan_padded_kernel(int* __restrict__ row_of_pair, int* __restrict__ w_rows1,
 // out[row_of_pair[p], :] = in[p / top, :], bfloat16 rows of d elements (d a multiple of 8); a warp per pair.  With
 // row_scale: row_scale[row_of_pair[p]] = weights[p].
 __global__ void __launch_bounds__(256)
-moe_gather_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ in, long long in_stride,
-                  const int* __restrict__ row_of_pair, float* __restrict__ row_scale, const float* __restrict__ weights, int P,
+moe_gather_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* in, long long in_stride,
+                  const int* row_of_pair, float* __restrict__ row_scale, const float* weights, int P,
                   int top, int d) {
   pdl_trigger();
   pdl_wait();
@@ -285,9 +285,9 @@ constexpr int BN = 64, BK = 32;
 
 template <typename T, typename O, bool GLU>
 __global__ void __launch_bounds__(256)
-moe_gemm_kernel(O* __restrict__ out, const T* __restrict__ a, long long a_stride, const T* __restrict__ w,
-                const int* __restrict__ sorted, const int* __restrict__ tiles, int top, int gather, int scatter, int N,
-                int N_w, int Kd, float limit, float slope, float plus, int act, const float* __restrict__ early) {
+moe_gemm_kernel(O* __restrict__ out, const T* a, long long a_stride, const T* __restrict__ w,
+                const int* sorted, const int* tiles, int top, int gather, int scatter, int N,
+                int N_w, int Kd, float limit, float slope, float plus, int act, const float* early) {
   __shared__ float factor[TILE_ROWS];
   __shared__ float As[BK][TILE_ROWS + 1];
   __shared__ float Bs[GLU ? 2 : 1][BK][BN + 1];
@@ -380,10 +380,10 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 
 template <typename O, bool GLU>
 __global__ void __launch_bounds__(128)
-moe_gemm_mma_kernel(O* __restrict__ out, const __nv_bfloat16* __restrict__ a, long long a_stride,
-                    const __nv_bfloat16* __restrict__ w, const int* __restrict__ sorted, const int* __restrict__ tiles,
+moe_gemm_mma_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
+                    const __nv_bfloat16* __restrict__ w, const int* sorted, const int* tiles,
                     int top, int gather, int scatter, int N, int N_w, int Kd, float limit, float slope, float plus, int act,
-                    const float* __restrict__ early) {
+                    const float* early) {
   __shared__ float factor[TILE_ROWS];
   __shared__ __align__(16) __nv_bfloat16 As[TILE_ROWS][TLD];
   __shared__ __align__(16) __nv_bfloat16 Bs[GLU ? 2 : 1][BN][TLD];
@@ -507,8 +507,6 @@ __global__ void __launch_bounds__(256, GLU ? 2 : 4)
 moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
                 const __nv_bfloat16* __restrict__ w, const int* ids, int top, int gather, int N, int N_w,
                 int Kd, float limit, float slope, float plus, int act, const float* early) {
-  // (what kernels before this one write has no __restrict__: a load that the compiler takes for constant may be moved ahead
-  // of the wait below)
   constexpr int STREAMS = GLU ? 4 : 2, STEPS = 4, PER_WARP = gv_cols(GLU) / 8;
   extern __shared__ __align__(16) float xs[];          // [Kd]
   pdl_wait();
@@ -589,8 +587,8 @@ moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
 // out[t, c] = act(f in[t, c], f in[t, n + c]) for the dense (shared) expert, f = row_scale[t] (null: 1).
 template <typename I, typename O>
 __global__ void __launch_bounds__(256)
-glu_limited_kernel(O* __restrict__ out, const I* __restrict__ in, long long stride, int n, float limit, float slope, float plus,
-                   const float* __restrict__ row_scale) {
+glu_limited_kernel(O* __restrict__ out, const I* in, long long stride, int n, float limit, float slope, float plus,
+                   const float* row_scale) {
   pdl_trigger();
   pdl_wait();
   const I* row = in + (size_t)blockIdx.x * stride;
@@ -613,8 +611,8 @@ __device__ __forceinline__ void load_four(const __nv_bfloat16* p, float (&v)[4])
 
 template <typename I, typename O>
 __global__ void __launch_bounds__(256)
-glu_limited_vec_kernel(O* __restrict__ out, const I* __restrict__ in, long long stride, int n, float limit, float slope, float plus,
-                       const float* __restrict__ row_scale) {
+glu_limited_vec_kernel(O* __restrict__ out, const I* in, long long stride, int n, float limit, float slope, float plus,
+                       const float* row_scale) {
   pdl_trigger();
   pdl_wait();
   const int c = (blockIdx.y * 256 + threadIdx.x) * 4;

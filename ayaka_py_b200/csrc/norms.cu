@@ -85,7 +85,7 @@ __device__ __forceinline__ void block_sums_upto(float (&v)[N], float* red, int n
 // is that many runs of d numbers side by side, each divided by its own root mean square.
 template <typename O>
 __global__ void __launch_bounds__(THREADS)
-rmsnorm_kernel(O* __restrict__ out, long long out_stride, const float* __restrict__ x, long long x_stride,
+rmsnorm_kernel(O* __restrict__ out, long long out_stride, const float* x, long long x_stride,
                const float* __restrict__ w, const int* __restrict__ rows, int d, float eps) {
   __shared__ float red[4];
   pdl_trigger();
@@ -117,8 +117,8 @@ constexpr int VEC_TAPS = 8;
 
 template <typename O>
 __global__ void __launch_bounds__(1024)
-rmsnorm_conv_kernel(O* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w,
-                    const float* __restrict__ taps_w, float* __restrict__ state, const int* __restrict__ row_req,
+rmsnorm_conv_kernel(O* __restrict__ out, const float* x, const float* __restrict__ w,
+                    const float* __restrict__ taps_w, float* state, const int* __restrict__ row_req,
                     const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int d, int taps, float eps,
                     int inline_state) {
   __shared__ float red[32 * MAX_TAPS];
@@ -191,8 +191,8 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float a, float b, float
 
 template <typename O, int VT>      // VT: the most taps this instance holds rows for
 __global__ void __launch_bounds__(512, 2)
-rmsnorm_conv_vec_kernel(O* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w,
-                        const float* __restrict__ taps_w, float* __restrict__ state, const int* __restrict__ row_req,
+rmsnorm_conv_vec_kernel(O* __restrict__ out, const float* x, const float* __restrict__ w,
+                        const float* __restrict__ taps_w, float* state, const int* __restrict__ row_req,
                         const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int d, int taps, float eps,
                         int inline_state) {
   __shared__ float red[32 * VT];
@@ -270,7 +270,7 @@ rmsnorm_conv_vec_kernel(O* __restrict__ out, const float* __restrict__ x, const 
 // The state after a step: the last taps - 1 of (old state, the portion's inputs h).  One block
 // per request; a thread reads what it needs of its channels before it writes them.
 __global__ void __launch_bounds__(1024)
-conv_state_kernel(float* __restrict__ state, const float* __restrict__ x, const float* __restrict__ w,
+conv_state_kernel(float* state, const float* x, const float* __restrict__ w,
                   const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int d, int taps, float eps) {
   __shared__ float red[32 * MAX_TAPS];
   pdl_trigger();
@@ -313,46 +313,40 @@ conv_state_kernel(float* __restrict__ state, const float* __restrict__ x, const 
 // ------------------------------------------------------ normed residual sum --
 // x[t, :] += mult * y[t, :] / rms(y[t, :]) * w; with several groups (grid y) a row is that many runs of d
 // numbers, each with its own root mean square.
-__global__ void __launch_bounds__(THREADS)
-rmsnorm_residual_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w, int d,
-                        float eps, float mult) {
-  __shared__ float red[4];
-  pdl_trigger();
-  const size_t at = ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * d;
-  w += (size_t)blockIdx.y * d;
-  pdl_wait();
-  const float* src = y + at;
+//
+// The kernels that update rows in place read and write through `__restrict__` in functions of their own that begin behind
+// the wait (see pdl_wait): the loads of a loop then still go ahead of its stores, but none ahead of the wait.
+__device__ __forceinline__ void rmsnorm_residual(float* __restrict__ dst, const float* __restrict__ src, const float* __restrict__ w, int d,
+                                                 float eps, float mult, float* red) {
   float s = 0.f;
   for (int i = threadIdx.x; i < d; i += THREADS) {
     const float v = src[i];
     s = fmaf(v, v, s);
   }
   const float inv = 1.0f / sqrtf(block_sum_128(s, red) / (float)d + eps);
-  float* dst = x + at;
   for (int i = threadIdx.x; i < d; i += THREADS) dst[i] += mult * (src[i] * inv * w[i]);
+}
+__global__ void __launch_bounds__(THREADS)
+rmsnorm_residual_kernel(float* x, const float* y, const float* __restrict__ w, int d, float eps, float mult) {
+  __shared__ float red[4];
+  pdl_trigger();
+  const size_t at = ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * d;
+  pdl_wait();
+  rmsnorm_residual(x + at, y + at, w + (size_t)blockIdx.y * d, d, eps, mult, red);
 }
 
 // The same, and the next norm of the updated stream in the same pass: out[t, :] = x[t, :] / rms(x[t, :]) * w2
 // with x as just updated (same runs, each with its own root mean square; eps2 under the root).
 template <typename O>
-__global__ void __launch_bounds__(THREADS)
-rmsnorm_residual_norm_kernel(float* __restrict__ x, O* __restrict__ out, const float* __restrict__ y,
-                             const float* __restrict__ w, const float* __restrict__ w2, int d, float eps, float mult,
-                             float eps2) {
-  __shared__ float red[4], red2[4];
-  pdl_trigger();
-  const size_t at = ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * d;
-  w += (size_t)blockIdx.y * d;
-  w2 += (size_t)blockIdx.y * d;
-  pdl_wait();
-  const float* src = y + at;
+__device__ __forceinline__ void rmsnorm_residual_norm(float* __restrict__ dst, O* __restrict__ o, const float* __restrict__ src,
+                                                      const float* __restrict__ w, const float* __restrict__ w2, int d, float eps,
+                                                      float mult, float eps2, float* red, float* red2) {
   float s = 0.f;
   for (int i = threadIdx.x; i < d; i += THREADS) {
     const float v = src[i];
     s = fmaf(v, v, s);
   }
   const float inv = 1.0f / sqrtf(block_sum_128(s, red) / (float)d + eps);
-  float* dst = x + at;
   float s2 = 0.f;
   for (int i = threadIdx.x; i < d; i += THREADS) {
     const float v = dst[i] + mult * (src[i] * inv * w[i]);
@@ -360,8 +354,17 @@ rmsnorm_residual_norm_kernel(float* __restrict__ x, O* __restrict__ out, const f
     s2 = fmaf(v, v, s2);
   }
   const float inv2 = 1.0f / sqrtf(block_sum_128(s2, red2) / (float)d + eps2);
-  O* o = out + at;
   for (int i = threadIdx.x; i < d; i += THREADS) o[i] = from_float<O>(dst[i] * inv2 * w2[i]);     // each thread reads back its own stores
+}
+template <typename O>
+__global__ void __launch_bounds__(THREADS)
+rmsnorm_residual_norm_kernel(float* x, O* __restrict__ out, const float* y, const float* __restrict__ w, const float* __restrict__ w2,
+                             int d, float eps, float mult, float eps2) {
+  __shared__ float red[4], red2[4];
+  pdl_trigger();
+  const size_t at = ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * d;
+  pdl_wait();
+  rmsnorm_residual_norm(x + at, out + at, y + at, w + (size_t)blockIdx.y * d, w2 + (size_t)blockIdx.y * d, d, eps, mult, eps2, red, red2);
 }
 
 // ---------------------------------------------- layer-normed residual sum --
@@ -369,15 +372,10 @@ rmsnorm_residual_norm_kernel(float* __restrict__ x, O* __restrict__ out, const f
 // deviations, made in a second pass over the row); b may be null.  With ``out``: the next layer norm of the
 // updated stream in the same kernel, out[t, :] = (x - mean(x)) / sqrt(var(x) + eps2) * w2 + b2.
 template <typename O>
-__global__ void __launch_bounds__(THREADS)
-layernorm_residual_kernel(float* __restrict__ x, O* __restrict__ out, const float* __restrict__ y,
-                          const float* __restrict__ w, const float* __restrict__ b, const float* __restrict__ w2,
-                          const float* __restrict__ b2, int d, float eps, float eps2) {
-  __shared__ float red[4], red2[4], red3[4], red4[4];
-  pdl_trigger();
-  const size_t at = (size_t)blockIdx.x * d;
-  pdl_wait();
-  const float* src = y + at;
+__device__ __forceinline__ void layernorm_residual(float* __restrict__ dst, O* __restrict__ o, const float* __restrict__ src,
+                                                   const float* __restrict__ w, const float* __restrict__ b, const float* __restrict__ w2,
+                                                   const float* __restrict__ b2, int d, float eps, float eps2, float* red, float* red2,
+                                                   float* red3, float* red4) {
   const float inv_d = 1.0f / (float)d;
   float s = 0.f;
   for (int i = threadIdx.x; i < d; i += THREADS) s += src[i];
@@ -388,14 +386,13 @@ layernorm_residual_kernel(float* __restrict__ x, O* __restrict__ out, const floa
     q = fmaf(c, c, q);
   }
   const float inv = 1.0f / sqrtf(block_sum_128(q, red2) * inv_d + eps);
-  float* dst = x + at;
   float s2 = 0.f;
   for (int i = threadIdx.x; i < d; i += THREADS) {
     const float v = dst[i] + fmaf((src[i] - mean) * inv, w[i], b ? b[i] : 0.f);
     dst[i] = v;
     s2 += v;
   }
-  if (!out) return;
+  if (!o) return;
   const float mean2 = block_sum_128(s2, red3) * inv_d;
   float q2 = 0.f;
   for (int i = threadIdx.x; i < d; i += THREADS) {         // each thread reads back its own stores
@@ -403,8 +400,17 @@ layernorm_residual_kernel(float* __restrict__ x, O* __restrict__ out, const floa
     q2 = fmaf(c, c, q2);
   }
   const float inv2 = 1.0f / sqrtf(block_sum_128(q2, red4) * inv_d + eps2);
-  O* o = out + at;
   for (int i = threadIdx.x; i < d; i += THREADS) o[i] = from_float<O>(fmaf((dst[i] - mean2) * inv2, w2[i], b2 ? b2[i] : 0.f));
+}
+template <typename O>
+__global__ void __launch_bounds__(THREADS)
+layernorm_residual_kernel(float* x, O* __restrict__ out, const float* y, const float* __restrict__ w, const float* __restrict__ b,
+                          const float* __restrict__ w2, const float* __restrict__ b2, int d, float eps, float eps2) {
+  __shared__ float red[4], red2[4], red3[4], red4[4];
+  pdl_trigger();
+  const size_t at = (size_t)blockIdx.x * d;
+  pdl_wait();
+  layernorm_residual(x + at, out ? out + at : nullptr, y + at, w, b, w2, b2, d, eps, eps2, red, red2, red3, red4);
 }
 
 // ------------------------------------------------- short groups: a warp each --
@@ -413,7 +419,7 @@ layernorm_residual_kernel(float* __restrict__ x, O* __restrict__ out, const floa
 // block per unit: more threads on each).
 template <typename O>
 __global__ void __launch_bounds__(THREADS)
-rmsnorm_warp_kernel(O* __restrict__ out, long long out_stride, const float* __restrict__ x, long long x_stride,
+rmsnorm_warp_kernel(O* __restrict__ out, long long out_stride, const float* x, long long x_stride,
                     const float* __restrict__ w, const int* __restrict__ rows, int d, int groups, int units, float eps) {
   pdl_trigger();
   const int u = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -432,38 +438,40 @@ rmsnorm_warp_kernel(O* __restrict__ out, long long out_stride, const float* __re
 
 // x += mult * norm(y) * w; with ``out`` also out = norm(x) * w2 of the updated rows.
 template <typename O>
+__device__ __forceinline__ void rmsnorm_residual_warp(float* __restrict__ dst, O* __restrict__ o, const float* __restrict__ src,
+                                                      const float* __restrict__ w, const float* __restrict__ w2, int d, int lane,
+                                                      float eps, float mult, float eps2) {
+  float s = 0.f;
+  for (int i = lane; i < d; i += 32) s = fmaf(src[i], src[i], s);
+  const float inv = 1.0f / sqrtf(warp_sum(s) / (float)d + eps);
+  float s2 = 0.f;
+  for (int i = lane; i < d; i += 32) {
+    const float v = dst[i] + mult * (src[i] * inv * w[i]);
+    dst[i] = v;
+    s2 = fmaf(v, v, s2);
+  }
+  if (!o) return;
+  const float inv2 = 1.0f / sqrtf(warp_sum(s2) / (float)d + eps2);
+  for (int i = lane; i < d; i += 32) o[i] = from_float<O>(dst[i] * inv2 * w2[i]);     // each lane reads back its own stores
+}
+template <typename O>
 __global__ void __launch_bounds__(THREADS)
-rmsnorm_residual_warp_kernel(float* __restrict__ x, O* __restrict__ out, const float* __restrict__ y,
-                             const float* __restrict__ w, const float* __restrict__ w2, int d, int groups, int units,
-                             float eps, float mult, float eps2) {
+rmsnorm_residual_warp_kernel(float* x, O* __restrict__ out, const float* y, const float* __restrict__ w, const float* __restrict__ w2,
+                             int d, int groups, int units, float eps, float mult, float eps2) {
   pdl_trigger();
   const int u = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (u >= units) return;
   pdl_wait();
   const size_t at = (size_t)u * d;              // rows are dense: unit u starts at u * d
   const int grp_at = (u % groups) * d;
-  const float* src = y + at;
-  float s = 0.f;
-  for (int i = lane; i < d; i += 32) s = fmaf(src[i], src[i], s);
-  const float inv = 1.0f / sqrtf(warp_sum(s) / (float)d + eps);
-  float* dst = x + at;
-  float s2 = 0.f;
-  for (int i = lane; i < d; i += 32) {
-    const float v = dst[i] + mult * (src[i] * inv * w[grp_at + i]);
-    dst[i] = v;
-    s2 = fmaf(v, v, s2);
-  }
-  if (!out) return;
-  const float inv2 = 1.0f / sqrtf(warp_sum(s2) / (float)d + eps2);
-  O* o = out + at;
-  for (int i = lane; i < d; i += 32) o[i] = from_float<O>(dst[i] * inv2 * w2[grp_at + i]);     // each lane reads back its own stores
+  rmsnorm_residual_warp(x + at, out ? out + at : nullptr, y + at, w + grp_at, w2 ? w2 + grp_at : nullptr, d, lane, eps, mult, eps2);
 }
 
 // ---------------------------------------------------------------- polynorm --
 // out = a z / rms(z) + b z^2 / rms(z^2) + c z^3 / rms(z^3) + e over a row of width n.
 template <typename I, typename O>
 __global__ void __launch_bounds__(THREADS)
-polynorm_kernel(O* __restrict__ out, const I* __restrict__ z, const float* __restrict__ coeff, int n, float eps) {
+polynorm_kernel(O* __restrict__ out, const I* z, const float* __restrict__ coeff, int n, float eps) {
   __shared__ float red[12];
   pdl_trigger();
   const float a = coeff[0], b = coeff[1], c = coeff[2], e = coeff[3];
@@ -491,7 +499,7 @@ polynorm_kernel(O* __restrict__ out, const I* __restrict__ z, const float* __res
 
 // ------------------------------------------------------------ scaled embed --
 template <typename W>
-__global__ void embed_scaled_kernel(float* __restrict__ out, const int* __restrict__ tok, const W* __restrict__ table,
+__global__ void embed_scaled_kernel(float* __restrict__ out, const int* tok, const W* __restrict__ table,
                                     int d, float scale) {
   pdl_trigger();
   pdl_wait();

@@ -21,8 +21,8 @@ __device__ __forceinline__ float softplusf(float z) { return z > 20.f ? z : log1
 // conversion of the rows.
 template <typename O>
 __global__ void __launch_bounds__(256)
-token_shift_kernel(O* __restrict__ out, const float* __restrict__ x, const float* __restrict__ mu,
-                   float* __restrict__ state, const int* __restrict__ row_req, const int* __restrict__ req_q_start,
+token_shift_kernel(O* __restrict__ out, const float* x, const float* __restrict__ mu,
+                   float* state, const int* __restrict__ row_req, const int* __restrict__ req_q_start,
                    const int* __restrict__ req_slot, int d) {
   pdl_trigger();
   const int t = blockIdx.x;
@@ -58,8 +58,8 @@ token_shift_kernel(O* __restrict__ out, const float* __restrict__ x, const float
 constexpr int MAX_TAPS = 16;
 
 __global__ void __launch_bounds__(256)
-causal_conv_kernel(float* __restrict__ out, const float* __restrict__ in, long long in_stride,
-                   const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ state,
+causal_conv_kernel(float* __restrict__ out, const float* in, long long in_stride,
+                   const float* __restrict__ w, const float* __restrict__ bias, const float* state,
                    long long slot_stride, const int* __restrict__ row_req, const int* __restrict__ req_q_start,
                    const int* __restrict__ req_slot, int C, int taps) {
   pdl_trigger();
@@ -84,7 +84,7 @@ causal_conv_kernel(float* __restrict__ out, const float* __restrict__ in, long l
 // channel of a request and moves forward through the slots, so an old value is read before
 // its place is written.
 __global__ void __launch_bounds__(256)
-conv_state_kernel(float* __restrict__ state, long long slot_stride, const float* __restrict__ in, long long in_stride,
+conv_state_kernel(float* state, long long slot_stride, const float* in, long long in_stride,
                   const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int C, int taps) {
   pdl_trigger();
   const int req = blockIdx.y;
@@ -185,7 +185,7 @@ constexpr int SEG = 8;
 
 template <typename O, typename Gate, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
-scan_kernel(O* __restrict__ out, float* __restrict__ state, long long slot_stride, Gate gate,
+scan_kernel(O* __restrict__ out, float* state, long long slot_stride, Gate gate,
             const int* __restrict__ req_q_start, const int* __restrict__ req_slot, int W) {
   __shared__ float fold_a[WARPS][32], fold_b[WARPS][32];
   pdl_trigger();
@@ -253,7 +253,7 @@ int launch_scan(void* out, float* state, long long slot_stride, const Gate& gate
 }
 
 // x *= factor
-__global__ void scale_kernel(float* __restrict__ x, long long n, float factor) {
+__global__ void scale_kernel(float* x, long long n, float factor) {
   pdl_trigger();
   pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)

@@ -16,9 +16,9 @@ namespace {
 // values and the other layer's values start are multiples of 4, all tensors 16-byte aligned.
 template <typename C, int VEC, bool NEIGHBOURS>
 __global__ void __launch_bounds__(256)
-rotary_prepare_kernel(C* __restrict__ qout, C* __restrict__ kpages, C* __restrict__ vpages, const float* __restrict__ proj,
+rotary_prepare_kernel(C* __restrict__ qout, C* __restrict__ kpages, C* __restrict__ vpages, const float* proj,
                       long long stride, const float* __restrict__ qw, const float* __restrict__ kw, float eps,
-                      const float* __restrict__ freq, float gain, int rot, const float* __restrict__ first,
+                      const float* __restrict__ freq, float gain, int rot, const float* first,
                       long long first_stride, float keep, float mix, const int* __restrict__ row_req,
                       const int* __restrict__ positions, const int* __restrict__ table, int table_stride, int page_size,
                       int H, int G, int D, int v_width, int writes) {

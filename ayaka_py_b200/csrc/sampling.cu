@@ -180,10 +180,10 @@ __device__ uint32_t select_nucleus(const float* row, int V, float inv_t, float z
 }
 
 __global__ void __launch_bounds__(THREADS)
-sample_kernel(int* __restrict__ out, const float* __restrict__ logits, int V,
-              const float* __restrict__ temperature, const long long* __restrict__ seed,
-              const long long* __restrict__ offset, const long long* __restrict__ top_k,
-              const float* __restrict__ top_p, const float* __restrict__ min_p) {
+sample_kernel(int* __restrict__ out, const float* logits, int V,
+              const float* temperature, const long long* seed,
+              const long long* offset, const long long* top_k,
+              const float* top_p, const float* min_p) {
   __shared__ MaxIdx red[THREADS / 32];
   __shared__ double partial[THREADS];
   __shared__ int chosen_thread;

@@ -250,8 +250,8 @@ stream_update_kernel(StreamArgs a) {
 // out[t, j] = gelu_tanh(sum_c w[j, c] x[t, c]) * table[tok[t], col0 + j]: a warp per (row, j), for a handful of rows.
 template <typename W>
 __global__ void __launch_bounds__(256)
-token_gate_kernel(W* __restrict__ out, const float* __restrict__ x, const W* __restrict__ w, const W* __restrict__ table,
-                  long long table_stride, int col0, const int* __restrict__ tok, int d, int n, int vec) {
+token_gate_kernel(W* __restrict__ out, const float* x, const W* __restrict__ w, const W* __restrict__ table,
+                  long long table_stride, int col0, const int* tok, int d, int n, int vec) {
   pdl_trigger();
   const int t = blockIdx.x, lane = threadIdx.x & 31, j = blockIdx.y * 8 + (threadIdx.x >> 5);
   pdl_wait();
@@ -284,8 +284,8 @@ token_gate_kernel(W* __restrict__ out, const float* __restrict__ x, const W* __r
 // The same from a product already made: out[t, j] = gelu_tanh(z[t, j]) * table[tok[t], col0 + j].
 template <typename W>
 __global__ void __launch_bounds__(256)
-token_gate_mul_kernel(W* __restrict__ out, const float* __restrict__ z, const W* __restrict__ table, long long table_stride, int col0,
-                      const int* __restrict__ tok, int n, long long total) {
+token_gate_mul_kernel(W* __restrict__ out, const float* z, const W* __restrict__ table, long long table_stride, int col0,
+                      const int* tok, int n, long long total) {
   pdl_trigger();
   pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -294,14 +294,14 @@ token_gate_mul_kernel(W* __restrict__ out, const float* __restrict__ z, const W*
   }
 }
 
-__global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ x, long long n, float cap) {
+__global__ void __launch_bounds__(256) softcap_kernel(float* x, long long n, float cap) {
   pdl_trigger();
   pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     x[i] = cap * tanhf(x[i] / cap);
 }
 
-__global__ void __launch_bounds__(256) softcap_vec_kernel(float4* __restrict__ x, long long n4, float cap) {
+__global__ void __launch_bounds__(256) softcap_vec_kernel(float4* x, long long n4, float cap) {
   pdl_trigger();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
