@@ -51,6 +51,7 @@ struct LatentArgs {
   const int* req_pos0;
   int* error;
   int table_stride, num_req, H, HG, BR, rank, rot, page_shift, window, own;      // own: chunks whose columns a CTA sums
+  int rows_end;                       // rows of the pages: a copy from there on brings zeros
   float scale_log2;
 };
 
@@ -194,7 +195,9 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
       const int kp = k_begin + t * NK + mine * box;
       const int logical = kp >> args.page_shift;
       const int page = (kp <= last_pos && logical < args.table_stride) ? my_table[logical] : 0;
-      return (page << args.page_shift) + (kp & ((1 << args.page_shift) - 1) & (page > 0 ? ~0 : 0));
+      // a position on no page (one that a window has passed) has weight 0, but what is copied for it enters P C all the
+      // same and has to be finite: zeros from behind the pages' end, not the padding page's contents
+      return page > 0 ? (page << args.page_shift) + (kp & ((1 << args.page_shift) - 1)) : args.rows_end;
     };
     auto bring = [&](int t, int row, bool owned) -> bool {
       const int b = t & 1;
@@ -527,7 +530,7 @@ AYK_EXPORT int ayk_latent_attention_tc(float* out, const float* query, const voi
   dim3 grid(halves, total_rows / BR + num_req, (H + HG - 1) / HG);      // the halves of a tile side by side: they read the same keys
   AYK_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "ayk_latent_attention_tc: %d rows, %d requests, %d heads", total_rows, num_req, H);
   LatentArgs args{out, query, table, req_q_start, req_pos0, g_error_dev, table_stride, num_req, H, HG, BR, rank, rot, shift, window,
-                  rank / 64 / halves, scale * 1.4426950408889634f};
+                  rank / 64 / halves, pages * page_size, scale * 1.4426950408889634f};
   const size_t smem = smem_bytes((rank + rot) / 64);
   if (rank == 512 && rot == 64) ayk_launch(latent_tc_kernel<5, 4>, grid, dim3(THREADS), smem, stream, ml, mr, args);
   else if (rank == 512 && rot == 0) ayk_launch(latent_tc_kernel<4, 4>, grid, dim3(THREADS), smem, stream, ml, mr, args);

@@ -487,6 +487,34 @@ def test_latent_attention_on_tcgen05_tile_edges(H, rank, rot, P, window):
         cache.commit(res)
 
 
+def test_latent_attention_on_tcgen05_beside_released_pages():
+    """Keys that a window has passed lie on pages that were given back (table entry 0); the first tile of a portion begins
+    among them.  Whatever the padding page holds, numbers or not, has no part in the sums."""
+    from ayaka_py_b200 import ops
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts import KVNeed
+    H, rank, rot, P, window = 8, 128, 64, 8, 40
+    cache, runner = context_for([CacheGroupSpec("g", KVNeed(1, rot, window, 1, rank), 1)], "bfloat16", max_requests=4, page_size=P,
+                                pages=256, positions=1024)
+    rope, lat = (t[:, :, 0] for t in cache.kv_layer(0, 0))
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    lat.copy_(torch.randn(lat.shape, generator=gen, device="cuda"))
+    rope.copy_(torch.randn(rope.shape, generator=gen, device="cuda"))
+    lat[0] = float("nan")
+    rope[0] = float("nan")
+    for plan in ({0: 100, 1: 203, 2: 64}, {0: 5, 1: 33, 2: 2}, {0: 64, 1: 1, 2: 31}):
+        ctx, res = step_of(cache, runner, plan)
+        first = [max(0, int(a) - window + 1) // 32 * 32 for a in ctx.host["pos0"]]
+        released = [int(row[a // P]) == 0 for row, a in zip(ctx.tables[0].cpu(), first)]
+        assert any(released) or not ctx.host["pos0"].any()
+        q = torch.randn(ctx.num_rows, H, rank + rot, generator=gen, device="cuda") * 0.5
+        a = ops.latent_attention(q, lat, rope, ctx.tables[0], ctx, 0.2, tensor_cores=False, window=window)
+        b = ops.latent_attention(q, lat, rope, ctx.tables[0], ctx, 0.2, tensor_cores=True, window=window)
+        assert torch.isfinite(b).all()
+        assert float((a - b).abs().max()) < 0.01 * float(a.abs().max()) + 1e-3, plan
+        cache.commit(res)
+
+
 @pytest.mark.parametrize("T,H,N,K,wide_gate", [(64, 2, 128, 64, None), (127, 3, 129, 72, True), (129, 1, 512, 128, False), (300, 2, 8, 520, True),
                                                (128, 5, 136, 512, None)])
 def test_per_head_products_on_tcgen05(T, H, N, K, wide_gate):
