@@ -52,6 +52,7 @@ struct LatentArgs {
   int* error;
   int table_stride, num_req, H, HG, BR, rank, rot, page_shift, window, own;      // own: chunks whose columns a CTA sums
   int rows_end;                       // rows of the pages: a copy from there on brings zeros
+  int two_halves;                     // 1: a CTA sums one half of the latent's columns; blocks 2 i and 2 i + 1 are tile i's
   float scale_log2;
 };
 
@@ -88,7 +89,7 @@ template <int FOREIGN, int OWN>
 __global__ void __launch_bounds__(THREADS, 1)
 latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_constant__ CUtensorMap map_rope, const LatentArgs args) {
   // Tiles of the requests' last rows see the most keys: they start first (blocks are handed out in order).
-  int tile = gridDim.y - 1 - blockIdx.y, req = -1, q0 = 0, q_len = 0;
+  int tile = (int)(gridDim.x >> args.two_halves) - 1 - (int)(blockIdx.x >> args.two_halves), req = -1, q0 = 0, q_len = 0;
   for (int r = 0; r < args.num_req; ++r) {
     const int len = args.req_q_start[r + 1] - args.req_q_start[r];
     const int n = (len + args.BR - 1) / args.BR;
@@ -97,7 +98,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
   }
   if (req < 0) return;
   const int H = args.H, HG = args.HG, rank = args.rank, rot = args.rot, Dk = rank + rot;
-  const int half = blockIdx.x, h0 = blockIdx.z * HG;
+  const int half = args.two_halves ? (int)(blockIdx.x & 1) : 0, h0 = blockIdx.y * HG;
   const int heads = min(HG, H - h0);
   const int rows = min(args.BR, q_len - q0);
   const int row0 = args.req_q_start[req] + q0;
@@ -500,9 +501,9 @@ AYK_EXPORT int ayk_latent_tc_error() { return g_error_host ? *g_error_host : 0; 
 
 // Whether the tcgen05 kernel takes this geometry: keys in whole chunks of 64 numbers, at most nine; latents beyond 256 in two
 // equal halves of whole chunks; pages of at least the swizzle's 8 rows.
-AYK_EXPORT int ayk_latent_attention_tc_takes(int rank, int rot, int page_size, const void* query, const void* latent_pages, const void* rope_pages) {
+AYK_EXPORT int ayk_latent_attention_tc_takes(int rank, int rot, int pages, int page_size, const void* query, const void* latent_pages, const void* rope_pages) {
   if (rank < 64 || rank % 64 != 0 || rank > 512 || (rank > 256 && rank % 128 != 0) || rot < 0 || rot % 64 != 0 || rank + rot > 64 * MAX_CHUNKS) return 0;
-  if (page_size < 8 || (page_size & (page_size - 1)) != 0) return 0;
+  if (page_size < 8 || (page_size & (page_size - 1)) != 0 || (long long)pages * page_size >= (1ll << 31)) return 0;
   return (uintptr_t)query % 16 == 0 && (uintptr_t)latent_pages % 16 == 0 && (uintptr_t)rope_pages % 16 == 0;
 }
 
@@ -512,9 +513,9 @@ AYK_EXPORT int ayk_latent_attention_tc(float* out, const float* query, const voi
                                        int total_rows, int H, int rank, int rot, int page_size, float scale, int window,
                                        cudaStream_t stream) {
   if (num_req == 0 || total_rows == 0) return 0;
-  AYK_REQUIRE(ayk_latent_attention_tc_takes(rank, rot, page_size, query, latent_pages, rope_pages) && (uintptr_t)out % 16 == 0,
+  AYK_REQUIRE(ayk_latent_attention_tc_takes(rank, rot, pages, page_size, query, latent_pages, rope_pages) && (uintptr_t)out % 16 == 0,
               "ayk_latent_attention_tc: latent %d + %d, pages of %d, or the operands' alignment, are not taken", rank, rot, page_size);
-  AYK_REQUIRE((long long)pages * page_size < (1ll << 31) && H >= 1, "ayk_latent_attention_tc: %d pages of %d, %d heads", pages, page_size, H);
+  AYK_REQUIRE(H >= 1, "ayk_latent_attention_tc: %d heads", H);
   {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (setup() != 0) return -1;
@@ -527,10 +528,11 @@ AYK_EXPORT int ayk_latent_attention_tc(float* out, const float* query, const voi
   if (rot > 0) { if (encode(&mr, rope_pages, (long long)pages * page_size, rot, box) != 0) return -1; }
   else mr = ml;
   const int HG = H < AQ ? H : AQ, BR = AQ / HG, halves = rank > 256 ? 2 : 1;
-  dim3 grid(halves, total_rows / BR + num_req, (H + HG - 1) / HG);      // the halves of a tile side by side: they read the same keys
-  AYK_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "ayk_latent_attention_tc: %d rows, %d requests, %d heads", total_rows, num_req, H);
+  // the halves of a tile side by side (they read the same keys); tiles along x, where a grid has room for any step's rows
+  dim3 grid((unsigned)halves * (unsigned)(total_rows / BR + num_req), (H + HG - 1) / HG);
+  AYK_REQUIRE(grid.y <= 65535, "ayk_latent_attention_tc: %d heads", H);
   LatentArgs args{out, query, table, req_q_start, req_pos0, g_error_dev, table_stride, num_req, H, HG, BR, rank, rot, shift, window,
-                  rank / 64 / halves, pages * page_size, scale * 1.4426950408889634f};
+                  rank / 64 / halves, pages * page_size, halves - 1, scale * 1.4426950408889634f};
   const size_t smem = smem_bytes((rank + rot) / 64);
   if (rank == 512 && rot == 64) ayk_launch(latent_tc_kernel<5, 4>, grid, dim3(THREADS), smem, stream, ml, mr, args);
   else if (rank == 512 && rot == 0) ayk_launch(latent_tc_kernel<4, 4>, grid, dim3(THREADS), smem, stream, ml, mr, args);

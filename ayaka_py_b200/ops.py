@@ -539,7 +539,8 @@ def latent_attention(query: torch.Tensor, latent_pages: torch.Tensor, rope_pages
     elif tensor_cores and not takes:
         raise KernelError(f"latent_attention: the tensor-core kernel does not take {latent_pages.dtype} pages of {rank} + {rot}")
     if tensor_cores and ctx.max_q_len > 1 and lib.ayk_latent_attention_tc_takes(
-            ctypes.c_int(rank), ctypes.c_int(rot), ctypes.c_int(latent_pages.shape[1]), _ptr(query), _ptr(latent_pages), _ptr(rope_pages)):
+            ctypes.c_int(rank), ctypes.c_int(rot), ctypes.c_int(latent_pages.shape[0]), ctypes.c_int(latent_pages.shape[1]), _ptr(query),
+            _ptr(latent_pages), _ptr(rope_pages)):
         _launch(lib.ayk_latent_attention_tc(_ptr(out), _ptr(query), _ptr(latent_pages), _ptr(rope_pages), ctypes.c_int(latent_pages.shape[0]),
                                             _ptr(_i32(table, "table")), ctypes.c_int(table.stride(0)), _ptr(ctx.req_q_start),
                                             _ptr(ctx.req_pos0), ctypes.c_int(ctx.num_requests), ctypes.c_int(T), ctypes.c_int(H),

@@ -515,6 +515,24 @@ def test_latent_attention_on_tcgen05_beside_released_pages():
         cache.commit(res)
 
 
+def test_latent_attention_on_tcgen05_of_more_rows_than_a_grid_has_room_for_along_y():
+    """More than 64 heads take one row per tile: a step of more than 65,535 rows is as many tiles."""
+    from ayaka_py_b200 import ops
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts import KVNeed
+    H, rank, P, window, rows = 65, 64, 64, 8, 65600
+    cache, runner = context_for([CacheGroupSpec("g", KVNeed(1, 0, window, 1, rank), 1)], "bfloat16", max_requests=2, page_size=P,
+                                pages=rows // P + 4, positions=rows)
+    rope, lat = (t[:, :, 0] for t in cache.kv_layer(0, 0))
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    lat.copy_(torch.randn(lat.shape, generator=gen, device="cuda"))
+    ctx, res = step_of(cache, runner, {0: rows})
+    q = torch.randn(rows, H, rank, generator=gen, device="cuda") * 0.5
+    b = ops.latent_attention(q, lat, rope, ctx.tables[0], ctx, 0.2, tensor_cores=True, window=window)
+    a = ops.latent_attention(q, lat, rope, ctx.tables[0], ctx, 0.2, tensor_cores=False, window=window)
+    assert float((a - b).abs().max()) < 0.01 * float(a.abs().max()) + 1e-3
+
+
 @pytest.mark.parametrize("T,H,N,K,wide_gate", [(64, 2, 128, 64, None), (127, 3, 129, 72, True), (129, 1, 512, 128, False), (300, 2, 8, 520, True),
                                                (128, 5, 136, 512, None)])
 def test_per_head_products_on_tcgen05(T, H, N, K, wide_gate):
