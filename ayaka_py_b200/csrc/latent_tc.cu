@@ -40,8 +40,8 @@ constexpr int NK = 32;                // keys per tile
 constexpr int MAX_CHUNKS = 9;         // runs of 64 numbers of a key: 512 + 64
 constexpr int Q_CHUNK = AQ * 128, K_CHUNK = NK * 128, P_BYTES = AQ * NK * 2;
 constexpr int THREADS = 192;
-constexpr int TMEM_COLS = 512;        // O: columns 0..255; S: two buffers of 32 from column 256 on
-constexpr uint32_t S_COL = 256;
+// Tensor memory: O in columns 0 .. 64 own - 1, two buffers of 32 for S behind it; the next power of two is asked for.
+__host__ __device__ constexpr uint32_t tmem_columns(int own) { return own <= 1 ? 128u : (own <= 3 ? 256u : 512u); }
 
 struct LatentArgs {
   float* out;                         // [T, H, rank]
@@ -110,6 +110,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
   const int* my_table = args.table + (size_t)req * args.table_stride;
   const int own = OWN ? OWN : args.own, chunks = OWN ? OWN + FOREIGN : Dk / 64, foreign = chunks - own, lat_chunks = rank / 64;
   const int own_first = half * own;                    // chunk numbers: latent first, then the rotated part
+  const uint32_t s_col = 64u * (uint32_t)own;
   // the i-th foreign chunk's number
   auto foreign_chunk = [&](int i) { return i < own_first ? i : i + own; };
 
@@ -140,7 +141,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 5) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(tmem_columns(own)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();
@@ -275,7 +276,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
           const uint64_t da = make_desc(q_tile + (uint32_t)number * Q_CHUNK), db = make_desc(from + (uint32_t)c * K_CHUNK);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma(tmem + S_COL + 32u * b, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), IDESC_S, (opens && c == 0 && k == 0) ? 0u : 1u);
+            umma(tmem + s_col + 32u * b, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), IDESC_S, (opens && c == 0 && k == 0) ? 0u : 1u);
         }
         if (!owned) umma_commit(foreign_empty + 8 * b);
         else umma_commit(s_full + 8 * b);
@@ -336,7 +337,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
       if (!ok) break;
       tc_fence_after();
       uint32_t s[32];
-      tmem_ld32(tmem + S_COL + 32u * b + lane_addr, s);
+      tmem_ld32(tmem + s_col + 32u * b + lane_addr, s);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
@@ -439,7 +440,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap map_latent, const __grid_co
   tc_fence_before();
   __syncthreads();
   if (warp == 5) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_columns(own)) : "memory");
   }
 }
 
@@ -454,7 +455,13 @@ int* g_error_dev = nullptr;
 std::mutex g_mutex;
 AykPerDevice g_configured;
 
-constexpr size_t smem_bytes(int chunks) { return (size_t)chunks * (Q_CHUNK + 2 * K_CHUNK) + P_BYTES + 128; }
+// No more CTAs may share a multiprocessor than its 512 tensor-memory columns serve: one more would wait for them until
+// another is through, while a multiprocessor beside it has none (measured, latent 256 without a rotated part: 101 requests'
+// tiles over 500 keys 125 us, two to a multiprocessor where 62 were to be had).  Shared memory holds them off.
+constexpr size_t smem_bytes(int chunks, int own) {
+  const size_t used = (size_t)chunks * (Q_CHUNK + 2 * K_CHUNK) + P_BYTES + 128, apart = (228 * 1024) / (512 / tmem_columns(own) + 1) + 128;
+  return used > apart ? used : apart;
+}
 
 int setup() {
   if (!g_encode) {
@@ -473,10 +480,10 @@ int setup() {
     if (err != cudaSuccess) return ayk_fail("ayk_latent_attention_tc: cudaHostGetDevicePointer: %s", cudaGetErrorString(err));
   }
   if (!g_configured.here()) {
-    cudaError_t err = cudaFuncSetAttribute(latent_tc_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(MAX_CHUNKS));
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(latent_tc_kernel<5, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(9));
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(latent_tc_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(8));
-    if (err != cudaSuccess) return ayk_fail("ayk_latent_attention_tc: shared memory %zu: %s", smem_bytes(MAX_CHUNKS), cudaGetErrorString(err));
+    cudaError_t err = cudaFuncSetAttribute(latent_tc_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(MAX_CHUNKS, 4));
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(latent_tc_kernel<5, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(9, 4));
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(latent_tc_kernel<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(8, 4));
+    if (err != cudaSuccess) return ayk_fail("ayk_latent_attention_tc: shared memory %zu: %s", smem_bytes(MAX_CHUNKS, 4), cudaGetErrorString(err));
     g_configured.here() = true;
   }
   return 0;
@@ -533,7 +540,7 @@ AYK_EXPORT int ayk_latent_attention_tc(float* out, const float* query, const voi
   AYK_REQUIRE(grid.y <= 65535, "ayk_latent_attention_tc: %d heads", H);
   LatentArgs args{out, query, table, req_q_start, req_pos0, g_error_dev, table_stride, num_req, H, HG, BR, rank, rot, shift, window,
                   rank / 64 / halves, pages * page_size, halves - 1, scale * 1.4426950408889634f};
-  const size_t smem = smem_bytes((rank + rot) / 64);
+  const size_t smem = smem_bytes((rank + rot) / 64, rank / 64 / halves);
   if (rank == 512 && rot == 64) ayk_launch(latent_tc_kernel<5, 4>, grid, dim3(THREADS), smem, stream, ml, mr, args);
   else if (rank == 512 && rot == 0) ayk_launch(latent_tc_kernel<4, 4>, grid, dim3(THREADS), smem, stream, ml, mr, args);
   else ayk_launch(latent_tc_kernel<0, 0>, grid, dim3(THREADS), smem, stream, ml, mr, args);
