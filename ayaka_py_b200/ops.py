@@ -9,9 +9,11 @@ raises.  Every function launches on torch's current stream.
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 import threading
 
+import numpy as np
 import torch
 
 from .csrc import build as _build
@@ -519,14 +521,59 @@ LATENT_WINDOW_WHOLE = 32  # a window of up to this many keys is one partition
 LATENT_PARTS = 64        # at most this many partitions of the context when every request brings one row
 
 
+def _latent_tiles(ctx, rows: int, window: int | None) -> tuple[int, float, float]:
+    """A step's tiles of ``rows`` rows of one request, the 32-key tiles that they read together, and those of the longest;
+    worked out once per step."""
+    key = ("latent_tiles", rows, window)
+    if key not in ctx.host:
+        counts, pos0 = ctx.host["counts"], ctx.host["pos0"]
+        most = math.inf if window is None else (window + rows) / 32 + 1
+        tiles = -(-counts // rows)
+        keys = np.minimum((2 * pos0 + counts) / 64 + 0.5, most)
+        ctx.host[key] = int(tiles.sum()), float((tiles * keys).sum()), min(ctx.max_kv_len / 32 + 0.5, most)
+    return ctx.host[key]
+
+
+def _latent_tc_pays(ctx, heads: int, rank: int, rot: int, window: int | None, sms: int) -> bool:
+    """Whether the tcgen05 form of the latent attention is the faster one for a step that brings more than one row of some
+    request.  It takes 128 pairs to a tile (and with a latent beyond 256 two blocks to each) where the mma.sync form takes
+    64, starts later and has fewer blocks to a multiprocessor, but passes a tile of keys in half the time.  The estimates
+    (us: a block's start, its time per 32 keys, blocks that a multiprocessor works off side by side, what the last ones add)
+    are fitted to 27 steps x 26 shapes (64 to 512 + 0 or 64, 2 to 200 heads; contexts of 64 to 2,048; short portions, many
+    single rows beside one).  Of the 702 the choice is more than 3 % slower than mma.sync in 3, by 11 % at most (128 heads,
+    latent 64), and on average 0.6 % behind the better of the two.  Measured, mma.sync and tcgen05, 16 heads, 512 + 64: one
+    prompt of 32 rows 13.6, 18.9; of 128 27.6, 25.9; 2 x 1,024 rows 316, 205; 100 single rows of 100 keys beside 64 rows 36, 58."""
+    def time(base, start, step, at_once, tail, tiles, keys, longest):
+        one = start + step * longest
+        return base + max(one, (start * tiles + step * keys) / (sms * at_once) + (tail * one if tiles > sms * at_once else 0.0))
+
+    def work(pairs, halves):
+        group = min(heads, pairs)
+        tiles, keys, longest = _latent_tiles(ctx, pairs // group, window)
+        blocks = -(-heads // group) * halves
+        return tiles * blocks, keys * blocks, longest
+
+    if "counts" not in ctx.host:
+        return True
+    if rank > 256:
+        return time(0.0, 14.8, 2.4, 0.87, 0.46, *work(128, 2)) < 0.97 * time(0.0, 2.8, 5.7, 0.9, 0.29, *work(64, 1))
+    step = 2.3 + 0.22 * (rank // 64) if rot == 0 else 1.7 + 0.3 * (rank // 64)
+    ours = time(2.8, 8.9, step, 1.1, 0.5, *work(128, 1))
+    theirs = time(1.5, 2.7, 1.5 + 0.73 * ((rank + rot) // 64), 1.7, 0.5, *work(64, 1))
+    if rank <= 128:                    # as fast per tile without a rotated part, hardly faster with one
+        return rot > 0 and ctx.max_kv_len > 128 and ours < 0.9 * theirs
+    return ours < 0.97 * theirs
+
+
 def latent_attention(query: torch.Tensor, latent_pages: torch.Tensor, rope_pages: torch.Tensor, table: torch.Tensor,
                      ctx, scale: float, tensor_cores: bool | None = None, window: int | None = None) -> torch.Tensor:
     """Causal attention of the step's rows over cached (latent, rotated key part) pairs shared by
     all heads: query [T, H, rank + rot] float32; returns sum_j p_j latent_j as float32 [T, H, rank].  ``window``: a
     row sees its own position and the window - 1 before it.
-    bfloat16 pages whose rows are whole 16-byte pieces go through the tensor-core kernels (tcgen05 for prompt portions
-    whose latent and rotated part are whole runs of 64 numbers; else mma.sync, a decode step's context cut into
-    partitions and merged); 32-bit pages and other sizes through the kernel on the FP32 pipes."""
+    bfloat16 pages whose rows are whole 16-byte pieces go through the tensor-core kernels (tcgen05 for steps with portions
+    of more than one row whose latent and rotated part are whole runs of 64 numbers, where it is the faster one, and with
+    ``tensor_cores`` True wherever it can; else mma.sync, a decode step's context cut into partitions and merged); 32-bit
+    pages and other sizes through the kernel on the FP32 pipes."""
     lib = _ready()
     T, H, Dk = query.shape
     rank, rot = latent_pages.shape[-1], rope_pages.shape[-1]
@@ -534,13 +581,14 @@ def latent_attention(query: torch.Tensor, latent_pages: torch.Tensor, rope_pages
         raise KernelError("latent_attention: query must be contiguous float32 [T, H, rank + rot]")
     out = torch.empty((T, H, rank), dtype=torch.float32, device=query.device)
     takes = latent_pages.dtype == torch.bfloat16 and bool(lib.ayk_latent_attention_mma_takes(ctypes.c_int(rank), ctypes.c_int(rot)))
-    if tensor_cores is None:
+    by_time = tensor_cores is None
+    if by_time:
         tensor_cores = takes
     elif tensor_cores and not takes:
         raise KernelError(f"latent_attention: the tensor-core kernel does not take {latent_pages.dtype} pages of {rank} + {rot}")
     if tensor_cores and ctx.max_q_len > 1 and lib.ayk_latent_attention_tc_takes(
             ctypes.c_int(rank), ctypes.c_int(rot), ctypes.c_int(latent_pages.shape[0]), ctypes.c_int(latent_pages.shape[1]), _ptr(query),
-            _ptr(latent_pages), _ptr(rope_pages)):
+            _ptr(latent_pages), _ptr(rope_pages)) and (not by_time or _latent_tc_pays(ctx, H, rank, rot, window, sm_count())):
         _launch(lib.ayk_latent_attention_tc(_ptr(out), _ptr(query), _ptr(latent_pages), _ptr(rope_pages), ctypes.c_int(latent_pages.shape[0]),
                                             _ptr(_i32(table, "table")), ctypes.c_int(table.stride(0)), _ptr(ctx.req_q_start),
                                             _ptr(ctx.req_pos0), ctypes.c_int(ctx.num_requests), ctypes.c_int(T), ctypes.c_int(H),

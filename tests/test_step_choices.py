@@ -1,0 +1,38 @@
+"""Which kernel a step takes where more than one can: the rules that look at a step's rows and contexts, at points where both
+sides were measured.  Nothing is launched."""
+
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+
+from ayaka_py_b200 import ops
+
+SMS = 148
+
+
+def step(plan):
+    """A step's context for [(cached tokens, rows brought)], single rows first."""
+    pos0, counts = (np.array(x, dtype=np.int64) for x in zip(*sorted(plan, key=lambda e: e[1] != 1)))
+    return SimpleNamespace(host={"pos0": pos0, "counts": counts}, num_requests=len(plan), num_rows=int(counts.sum()),
+                           num_single=int((counts == 1).sum()), max_q_len=int(counts.max()), max_kv_len=int((pos0 + counts).max()))
+
+
+@pytest.mark.parametrize("heads,rank,rot,plan,tcgen05", [
+    (16, 512, 64, [(0, 1024), (0, 777)], True), (16, 512, 64, [(512, 512)], True), (16, 512, 64, [(500, 2)], True),
+    (16, 512, 64, [(0, 32)], False), (16, 512, 64, [(0, 64)], False), (16, 512, 64, [(20, 3)] * 200, False),
+    (16, 512, 64, [(100, 1)] * 100 + [(0, 64)], False), (16, 512, 64, [(250, 3)] * 100, False),
+    (16, 512, 64, [(500, 1)] * 64 + [(0, 512)], True), (8, 512, 64, [(500, 1)] * 200 + [(0, 512)], False),
+    (128, 512, 64, [(0, 128)], False), (128, 512, 64, [(0, 384)], True), (130, 512, 64, [(0, 256)], False),
+    (16, 256, 64, [(0, 1024)] * 2, True), (16, 256, 64, [(400, 2)] * 200, False), (40, 192, 0, [(0, 1024)] * 2, True),
+    (16, 128, 64, [(0, 1024)] * 2, True), (16, 128, 64, [(0, 128)], False), (16, 64, 64, [(900, 4)] * 32, True),
+    (16, 64, 0, [(0, 1024)] * 2, False)])
+def test_latent_attention_takes_the_faster_of_its_tensor_core_forms(heads, rank, rot, plan, tcgen05):
+    assert ops._latent_tc_pays(step(plan), heads, rank, rot, None, SMS) is tcgen05
+
+
+def test_a_window_bounds_the_keys_that_a_tile_is_thought_to_read():
+    ctx = step([(900, 4)] * 32)
+    assert ops._latent_tc_pays(ctx, 16, 512, 64, None, SMS)
+    assert not ops._latent_tc_pays(ctx, 16, 512, 64, 16, SMS)
+    assert ops._latent_tiles(ctx, 8, None)[1] > ops._latent_tiles(ctx, 8, 16)[1]
