@@ -19,6 +19,7 @@ import time
 
 import torch
 
+from .. import ops
 from ..cache.manager import CacheManager, pages_for_budget
 from ..config.engine import EngineConfig
 from ..sampling.sampler import Sampler
@@ -154,6 +155,9 @@ class Engine:
             t0 = time.perf_counter()
             torch.cuda.synchronize()
             self._waited = getattr(self, "_waited", 0.0) + time.perf_counter() - t0
+        code = ops.tc_error()
+        if code:
+            raise ops.KernelError(f"a wait inside a tensor-core kernel ran out (code {code}): the step's results cannot be trusted")
         done = self.scheduler.resolve(launched.plan, sampled)
         results = [self.scheduler.result_of(s) for s in done]
         for r in results:

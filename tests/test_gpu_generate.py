@@ -229,6 +229,23 @@ def test_lookahead_gives_the_same_tokens(model_folders, graph):
     assert want["r0"][1] == "stop" and len(want["r0"][0]) <= 14
 
 
+def test_a_wait_that_ran_out_ends_the_step_with_an_error(model_folders, monkeypatch):
+    """A kernel whose bounded wait runs out leaves a code; the engine must not hand out tokens of that step."""
+    import torch
+    from ayaka_py_b200 import EngineConfig, Request, SamplingParams, StopCriteria, ops
+    from ayaka_py_b200.engine.engine import Engine
+    from ayaka_py_b200.engine.loading import load_model
+    folder, cfg, weights = model_folders["B"]
+    _, model = load_model(folder, "bfloat16", "cuda")
+    engine = Engine(model, EngineConfig(dtype="bfloat16", page_size=8, kv_pages=64, batch_tokens=64, prefill_chunk=32), eos_token_id=None)
+    engine.submit(Request("r", tiny_models.prompts(cfg, [9], seed=31)[0], SamplingParams(temperature=0.0), StopCriteria(max_tokens=5, ignore_eos=True)))
+    engine.step()
+    monkeypatch.setattr(ops, "tc_error", lambda: 53)
+    with pytest.raises(ops.KernelError, match="53"):
+        engine.step()
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_lookahead_past_prompt_portions_and_page_pressure(model_folders, dtype):
     """Steps planned ahead that hold prompt portions and newly admitted requests beside the decoding ones,
