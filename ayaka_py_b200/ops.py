@@ -657,7 +657,44 @@ def mlstm_head_floats(dim: int, vdim: int) -> int:
     return dim * vdim + dim + 4
 
 
-MLSTM_LONG = 64          # rows of one request from which on its chunks go side by side
+MLSTM_LONG = 64          # rows of one request from which on its chunks may go side by side
+MLSTM_SINGLES = 128      # (single row, head) pairs of a step from which on they are a launch of their own beside long portions
+
+
+def _mlstm_singles(ctx, heads: int) -> int:
+    """The leading single-row requests that the token-by-token kernel takes in a step whose portions have their chunks side
+    by side.  As chunks of one row they move their memory four times, through a scratch with a whole memory for each; the
+    launch costs 7 us.  Measured, 16 heads of 128 x 128 beside 512 rows, in one and apart: 8 single rows 70, 51 us; 64 275,
+    111; 250 1,414, 309; 4 heads beside 128 rows: 8 43, 49; 32 54, 49."""
+    singles = getattr(ctx, "num_single", 0)
+    return singles if singles * heads >= MLSTM_SINGLES else 0
+
+
+def _mlstm_long_pays(ctx, heads: int, dim: int, vdim: int) -> bool:
+    """Whether chunks side by side are faster than the walk over 16-token chunks for a step with a portion of MLSTM_LONG
+    rows or more.  The walk's time is its longest portion's chain, and a memory's way in and out for every other request, or,
+    when that fills the chip, all its chunks over the blocks that run at once; three kernels side by side take about 40 us
+    however few the chunks, and their grid grows with the requests.  The estimates (us) are fitted to steps of one to 250
+    requests of 1 to 1,024 rows, heads of 32 x 32 to 128 x 128, 4 to 16 of them.  Measured, walk and side by side, 16 heads of
+    128 x 128: one portion of 64 rows 25, 42; of 100 38, 43; of 128 43, 41; of 1,024 309, 63; 8 of 64 78, 68; 64 of 64 546, 375;
+    100 of 3 beside 64 280, 420; 250 single rows beside 64 618, 306; 16 heads of 32 x 32, 64 of 64 rows 134, 202."""
+    if "counts" not in ctx.host:
+        return True
+    key = ("mlstm_long", heads, dim, vdim)
+    if key not in ctx.host:
+        counts = ctx.host["counts"]
+        chunks = -(-counts // 16)
+        blocks, size = heads * -(-vdim // 32), dim * vdim
+        each = (0.0135 + 0.000163 * dim) * blocks
+        walk = 8.0 + max((2.6 + 0.0172 * dim) * int(chunks.max()) + each * (len(counts) - 1), each * int(chunks.sum()))
+        singles = _mlstm_singles(ctx, heads)
+        requests, rows = len(counts) - singles, int(counts.sum()) - singles
+        grid = (rows // 64 + requests) * heads
+        long = 27.0 + 0.115 * dim + max(0, grid - 148) * (0.1 + 6e-6 * size + 0.0002 * requests)
+        if singles:
+            long += 7.0 + (0.032 + 2.1e-6 * size) * heads * singles
+        ctx.host[key] = long < 0.92 * walk
+    return ctx.host[key]
 
 
 def mlstm(proj: torch.Tensor, state: torch.Tensor, norm_weight: torch.Tensor, ctx, heads: int, dim: int, vdim: int,
@@ -667,8 +704,8 @@ def mlstm(proj: torch.Tensor, state: torch.Tensor, norm_weight: torch.Tensor, ct
     rows [q | k | v | z_i (heads) | z_f (heads) | gate (heads * vdim)]; returns [T, heads * vdim] in
     ``out_dtype``.  ``chunked``: the kernel that takes 16 tokens at a time (default: whenever a request brings
     more than one row, or the values are wider than the token-by-token kernel's 256 numbers, and the head size
-    fits it; from ``MLSTM_LONG`` rows of one request on, heads of up to 128 x 128 have their chunks of 64 tokens side by
-    side); ``slice_cols``: value columns per block of that kernel, 16 or 32 (0: 32, or 16 where blocks of 32
+    fits it; with ``MLSTM_LONG`` rows or more of one request, heads of up to 128 x 128 have their chunks of 64 tokens side by
+    side where that is faster, and always with ``chunked`` True); ``slice_cols``: value columns per block of that kernel, 16 or 32 (0: 32, or 16 where blocks of 32
     would leave most SMs idle)."""
     lib = _ready()
     lib.ayk_mlstm_slice_cols(ctypes.c_int(slice_cols))
@@ -679,7 +716,8 @@ def mlstm(proj: torch.Tensor, state: torch.Tensor, norm_weight: torch.Tensor, ct
         raise KernelError("mlstm: projection rows, state or norm weight do not fit")
     out = torch.empty((T, heads * vdim), dtype=out_dtype, device=proj.device)
     takes = bool(lib.ayk_mlstm_chunk_takes(ctypes.c_int(dim)))
-    if chunked is None:
+    by_time = chunked is None
+    if by_time:
         chunked = (ctx.max_q_len > 1 or vdim > 256) and takes
     elif chunked and not takes:
         raise KernelError(f"mlstm: the chunked kernel does not take heads of {dim} numbers")
@@ -688,13 +726,20 @@ def mlstm(proj: torch.Tensor, state: torch.Tensor, norm_weight: torch.Tensor, ct
     global launches
     scratch = None
     if (chunked and slice_cols == 0 and ctx.max_q_len >= MLSTM_LONG and state.data_ptr() % 16 == 0 and
-            lib.ayk_mlstm_long_takes(ctypes.c_int(heads), ctypes.c_int(dim), ctypes.c_int(vdim), ctypes.c_longlong(proj.stride(0)), _ptr(proj))):
+            lib.ayk_mlstm_long_takes(ctypes.c_int(heads), ctypes.c_int(dim), ctypes.c_int(vdim), ctypes.c_longlong(proj.stride(0)), _ptr(proj)) and
+            (not by_time or _mlstm_long_pays(ctx, heads, dim, vdim))):
+        singles = _mlstm_singles(ctx, heads)
+        if singles:
+            _launch(lib.ayk_mlstm(_ptr(out), _ptr(state), _ptr(proj), ctypes.c_longlong(proj.stride(0)), _ptr(norm_weight),
+                                  _ptr(ctx.row_req), _ptr(ctx.req_q_start), _ptr(ctx.req_slot), ctypes.c_int(singles),
+                                  ctypes.c_int(singles), ctypes.c_int(heads), ctypes.c_int(dim), ctypes.c_int(vdim),
+                                  ctypes.c_float(cap), ctypes.c_float(eps), _ptr(None), ctypes.c_int(_tag(out_dtype)), _stream()))
         lib.ayk_mlstm_long_scratch_floats.restype = ctypes.c_longlong
-        floats = int(lib.ayk_mlstm_long_scratch_floats(ctypes.c_int(T), ctypes.c_int(ctx.num_requests), ctypes.c_int(heads),
-                                                       ctypes.c_int(dim), ctypes.c_int(vdim)))
+        requests, rows = ctypes.c_int(ctx.num_requests - singles), ctypes.c_int(T - singles)
+        floats = int(lib.ayk_mlstm_long_scratch_floats(rows, requests, ctypes.c_int(heads), ctypes.c_int(dim), ctypes.c_int(vdim)))
         scratch = torch.empty((floats,), dtype=torch.float32, device=proj.device)
         _launch(lib.ayk_mlstm_long(_ptr(out), _ptr(state), _ptr(proj), ctypes.c_longlong(proj.stride(0)), _ptr(norm_weight),
-                                   _ptr(ctx.req_q_start), _ptr(ctx.req_slot), ctypes.c_int(ctx.num_requests), ctypes.c_int(T),
+                                   _ptr(ctx.req_q_start[singles:]), _ptr(ctx.req_slot[singles:]), requests, rows,
                                    ctypes.c_int(heads), ctypes.c_int(dim), ctypes.c_int(vdim), ctypes.c_float(cap), ctypes.c_float(eps),
                                    _ptr(scratch), ctypes.c_int(_tag(out_dtype)), _stream()))
         launches += 2

@@ -442,6 +442,52 @@ def test_mlstm_chunks_side_by_side(H, D, Dv):
         cache.commit(res)
 
 
+@pytest.mark.parametrize("H,D,Dv", [(3, 128, 128), (2, 64, 128), (1, 12, 20), (2, 128, 36)])
+def test_mlstm_chunks_side_by_side_where_the_walk_would_be_faster(monkeypatch, H, D, Dv):
+    from ayaka_py_b200 import ops
+    monkeypatch.setattr(ops, "_mlstm_long_pays", lambda *a: True)
+    test_mlstm_chunks_side_by_side(H, D, Dv)
+
+
+@pytest.mark.parametrize("f_bias,i_gain", [(2.0, 1.0), (-6.0, 8.0)])
+def test_mlstm_single_rows_beside_a_long_portion(f_bias, i_gain):
+    """Many requests of one row beside portions that take the form for long ones, gates usual and strong: the single rows and
+    their memories have the bits that a decode step gives them, and the step's scratch has no memory for them."""
+    from ayaka_py_b200 import ops
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts import StateNeed
+    H, D, Dv, n = 4, 64, 128, 40
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    width = 2 * H * D + 2 * H * Dv + 2 * H
+    w = torch.rand(H * Dv, generator=gen, device="cuda") + 0.5
+    spec = CacheGroupSpec("g", StateNeed((H, ops.mlstm_head_floats(D, Dv)), torch.float32), 1)
+    cache, runner = context_for([spec], "float32", max_requests=n + 2, page_size=8, pages=8)
+    state = cache.state_layer(0, 0)
+    for plan in ({i: 3 for i in range(n + 2)}, {**{i: 1 for i in range(n)}, n: 300, n + 1: 5}):
+        ctx, res = step_of(cache, runner, plan)
+        proj = torch.randn(ctx.num_rows, width, generator=gen, device="cuda")
+        gates = proj[:, 2 * H * D + H * Dv:2 * H * D + H * Dv + 2 * H]
+        gates[:, :H] *= i_gain
+        gates[:, H:] += f_bias
+        before = state.clone()
+        walk = ops.mlstm(proj, state, w, ctx, H, D, Dv, 10.0, 1e-5, torch.float32, chunked=False)
+        walked = state.clone()
+        state.copy_(before)
+        torch.cuda.synchronize()
+        held = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        out = ops.mlstm(proj, state, w, ctx, H, D, Dv, 10.0, 1e-5, torch.float32)
+        taken = torch.cuda.max_memory_allocated() - held
+        assert float((out - walk).abs().max()) < 1e-4 * float(walk.abs().max())
+        used = [cache.slot_of[i] for i in plan]
+        assert float((state - walked)[used].abs().max()) < 1e-4 * max(1.0, float(walked[used].abs().max()))
+        if ctx.num_single:
+            alone = [cache.slot_of[i] for i in range(n)]
+            assert torch.equal(out[:n], walk[:n]) and torch.equal(state[alone], walked[alone])
+            assert taken < 20 * H * ops.mlstm_head_floats(D, Dv) * 4          # 6 chunks, and the rows; 47 memories before
+        cache.commit(res)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,D,Dv,rank", [(3, 12, 10, 20), (2, 32, 16, 40), (4, 64, 64, 128), (1, 16, 48, 8), (8, 64, 48, 96), (2, 24, 256, 36)])
 def test_latent_attention_without_rotation_alone(dtype, H, D, Dv, rank):

@@ -36,3 +36,17 @@ def test_a_window_bounds_the_keys_that_a_tile_is_thought_to_read():
     assert ops._latent_tc_pays(ctx, 16, 512, 64, None, SMS)
     assert not ops._latent_tc_pays(ctx, 16, 512, 64, 16, SMS)
     assert ops._latent_tiles(ctx, 8, None)[1] > ops._latent_tiles(ctx, 8, 16)[1]
+
+
+@pytest.mark.parametrize("heads,dim,vdim,plan,long,apart", [
+    (16, 128, 128, [(0, 64)], False, 0), (16, 128, 128, [(0, 256)], True, 0), (4, 128, 128, [(0, 64)], False, 0),
+    (16, 128, 128, [(0, 1024), (0, 777)], True, 0), (16, 128, 128, [(0, 64)] * 8, True, 0), (4, 128, 128, [(0, 64)] * 8, False, 0),
+    (4, 128, 128, [(0, 64)] * 64, True, 0), (16, 32, 32, [(0, 64)] * 64, False, 0), (16, 32, 32, [(0, 64)] * 250, False, 0),
+    (16, 128, 128, [(9, 1)] * 8 + [(0, 64)], False, 8), (16, 128, 128, [(9, 1)] * 8 + [(0, 256)], True, 8),
+    (16, 128, 128, [(9, 1)] * 250 + [(0, 64)], True, 250), (4, 128, 128, [(9, 1)] * 8 + [(0, 256)], True, 0),
+    (16, 32, 32, [(9, 1)] * 64 + [(0, 64)], False, 64), (16, 128, 128, [(9, 3)] * 100 + [(0, 64)], False, 0),
+    (16, 128, 128, [(9, 3)] * 30 + [(0, 256)], True, 0)])
+def test_mlstm_takes_the_faster_of_its_forms_for_portions(heads, dim, vdim, plan, long, apart):
+    ctx = step(plan)
+    assert ops._mlstm_long_pays(ctx, heads, dim, vdim) is long
+    assert ops._mlstm_singles(ctx, heads) == apart
