@@ -917,16 +917,29 @@ def sigmoid_attention(q: torch.Tensor, kpages: torch.Tensor, vpages: torch.Tenso
 def grouped_part(max_len: int, blocks: int = 0) -> int:
     """Keys per partition of the context when every request brings one row: 64, or the power of two that
     leaves at most 64 partitions of the longest context the cache holds.  ``blocks`` (requests times groups of heads; 0:
-    unknown): larger partitions, up to 256 keys and a quarter of the context, while they leave two blocks to every
-    multiprocessor.  A block of one 64-key tile has nothing to load while it computes, and the merge reads 520 bytes per
-    head and partition; measured for 32 requests of 16 heads over 4 key heads, 1,900 keys each (us for the layer): 86 with
-    64 keys, 71 with 128, 64 with 256, 69 with 512; 8 requests 39, 33, 30, 39; 4 requests over 1,000 keys 22.6, 24.7, 24.7."""
+    leave it at that): larger partitions, up to 256 keys and a quarter of what the cache holds, when there is a block for four of
+    five multiprocessors even if every context fits one partition.  The contexts are not looked at (a captured step is replayed
+    as they grow), so a line that counted the cache's partitions left short contexts with too few blocks.  A row's sums, and so
+    their order, are those of its step's partition size, which goes with the step's number of requests.
+    A block of one 64-key tile has nothing to load while it computes, and the merge reads 520 bytes per head and partition.
+    Measured, 16 heads over 4 key heads of 128, a cache of 2,048 keys (us; 64, 128, 256 keys): 32 requests of 1,948 keys 74.7, 59.3, 54.2;
+    of 250 19.1, 13.7, 15.4; 128 requests of 100 48.6, 29.7, 22.4; but 8 requests of 250 8.6, 10.8, 14.7, of 1,948 26.3, 20.1, 17.1."""
     part = 64
     while part * 64 < max_len:
         part *= 2
-    while blocks and part < 256 and part * 8 <= max_len and blocks * -(-max_len // (2 * part)) >= 2 * sm_count():
+    while blocks * 5 >= sm_count() * 4 and part < 256 and part * 8 <= max_len:
         part *= 2
     return part
+
+
+def _grouped_blocks(rows: int, heads: int, groups: int, key_dim: int, vdim: int, tensor_cores: bool) -> int:
+    """``blocks`` of ``grouped_part`` for a step of single rows.  The kernel on the FP32 pipes has a block to each head and
+    takes 3 us a key tile, so larger partitions pay there from twelve blocks to a multiprocessor on only: float32, 16 heads,
+    contexts of 250 and 1,948 keys of 2,048 (us; 64, 128, 256 keys): 32 requests 439, 481, 592 and 2,888, 2,811, 2,850; 128 requests 2,129,
+    1,760, 1,621 and 11,541, 11,020, 10,846."""
+    if tensor_cores and heads // groups <= 64 and key_dim % 8 == 0 and vdim % 8 == 0 and vdim <= 128:
+        return rows * groups
+    return rows * heads if rows * heads >= 12 * sm_count() else 0
 
 
 def head_norm_prepare(proj: torch.Tensor, kpages: torch.Tensor, vpages: torch.Tensor, q_norm: torch.Tensor, k_norm: torch.Tensor,
@@ -997,7 +1010,7 @@ def grouped_attention(q: torch.Tensor, kpages: torch.Tensor, vpages: torch.Tenso
     if sinks is not None and _f32(sinks, "sinks").numel() != heads:
         raise KernelError("grouped_attention: one sink per query head")
     span, from_first = ctx.cache.max_len, False
-    blocks = T * max(key_heads, VH)
+    blocks = _grouped_blocks(T, heads, max(key_heads, VH), key_dim, DV, tensor_cores and q.dtype == torch.bfloat16)
     part_keys = grouped_part(span, blocks)
     parts = max(1, -(-span // part_keys)) if ctx.max_q_len == 1 else 1
     reach = min(n for n in (span, window or span, chunk or span))

@@ -50,3 +50,12 @@ def test_mlstm_takes_the_faster_of_its_forms_for_portions(heads, dim, vdim, plan
     ctx = step(plan)
     assert ops._mlstm_long_pays(ctx, heads, dim, vdim) is long
     assert ops._mlstm_singles(ctx, heads) == apart
+
+
+@pytest.mark.parametrize("rows,heads,groups,tensor_cores,max_len,keys", [
+    (8, 16, 4, True, 2048, 64), (8, 16, 4, True, 8192, 128), (8, 32, 8, True, 2048, 64), (32, 16, 4, True, 2048, 256),
+    (32, 16, 4, True, 8192, 256), (8, 16, 16, True, 2048, 256), (128, 16, 4, True, 512, 128), (128, 16, 4, True, 100, 64),
+    (32, 32, 1, True, 2048, 64), (32, 16, 4, False, 2048, 64), (128, 16, 4, False, 2048, 256)])
+def test_partitions_grow_where_short_contexts_leave_no_multiprocessor_without_a_block(monkeypatch, rows, heads, groups, tensor_cores, max_len, keys):
+    monkeypatch.setattr(ops, "sm_count", lambda: SMS)
+    assert ops.grouped_part(max_len, ops._grouped_blocks(rows, heads, groups, 128, 128, tensor_cores)) == keys
