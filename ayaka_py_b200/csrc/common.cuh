@@ -102,16 +102,16 @@ __device__ __forceinline__ float apply_activation_tc(float x, int act) {
 // Without the attribute both are no-ops.
 //
 // Blocks that are placed early go where the running kernel has left room, several to one multiprocessor and none to
-// others, and stay there, and they take that room from blocks of the running kernel that are still to come.  Kernels of a
-// few blocks (a decode step's) gain the launch latency; kernels whose time is that of their fullest multiprocessor
-// (several blocks to each, bound by its pipes) lose more by the uneven places.  So those neither trigger before their
+// others, and stay there.  (They are placed once every block of the running kernel has triggered or ended, so they take
+// nothing from it.)  Kernels of a few blocks (a decode step's) gain the launch latency; kernels whose time is that of their
+// fullest multiprocessor (several blocks to each, bound by its pipes) lose more by the uneven places.  So those neither trigger before their
 // end nor, where it was measured to cost, are launched before the end of the kernel in front (ayk_launch_after).
 // Measured: a float32 GPT-2 layer over 377 rows 952 -> 538 us, an mLSTM layer over 1,801 rows 614 -> 471, the routed
 // experts of a decode step of 8 rows 108.6 -> 98.5, latent attention of a decode step of 8 rows 58.6 -> 55.2.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-constexpr unsigned AYK_FEW_BLOCKS = 74;      // at most one block to every second multiprocessor: early launches cannot crowd one
+constexpr unsigned AYK_FEW_BLOCKS = 74;      // half of the B200's 148 multiprocessors: so few blocks crowd none, wherever they are placed
 
 int ayk_pdl_enabled();
 int ayk_sm_count();          // streaming multiprocessors of the current device

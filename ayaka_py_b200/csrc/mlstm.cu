@@ -438,11 +438,12 @@ mlstm_finish_kernel(C* __restrict__ out, float* state, const float* raw, const f
 //   mlstm_long_scan   per cell of the memory, over the chunks: leaves every chunk's S_0, n_0, m_0 in the place of its dS
 //                     (S' = e^(m - m') S + e^(G - m') dS with m' = max(m, G), then m = B + m'), and files the last into the state
 //   mlstm_long_out    a chunk's outputs from its S_0, n_0, m_0 (formulas above), with the head's norm and gate applied
-// All three are float32; the products are register tiles fed with float4 from shared memory (8 x 8 sums a thread,
-// 8 x 4 for the pairs' weights), bound by the FP32 pipes and shared memory; the memories' round trips
+// All three are float32; the products are register tiles fed with float4 from shared memory (8 x 8 sums a thread in the
+// first kernel; 4 x 8, and 4 x 4 for the pairs' weights, in the last), bound by the FP32 pipes and shared memory; the memories' round trips
 // (4 x 64 KB a chunk and head of 128 x 128) stay in the L2 for portions of a few thousand tokens.
 // Measured for the layer at 16 heads of 128 x 128 (us; before: the chunked form): 1,024 and 777 tokens 471 -> 261; at 8 heads
-// 2 x 1,024 tokens 461 -> 131, 2 x 200 113 -> 70, 2 x 17 (the chunked form) 64.  The line lies at one whole chunk: 64 tokens.
+// 2 x 1,024 tokens 461 -> 131, 2 x 200 113 -> 70, 2 x 17 (the chunked form) 64; the outputs by two blocks to a multiprocessor then
+// brought the first to 218.  Which form a step takes is estimated from its portions (ops.py), from one whole chunk (64 tokens) on.
 constexpr int LC = 64, LMAX = 128, LLD = LMAX + 4, LTHREADS = 256;
 
 __device__ __forceinline__ void cp_async_16(float* dst, const float* src, bool on) {

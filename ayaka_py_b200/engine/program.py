@@ -7,7 +7,7 @@ of operations, and a step is then one call into the library, which lays the buff
 in a workspace for the step's row counts, picks each kernel by the rules of
 ``ops.linear`` / ``ops.attention`` and launches it.  The kernels, their arguments and
 their order are those of ``Model.forward``; only the interpreter is out of the loop
-(about 20 us per launch from Python against 2 us from native code, which is what
+(about 13 us per launch from Python against 2 us from native code, which is what
 bounds prompt and mixed steps of small models).
 
 A part without ``lower`` (a toy part of a test, an attention with a position encoding
