@@ -923,7 +923,8 @@ def grouped_part(max_len: int, blocks: int = 0) -> int:
     their order, are those of its step's partition size, which goes with the step's number of requests.
     A block of one 64-key tile has nothing to load while it computes, and the merge reads 520 bytes per head and partition.
     Measured, 16 heads over 4 key heads of 128, a cache of 2,048 keys (us; 64, 128, 256 keys): 32 requests of 1,948 keys 74.7, 59.3, 54.2;
-    of 250 19.1, 13.7, 15.4; 128 requests of 100 48.6, 29.7, 22.4; but 8 requests of 250 8.6, 10.8, 14.7, of 1,948 26.3, 20.1, 17.1."""
+    of 250 19.1, 13.7, 15.4; 128 requests of 100 48.6, 29.7, 22.4; but 8 requests of 250 8.6, 10.8, 14.7, of 1,948 26.3, 20.1, 17.1.
+    Keys of 512 numbers (tiles of 32): 30 requests of 250 38.0, 29.3, 25.1, of 1,948 178, 156, 148."""
     part = 64
     while part * 64 < max_len:
         part *= 2
