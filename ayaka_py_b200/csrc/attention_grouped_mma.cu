@@ -397,6 +397,245 @@ int launch(const GroupedArgs& a, int page_shift, int tq, int DKP, int qrows, siz
   return ayk_check_launch("ayk_grouped_attention (tensor cores)");
 }
 
+// ------------------------------------------------------- steps of single rows --
+// A decode step is bound by the stream of the cached keys and values, and the products of a row's heads are small.  A block takes
+// (request, group of at most 8 heads, part of the context); each of its four warps takes every fourth 16 keys of the part on its own, with a
+// running softmax and sums that meet at the end, and copies them into its own GD_STAGES places of shared memory, the next under the
+// products of the present, so that no warp waits for another.  The pages of the part are looked up once, 32 by 32:
+// a load of the table between the copies would be answered behind them.  S has the heads as rows (m16n8k16, the upper half empty); its
+// fragments are those of the weights as second operand of O^T += V^T P^T, whose columns are the heads: half of the products
+// and registers of O += P V.  A piece of 16 bytes lies at its number XOR the low bits of its key, which leaves ldmatrix without bank
+// conflicts.  Three blocks to a multiprocessor (64 KB each for heads of 128).
+// Measured, the rotary layer of width 2,048, 16 heads over 4 key heads of 128, against the form of the kernel above in which the
+// block's warps share each tile of 64 keys behind a barrier (us): 32 requests of 1,900 keys 64.0 -> 46.7 (this kernel 47 -> 26, 4.2 TB/s),
+// 17 of 1,900 56.9 -> 40.9, 8 of 1,900 39.0 -> 28.7, 32 of 250 29.1 -> 24.0, 1 of 30 18.5 -> 16.4; none of 80 steps slower.  A warp to an
+// item, with no sums to meet, was slower for short parts (8 of 250: 22.6 against 19.9) and no faster for long ones (47.2).
+constexpr int GD_WARPS = 4, GD_STAGES = 2, GD_KEYS = 16, GD_HEADS = 8;
+constexpr size_t gd_smem(int d) { return (size_t)GD_WARPS * GD_STAGES * GD_KEYS * 2 * d * sizeof(__nv_bfloat16); }
+
+template <int D>
+__global__ void __launch_bounds__(GD_WARPS * 32, 3)
+grouped_decode_kernel(GroupedArgs a, int page_shift) {
+  constexpr int PIECES = D / 8, PER = 32 / PIECES, HALF = GD_KEYS * D;      // keys that a copy instruction covers; elements of 16 keys
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+  __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(smem_raw) + (size_t)warp * GD_STAGES * 2 * HALF;      // [stage]: keys, values
+  const int QH = a.QH, NG = max(a.KH, a.VH), hpg = QH / NG;
+  const int req = blockIdx.x, g = blockIdx.y, part = blockIdx.z;
+  const int kh = g / (NG / a.KH), vh = g / (NG / a.VH);
+  const int row = a.req_q_start[req], pos = a.req_pos0[req];
+  const int base_part = a.parts_from_first ? grouped_base_part(pos, a.window, a.chunk, a.part_keys) : 0;
+  const int k_first = a.part_keys > 0 ? (base_part + part) * a.part_keys : 0;
+  const int k_last = a.part_keys > 0 ? min(pos, k_first + a.part_keys - 1) : pos;
+  const int* my_table = a.table + (size_t)req * a.table_stride;
+  int page_base = 0;
+  auto lookup = [&](int base) {                         // lane i: the page of the part's (base + i)-th 16 keys
+    const int k = k_first + (base + lane) * GD_KEYS;
+    return k <= k_last ? my_table[k >> page_shift] : 0;
+  };
+  int pages = lookup(0);
+  pdl_wait();
+  if (k_first > pos) return;                            // the merge does not read parts beyond the context
+  const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(a.q);
+  const int piece = lane % PIECES, sub = lane / PIECES;
+  const __nv_bfloat16* kcache = reinterpret_cast<const __nv_bfloat16*>(a.kcache) + ((size_t)sub * a.KH + kh) * D + piece * 8;
+  const __nv_bfloat16* vcache = reinterpret_cast<const __nv_bfloat16*>(a.vcache) + ((size_t)sub * a.VH + vh) * D + piece * 8;
+  const float scale2 = a.scale * LOG2E;
+  // where this lane's rows of an ldmatrix lie, and its first piece
+  const int krow = (lane >> 4) * 8 + (lane & 7), kpiece = (lane >> 3) & 1;
+  const int vrow = (lane >> 4) * 8 + (lane & 7), vpiece = (lane >> 3) & 1;
+  const GroupedTiles walk(k_first, k_last, pos, a.window, a.keep_first, GD_KEYS, a.chunk);
+  auto mine = [&](int k0, int steps) {                  // 16 keys further, ``steps`` times
+    for (int i = 0; i < steps; ++i) k0 = walk.next(k0);
+    return k0;
+  };
+  int ask_k = mine(walk.first(), warp), ask_slot = 0, on_page = 0;      // on_page: a bit to a stage, the next to be read lowest
+  auto ask = [&]() {
+    if (ask_k <= k_last) {
+      const int unit = (ask_k - k_first) / GD_KEYS;
+      if ((unit & ~31) != page_base) {
+        page_base = unit & ~31;
+        pages = lookup(page_base);
+      }
+      const int page = __shfl_sync(0xffffffffu, pages, unit & 31);
+      const int bytes = page > 0 ? 16 : 0;              // no page: zeros
+      const size_t cell = page > 0 ? ((size_t)page << page_shift) + (ask_k & ((1 << page_shift) - 1)) : 0;
+      const __nv_bfloat16* kfrom = kcache + cell * a.KH * D;
+      const __nv_bfloat16* vfrom = vcache + cell * a.VH * D;
+      const uint32_t to = (uint32_t)__cvta_generic_to_shared(ring + (size_t)ask_slot * 2 * HALF);
+#pragma unroll
+      for (int i = 0; i < GD_KEYS / PER; ++i) {
+        const int key = i * PER + sub;
+        const uint32_t at = to + (uint32_t)(key * D * 2 + ((piece ^ (key & 7)) << 4));
+        const int live = ask_k + key <= k_last ? bytes : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(kfrom + (live ? (size_t)i * PER * a.KH * D : 0)), "r"(live) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + HALF * 2), "l"(vfrom + (live ? (size_t)i * PER * a.VH * D : 0)), "r"(live) : "memory");
+      }
+      on_page |= (page > 0) << (GD_STAGES - 1);
+      ask_k = mine(ask_k, GD_WARPS);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");          // a group a tile, or its absence
+    ask_slot = ask_slot + 1 == GD_STAGES ? 0 : ask_slot + 1;
+  };
+#pragma unroll
+  for (int i = 0; i < GD_STAGES - 1; ++i) {
+    ask();
+    on_page >>= 1;
+  }
+  const bool head_row = gid < hpg;
+  uint32_t qf[D / 16][2];                               // row gid of the first operand: the group's head gid
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      qf[ks][r] = head_row ? *reinterpret_cast<const uint32_t*>(q + ((size_t)row * QH + g * hpg + gid) * D + ks * 16 + r * 8 + tig * 2) : 0u;
+  const float slope2 = a.slopes && head_row ? a.slopes[g * hpg + gid] * LOG2E : 0.f;
+  float m_run = -INFINITY, l_run = 0.f;                 // l: this thread's share of the head's denominator
+  if (a.sinks && part == 0 && warp == 0 && head_row) {  // the sink counts once per row: in the first part, one of the row's four threads
+    m_run = a.sinks[g * hpg + gid] * LOG2E;
+    l_run = tig == 0 ? 1.f : 0.f;
+  }
+  const int chunk_start = a.chunk > 0 ? pos / a.chunk * a.chunk : 0;
+  float o[D / 16][4];                                   // rows: dimensions gid and gid + 8 of 16; columns: heads 2 tig and 2 tig + 1
+#pragma unroll
+  for (int mt = 0; mt < D / 16; ++mt)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) o[mt][c] = 0.f;
+  int slot = 0;
+#pragma unroll 1
+  for (int k0 = mine(walk.first(), warp); k0 <= k_last; k0 = mine(k0, GD_WARPS)) {
+    ask();
+    asm volatile("cp.async.wait_group %0;" ::"n"(GD_STAGES - 1) : "memory");
+    __syncwarp();
+    const uint32_t kat = (uint32_t)__cvta_generic_to_shared(ring + (size_t)slot * 2 * HALF), vat = kat + HALF * 2;
+    const bool on = on_page & 1;
+    on_page >>= 1;
+    slot = slot + 1 == GD_STAGES ? 0 : slot + 1;
+    float sc[2][2][4];                                  // two sums a tile of 8 keys (even and odd 16s of the head), for shorter chains
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sc[nt][0][c] = sc[nt][1][c] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ++ks) {
+      uint32_t b0, b1, b2, b3;
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3) : "r"(kat + (uint32_t)(krow * D * 2 + (((ks * 2 + kpiece) ^ (krow & 7)) << 4))));
+      const uint32_t qa[4] = {qf[ks][0], 0u, qf[ks][1], 0u};
+      mma_bf16(sc[0][ks & 1], qa, b0, b1);
+      mma_bf16(sc[1][ks & 1], qa, b2, b3);
+    }
+    const bool inside = on && k0 + GD_KEYS - 1 <= k_last && (a.window <= 0 || pos - k0 < a.window) && k0 >= chunk_start;
+    float s[2][2], mx = -INFINITY;                      // this thread's keys: k0 + 8 nt + 2 tig + c
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int key = k0 + nt * 8 + tig * 2 + c;
+        float v = fmaf(-slope2, (float)(pos - key), (sc[nt][0][c] + sc[nt][1][c]) * scale2);
+        if (!inside) {
+          const bool seen = on && key <= k_last && (a.window <= 0 || pos - key < a.window || key < a.keep_first) && key >= chunk_start;
+          v = seen ? v : -INFINITY;
+        }
+        s[nt][c] = v;
+        mx = fmaxf(mx, v);
+      }
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const float m_new = fmaxf(m_run, mx);
+    const float alpha = m_new > -INFINITY ? fast_exp2(m_run - m_new) : 1.f;         // 2^(-inf) = 0 on the first visible tile
+    m_run = m_new;
+    const float base = m_new > -INFINITY ? m_new : 0.f;                             // nothing seen yet: every weight is 2^(-inf) = 0
+    float sum = 0.f;
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        s[nt][c] = fast_exp2(s[nt][c] - base);
+        sum += s[nt][c];
+      }
+    l_run = fmaf(l_run, alpha, sum);
+    if (__any_sync(0xffffffffu, alpha != 1.f)) {
+      const float a0 = __shfl_sync(0xffffffffu, alpha, tig * 8), a1 = __shfl_sync(0xffffffffu, alpha, tig * 8 + 4);
+#pragma unroll
+      for (int mt = 0; mt < D / 16; ++mt) {
+        o[mt][0] *= a0; o[mt][1] *= a1;
+        o[mt][2] *= a0; o[mt][3] *= a1;
+      }
+    }
+    // O^T += V^T P^T: the 32-bit weights enter the product rounded to bfloat16, as the values they multiply are
+    const uint32_t p0 = pack_bf16(s[0][0], s[0][1]), p1 = pack_bf16(s[1][0], s[1][1]);
+#pragma unroll
+    for (int mt = 0; mt < D / 16; ++mt) {
+      uint32_t va[4];
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(va[0]), "=r"(va[1]), "=r"(va[2]), "=r"(va[3]) : "r"(vat + (uint32_t)(vrow * D * 2 + (((mt * 2 + vpiece) ^ (vrow & 7)) << 4))));
+      mma_bf16(o[mt], va, p0, p1);
+    }
+    __syncwarp();                                       // this place is refilled by the next ask
+  }
+
+  // the warps' maxima, sums and O meet in the places of the keys, in warp order
+  constexpr int LDO = D + 4;
+  float* So = reinterpret_cast<float*>(smem_raw);       // [4 warps][8 heads][LDO]
+  float2* Sml = reinterpret_cast<float2*>(So + GD_WARPS * GD_HEADS * LDO);
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+  __syncthreads();
+  if (tig == 0) Sml[warp * GD_HEADS + gid] = make_float2(m_run, l_run);
+#pragma unroll
+  for (int mt = 0; mt < D / 16; ++mt)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) So[(warp * GD_HEADS + tig * 2 + (c & 1)) * LDO + mt * 16 + gid + (c >> 1) * 8] = o[mt][c];
+  __syncthreads();
+  for (int i = tid; i < hpg * (D / 4); i += GD_WARPS * 32) {
+    const int h = i / (D / 4), col = (i - h * (D / 4)) * 4;
+    float m = -INFINITY, l = 0.f;
+#pragma unroll
+    for (int w = 0; w < GD_WARPS; ++w) m = fmaxf(m, Sml[w * GD_HEADS + h].x);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < GD_WARPS; ++w) {
+      const float2 ml = Sml[w * GD_HEADS + h];
+      const float f = m > -INFINITY ? fast_exp2(ml.x - m) : 0.f;
+      const float4 x = *reinterpret_cast<const float4*>(So + (w * GD_HEADS + h) * LDO + col);
+      l = fmaf(ml.y, f, l);
+      v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
+    }
+    const int head = g * hpg + h;
+    const size_t head_at = (size_t)row * QH + head;
+    if (a.partial_o) {
+      *reinterpret_cast<float4*>(a.partial_o + ((size_t)part * a.total_rows * QH + head_at) * D + col) = v;
+      if (col == 0) {
+        float* pml = a.partial_ml + ((size_t)part * a.total_rows * QH + head_at) * 2;
+        pml[0] = m * LN2;                               // the merge works in base e
+        pml[1] = l;
+      }
+    } else {
+      const float inv = l > 0.f ? 1.0f / l : 0.f;
+      v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+      if (a.gate) {
+        const float* gate = a.gate + (size_t)row * a.gate_stride + (size_t)head * D + col;
+        v.x = __fdividef(v.x, 1.0f + __expf(-gate[0])); v.y = __fdividef(v.y, 1.0f + __expf(-gate[1]));
+        v.z = __fdividef(v.z, 1.0f + __expf(-gate[2])); v.w = __fdividef(v.w, 1.0f + __expf(-gate[3]));
+      }
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(a.out) + head_at * D + col) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    }
+  }
+}
+
+template <int D>
+int launch_single(const GroupedArgs& a, int page_shift, int NG, cudaStream_t stream) {
+  static AykPerDevice granted;
+  if (!granted.here()) {
+    cudaError_t e = cudaFuncSetAttribute(grouped_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gd_smem(D));
+    if (e != cudaSuccess) return ayk_fail("ayk_grouped_attention: shared memory %zu: %s", gd_smem(D), cudaGetErrorString(e));
+    granted.here() = true;
+  }
+  ayk_launch(grouped_decode_kernel<D>, dim3(a.num_req, NG, a.parts), dim3(GD_WARPS * 32), gd_smem(D), stream, a, page_shift);
+  return ayk_check_launch("ayk_grouped_attention (single rows)");
+}
+
 size_t smem_bytes(int DKP, int DVT, int KT, int qrows) {
   return ((size_t)qrows * (DKP + 8) + (size_t)NBUF * KT * (DKP + 8 + DVT + 8)) * sizeof(__nv_bfloat16) + NBUF * KT;
 }
@@ -412,6 +651,11 @@ int ayk_grouped_attention_mma(const GroupedArgs& a, cudaStream_t stream) {
   int page_shift = 0;
   while ((1 << page_shift) < a.page_size) ++page_shift;
   if ((1 << page_shift) != a.page_size) return 1;
+  // heads of 64 or 128 numbers, 16 keys within a page; wider groups and other sizes take the tiles below
+  if (a.total_rows == a.num_req && hpg <= GD_HEADS && a.DK == a.DV && a.page_size >= GD_KEYS) {
+    if (a.DK == 128) return launch_single<128>(a, page_shift, NG, stream);
+    if (a.DK == 64) return launch_single<64>(a, page_shift, NG, stream);
+  }
   const int DKP = (a.DK + 15) & ~15;
   const int DVT = a.DV <= 32 ? 32 : (a.DV <= 64 ? 64 : 128);
   // every request brings one row: a tile holds the heads of one token, and only their rows are staged

@@ -1,0 +1,42 @@
+"""Steps of single tokens: the kernels that stream weights and cached keys, at the edges of what they take."""
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from test_gpu_vedadra import context_for, step_of        # noqa: E402
+
+
+@pytest.mark.parametrize("H,G,D,page,window,keep,chunk,cut", [
+    (16, 4, 128, 16, None, 0, None, True), (8, 1, 128, 32, None, 0, None, True), (6, 2, 128, 16, 70, 9, None, True),
+    (16, 2, 64, 64, 300, 0, None, True), (8, 4, 128, 16, None, 0, 100, True), (4, 4, 64, 16, 1, 0, None, True), (16, 4, 128, 16, None, 0, None, False)])
+def test_single_rows_of_heads_that_share_their_keys(H, G, D, page, window, keep, chunk, cut):
+    """The tensor-core kernel against the FP32 pipes on the same bfloat16 pages: contexts that end at the edges of the warps'
+    16 keys and of partitions, a window far into a part, windows, kept first keys, chunks, sinks, gates."""
+    from ayaka_py_b200 import ops
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts.base import KVNeed
+    torch.manual_seed(H + D)
+    need = KVNeed(kv_heads=G, head_dim=D, window=window if not chunk else None, value_heads=G, value_dim=D, keep_first=keep if window else 0)
+    before = [0, 1, 15, 16, 17, 63, 64, 127, 128, 255, 256, 511, 1000] if cut else [0, 15, 16, 63]
+    cache, runner = context_for([CacheGroupSpec("g", need, 1)], "bfloat16", max_requests=len(before), page_size=page,
+                                pages=sum(-(-(n + 1) // page) for n in before) + 2, positions=1024 if cut else 64)
+    kpages, vpages = cache.kv_layer(0, 0)
+    kpages.copy_(torch.randn(kpages.shape, device="cuda") * 0.7)
+    vpages.copy_(torch.randn(vpages.shape, device="cuda"))
+    for i, n in enumerate(before):
+        slot = cache.open(i)
+        if n:
+            cache.commit(cache.reserve([(slot, 0, n)]))
+    ctx, res = step_of(cache, runner, {i: 1 for i in range(len(before))})
+    q = (torch.randn(ctx.num_rows, H * D, device="cuda") * 0.3).to(torch.bfloat16)
+    for sinks, slopes in ((torch.randn(H, device="cuda"), None), (None, torch.rand(H, device="cuda") * 0.05)):
+        kw = dict(heads=H, key_heads=G, key_dim=D, scale=0.6, window=window, keep_first=keep, chunk=chunk, sinks=sinks, slopes=slopes,
+                  gate=torch.randn(ctx.num_rows, H * D, device="cuda"))
+        got = ops.grouped_attention(q, kpages, vpages, ctx.tables[0], ctx, tensor_cores=True, **kw).float()
+        want = ops.grouped_attention(q, kpages, vpages, ctx.tables[0], ctx, tensor_cores=False, **kw).float()
+        assert torch.isfinite(got).all()
+        # the weights enter the second product as bfloat16 (2^-9 of each), the result is rounded to bfloat16 twice
+        assert float((got - want).abs().max()) < 1.5e-2 * float(want.abs().max())
+    cache.rollback(res)
