@@ -480,7 +480,7 @@ moe_gemm_mma_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_str
 
 // --------------------------------------------- few pairs: matrix times vector --
 // A step of single tokens has a handful of (token, choice) pairs, most on experts of their own: each pair
-// then streams its expert's matrix once, and the product is bound by that stream.  A block takes one pair and
+// then streams its expert's matrix once, and little else happens (moe_gemv_kernel below takes over where the matrices are many).  A block takes one pair and
 // 64 output features (32 with the activation); the pair's activation row waits in shared memory as float32; a warp takes 8 (4)
 // features, two at a time, its lanes striding along K in 16-byte pieces of the weight rows (with the activation, both the gate
 // row and the up row of a feature), sixteen pieces (eight without the activation, by twice as
@@ -488,7 +488,7 @@ moe_gemm_mma_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_str
 // Measured, the routed layer of width 2,048 (us; before: 64 features a block, four pieces at a time): 1 row 65 -> 33, 3 rows
 // 92 -> 62, 8 rows 99 -> 92; of width 1,024 1 row 33 -> 25, 8 rows 44 -> 34.  The first product of the 8 rows 56 -> 37; the second
 // 20 -> 24 with sixteen pieces, and the layer 89 -> 85 with eight and four blocks to a multiprocessor.
-constexpr int gv_cols(bool glu) { return glu ? 32 : 64; }
+constexpr int pv_cols(bool glu) { return glu ? 32 : 64; }
 
 __device__ __forceinline__ float dot8(const uint4& w, const float4& x0, const float4& x1) {
   // a bfloat16 is the upper half of a float
@@ -504,10 +504,10 @@ __device__ __forceinline__ float dot8(const uint4& w, const float4& x0, const fl
 
 template <typename O, bool GLU>
 __global__ void __launch_bounds__(256, GLU ? 2 : 4)
-moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
+moe_pair_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
                 const __nv_bfloat16* __restrict__ w, const int* ids, int top, int gather, int N, int N_w,
                 int Kd, float limit, float slope, float plus, int act, const float* early) {
-  constexpr int STREAMS = GLU ? 4 : 2, STEPS = 4, PER_WARP = gv_cols(GLU) / 8;
+  constexpr int STREAMS = GLU ? 4 : 2, STEPS = 4, PER_WARP = pv_cols(GLU) / 8;
   extern __shared__ __align__(16) float xs[];          // [Kd]
   pdl_wait();
   const int pair = blockIdx.x;
@@ -579,6 +579,205 @@ moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
       out[(size_t)pair * N + n0] = from_float<O>(GLU ? glu_limited(sum[0], sum[STREAMS - 2], limit, slope, plus) : apply_activation(sum[0], act));
       if (n1 < N)
         out[(size_t)pair * N + n1] = from_float<O>(GLU ? glu_limited(sum[1], sum[STREAMS - 1], limit, slope, plus) : apply_activation(sum[1], act));
+    }
+  }
+}
+
+// ----------------------------------------------- few pairs: a stream of weights --
+// A step of single tokens has a handful of (token, choice) pairs, and the product is bound by the stream of their experts'
+// matrices.  The pairs are grouped by expert, up to eight to a group, so that an expert that several rows chose is streamed once
+// for them (8 rows of 2 of 16 experts choose 10.5 experts on average, in 16 pairs).  The work is cut into (group, 16 weight rows): with the
+// activation the gate and up rows of eight features, else the rows of sixteen; in equal runs to the blocks, one block of eight warps to a
+// multiprocessor, and a run's K in steps of 32 to the warps in turn.  A lane copies the 16-byte pieces that it multiplies itself into its own places of shared
+// memory, GV_STAGES stages of two steps deep and across the ends of the units, and waits for nothing but its own copies:
+// no registers are held for pieces on their way, and 128 KB of a multiprocessor's share are always asked for.  The weight rows are the rows of
+// m16n8k16, the group's activation rows its columns; which of the K numbers of a step sits at which place of the product does not matter, so
+// a piece of eight numbers goes into two products as it lies.  A unit's sums of the eight warps meet in shared memory.  What the loop reads besides lies in
+// shared memory too: a load from global memory is answered behind the copies asked for before it, even when it hits the L1.  No
+// sorting of rows: pair p reads row p / top (gather) or p, and writes row p; a pair's sum does not depend on its group.
+// Where the line to moe_pair_gemv_kernel lies: this kernel needs the list of groups and most of a multiprocessor's shared memory before its
+// first copy, about 2 us a launch.  Measured, the routed layer, 2 of 16 experts (us; pair by pair, grouped): width 2,048 2 rows 39.0, 41.5, 3 rows
+// 57.1, 54.2, 8 rows 83.2, 68.8, 31 rows 210, 99; width 1,024 8 rows 30.8, 32.8, 12 rows 40.9, 38.6, 31 rows 74.3, 50.0; width 512 24 rows 32.8,
+// 34.9.  Summing on the FP32 pipes in place of the tensor cores took 82 at 8 rows: the blocks whose experts had three and four rows were late.
+constexpr long long GV_LINE = 20LL << 20;                // pairs times the numbers of a result's matrix, from which on the grouped kernel is the faster
+constexpr int GV_WARPS = 8, GV_STAGES = 9, GV_STEP = 32, GV_GROUP = 8;
+constexpr int GV_MOST = 128;                             // pairs of one launch
+constexpr int GV_PAD = 32;                               // numbers between two activation rows: eight lanes' pieces of two rows lie in different banks
+constexpr size_t GV_RING = (size_t)GV_WARPS * GV_STAGES * 4 * 32 * sizeof(uint4);        // two steps of two rows a lane
+constexpr size_t GV_SUMS = (size_t)2 * GV_WARPS * 128 * sizeof(float);
+constexpr int gv_group(int Kd) { return Kd <= 4096 ? 8 : Kd <= 8192 ? 4 : 2; }            // pairs of a group: as many rows as fit
+constexpr int gv_held(int Kd) { return Kd <= 2048 ? 2 : 1; }      // groups whose rows are held: a block's run rarely meets more than two
+constexpr size_t gv_smem(int Kd) {
+  return GV_RING + GV_SUMS + 4 * GV_MOST * sizeof(int) + (size_t)gv_held(Kd) * gv_group(Kd) * (Kd + GV_PAD) * sizeof(__nv_bfloat16);
+}
+static_assert(gv_smem(2048) <= 227 * 1024 && gv_smem(4096) <= 227 * 1024 && gv_smem(8192) <= 227 * 1024 && gv_smem(12288) <= 227 * 1024,
+              "the places of the copies and the activation rows share a multiprocessor");
+
+__device__ __forceinline__ void gv_copy(void* dst, const __nv_bfloat16* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void gv_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+template <typename O, bool GLU>
+__global__ void __launch_bounds__(GV_WARPS * 32, 1)
+moe_gemv_kernel(O* __restrict__ out, const __nv_bfloat16* a, long long a_stride,
+                const __nv_bfloat16* __restrict__ w, const int* ids, int pairs, int top, int gather, int N, int N_w,
+                int Kd, int held, int most, float limit, float slope, float plus, int act, const float* early) {
+  constexpr int COLS = GLU ? 8 : 16;                     // features of a unit
+  extern __shared__ __align__(16) unsigned char gv_shared[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+  uint4* ring = reinterpret_cast<uint4*>(gv_shared) + (size_t)warp * GV_STAGES * 4 * 32 + lane;      // [stage][step, row][lane]
+  float* sums = reinterpret_cast<float*>(gv_shared + GV_RING);    // [2][warp][16 rows][8 pairs]
+  int* id_of = reinterpret_cast<int*>(gv_shared + GV_RING + GV_SUMS);      // [pairs]
+  int* sorted = id_of + GV_MOST;                                  // the pairs, by expert
+  int* start = sorted + GV_MOST;                                  // place in ``sorted`` at which a group starts
+  float* factor = reinterpret_cast<float*>(start + GV_MOST);      // [pairs]
+  __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(factor + GV_MOST);      // [held][most][Kd + GV_PAD]
+  pdl_wait();
+  if (tid < GV_MOST) {
+    id_of[tid] = tid < pairs ? ids[tid] : 0x7fffffff;
+    factor[tid] = early && tid < pairs ? early[tid] : 1.f;
+    sorted[tid] = -1;
+  }
+  __syncthreads();
+  if (tid < pairs) {                                              // place of a pair: those of lower experts, then those before it
+    const int id = id_of[tid];
+    int lower = 0, same = 0;
+    for (int q = 0; q < pairs; q += 4) {
+      const int4 v = *reinterpret_cast<const int4*>(id_of + q);
+      lower += (v.x < id) + (v.y < id) + (v.z < id) + (v.w < id);
+      same += (v.x == id && q < tid) + (v.y == id && q + 1 < tid) + (v.z == id && q + 2 < tid) + (v.w == id && q + 3 < tid);
+    }
+    sorted[lower + same] = same % most == 0 ? tid : ~tid;         // a group's first pair as it is, the others inverted
+  }
+  __syncthreads();
+  const bool starts = tid < pairs && sorted[tid] >= 0;
+  if (starts) {
+    int at = 0;
+    for (int j = 0; j < tid; j += 4) {
+      const int4 v = *reinterpret_cast<const int4*>(sorted + j);
+      at += (v.x >= 0) + (v.y >= 0 && j + 1 < tid) + (v.z >= 0 && j + 2 < tid) + (v.w >= 0 && j + 3 < tid);
+    }
+    start[at] = tid;
+  }
+  const int groups = __syncthreads_count(starts);
+
+  const int units = (N + COLS - 1) / COLS;               // of a group
+  const long long total = (long long)groups * units;
+  const int begin = (int)(total * blockIdx.x / gridDim.x), end = (int)(total * (blockIdx.x + 1) / gridDim.x);
+  if (begin == end) return;
+  auto pair_at = [&](int i) { const int p = sorted[i]; return p < 0 ? ~p : p; };
+  auto members_of = [&](int g) { return (g + 1 < groups ? start[g + 1] : pairs) - start[g]; };
+  const int g_first = begin / units, g_last = (end - 1) / units;
+  auto bring_rows = [&](int g_from) {                    // the activation rows of the next ``held`` groups
+    for (int g = g_from; g <= g_last && g < g_from + held; ++g)
+      for (int m = 0; m < members_of(g); ++m) {
+        const int p = pair_at(start[g] + m);
+        const __nv_bfloat16* from = a + (size_t)(gather ? p / top : p) * a_stride;
+        __nv_bfloat16* to = rows + (size_t)((g - g_from) * most + m) * (Kd + GV_PAD);
+        for (int i = tid * 8; i < Kd; i += GV_WARPS * 32 * 8) gv_copy(to + i, from + i);
+      }
+    gv_commit();
+  };
+  bring_rows(g_first);
+  // the copies of the weights run ahead of the products: their own unit, first K number and rows
+  const int k_mine = warp * GV_STEP + tig * 8;           // of a stage: this lane's piece of the first step; the second step lies 8 warps on
+  constexpr int STAGE_K = 2 * GV_WARPS * GV_STEP;
+  int ask_unit = begin, ask_k = 0, ask_slot = 0, ask_g = g_first, ask_f = (begin - g_first * units) * COLS;
+  const __nv_bfloat16 *ask0 = w, *ask1 = w;
+  auto ask_rows = [&]() {
+    const __nv_bfloat16* we = w + (size_t)id_of[sorted[start[ask_g]]] * N_w * Kd + k_mine;
+    const int f0 = min(ask_f + gid, N - 1), f1 = GLU ? f0 + N : min(ask_f + 8 + gid, N - 1);       // past the last feature the last one's again
+    ask0 = we + (size_t)f0 * Kd;
+    ask1 = we + (size_t)f1 * Kd;
+  };
+  auto ask = [&]() {
+    if (ask_unit < end) {
+      uint4* to = ring + ask_slot * 4 * 32;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (ask_k + i * (STAGE_K / 2) + k_mine < Kd) {
+          gv_copy(to + i * 64, ask0 + ask_k + i * (STAGE_K / 2));
+          gv_copy(to + i * 64 + 32, ask1 + ask_k + i * (STAGE_K / 2));
+        }
+      ask_k += STAGE_K;
+      if (ask_k >= Kd) {
+        ask_k = 0;
+        ask_f += COLS;
+        if (ask_f >= N) {
+          ask_f = 0;
+          ++ask_g;
+        }
+        if (++ask_unit < end) ask_rows();
+      }
+    }
+    gv_commit();                                         // one group a stage, so that "all but the last ones" means the oldest stage
+    ask_slot = ask_slot + 1 == GV_STAGES ? 0 : ask_slot + 1;
+  };
+  ask_rows();
+#pragma unroll
+  for (int i = 0; i < GV_STAGES - 1; ++i) ask();
+  asm volatile("cp.async.wait_group %0;" ::"n"(GV_STAGES - 1) : "memory");        // the activation rows
+  __syncthreads();
+
+  int slot = 0, g_from = g_first, g = g_first, f = (begin - g_first * units) * COLS;
+#pragma unroll 1
+  for (int unit = begin; unit < end; ++unit) {
+    const int members = members_of(g);
+    const __nv_bfloat16* x = rows + (size_t)((g - g_from) * most + gid) * (Kd + GV_PAD) + k_mine;
+    float acc[2][4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[0][c] = acc[1][c] = 0.f;
+#pragma unroll 1
+    for (int k = 0; k < Kd; k += STAGE_K) {
+      ask();
+      asm volatile("cp.async.wait_group %0;" ::"n"(GV_STAGES - 1) : "memory");
+      const uint4* from = ring + slot * 4 * 32;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int at = k + i * (STAGE_K / 2);
+        if (at + warp * GV_STEP >= Kd) break;            // warp-uniform
+        uint4 w0 = make_uint4(0u, 0u, 0u, 0u), w1 = w0, v = w0;
+        if (at + k_mine < Kd) {
+          w0 = from[i * 64];
+          w1 = from[i * 64 + 32];
+          if (gid < members) v = *reinterpret_cast<const uint4*>(x + at);
+        }
+        const uint32_t a0[4] = {w0.x, w1.x, w0.y, w1.y}, a1[4] = {w0.z, w1.z, w0.w, w1.w};
+        const uint32_t b0[2] = {v.x, v.y}, b1[2] = {v.z, v.w};
+        mma_bf16(acc[0], a0, b0);
+        mma_bf16(acc[1], a1, b1);
+      }
+      slot = slot + 1 == GV_STAGES ? 0 : slot + 1;
+    }
+    float* meet = sums + (unit & 1) * (GV_WARPS * 128);  // in turns: a unit's readers are through at the next unit's barrier
+    float* to = meet + warp * 128 + gid * 8 + tig * 2;
+    *reinterpret_cast<float2*>(to) = make_float2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
+    *reinterpret_cast<float2*>(to + 64) = make_float2(acc[0][2] + acc[1][2], acc[0][3] + acc[1][3]);
+    __syncthreads();
+    const int m = tid / COLS, j = tid % COLS;            // a pair and a feature to a thread
+    if (m < members && f + j < N) {
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int i = 0; i < GV_WARPS; ++i) {
+        s0 += meet[i * 128 + j * 8 + m];
+        if (GLU) s1 += meet[i * 128 + 64 + j * 8 + m];
+      }
+      const int p = pair_at(start[g] + m);
+      const float by = factor[p];
+      out[(size_t)p * N + f + j] = from_float<O>(GLU ? glu_limited(by * s0, by * s1, limit, slope, plus) : apply_activation(by * s0, act));
+    }
+    f += COLS;
+    if (f >= N) {
+      f = 0;
+      ++g;
+      if (g - g_from == held && unit + 1 < end) {        // a run over more groups than are held
+        g_from = g;
+        __syncthreads();
+        bring_rows(g_from);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+      }
     }
   }
 }
@@ -821,10 +1020,39 @@ AYK_EXPORT int ayk_moe_combine(float* shared, const float* picked, const int* ro
   return ayk_check_launch("ayk_moe_combine");
 }
 
-// The products of a few pairs, pair by pair (see moe_gemv_kernel): bfloat16 a and w, K a multiple of 8 and at most
+// The products of a few pairs (see moe_gemv_kernel): bfloat16 a and w, K a multiple of 8 and at most
 // 12,288.  gather: pair p reads row p / top of a, else row p.  glu: out [pairs, N] bfloat16 = activation of (gate, up)
 // rows of w [E, 2 N, K]; else out [pairs, N] (out_dtype) = act(row times w [E, N, K]).
 AYK_EXPORT int ayk_moe_gemv_takes(int Kd, long long a_stride) { return Kd % 8 == 0 && a_stride % 8 == 0 && Kd <= 12288; }
+
+namespace {
+template <typename O, bool GLU>
+int gemv(O* out, const __nv_bfloat16* a, long long a_stride, const __nv_bfloat16* w, const int* ids, int pairs, int top, int gather, int N,
+         int N_w, int Kd, float limit, float slope, float plus, int act, const float* early, cudaStream_t stream) {
+  if ((long long)pairs * N * Kd < GV_LINE) {
+    ayk_launch(moe_pair_gemv_kernel<O, GLU>, dim3(pairs, (N + pv_cols(GLU) - 1) / pv_cols(GLU)), dim3(256), (size_t)Kd * sizeof(float), stream,
+               out, a, a_stride, w, ids, top, gather, N, N_w, Kd, limit, slope, plus, act, early);
+    return ayk_check_launch("ayk_moe_gemv");
+  }
+  static AykPerDevice granted;
+  if (!granted.here()) {
+    cudaError_t e = cudaFuncSetAttribute(moe_gemv_kernel<O, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return ayk_fail("ayk_moe_gemv: shared memory: %s", cudaGetErrorString(e));
+    granted.here() = true;
+  }
+  const int units = (N + (GLU ? 7 : 15)) / (GLU ? 8 : 16);
+  const int most = GV_MOST / top * top;                  // whole tokens a launch
+  for (int p = 0; p < pairs; p += most) {
+    const int n = pairs - p < most ? pairs - p : most;
+    const long long blocks = (long long)n * units;
+    const int sms = ayk_sm_count();
+    ayk_launch(moe_gemv_kernel<O, GLU>, dim3((unsigned)(blocks < sms ? blocks : sms)), dim3(GV_WARPS * 32), gv_smem(Kd), stream, out + (size_t)p * N,
+               a + (size_t)(gather ? p / top : p) * a_stride, a_stride, w, ids + p, n, top, gather, N, N_w, Kd, gv_held(Kd), gv_group(Kd), limit, slope, plus, act,
+               early ? early + p : nullptr);
+  }
+  return ayk_check_launch("ayk_moe_gemv");
+}
+}  // namespace
 
 AYK_EXPORT int ayk_moe_gemv(void* out, const void* a, long long a_stride, const void* w, const int* ids, int pairs, int top,
                             int N, int N_w, int Kd, int gather, int glu, float limit, float slope, float plus, int act, const float* early,
@@ -832,16 +1060,11 @@ AYK_EXPORT int ayk_moe_gemv(void* out, const void* a, long long a_stride, const 
                             cudaStream_t stream) {
   if (pairs == 0 || N == 0) return 0;
   AYK_REQUIRE(ayk_moe_gemv_takes(Kd, a_stride), "ayk_moe_gemv: rows of %d elements (stride %lld)", Kd, a_stride);
-  dim3 grid(pairs, (N + gv_cols(glu) - 1) / gv_cols(glu));
-  const size_t smem = (size_t)Kd * sizeof(float);
+  AYK_REQUIRE(top >= 1 && top <= GV_MOST, "ayk_moe_gemv: %d choices a row", top);
+  const __nv_bfloat16 *rows = (const __nv_bfloat16*)a, *weights = (const __nv_bfloat16*)w;
   if (glu)
-    ayk_launch(moe_gemv_kernel<__nv_bfloat16, true>, grid, dim3(256), smem, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)a,
-               a_stride, (const __nv_bfloat16*)w, ids, top, gather, N, N_w, Kd, limit, slope, plus, act, early);
-  else if (out_dtype == AYK_DTYPE_BF16)
-    ayk_launch(moe_gemv_kernel<__nv_bfloat16, false>, grid, dim3(256), smem, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)a,
-               a_stride, (const __nv_bfloat16*)w, ids, top, gather, N, N_w, Kd, limit, slope, plus, act, early);
-  else
-    ayk_launch(moe_gemv_kernel<float, false>, grid, dim3(256), smem, stream, (float*)out, (const __nv_bfloat16*)a, a_stride,
-               (const __nv_bfloat16*)w, ids, top, gather, N, N_w, Kd, limit, slope, plus, act, early);
-  return ayk_check_launch("ayk_moe_gemv");
+    return gemv<__nv_bfloat16, true>((__nv_bfloat16*)out, rows, a_stride, weights, ids, pairs, top, gather, N, N_w, Kd, limit, slope, plus, act, early, stream);
+  if (out_dtype == AYK_DTYPE_BF16)
+    return gemv<__nv_bfloat16, false>((__nv_bfloat16*)out, rows, a_stride, weights, ids, pairs, top, gather, N, N_w, Kd, limit, slope, plus, act, early, stream);
+  return gemv<float, false>((float*)out, rows, a_stride, weights, ids, pairs, top, gather, N, N_w, Kd, limit, slope, plus, act, early, stream);
 }

@@ -8,6 +8,41 @@ pytestmark = pytest.mark.gpu
 from test_gpu_vedadra import context_for, step_of        # noqa: E402
 
 
+@pytest.mark.parametrize("T,E,top,N,K", [(31, 16, 2, 2048, 2048),       # groups of several sizes
+                                         (40, 2, 2, 1016, 1000),        # far more than eight pairs an expert, features and K with remainders
+                                         (70, 5, 2, 264, 2056),         # more pairs than a launch takes
+                                         (9, 4, 3, 250, 8200),          # long rows: groups of two pairs
+                                         (6, 1, 1, 2100, 4096)])        # one group, rows held for one group at a time
+@pytest.mark.parametrize("form", ["gate", "act", "plain"])
+def test_the_grouped_stream_of_a_few_pairs(T, E, top, N, K, form):
+    """Against the same operands in 64 bits.  A float32 sum of K products in any order is off by at most K 2^-24 of the
+    sum of their sizes (far less in practice: 2^-17 is stated); a bfloat16 result by 2^-8 of itself more."""
+    from ayaka_py_b200 import ops
+    assert T * top * N * K >= 20 << 20                   # the grouped kernel's side of the line
+    gen = torch.Generator(device="cuda").manual_seed(T + N)
+    pairs, first = T * top, form != "plain"
+    a = torch.randn(T if first else pairs, K, generator=gen, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(E, 2 * N if form == "gate" else N, K, generator=gen, device="cuda") / K ** 0.5).to(torch.bfloat16)
+    route = ops.moe_route(torch.randn(T, E, generator=gen, device="cuda") * 2, E, top, plan=False)
+    glu = (1.5, 1.702, 1.0) if form == "gate" else None
+    got = ops.moe_gemv(a, w, route, glu=glu, activation="relu2" if form == "act" else None, weigh_input=form == "gate").double()
+    x = a.double()
+    for p in range(pairs):
+        t, k = divmod(p, top)
+        row, m = x[t if first else p], w[int(route.ids[t, k])].double()
+        z, size = m @ row, m.abs() @ row.abs()
+        if form == "gate":
+            z, size = z * float(route.weights[t, k]), size * float(route.weights[t, k])
+            g, u = z[:N].clamp(max=1.5), z[N:].clamp(-1.5, 1.5)
+            want, room = g * torch.sigmoid(1.702 * g) * (u + 1.0), (size[:N] * 2.5 * 1.5 + size[N:] * 1.5)
+        elif form == "act":
+            want, room = z.clamp(min=0.0) ** 2, 2 * z.abs() * size
+        else:
+            want, room = z, size
+        assert ((got[p] - want).abs() <= room * 2.0 ** -17 + (want.abs() * 2.0 ** -8 if first else 0.0) + 1e-6).all(), p
+    assert ops.tc_error() == 0
+
+
 @pytest.mark.parametrize("H,G,D,page,window,keep,chunk,cut", [
     (16, 4, 128, 16, None, 0, None, True), (8, 1, 128, 32, None, 0, None, True), (6, 2, 128, 16, 70, 9, None, True),
     (16, 2, 64, 64, 300, 0, None, True), (8, 4, 128, 16, None, 0, 100, True), (4, 4, 64, 16, 1, 0, None, True), (16, 4, 128, 16, None, 0, None, False)])
