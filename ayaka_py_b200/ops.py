@@ -977,11 +977,39 @@ def head_norm_prepare(proj: torch.Tensor, kpages: torch.Tensor, vpages: torch.Te
     return q
 
 
+def _grouped_wide_pays(ctx, heads: int, groups: int, window: int | None, chunk: int | None, sms: int) -> bool:
+    """Whether a step that brings more than one row of some request takes the tcgen05 form of the grouped attention (two tiles of
+    128 rows to a block, one block to a multiprocessor) or the mma.sync form (64 (row, head) pairs to a block, three).  The estimates
+    (us: a block's start and its time a key, alone and where blocks share the multiprocessors) are fitted to 520 steps of 5 shapes (8 to 32 heads
+    over 2 to 8 key heads; 1 to 32 requests of 2 to 1,024 rows, contexts of 2 to 1,924 keys): the choice is on average
+    0.3 % behind the faster form, more than 6 % in 6 of them.  Measured, mma.sync and tcgen05, 16 heads over 4: one prompt of 32 rows 7.5, 7.9, of
+    128 12.0, 9.8, of 1,024 63, 28; 8 of 512 78, 27; 2 rows behind 500 keys 25, 19; 32 requests of 2 rows behind 500 26, 38."""
+    if "counts" not in ctx.host:
+        return True
+    key = ("grouped_wide", heads, groups, window, chunk)
+    if key not in ctx.host:
+        counts, pos0 = ctx.host["counts"], ctx.host["pos0"]
+        reach = min(window or math.inf, chunk or math.inf)
+        hpg = heads // groups
+
+        def work(rows, blocks):        # (the longest context a block reads, blocks and the keys they read to a multiprocessor)
+            tiles = -(-counts // rows)
+            keys = np.minimum(np.minimum(pos0 + (counts + rows) / 2, pos0 + counts), reach + rows)
+            return min(ctx.max_kv_len, reach + rows), float(tiles.sum()) * blocks / sms, float((tiles * keys).sum()) * blocks / sms
+
+        longest, blocks, keys = work(128 if hpg % 2 == 0 else 256, heads // 2 if hpg % 2 == 0 else heads)
+        wide = max(6.0 + 0.0226 * longest, 0.85 * (6.0 * blocks + 0.0226 * keys))
+        longest, blocks, keys = work(max(1, 64 // hpg), groups)
+        ctx.host[key] = wide < 0.95 * max(5.8 + 0.041 * longest, 2.2 * blocks + 0.031 * keys)
+    return ctx.host[key]
+
+
 def grouped_attention(q: torch.Tensor, kpages: torch.Tensor, vpages: torch.Tensor, table: torch.Tensor, ctx, heads: int,
                       key_heads: int, key_dim: int, scale: float, slopes: torch.Tensor | None = None,
                       window: int | None = None, keep_first: int = 0, gate: torch.Tensor | None = None,
                       maps: int = 1, lam: float = 0.0, post_scale: float = 1.0, eps: float = 0.0,
-                      tensor_cores: bool = True, chunk: int | None = None, sinks: torch.Tensor | None = None) -> torch.Tensor:
+                      tensor_cores: bool = True, chunk: int | None = None, sinks: torch.Tensor | None = None,
+                      wide: bool | None = None) -> torch.Tensor:
     """Softmax attention of the step's rows over the paged cache with keys and values grouped separately:
     ``heads`` query heads of ``key_dim`` read ``key_heads`` key heads (the pages' rows taken as
     [key_heads, key_dim]) and the value heads of ``vpages``; score (q . k) scale - slopes[h] (i - j); key j
@@ -991,7 +1019,8 @@ def grouped_attention(q: torch.Tensor, kpages: torch.Tensor, vpages: torch.Tenso
     head o1 - lam o2, divided by its root mean square (``eps`` under the root), times ``post_scale``; a
     gate then has one number per output head.  When every request brings one row the context is cut into parts that a
     second kernel merges (with a window that keeps no first keys, or a chunk, the parts that it can reach).  ``sinks``
-    float32 [heads]: exp(sinks[h]) more in every denominator (a key that is always seen and has no value).
+    float32 [heads]: exp(sinks[h]) more in every denominator (a key that is always seen and has no value).  ``wide``: steps with
+    portions of bfloat16 heads of 128, one map, no slopes and no kept first keys, through the tcgen05 kernel (None: where it is the faster one).
     Returns [T, heads / maps * vdim] of the pages' dtype."""
     lib = _ready()
     lib.ayk_grouped_attention_tensor_cores(ctypes.c_int(1 if tensor_cores else 0))
@@ -1010,6 +1039,16 @@ def grouped_attention(q: torch.Tensor, kpages: torch.Tensor, vpages: torch.Tenso
     out = torch.empty((T, out_heads * DV), dtype=q.dtype, device=q.device)
     if sinks is not None and _f32(sinks, "sinks").numel() != heads:
         raise KernelError("grouped_attention: one sink per query head")
+    if wide is not False and tensor_cores and ctx.max_q_len > 1 and key_dim == 128 and DV == 128 and maps == 1 and slopes is None \
+            and not keep_first and key_heads == VH and scale > 0 and q.dtype == torch.bfloat16 \
+            and (wide or _grouped_wide_pays(ctx, heads, VH, window, chunk, sm_count())) and lib.ayk_attention_wide_tc_takes(
+                ctypes.c_int(key_dim), ctypes.c_int(DV), ctypes.c_int(pages), ctypes.c_int(P), _ptr(q), _ptr(kpages), _ptr(vpages)):
+        _launch(lib.ayk_attention_wide_tc(_ptr(out), _ptr(q), _ptr(kpages), _ptr(vpages), ctypes.c_int(pages), _ptr(_i32(table, "table")),
+                                          ctypes.c_int(table.stride(0)), _ptr(ctx.req_q_start), _ptr(ctx.req_pos0), ctypes.c_int(ctx.num_requests),
+                                          ctypes.c_int(T), ctypes.c_int(heads), ctypes.c_int(VH), ctypes.c_int(P), ctypes.c_float(scale),
+                                          _ptr(sinks), ctypes.c_int(window or 0), ctypes.c_int(chunk or 0), _ptr(gate),
+                                          ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _stream()))
+        return out
     span, from_first = ctx.cache.max_len, False
     blocks = _grouped_blocks(T, heads, max(key_heads, VH), key_dim, DV, tensor_cores and q.dtype == torch.bfloat16)
     part_keys = grouped_part(span, blocks)
@@ -1719,10 +1758,11 @@ MIXED_DECODE_MIN = 1     # single-token requests in a mixed step from which they
 
 def tc_error() -> int:
     """0, or the code of the bounded wait that ran out in a tensor-core kernel
-    (1-4: matrix product, 11-17: attention, 51-58: latent attention, 61-68: per-head products)."""
+    (1-4: matrix product, 11-17: attention, 51-58: latent attention, 61-68: per-head products, 80-91: attention of wide heads)."""
     lib = library()
     return (int(lib.ayk_gemm_tc_error()) or int(lib.ayk_attention_tc_error())
-            or int(lib.ayk_gemm_tc_prefill_error()) or int(lib.ayk_latent_tc_error()) or int(lib.ayk_head_tc_error()))
+            or int(lib.ayk_gemm_tc_prefill_error()) or int(lib.ayk_latent_tc_error()) or int(lib.ayk_head_tc_error())
+            or int(lib.ayk_attention_wide_tc_error()))
 
 
 def attention(q, kcache, vcache, table, ctx, num_heads: int, scale: float,

@@ -59,3 +59,12 @@ def test_mlstm_takes_the_faster_of_its_forms_for_portions(heads, dim, vdim, plan
 def test_partitions_grow_where_short_contexts_leave_no_multiprocessor_without_a_block(monkeypatch, rows, heads, groups, tensor_cores, max_len, keys):
     monkeypatch.setattr(ops, "sm_count", lambda: SMS)
     assert ops.grouped_part(max_len, ops._grouped_blocks(rows, heads, groups, 128, 128, tensor_cores)) == keys
+
+
+@pytest.mark.parametrize("heads,groups,window,chunk,plan,tcgen05", [
+    (16, 4, None, None, [(0, 1024)] * 2, True), (16, 4, None, 512, [(0, 1024)] * 2, True), (16, 4, None, None, [(0, 128)], True),
+    (16, 4, None, None, [(0, 16)], False), (16, 4, None, None, [(500, 2)], True), (16, 4, None, None, [(500, 2)] * 32, False),
+    (8, 8, None, None, [(0, 512)] * 8, True), (32, 8, None, None, [(0, 8)] * 32, False), (16, 4, None, None, [(1900, 64)], True),
+    (12, 4, None, None, [(0, 128)] * 8, True)])
+def test_grouped_attention_takes_the_faster_of_its_forms_for_portions(heads, groups, window, chunk, plan, tcgen05):
+    assert ops._grouped_wide_pays(step(plan), heads, groups, window, chunk, SMS) is tcgen05
