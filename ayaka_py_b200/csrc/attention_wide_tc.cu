@@ -9,8 +9,8 @@
 // scales its rows' O where one of their maxima has grown.
 //
 // Keys have KC chunks of 64 numbers.  Two sources: a paged cache (pages found through the block table; positions on no page are read
-// behind the pages' end as zeros, positions behind the last row's are wiped from the values), or rows side by side (key_row: a request's first
-// row), whose third chunk, a part that all heads share, comes from pages.  F16: queries, keys, weights and values are float16
+// behind the pages' end as zeros, positions behind the last row's are wiped from the values), or rows side by side (latent_expand.cu),
+// whose third chunk, a part that all heads share, comes from pages.  F16: queries, keys, weights and values are float16
 // (the shared third chunk bfloat16 on both sides), with a factor per row and head on the scores (q_scale); else bfloat16.
 //
 // Warps 0-3: rows of tile A, 4-7: of tile B; 8: TMA; 9 and 10: MMA issue of A and of B (9: tensor memory).  One block to a multiprocessor (192 or 224 KB).  Every wait
@@ -46,13 +46,13 @@ struct WideArgs {
   const int* table;              // [R, table_stride]
   const int* req_q_start;        // [R + 1]
   const int* req_pos0;           // [R]
-  const int* key_row;            // [R] or null: keys and values lie side by side from this row on
   const float* sinks;            // [H] or null: the score of one more key without a value
   const float* gate;             // float32 rows or null: the output is multiplied by sigmoid of the row's number at h * gate_head + d * gate_col
   const float* q_scale;          // [T, H] or null: the factor of a row's scores
   int* error;
   long long gate_stride;
   int gate_head, gate_col;
+  int side_by_side;              // keys and values lie side by side, request after request (latent_expand.cu), instead of in pages
   int table_stride, num_req, H, heads_per_key, v_head0, page_shift, rows_end, window, chunk, pair_heads;
   float scale_log2;
 };
@@ -129,7 +129,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   const int end_a = (pos_a + rows_a - 1 - k_begin) / KEYS + 1;
   const int start_b = rows_b > 0 ? (first_key(pos_b) - k_begin) / KEYS : 0;
   const int end_b = rows_b > 0 ? (pos_b + rows_b - 1 - k_begin) / KEYS + 1 : 0;
-  const bool wipes = args.key_row == nullptr && (last_key - k_begin + 1) % KEYS != 0;      // the last tile holds positions behind the last row's
+  const bool wipes = !args.side_by_side && (last_key - k_begin + 1) % KEYS != 0;      // the last tile holds positions behind the last row's
   const int num_tiles = max(end_a, end_b);             // no tile is read by neither: B's first key is at most the one behind A's last
 
   if (threadIdx.x == 0) {
@@ -165,8 +165,13 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     // ---- TMA
     const int* my_table = args.table + (size_t)req * args.table_stride;
     const int box = min(KEYS, 1 << args.page_shift), boxes = KEYS / box;
-    const bool paged = args.key_row == nullptr;
-    const int k_row0 = paged ? 0 : args.key_row[req];
+    const bool paged = !args.side_by_side;
+    int k_row0 = 0;                                    // the row of key 0 (rows start at a request's first visible 64 keys)
+    if (!paged) {
+      auto from = [&](int r) { return args.window > 0 ? max(0, args.req_pos0[r] - args.window + 1) / KEYS * KEYS : 0; };
+      for (int r = lane; r < req; r += 32) k_row0 += args.req_pos0[r] - from(r) + args.req_q_start[r + 1] - args.req_q_start[r];
+      k_row0 = (int)__reduce_add_sync(0xffffffffu, (unsigned)k_row0) - from(req);
+    }
     const int kh = args.pair_heads || args.heads_per_key > 1 ? h0 / args.heads_per_key : h0;
     auto cell_of = [&](int t) {                        // lane i: where the i-th box of tile t lies in the pages
       const int k = k_begin + t * KEYS + lane * box;
@@ -470,7 +475,8 @@ int setup() {
   }
   if (!g_configured.here()) {
     cudaError_t err = cudaFuncSetAttribute(attention_wide_tc_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(2));
-    if (err != cudaSuccess) return ayk_fail("ayk_attention_wide_tc: shared memory %zu: %s", smem_bytes(2), cudaGetErrorString(err));
+    if (err == cudaSuccess) err = cudaFuncSetAttribute(attention_wide_tc_kernel<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(3));
+    if (err != cudaSuccess) return ayk_fail("ayk_attention_wide_tc: shared memory %zu: %s", smem_bytes(3), cudaGetErrorString(err));
     g_configured.here() = true;
   }
   return 0;
@@ -536,9 +542,36 @@ AYK_EXPORT int ayk_attention_wide_tc(void* out, const void* q, const void* kcach
   CUtensorMap mq, mk, mv;
   if (encode_rows(&mq, q, total_rows, H * 128, false) || encode(&mk, kcache, cells, G, 128, box, false) || encode(&mv, vcache, cells, G, 128, box, false)) return -1;
   const int pair = (H / G) % 2 == 0 ? 1 : 0, span = pair ? ROWS : 2 * ROWS;
-  WideArgs args{(__nv_bfloat16*)out, table, req_q_start, req_pos0, nullptr, sinks, gate, nullptr, g_error_dev, gate_stride, 128, 1,
+  WideArgs args{(__nv_bfloat16*)out, table, req_q_start, req_pos0, sinks, gate, nullptr, g_error_dev, gate_stride, 128, 1, 0,
                 table_stride, num_req, H, H / G, 0, shift, (int)cells, window, chunk, pair, scale * 1.4426950408889634f};
   AYK_REQUIRE(total_rows / span + num_req <= 65535, "ayk_attention_wide_tc: too many row tiles (%d rows, %d requests)", total_rows, num_req);
   ayk_launch(attention_wide_tc_kernel<2, false>, dim3(pair ? H / 2 : H, total_rows / span + num_req), dim3(THREADS), smem_bytes(2), stream, mq, mq, mk, mv, mk, args);
   return ayk_check_launch("ayk_attention_wide_tc");
+}
+
+// The expanded latent attention: out [T, H * 128] bfloat16; q16, q_rot, q_scale as latent_expand.cu makes them; kv [kv_rows, 2 H, 128] float16, keys of
+// every head and then values; rope_pages [pages, page_size, 64] bfloat16, shared by the heads.  gate: float32 rows of gate_stride, the number at
+// h * gate_head + d * gate_col, or null.
+AYK_EXPORT int ayk_attention_expanded_tc(void* out, const void* q16, const void* q_rot, const float* q_scale, const void* kv, int kv_rows, const void* rope_pages,
+                                         int pages, const int* table, int table_stride, const int* req_q_start, const int* req_pos0, int num_req,
+                                         int total_rows, int H, int page_size, float scale, int window, const float* gate, long long gate_stride,
+                                         int gate_head, int gate_col, cudaStream_t stream) {
+  if (num_req == 0 || total_rows == 0) return 0;
+  AYK_REQUIRE(page_size >= 8 && page_shift_of(page_size) >= 0 && (long long)pages * page_size < (1ll << 31) && scale > 0.f && H >= 1,
+              "ayk_attention_expanded_tc: pages of %d are not taken", page_size);
+  AYK_REQUIRE((((uintptr_t)out | (uintptr_t)q16 | (uintptr_t)q_rot | (uintptr_t)kv | (uintptr_t)rope_pages) & 15) == 0, "ayk_attention_expanded_tc: operands must be 16-byte aligned");
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (setup() != 0) return -1;
+  }
+  const int shift = page_shift_of(page_size), box = page_size < KEYS ? page_size : KEYS;
+  const long long cells = (long long)pages * page_size;
+  CUtensorMap mq, mr, mkv, ms;
+  if (encode_rows(&mq, q16, total_rows, H * 128, true) || encode_rows(&mr, q_rot, total_rows, H * 64, false) ||
+      encode(&mkv, kv, kv_rows, 2 * H, 128, KEYS, true) || encode(&ms, rope_pages, cells, 1, 64, box, false)) return -1;
+  WideArgs args{(__nv_bfloat16*)out, table, req_q_start, req_pos0, nullptr, gate, q_scale, g_error_dev, gate_stride, gate_head, gate_col, 1,
+                table_stride, num_req, H, 1, H, shift, (int)cells, window, 0, 0, scale * 1.4426950408889634f};
+  AYK_REQUIRE(total_rows / (2 * ROWS) + num_req <= 65535, "ayk_attention_expanded_tc: too many row tiles (%d rows, %d requests)", total_rows, num_req);
+  ayk_launch(attention_wide_tc_kernel<3, true>, dim3(H, total_rows / (2 * ROWS) + num_req), dim3(THREADS), smem_bytes(3), stream, mq, mr, mkv, mkv, ms, args);
+  return ayk_check_launch("ayk_attention_expanded_tc");
 }

@@ -8,6 +8,7 @@
 
 #define AYK_DTYPE_F32 0
 #define AYK_DTYPE_BF16 1
+#define AYK_DTYPE_F16 2      // keys and values of the expanded latent attention only
 
 #define AYK_ACT_NONE 0
 #define AYK_ACT_GELU_ERF 1

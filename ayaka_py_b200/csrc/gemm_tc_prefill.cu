@@ -25,6 +25,7 @@
 // the two-SM form) in the error word of the tensor-core kernels and the CTA
 // winds down.
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include <cstdlib>
 #include <mutex>
@@ -105,7 +106,16 @@ __device__ __forceinline__ long long cache_place(const PrefillArgs& a, int row) 
 // uses are compiled on their own (MODE): 0 = bfloat16 out, no activation, no residual; 1 = float32
 // out with residual; 2 = bfloat16 out with tanh-GELU; 3 = anything, decided at run time; 4 = as 0, and
 // the key and value columns go into the paged cache as well (`place`: where this row's do, or -1); 5 = bfloat16
-// out with the squared ReLU; 6 = bfloat16 out with SiLU.
+// out with the squared ReLU; 6 = bfloat16 out with SiLU; 7 = as 0 in float16.
+template <bool F16>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
+  if (F16) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 template <int W, int MODE>
 __device__ __forceinline__ void epilogue_chunk(const PrefillArgs& a, uint32_t taddr, int row, int n, bool row_ok,
                                                long long place) {
@@ -149,10 +159,7 @@ __device__ __forceinline__ void epilogue_chunk(const PrefillArgs& a, uint32_t ta
       if (out_bf16) {
         uint32_t w[4];
 #pragma unroll
-        for (int u = 0; u < 8; u += 2) {
-          __nv_bfloat162 p = __floats2bfloat162_rn(y[u], y[u + 1]);
-          w[u >> 1] = *reinterpret_cast<uint32_t*>(&p);
-        }
+        for (int u = 0; u < 8; u += 2) w[u >> 1] = pack_pair<MODE == 7>(y[u], y[u + 1]);
         *reinterpret_cast<uint4*>((__nv_bfloat16*)a.C + idx + j) = make_uint4(w[0], w[1], w[2], w[3]);
         if (MODE == 4) {
           const int off = n + j - a.kv_col0;         // kv_col0 and kv_width are multiples of 8: a piece is all key or all value
@@ -204,6 +211,7 @@ __device__ __forceinline__ void epilogue_row_any(const PrefillArgs& a, uint32_t 
   else if (a.mode == 4) epilogue_row<4>(a, taddr, row, n, cols, row_ok, place);
   else if (a.mode == 5) epilogue_row<5>(a, taddr, row, n, cols, row_ok, place);
   else if (a.mode == 6) epilogue_row<6>(a, taddr, row, n, cols, row_ok, place);
+  else if (a.mode == 7) epilogue_row<7>(a, taddr, row, n, cols, row_ok, place);
   else epilogue_row<3>(a, taddr, row, n, cols, row_ok, place);
 }
 
@@ -282,8 +290,7 @@ __device__ __forceinline__ void finish_split_cols(const PrefillArgs& a, uint32_t
       uint32_t w[4];
 #pragma unroll
       for (int u = 0; u < 8; u += 2) {
-        __nv_bfloat162 pr = __floats2bfloat162_rn(y[u], y[u + 1]);
-        w[u >> 1] = *reinterpret_cast<uint32_t*>(&pr);
+        w[u >> 1] = a.mode == 7 ? pack_pair<true>(y[u], y[u + 1]) : pack_pair<false>(y[u], y[u + 1]);
       }
       *reinterpret_cast<uint4*>((__nv_bfloat16*)a.C + idx) = make_uint4(w[0], w[1], w[2], w[3]);
       if (a.mode == 4) {
@@ -1125,10 +1132,12 @@ int prefill_product(void* C, const void* X, const void* W, const float* bias, co
   AYK_REQUIRE(K >= 8 && K % 8 == 0, "ayk_gemm_tc_prefill: K = %d must be a positive multiple of 8", K);
   AYK_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0) && ((uintptr_t)C % 16 == 0) &&
               (residual == nullptr || (uintptr_t)residual % 16 == 0), "ayk_gemm_tc_prefill: operands must be 16-byte aligned");
-  AYK_REQUIRE(out_dtype == AYK_DTYPE_F32 || out_dtype == AYK_DTYPE_BF16, "ayk_gemm_tc_prefill: unknown output dtype %d", out_dtype);
+  AYK_REQUIRE(out_dtype == AYK_DTYPE_F32 || out_dtype == AYK_DTYPE_BF16 || out_dtype == AYK_DTYPE_F16, "ayk_gemm_tc_prefill: unknown output dtype %d", out_dtype);
+  AYK_REQUIRE(out_dtype != AYK_DTYPE_F16 || (act == AYK_ACT_NONE && !bias && !residual && N % 8 == 0 && pair <= 0),
+              "ayk_gemm_tc_prefill: float16 out takes a plain product with rows of whole 16-byte pieces");
   AYK_REQUIRE(sms >= 1, "ayk_gemm_tc_prefill: sms must be positive");
   static const int pair_default = getenv("AYAKA_B200_GEMM_PAIR") ? atoi(getenv("AYAKA_B200_GEMM_PAIR")) : 0;
-  const bool use_pair = pair > 0 || (pair < 0 && pair_default && M > BM && sms >= 2);
+  const bool use_pair = out_dtype != AYK_DTYPE_F16 && (pair > 0 || (pair < 0 && pair_default && M > BM && sms >= 2));
   if (use_pair) {
     AYK_REQUIRE(M > 8 && sms >= 2, "ayk_gemm_tc_prefill: pairs of SMs need more than 8 rows and 2 SMs (got %d, %d)", M, sms);
     const int BN = tile_n > 0 ? tile_n : ayk_gemm_tc_pair_tile(M, N, sms);
@@ -1210,10 +1219,10 @@ int prefill_product(void* C, const void* X, const void* W, const float* bias, co
   }
   PrefillArgs args{};
   args.C = C; args.bias = bias; args.residual = residual; args.error = g_error_dev;
-  args.M = M; args.N = N; args.K = K; args.act = act; args.out_bf16 = out_dtype == AYK_DTYPE_BF16;
+  args.M = M; args.N = N; args.K = K; args.act = act; args.out_bf16 = out_dtype != AYK_DTYPE_F32;
   args.BN = BN;
   args.vec_ok = (N % 8 == 0) && (bias == nullptr || (uintptr_t)bias % 16 == 0);
-  args.mode = epilogue_mode(act, residual != nullptr, args.out_bf16);
+  args.mode = out_dtype == AYK_DTYPE_F16 ? 7 : epilogue_mode(act, residual != nullptr, args.out_bf16);
   if (take_cache_target(args, kv) != 0) return -1;
   args.box_m = box_m;
   args.m_tiles = (M + BM - 1) / BM;

@@ -18,7 +18,7 @@ import torch
 
 from .csrc import build as _build
 
-F32, BF16 = 0, 1
+F32, BF16, F16 = 0, 1, 2
 _DTYPE_TAG = {torch.float32: F32, torch.bfloat16: BF16}
 ACTIVATIONS = {"none": 0, "gelu_erf": 1, "gelu_tanh": 2, "quick_gelu": 3, "relu2": 4, "silu": 5}
 
@@ -534,15 +534,8 @@ def _latent_tiles(ctx, rows: int, window: int | None) -> tuple[int, float, float
     return ctx.host[key]
 
 
-def _latent_tc_pays(ctx, heads: int, rank: int, rot: int, window: int | None, sms: int) -> bool:
-    """Whether the tcgen05 form of the latent attention is the faster one for a step that brings more than one row of some
-    request.  It takes 128 pairs to a tile (and with a latent beyond 256 two blocks to each) where the mma.sync form takes
-    64, starts later and has fewer blocks to a multiprocessor, but passes a tile of keys in half the time.  The estimates
-    (us: a block's start, its time per 32 keys, blocks that a multiprocessor works off side by side, what the last ones add)
-    are fitted to 27 steps x 26 shapes (64 to 512 + 0 or 64, 2 to 200 heads; contexts of 64 to 2,048; short portions, many
-    single rows beside one).  Of the 702 the choice is more than 3 % slower than mma.sync in 3, by 11 % at most (128 heads,
-    latent 64), and on average 0.6 % behind the better of the two.  Measured, mma.sync and tcgen05, 16 heads, 512 + 64: one
-    prompt of 32 rows 13.6, 18.9; of 128 27.6, 25.9; 2 x 1,024 rows 316, 205; 100 single rows of 100 keys beside 64 rows 36, 58."""
+def _latent_times(ctx, heads: int, rank: int, rot: int, window: int | None, sms: int) -> tuple[float, float]:
+    """Estimated times (us) of the latent attention of a step, tcgen05 and mma.sync form (see ``_latent_tc_pays``)."""
     def time(base, start, step, at_once, tail, tiles, keys, longest):
         one = start + step * longest
         return base + max(one, (start * tiles + step * keys) / (sms * at_once) + (tail * one if tiles > sms * at_once else 0.0))
@@ -553,13 +546,24 @@ def _latent_tc_pays(ctx, heads: int, rank: int, rot: int, window: int | None, sm
         blocks = -(-heads // group) * halves
         return tiles * blocks, keys * blocks, longest
 
+    if rank > 256:
+        return time(0.0, 14.8, 2.4, 0.87, 0.46, *work(128, 2)), time(0.0, 2.8, 5.7, 0.9, 0.29, *work(64, 1))
+    step = 2.3 + 0.22 * (rank // 64) if rot == 0 else 1.7 + 0.3 * (rank // 64)
+    return time(2.8, 8.9, step, 1.1, 0.5, *work(128, 1)), time(1.5, 2.7, 1.5 + 0.73 * ((rank + rot) // 64), 1.7, 0.5, *work(64, 1))
+
+
+def _latent_tc_pays(ctx, heads: int, rank: int, rot: int, window: int | None, sms: int) -> bool:
+    """Whether the tcgen05 form of the latent attention is the faster one for a step that brings more than one row of some
+    request.  It takes 128 pairs to a tile (and with a latent beyond 256 two blocks to each) where the mma.sync form takes
+    64, starts later and has fewer blocks to a multiprocessor, but passes a tile of keys in half the time.  The estimates
+    (us: a block's start, its time per 32 keys, blocks that a multiprocessor works off side by side, what the last ones add)
+    are fitted to 27 steps x 26 shapes (64 to 512 + 0 or 64, 2 to 200 heads; contexts of 64 to 2,048; short portions, many
+    single rows beside one).  Of the 702 the choice is more than 3 % slower than mma.sync in 3, by 11 % at most (128 heads,
+    latent 64), and on average 0.6 % behind the better of the two.  Measured, mma.sync and tcgen05, 16 heads, 512 + 64: one
+    prompt of 32 rows 13.6, 18.9; of 128 27.6, 25.9; 2 x 1,024 rows 316, 205; 100 single rows of 100 keys beside 64 rows 36, 58."""
     if "counts" not in ctx.host:
         return True
-    if rank > 256:
-        return time(0.0, 14.8, 2.4, 0.87, 0.46, *work(128, 2)) < 0.97 * time(0.0, 2.8, 5.7, 0.9, 0.29, *work(64, 1))
-    step = 2.3 + 0.22 * (rank // 64) if rot == 0 else 1.7 + 0.3 * (rank // 64)
-    ours = time(2.8, 8.9, step, 1.1, 0.5, *work(128, 1))
-    theirs = time(1.5, 2.7, 1.5 + 0.73 * ((rank + rot) // 64), 1.7, 0.5, *work(64, 1))
+    ours, theirs = _latent_times(ctx, heads, rank, rot, window, sms)
     if rank <= 128:                    # as fast per tile without a rotated part, hardly faster with one
         return rot > 0 and ctx.max_kv_len > 128 and ours < 0.9 * theirs
     return ours < 0.97 * theirs
@@ -622,6 +626,82 @@ def latent_attention(query: torch.Tensor, latent_pages: torch.Tensor, rope_pages
                                      ctypes.c_int(ctx.num_requests), ctypes.c_int(T), ctypes.c_int(H), ctypes.c_int(rank),
                                      ctypes.c_int(rot), ctypes.c_int(latent_pages.shape[1]), ctypes.c_float(scale),
                                      ctypes.c_int(window or 0), ctypes.c_int(_tag(latent_pages.dtype)), _stream()))
+    return out
+
+
+def _latent_expanded_rows(ctx, window: int | None) -> int:
+    """Tokens whose keys and values the expanded latent attention of a step makes: every request's from the first visible 64 on."""
+    counts, pos0 = ctx.host["counts"], ctx.host["pos0"]
+    first = 0 if window is None else np.maximum(pos0 - window + 1, 0) // 64 * 64
+    return int((pos0 + counts - first).sum())
+
+
+LATENT_EXPANDED_BYTES = 256 << 20         # at most this much for a step's expanded keys and values
+
+
+def latent_expanded_pays(ctx, heads: int, rank: int, window: int | None, pages: torch.Tensor, sms: int) -> bool:
+    """Whether the latent attention (rotated part 64, heads of 128) of a step that brings more than one row of some request takes the form
+    with expanded keys and values.  That form takes one product over the tokens that the rows see and a fifth to a third of the attention's;
+    the other one makes two products per head of the rows alone.  The estimate (us that the expanded form is ahead) is fitted
+    to 631 steps (latent 512; 8, 16 and 32 heads; 1 to 64 requests of 2 to 1,024 rows behind 0 to 1,900 tokens, with and without a window):
+    the choice is on average 0.3 % behind the faster form, more than 5 % in 7 of them (many requests of a few rows behind long contexts).
+    Measured, the layer at 16 heads: 2 x 1,024 rows 317, 108; 2 x 1,024 behind 1,900 tokens 811, 165; 2 x 2 34.6, 25.8;
+    24 x 8 behind 500 95, 118; 64 x 2 behind 500 97, 150."""
+    P = pages.shape[1]
+    if ctx.max_q_len == 1 or "counts" not in ctx.host or P < 8 or P & (P - 1) or pages.shape[0] * P >= 1 << 31:
+        return False
+    key = ("latent_expanded", heads, rank, window)
+    if key not in ctx.host:
+        held = _latent_expanded_rows(ctx, window)
+        counts, pos0 = ctx.host["counts"], ctx.host["pos0"]
+        reach = math.inf if window is None else window + 256
+        tiles = -(-counts // 256)
+        keys = np.minimum(np.minimum(pos0 + (counts + 256) / 2, pos0 + counts), reach)
+        attention = max(6.0 + 0.024 * min(ctx.max_kv_len, reach), 0.8 * heads / sms * float((tiles * (6.0 + 0.024 * keys)).sum()))
+        ahead = 16.2 + min(_latent_times(ctx, heads, rank, 64, window, sms)) - attention - (0.62 * ctx.num_rows + 0.147 * held) * heads / 1000.0
+        ctx.host[key] = held * heads * 512 <= LATENT_EXPANDED_BYTES and ahead > 4.0
+    return ctx.host[key]
+
+
+def latent_expanded(proj: torch.Tensor, latent_pages: torch.Tensor, rope_pages: torch.Tensor, up_weight: torch.Tensor, norm_weight: torch.Tensor,
+                    freq: torch.Tensor, gain: float, rot_dims: int, ctx, table: torch.Tensor, heads: int, eps: float, halves: bool, scale: float,
+                    window: int | None, gate: torch.Tensor | None) -> torch.Tensor:
+    """The latent attention of a step's rows with keys and values expanded (``csrc/latent_expand.cu``): float32 projection rows
+    [q (heads x (128 + 64)) | down (rank + 64) | ...], the normed latents and rotated key parts go into their pages, ``up_weight``
+    [2 heads * 128, rank] makes keys (the first half) and values of every token that the rows see, in float16; returns the
+    heads' outputs [T, heads * 128] in the pages' dtype, times sigmoid(gate) (float32 [T, heads] or [T, heads * 128])."""
+    lib = _ready()
+    _f32(proj, "proj"); _f32(freq, "freq"); _f32(norm_weight, "norm_weight")
+    T, rank, P, pages = proj.shape[0], latent_pages.shape[-1], latent_pages.shape[1], latent_pages.shape[0]
+    if (latent_pages.dtype != torch.bfloat16 or rope_pages.dtype != torch.bfloat16 or up_weight.dtype != torch.bfloat16 or not up_weight.is_contiguous()
+            or up_weight.shape != (2 * heads * 128, rank) or rope_pages.shape[-1] != 64 or proj.shape[1] < heads * 192 + rank + 64 or proj.stride(1) != 1):
+        raise KernelError("latent_expanded: projection rows, weights or pages do not fit")
+    if gate is not None and (gate.dtype != torch.float32 or gate.shape not in ((T, heads), (T, heads * 128)) or gate.stride(1) != 1):
+        raise KernelError("latent_expanded: gate must be float32 [T, heads] or [T, heads * 128]")
+    held = _latent_expanded_rows(ctx, window)
+    dev = proj.device
+    q16 = torch.empty((T, heads, 128), dtype=torch.float16, device=dev)
+    q_rot = torch.empty((T, heads, 64), dtype=torch.bfloat16, device=dev)
+    q_scale = torch.empty((T, heads), dtype=torch.float32, device=dev)
+    side = torch.empty((held, rank), dtype=torch.bfloat16, device=dev)
+    kv = torch.empty((held, 2 * heads * 128), dtype=torch.float16, device=dev)
+    out = torch.empty((T, heads * 128), dtype=torch.bfloat16, device=dev)
+    table_ptr, stride, window_ = _ptr(_i32(table, "table")), ctypes.c_int(table.stride(0)), ctypes.c_int(window or 0)
+    starts, pos0, requests = _ptr(ctx.req_q_start), _ptr(ctx.req_pos0), ctypes.c_int(ctx.num_requests)
+    _launch(lib.ayk_latent_expand_prepare(_ptr(latent_pages), _ptr(rope_pages), _ptr(q16), _ptr(q_rot), _ptr(q_scale), _ptr(side), _ptr(proj),
+                                          ctypes.c_longlong(proj.stride(0)), _ptr(norm_weight), _ptr(freq), ctypes.c_float(gain),
+                                          ctypes.c_int(rot_dims), ctypes.c_int(1 if halves else 0), _ptr(ctx.row_req), _ptr(ctx.positions),
+                                          table_ptr, stride, ctypes.c_int(P), starts, pos0, requests, ctypes.c_int(T), ctypes.c_int(held - T),
+                                          ctypes.c_int(heads), ctypes.c_int(rank), ctypes.c_float(eps), window_, _stream()))
+    _launch(lib.ayk_gemm_tc_prefill(_ptr(kv), _ptr(side), _ptr(up_weight), None, None, ctypes.c_int(held), ctypes.c_int(2 * heads * 128),
+                                    ctypes.c_int(rank), ctypes.c_int(ACTIVATIONS["none"]), ctypes.c_int(F16), ctypes.c_int(0),
+                                    ctypes.c_int(sm_count()), ctypes.c_int(-1), _stream()))
+    gate_head, gate_col = (0, 0) if gate is None else (1, 0) if gate.shape[1] == heads else (128, 1)
+    _launch(lib.ayk_attention_expanded_tc(_ptr(out), _ptr(q16), _ptr(q_rot), _ptr(q_scale), _ptr(kv), ctypes.c_int(held), _ptr(rope_pages),
+                                          ctypes.c_int(pages), table_ptr, stride, starts, pos0, requests, ctypes.c_int(T), ctypes.c_int(heads),
+                                          ctypes.c_int(P), ctypes.c_float(scale), window_, _ptr(gate),
+                                          ctypes.c_longlong(gate.stride(0) if gate is not None else 0), ctypes.c_int(gate_head),
+                                          ctypes.c_int(gate_col), _stream()))
     return out
 
 

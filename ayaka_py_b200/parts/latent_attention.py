@@ -21,7 +21,8 @@ Only c and the rotated key part are cached (the cache manager's pages: "keys" ho
 the rotated part, "values" the latent, one head each).  The kernels never expand
 keys or values: with q' = U_k^T q_n the score is q' . c + q_r . k_r, and
 sum_j p_j U_v c_j = U_v sum_j p_j c_j, so attention runs over the cached pairs and
-U_v is applied once per row (``csrc/latent.cu``)."""
+U_v is applied once per row (``csrc/latent.cu``).  Except where a step's rows are many for the tokens they read: then one
+product makes the step's keys and values from the latents, and the rows attend to those (``ops.latent_expanded``)."""
 
 from __future__ import annotations
 
@@ -56,7 +57,7 @@ class LatentAttention(Mixer):
         self.rotary = None if rot is None else make_part(
             PartSpec("rotary", {"dims": rot["dims"], "base": rot["base"], "scaling": rot.get("scaling"),
                                 "layout": rot.get("layout", "interleaved")}), dtype, device)
-        self.no_freq = None
+        self.no_freq = self.up_weight = None
         self.q_width = heads * (dim + rot_dim)
         self.down_width = kv_rank + rot_dim if own_latent else 0
         self.in_weight = self.down_norm = None
@@ -88,6 +89,14 @@ class LatentAttention(Mixer):
             at += rows
         self.in_weight = fused
         self.uk_heads = self.uk_weight.view(H, self.dim, self.rank).transpose(1, 2).contiguous()      # [H, rank, dim]
+        if self.dtype == torch.bfloat16 and self.own_latent and (self.dim, self.rot_dim, self.vdim) == (128, 64, 128) and self.rank % 8 == 0 \
+                and self.scale > 0:
+            # keys over values for ``ops.latent_expanded``, whose keys and values are float16: a latent is at most sqrt(rank) times its
+            # norm's largest weight long, so no number of theirs can be larger than that times the longest row
+            up = torch.cat([self.uk_weight, self.uv_weight])
+            longest = float(up.float().norm(dim=1).max()) * float(self.down_norm.abs().max()) * self.rank ** 0.5
+            if longest < 30000.0:
+                self.up_weight, self.uk_weight, self.uv_weight = up, up[:H * self.dim], up[H * self.dim:]
         self.uv_heads = self.uv_weight.view(H, self.vdim, self.rank)                                   # [H, vdim, rank]
 
     def cache_need(self):
@@ -107,13 +116,17 @@ class LatentAttention(Mixer):
             freq, gain, rot_dims, halves = self.no_freq, 1.0, 0, False
         else:
             freq, gain, rot_dims, halves = self.rotary.freq, self.rotary.gain, self.rotary.dims, self.rotary.halves
+        first = self.q_width + self.down_width
+        gate = proj[:, first:first + self.gate_width] if self.gate_width else None
+        if self.up_weight is not None and ops.latent_expanded_pays(ctx, H, self.rank, self.window, latent_pages, ops.sm_count()):
+            o = ops.latent_expanded(proj, latent_pages, rope_pages, self.up_weight, self.down_norm, freq, gain, rot_dims, ctx, table, H, self.eps,
+                                    halves, self.scale, self.window, gate)
+            return ops.linear(o, self.out_weight, None, residual=residual, out_dtype=torch.float32, out=residual)
         query = ops.latent_prepare(proj, latent_pages, rope_pages, self.down_norm, freq, gain, rot_dims, ctx, table, H,
                                    self.dim, self.rot_dim, self.rank, self.eps, cache.writes, halves)
         q_plain = proj[:, :self.q_width].view(T, H, self.dim + self.rot_dim)[:, :, :self.dim]
         ops.head_matmul(q_plain, self.uk_heads, query[:, :, :self.rank])
         mixed = ops.latent_attention(query, latent_pages, rope_pages, table, ctx, self.scale, window=self.window)
-        first = self.q_width + self.down_width
-        gate = proj[:, first:first + self.gate_width] if self.gate_width else None
         o = torch.empty((T, H, self.vdim), dtype=self.dtype, device=h.device)
         ops.head_matmul(mixed, self.uv_heads, o, gate=gate)
         return ops.linear(o.view(T, H * self.vdim), self.out_weight, None, residual=residual,

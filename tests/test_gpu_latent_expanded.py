@@ -1,0 +1,91 @@
+"""The latent attention with keys and values expanded against the same in 64 bits, beside the form that never expands them."""
+
+import math
+from types import SimpleNamespace
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from test_gpu_vedadra import context_for, step_of        # noqa: E402
+
+RANK, ROT, DIM = 256, 64, 128
+
+
+def reference(x, w, H, rot, window, gate, start_rows):
+    """float64 rows of a whole sequence x [n, width]; the rows from start_rows on are returned."""
+    n = x.shape[0]
+    x = x.double()
+    q = (x @ w["q_weight"].double().T).view(n, H, DIM + ROT)
+    down = x @ w["down_weight"].double().T
+    c, kr = down[:, :RANK], down[:, None, RANK:]
+    c = c / torch.sqrt((c * c).mean(-1, keepdim=True) + 1e-6) * w["down_norm"].double()
+    freq = rot["base"] ** (-2.0 * torch.arange(rot["dims"] // 2, dtype=torch.float64, device=x.device) / rot["dims"])
+    angle = torch.arange(n, dtype=torch.float64, device=x.device)[:, None] * freq
+
+    def turn(v):
+        co, si = torch.cos(angle)[:, None], torch.sin(angle)[:, None]
+        out, d = v.clone(), rot["dims"]
+        a, b = (slice(0, d // 2), slice(d // 2, d)) if rot["layout"] == "halves" else (slice(0, d, 2), slice(1, d, 2))
+        out[..., a], out[..., b] = v[..., a] * co - v[..., b] * si, v[..., b] * co + v[..., a] * si
+        return out
+
+    qr, kr = turn(q[..., DIM:]), turn(kr)[:, 0]
+    k = torch.einsum("nr,hdr->nhd", c, w["uk_weight"].double().view(H, DIM, RANK))
+    v = torch.einsum("nr,hdr->nhd", c, w["uv_weight"].double().view(H, DIM, RANK))
+    i, j = torch.arange(n, device=x.device)[:, None], torch.arange(n, device=x.device)[None]
+    seen = (j <= i) & (i - j < (window or n + 1))
+    out = torch.empty(n, H, DIM, dtype=torch.float64, device=x.device)
+    for h in range(H):
+        s = ((q[:, h, :DIM] @ k[:, h].T + qr[:, h] @ kr.T) * (DIM + ROT) ** -0.5).masked_fill(~seen, -math.inf)
+        out[:, h] = torch.softmax(s, dim=1) @ v[:, h]
+    if gate:
+        g = torch.sigmoid(x @ w["gate_weight"].double().T)
+        out = out * (g[:, :, None] if gate == "head" else g.view(n, H, DIM))
+    return (out.reshape(n, H * DIM) @ w["out_weight"].double().T)[start_rows:]
+
+
+@pytest.mark.parametrize("H,page,window,gate,layout,dims,gain", [
+    (2, 16, None, None, "halves", 64, 1.0), (5, 8, 70, "head", "interleaved", 64, 1.0), (1, 64, None, "element", "halves", 32, 1.0),
+    (3, 128, 200, None, "interleaved", 16, 1.0),
+    (2, 16, None, None, "halves", 64, 3e4)])                # queries far beyond float16's range
+@pytest.mark.parametrize("before,brings", [([0], [2]), ([0], [65]), ([3, 300], [129, 257]), ([63, 64, 200], [1, 66, 2]), ([510], [5])])
+def test_expanded_keys_and_values(monkeypatch, H, page, window, gate, layout, dims, gain, before, brings):
+    from ayaka_py_b200 import ops
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts.latent_attention import LatentAttention
+    torch.manual_seed(H + page)
+    width = 256
+    rot = {"base": 50000.0, "dims": dims, "layout": layout}
+    part = LatentAttention(width, H, DIM, ROT, DIM, RANK, (DIM + ROT) ** -0.5, 1e-6, rot, gate=gate, window=window, dtype=torch.bfloat16)
+    w = {name: (torch.randn(d.shape, device="cuda") / d.shape[-1] ** 0.5).to(torch.bfloat16) if len(d.shape) == 2 else 1 + 0.1 * torch.randn(d.shape, device="cuda")
+         for name, d in part.tensors().items()}
+    w["q_weight"] *= gain
+    part.bind(w)
+    assert part.up_weight is not None
+    cache, runner = context_for([CacheGroupSpec("g", part.cache_need(), 1)], "bfloat16", max_requests=4, page_size=page,
+                                pages=sum(-(-(a + b) // page) for a, b in zip(before, brings)) + 2)
+    binding = SimpleNamespace(group=0, layer=0, writes=True)
+    rows = {i: torch.randn(a + b, width, device="cuda").to(torch.bfloat16) for i, (a, b) in enumerate(zip(before, brings))}
+    monkeypatch.setattr(ops, "latent_expanded_pays", lambda *a: False)
+    for i, n in enumerate(before):
+        cache.open(i)
+        if n:
+            ctx, res = step_of(cache, runner, {i: n})
+            part.forward(rows[i][:n], None, ctx, binding)
+            cache.commit(res)
+    ctx, res = step_of(cache, runner, dict(enumerate(brings)))
+    plan = sorted(range(len(brings)), key=lambda i: brings[i] != 1)       # a step's single rows come first
+    x = torch.cat([rows[i][before[i]:] for i in plan])
+    want = torch.cat([reference(rows[i], w, H, rot, window, gate, before[i]) for i in plan])
+    errors = []
+    for expanded in (False, True):
+        monkeypatch.setattr(ops, "latent_expanded_pays", lambda *a, e=expanded: e)
+        got = part.forward(x, None, ctx, binding).double()
+        assert torch.isfinite(got).all() and ops.tc_error() == 0
+        errors.append(float((got - want).norm() / want.norm()))
+    # bfloat16 products around the attention: 3e-3 on both sides; a far larger spread of the scores makes every rounding count for more
+    assert errors[1] < (8e-3 if gain == 1.0 else 0.2), errors
+    assert errors[1] < 1.2 * errors[0] + 1e-3, errors
+    cache.rollback(res)

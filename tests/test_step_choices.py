@@ -68,3 +68,14 @@ def test_partitions_grow_where_short_contexts_leave_no_multiprocessor_without_a_
     (12, 4, None, None, [(0, 128)] * 8, True)])
 def test_grouped_attention_takes_the_faster_of_its_forms_for_portions(heads, groups, window, chunk, plan, tcgen05):
     assert ops._grouped_wide_pays(step(plan), heads, groups, window, chunk, SMS) is tcgen05
+
+
+@pytest.mark.parametrize("heads,window,plan,expanded", [
+    (16, None, [(0, 1024), (0, 777)], True), (16, None, [(0, 2)] * 2, True), (16, None, [(1900, 2)] * 2, True), (16, 512, [(1900, 300)], True),
+    (16, None, [(500, 8)] * 24, False), (16, None, [(500, 2)] * 64, False), (32, None, [(500, 2)] * 24, False), (8, None, [(0, 130)] * 8, True),
+    (16, None, [(500, 1)] * 64 + [(0, 512)], False), (16, None, [(40000, 512)], False), (16, None, [(500, 1)] * 4, False)])
+def test_latent_attention_expands_keys_and_values_where_that_is_the_faster_form(heads, window, plan, expanded):
+    """The last but one needs more scratch memory than is given; the last is a decode step."""
+    pages = SimpleNamespace(shape=(4000, 16, 1, 512))
+    assert ops.latent_expanded_pays(step(plan), heads, 512, window, pages, SMS) is expanded
+    assert not ops.latent_expanded_pays(step(plan), heads, 512, window, SimpleNamespace(shape=(4000, 12, 1, 512)), SMS)
