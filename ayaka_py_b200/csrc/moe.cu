@@ -249,6 +249,7 @@ moe_plan_padded_kernel(int* __restrict__ row_of_pair, int* __restrict__ w_rows1,
         ++n;
       }
     }
+    w_rows1[max_tiles] = w_rows2[max_tiles] = min(n, max_tiles);       // tiles that hold rows: the products stop there
     for (; n < max_tiles; ++n) { w_rows1[n] = 0; w_rows2[n] = 0; }
   }
   __syncthreads();

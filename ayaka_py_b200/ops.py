@@ -1490,7 +1490,8 @@ def moe_experts_tc(h: torch.Tensor, in_weight: torch.Tensor, down_weight: torch.
     128-row tile against the matrix of its expert.  in_weight [experts, 2 inner, width] gate over up (or, with
     ``activation``, [experts, inner, width] and that activation in the first product's epilogue),
     down_weight [experts, width, inner].  ``weigh_input`` (with a gate): the pair's weight multiplies both halves of the
-    first product ahead of the activation.  Returns (float32 rows [padded, width], row of every pair)."""
+    first product ahead of the activation, which its epilogue makes.  Returns (float32 rows [padded, width], row of every pair); the
+    padded rows behind the last tile that holds any are not written."""
     lib = _ready()
     if weigh_input and activation is not None:
         raise KernelError("moe_experts_tc: weights in front of the activation take experts with a gate")
@@ -1502,7 +1503,7 @@ def moe_experts_tc(h: torch.Tensor, in_weight: torch.Tensor, down_weight: torch.
     max_tiles = pairs // pad + E
     dev_ = h.device
     row_of_pair = torch.empty((pairs,), dtype=torch.int32, device=dev_)
-    w_rows = torch.empty((2, max_tiles), dtype=torch.int32, device=dev_)
+    w_rows = torch.empty((2, max_tiles + 1), dtype=torch.int32, device=dev_)         # the last: how many tiles hold rows
     gathered = torch.empty((max_tiles * pad, d), dtype=torch.bfloat16, device=dev_)
     row_scale = torch.empty((max_tiles * pad,), dtype=torch.float32, device=dev_) if weigh_input else None
     _launch(lib.ayk_moe_plan_padded(_ptr(row_of_pair), _ptr(w_rows[0]), _ptr(w_rows[1]), _ptr(gathered), _ptr(row_scale),
@@ -1511,16 +1512,18 @@ def moe_experts_tc(h: torch.Tensor, in_weight: torch.Tensor, down_weight: torch.
                                     ctypes.c_int(d), ctypes.c_int(n1), ctypes.c_int(d), ctypes.c_int(max_tiles), _stream()))
     global launches
     launches += 1
-    both = torch.empty((max_tiles * pad, n1), dtype=torch.bfloat16, device=dev_)
-    _launch(lib.ayk_gemm_tc_prefill_grouped(_ptr(both), _ptr(gathered), _ptr(in_weight), _ptr(w_rows[0]), ctypes.c_int(max_tiles * pad),
-                                            ctypes.c_int(n1), ctypes.c_int(d), ctypes.c_int(E * n1),
-                                            ctypes.c_int(ACTIVATIONS[activation or "none"]), ctypes.c_int(BF16),
-                                            ctypes.c_int(sm_count()), _stream()))
-    hidden = both if activation is not None else glu_limited(both, inner, limit, slope, torch.bfloat16, plus, row_scale)
+    rows, sms = ctypes.c_int(max_tiles * pad), ctypes.c_int(sm_count())
+    expected = ctypes.c_int(min(max_tiles, max(min(E, pairs), pairs // pad + E // 2)) * pad)       # half a tile an expert lies empty, a whole one holds few rows
+    hidden = torch.empty((max_tiles * pad, inner), dtype=torch.bfloat16, device=dev_)
+    gated = activation is None
+    _launch(lib.ayk_gemm_tc_prefill_grouped(_ptr(hidden), _ptr(gathered), _ptr(in_weight), _ptr(w_rows[0]), rows, ctypes.c_int(inner), ctypes.c_int(d),
+                                            ctypes.c_int(E * n1), expected, ctypes.c_int(ACTIVATIONS[activation or "none"]), ctypes.c_int(BF16),
+                                            ctypes.c_int(1 if gated else 0), ctypes.c_float(limit), ctypes.c_float(slope), ctypes.c_float(plus),
+                                            _ptr(row_scale), sms, _stream()))
     picked = torch.empty((max_tiles * pad, d), dtype=torch.float32, device=dev_)
-    _launch(lib.ayk_gemm_tc_prefill_grouped(_ptr(picked), _ptr(hidden), _ptr(down_weight), _ptr(w_rows[1]), ctypes.c_int(max_tiles * pad),
-                                            ctypes.c_int(d), ctypes.c_int(inner), ctypes.c_int(E * d), ctypes.c_int(ACTIVATIONS["none"]),
-                                            ctypes.c_int(F32), ctypes.c_int(sm_count()), _stream()))
+    _launch(lib.ayk_gemm_tc_prefill_grouped(_ptr(picked), _ptr(hidden), _ptr(down_weight), _ptr(w_rows[1]), rows, ctypes.c_int(d), ctypes.c_int(inner),
+                                            ctypes.c_int(E * d), expected, ctypes.c_int(ACTIVATIONS["none"]), ctypes.c_int(F32), ctypes.c_int(0),
+                                            ctypes.c_float(0.0), ctypes.c_float(0.0), ctypes.c_float(0.0), None, sms, _stream()))
     return picked, row_of_pair
 
 
