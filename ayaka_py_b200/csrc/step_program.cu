@@ -200,6 +200,7 @@ AYK_EXPORT int ayk_program_run(const AykOp* ops, int n_ops, const AykBuffer* buf
               offset, step->workspace_bytes);
   auto at = [&](int id) -> uint8_t* {
     if (id == AYK_BUFFER_LOGITS) return (uint8_t*)step->logits;
+    if (id == AYK_BUFFER_STREAM) return (uint8_t*)step->stream;
     if (id < 0 || id >= n_buffers) return nullptr;
     return address[id];
   };
@@ -233,7 +234,7 @@ AYK_EXPORT int ayk_program_run(const AykOp* ops, int n_ops, const AykBuffer* buf
           kvp = &kv;
         }
         ++count;
-        rc = ayk_linear(at(op.out), at(op.in), op.p[0], (const float*)op.p[1], op.in2 >= 0 ? (const float*)at(op.in2) : nullptr,
+        rc = ayk_linear(at(op.out), at(op.in), op.p[0], (const float*)op.p[1], op.in2 != -1 ? (const float*)at(op.in2) : nullptr,
                         M, op.i[0], op.i[1], op.i[2], op.i[3], op.i[4], kvp, &filed, stream);
         if (op.i[6]) filed_flags[op.i[12] & 1023] = filed;
         break;

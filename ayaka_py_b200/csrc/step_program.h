@@ -13,6 +13,7 @@
 #define AYK_ROWS_WANTED 1     // ... over the S rows whose logits are wanted
 
 #define AYK_BUFFER_LOGITS (-2)    // the step's output, given by the caller
+#define AYK_BUFFER_STREAM (-3)    // the residual stream of a program of one block, given by the caller
 #define AYK_MAX_BUFFERS 64
 #define AYK_MAX_GROUPS 8
 
@@ -41,6 +42,7 @@ struct AykStep {
   void* logits;
   float* decode_scratch;
   long long decode_scratch_floats;
+  void* stream;
 };
 
 // Where the key and value columns of a fused q | k | v projection belong in the paged cache.

@@ -10,6 +10,8 @@ their order are those of ``Model.forward``; only the interpreter is out of the l
 (about 13 us per launch from Python against 2 us from native code, which is what
 bounds prompt and mixed steps of small models).
 
+A block of such parts called by itself (``BlockProgram``) runs the same way, over the caller's stream.
+
 A part without ``lower`` (a toy part of a test, an attention with a position encoding
 that turns queries and keys on the host's side) keeps the whole model on
 ``Model.forward``; nothing else changes for it.  ``AYAKA_B200_NATIVE_STEP=0`` does the
@@ -28,7 +30,7 @@ from ..parts.base import KVNeed, NotLowered
 
 OP_EMBED, OP_LAYERNORM, OP_LINEAR, OP_ATTENTION = 0, 1, 2, 3
 ROWS_ALL, ROWS_WANTED = 0, 1
-LOGITS = -2
+LOGITS, STREAM = -2, -3
 MAX_BUFFERS, MAX_GROUPS = 64, 8
 
 
@@ -49,11 +51,11 @@ class _Step(ctypes.Structure):
                 ("want_rows", ctypes.c_void_p), ("req_q_start", ctypes.c_void_p), ("req_pos0", ctypes.c_void_p),
                 ("tables", ctypes.c_void_p * MAX_GROUPS), ("table_stride", ctypes.c_int32 * MAX_GROUPS),
                 ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_longlong), ("logits", ctypes.c_void_p),
-                ("decode_scratch", ctypes.c_void_p), ("decode_scratch_floats", ctypes.c_longlong)]
+                ("decode_scratch", ctypes.c_void_p), ("decode_scratch_floats", ctypes.c_longlong), ("stream", ctypes.c_void_p)]
 
 
 def _bytes(dtype: torch.dtype) -> int:
-    return torch.empty((), dtype=dtype).element_size()
+    return dtype.itemsize
 
 
 class ProgramBuilder:
@@ -96,10 +98,8 @@ class ProgramBuilder:
     def _op(self, kind: int, src: int, src2: int, out: int, ints=(), floats=(), ptrs=()) -> None:
         op = _Op()
         op.kind, op.src, op.src2, op.out = kind, src, src2, out
-        for n, v in enumerate(ints):
-            op.i[n] = int(v)
-        for n, v in enumerate(floats):
-            op.f[n] = float(v)
+        op.i[:len(ints)] = ints
+        op.f[:len(floats)] = floats
         for n, v in enumerate(ptrs):
             op.p[n] = v or None
         self.ops.append(op)
@@ -215,10 +215,57 @@ class StepProgram:
         return logits
 
 
+def native_allowed(device) -> bool:
+    return os.environ.get("AYAKA_B200_NATIVE_STEP", "1") != "0" and str(device).startswith("cuda")
+
+
+class BlockProgram:
+    """The operations of one block over the caller's residual stream, for a caller that runs a layer by itself.  Nothing of a call is
+    kept: the workspace is the call's own, so calls on several streams and threads do not meet."""
+
+    def __init__(self, block, caches: dict, cache, dtype: torch.dtype):
+        builder = ProgramBuilder(cache, dtype)
+        if block.lower(builder, STREAM, caches) != STREAM:
+            raise NotLowered("the block does not keep its stream in place")
+        self.lib = ops._ready()
+        self.n_ops, self.row_bytes = len(builder.ops), [b for _, b in builder.buffers]
+        self.ops = (_Op * self.n_ops)(*builder.ops)
+        self.buffers = (_Buffer * max(1, len(builder.buffers)))(*[_Buffer(k, b) for k, b in builder.buffers])
+        self.keep, self.floats = builder.keep, builder.decode_floats_per_request
+        # the tensors that the operations were recorded with, as the parts hold them: a part that is given others needs a new program
+        self.bound = [(part, name.replace(".", "_"), getattr(part, name.replace(".", "_"))) for part in block.parts.values() for name in part.tensors()]
+
+    def current(self) -> bool:
+        return all(getattr(part, name) is tensor for part, name, tensor in self.bound)
+
+    def run(self, x: torch.Tensor, ctx) -> torch.Tensor:
+        T, cache, step = ctx.num_rows, ctx.cache, _Step()
+        if x.shape[0] != T:
+            raise ops.KernelError(f"a stream of {x.shape[0]} rows in a step of {T}")
+        workspace = torch.empty(sum((T * b + 255) // 256 * 256 for b in self.row_bytes) or 256, dtype=torch.uint8, device=x.device)
+        step.T, step.R, step.num_single, step.max_q_len = T, ctx.num_requests, ctx.num_single, ctx.max_q_len
+        step.max_context, step.settled = cache.max_len, 1 if ctx.earlier_rows_settled else 0
+        step.positions, step.row_req = ctx.positions.data_ptr(), ctx.row_req.data_ptr()
+        step.req_q_start, step.req_pos0 = ctx.req_q_start.data_ptr(), ctx.req_pos0.data_ptr()
+        for g, table in enumerate(ctx.tables[:MAX_GROUPS]):
+            if table is not None:
+                step.tables[g], step.table_stride[g] = table.data_ptr(), table.stride(0)
+        step.workspace, step.workspace_bytes, step.stream = workspace.data_ptr(), workspace.numel(), x.data_ptr()
+        if self.floats:
+            scratch = ops._decode_buffer(x.device, ctx.num_requests * self.floats * -(-cache.max_len // ops.DECODE_PART))
+            step.decode_scratch, step.decode_scratch_floats = scratch.data_ptr(), scratch.numel()
+        launched = ctypes.c_int(0)
+        code = self.lib.ayk_program_run(self.ops, self.n_ops, self.buffers, len(self.row_bytes), ctypes.byref(step), ctypes.byref(launched),
+                                        ops._stream())
+        ops.launches += launched.value
+        ops._check(code)
+        return x
+
+
 def lower_model(model, cache) -> StepProgram | None:
     """The model's step as a program, or None when a part of it cannot be lowered (then
     ``Model.forward`` runs the step) or AYAKA_B200_NATIVE_STEP=0 asks for the Python path."""
-    if os.environ.get("AYAKA_B200_NATIVE_STEP", "1") == "0" or not str(model.device).startswith("cuda"):
+    if not native_allowed(model.device):
         return None
     builder = ProgramBuilder(cache, model.dtype)
     try:
