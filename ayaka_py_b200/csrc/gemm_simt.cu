@@ -14,23 +14,25 @@ namespace {
 constexpr int BM = 64, BN = 64, BK = 16;
 
 // ---------------------------------------------------------------- float32 --
-// A tile of TM x 64 outputs; the block's 256 threads are four groups of 64, and of every slab of 32 k each group takes
-// its own eight, so that a tile keeps eight warps busy whatever its height: a group's thread holds TM / 8 x 8 sums and
-// reads, for four k at a time, TM / 8 + 8 float4 from shared memory for 32 * (TM / 8) products.  Slabs arrive by
-// cp.async, three ahead.  At the end the four groups' sums meet in shared memory and are added in one order,
-// (0 + 1) + (2 + 3), the same for every TM: the height is chosen by the row count, a row's result is not.
+// A tile of TM x 64 outputs: of every slab of 32 k each of the block's eight warps takes its own four, so that a tile keeps
+// eight warps busy whatever its height.  A thread holds TM / 4 x 8 sums and reads TM / 4 + 8 float4 from shared memory for
+// 32 * (TM / 4) products.  Slabs arrive by cp.async, three ahead; the next is asked for behind the first of a slab's products.
+// At the end the eight warps' sums meet in shared memory and are added in one order, ((0 + 1) + (2 + 3)) + ((4 + 5) + (6 + 7)),
+// the same for every TM: the height is chosen by the row count, a row's result is not.
 //
-// Bound by the FP32 pipes (128 FMA a clock and multiprocessor) and, per tile, by how many multiprocessors have one.  The
-// height is the one whose fullest multiprocessor has the least to do (f32_rows).  Measured for 377 rows, alone and cold
-// (us; before: 64-row tiles, slabs of 16 without copies ahead, 4 x 4 sums a thread): N 2304 K 768 71 -> 57, N 768 K 768
-// 56 -> 29, N 3072 K 768 74 -> 66, N 768 K 3072 207 -> 90; a GPT-2 small layer of 1 row 293 -> 139, of 130 rows 428 -> 286.  With the
-// copies' addresses worked out once and the groups' sums free of bank conflicts: the layer over 377 ragged rows 276 -> 236, over
-// 130 rows 197 -> 157.
-constexpr int FN = 64, FK = 32, FLD = FK + 4, FSTAGES = 4, FGROUPS = 4;      // rows of 36 floats: eight neighbours' 16-byte pieces lie on different banks
-constexpr int FSUM = FN + 8;             // floats per row of the groups' sums: a warp's four rows of eight lie on different banks
+// Bound by the FP32 pipes (128 FMA a clock and multiprocessor) and by what shared memory hands out, 128 bytes a clock: a
+// thread's 8 x 8 sums need four clocks for each of 16 float4 where the products need 64; and, per tile, by how many
+// multiprocessors have one.  Four groups of two warps and tiles of up to 64 rows gave a thread of 32 rows 4 x 8 sums, 12 float4
+// for 128 products.  Measured, weights cold, in a row (us; before, now): K 768, N 2304: 1 row 12.5, 9.9; 32 rows 13.1, 10.4;
+// 300 rows 49.8, 40.8; 377 rows 53.9, 40.8; 600 rows 74.9, 65.0; 1,200 rows 120, 125; N 3072: 377 rows 49.2, 52.4; 600 rows
+// 93.4, 88.6; K 3072, N 768: 1 row 42.5, 30.7; 130 rows 47.1, 36.5; 377 rows 62.0, 55.5; 1,200 rows 183, 187.  Tried beside it:
+// 16 x 8 sums a thread in tiles of 64 rows, one block to a multiprocessor (2,048 rows, N 4096, K 1024: 496 against 450);
+// fma.rn.f32x2 on pairs of k, which takes twice the registers and so 4 x 8 sums (526); slabs of 64 (526).
+constexpr int FN = 64, FK = 32, FLD = FK + 4, FSTAGES = 4, FWARPS = 8;       // rows of 36 floats: eight neighbours' 16-byte pieces lie on different banks
+constexpr int FSUM = FN + 8;             // floats per row of the warps' sums: a warp's four rows of eight lie on different banks
 constexpr int f32_stage_floats(int tm) { return (tm + FN) * FLD; }
 constexpr size_t f32_smem(int tm) {
-  const size_t ring = (size_t)FSTAGES * f32_stage_floats(tm), sums = (size_t)FGROUPS * tm * FSUM;
+  const size_t ring = (size_t)FSTAGES * f32_stage_floats(tm), sums = (size_t)FWARPS * tm * FSUM;
   return (ring > sums ? ring : sums) * sizeof(float);
 }
 
@@ -46,10 +48,10 @@ __global__ void __launch_bounds__(256, 2)
 gemm_f32_kernel(float* C, const float* A, const float* __restrict__ W, const float* __restrict__ bias,
                 const float* residual,               // C and residual may be one buffer (the residual stream in place)
                 int M, int N, int K, int act) {
-  constexpr int RM = TM / 8;
+  constexpr int RM = TM / 4;
   extern __shared__ __align__(16) float f32_tiles[];
   if (gridDim.x * gridDim.y <= AYK_FEW_BLOCKS) pdl_trigger();
-  const int tid = threadIdx.x, group = tid >> 6, tn = tid & 7, tm = (tid >> 3) & 7;
+  const int tid = threadIdx.x, warp = tid >> 5, tn = tid & 7, tm = (tid >> 3) & 3;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * FN;
   const int slabs = (K + FK - 1) / FK;
   // One slab into buffer b; rows past the matrices' ends and k past K are zeros.  In 16-byte pieces a thread always brings
@@ -101,35 +103,34 @@ gemm_f32_kernel(float* C, const float* A, const float* __restrict__ W, const flo
   for (int slab = 0; slab < slabs; ++slab) {
     asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
     __syncthreads();                                 // this slab is there for everybody; the one before has been read
-    if (slab + FSTAGES - 1 < slabs) fetch(slab + FSTAGES - 1, (slab + FSTAGES - 1) % FSTAGES);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const float* as = f32_tiles + (slab % FSTAGES) * f32_stage_floats(TM) + tm * FLD + group * 8;
-    const float* ws = f32_tiles + (slab % FSTAGES) * f32_stage_floats(TM) + (TM + tn) * FLD + group * 8;
+    const float* as = f32_tiles + (slab % FSTAGES) * f32_stage_floats(TM) + tm * FLD + warp * 4;
+    const float* ws = f32_tiles + (slab % FSTAGES) * f32_stage_floats(TM) + (TM + tn) * FLD + warp * 4;
+    float4 a[RM];
 #pragma unroll
-    for (int k = 0; k < 8; k += 4) {
-      float4 a[RM];
+    for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * 4 * FLD);
 #pragma unroll
-      for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * 8 * FLD + k);
+    for (int j = 0; j < 8; ++j) {
+      const float4 w = *reinterpret_cast<const float4*>(ws + j * 8 * FLD);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 w = *reinterpret_cast<const float4*>(ws + j * 8 * FLD + k);
-#pragma unroll
-        for (int i = 0; i < RM; ++i) {
-          acc[i][j] = fmaf(a[i].x, w.x, acc[i][j]);
-          acc[i][j] = fmaf(a[i].y, w.y, acc[i][j]);
-          acc[i][j] = fmaf(a[i].z, w.z, acc[i][j]);
-          acc[i][j] = fmaf(a[i].w, w.w, acc[i][j]);
-        }
+      for (int i = 0; i < RM; ++i) {
+        acc[i][j] = fmaf(a[i].x, w.x, acc[i][j]);
+        acc[i][j] = fmaf(a[i].y, w.y, acc[i][j]);
+        acc[i][j] = fmaf(a[i].z, w.z, acc[i][j]);
+        acc[i][j] = fmaf(a[i].w, w.w, acc[i][j]);
+      }
+      if (j == 0) {
+        if (slab + FSTAGES - 1 < slabs) fetch(slab + FSTAGES - 1, (slab + FSTAGES - 1) % FSTAGES);
+        asm volatile("cp.async.commit_group;" ::: "memory");
       }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();                                   // the ring is free for the sums
-  float* mine = f32_tiles + group * TM * FSUM;
+  float* mine = f32_tiles + warp * TM * FSUM;
 #pragma unroll
   for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) mine[(tm + 8 * i) * FSUM + tn + 8 * j] = acc[i][j];
+    for (int j = 0; j < 8; ++j) mine[(tm + 4 * i) * FSUM + tn + 8 * j] = acc[i][j];
   __syncthreads();
   const int col = tid & (FN - 1), n = n0 + col;
   if (n >= N) return;
@@ -139,7 +140,8 @@ gemm_f32_kernel(float* C, const float* A, const float* __restrict__ W, const flo
     const int m = m0 + r;
     if (m >= M) break;
     const float* at = f32_tiles + r * FSUM + col;
-    float v = ((at[0] + at[TM * FSUM]) + (at[2 * TM * FSUM] + at[3 * TM * FSUM])) + b;
+    auto sum = [&](int g) { return at[g * TM * FSUM]; };
+    float v = (((sum(0) + sum(1)) + (sum(2) + sum(3))) + ((sum(4) + sum(5)) + (sum(6) + sum(7)))) + b;
     v = apply_activation(v, act);
     if (residual) v += residual[(size_t)m * N + n];
     C[(size_t)m * N + n] = v;
@@ -148,13 +150,14 @@ gemm_f32_kernel(float* C, const float* A, const float* __restrict__ W, const flo
 
 // Rows per tile: the least work on the fullest multiprocessor, a multiprocessor taking whole tiles one after the other
 // (two at a time do not make it faster: the pipes are the bound).  Lower tiles read more of shared memory per product and
-// pay the same for a slab's barrier, which is what the factors say.
+// pay the same for a slab's barrier, which is what the factors say: 377 rows, K 768, N 3072 by tiles of 32, 16 and 8 rows take
+// 52, 63 and 90 us; 130 rows, N 2304 (180, 324 and 612 tiles) 26.8, 25.8 and 31.2; 32 rows 16.4, 12.3 and 10.4.
 int f32_rows(int M, int N, int sms) {
-  const int heights[4] = {64, 32, 16, 8};
-  const double factor[4] = {1.0, 1.2, 1.6, 2.6};
-  int best = 64;
+  const int heights[3] = {32, 16, 8};
+  const double factor[3] = {1.0, 1.25, 1.9};
+  int best = 32;
   double least = -1.0;
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 3; ++i) {
     const long tiles = (long)((M + heights[i] - 1) / heights[i]) * ((N + FN - 1) / FN);
     const double work = (double)((tiles + sms - 1) / sms) * heights[i] * factor[i];
     if (least < 0 || work < least) { least = work; best = heights[i]; }
@@ -172,10 +175,14 @@ int launch_f32(float* C, const float* A, const float* W, const float* bias, cons
     if (err != cudaSuccess) return ayk_fail("ayk_gemm_simt: shared memory %zu: %s", f32_smem(TM), cudaGetErrorString(err));
     done = true;
   }
-  dim3 grid((N + FN - 1) / FN, (M + TM - 1) / TM);
-  AYK_REQUIRE(grid.y <= 65535, "ayk_gemm_simt: M = %d exceeds %d rows", M, 65535 * TM);
-  ayk_launch_as(grid.x * grid.y <= AYK_FEW_BLOCKS, gemm_f32_kernel<TM, VEC>, grid, dim3(256), f32_smem(TM), stream, C, A, W, bias, residual,
-                M, N, K, act);
+  constexpr int MOST = 65535 * TM;                   // rows of one launch
+  for (int m = 0;; m += MOST) {
+    const int rows = M - m < MOST ? M - m : MOST;
+    dim3 grid((N + FN - 1) / FN, (rows + TM - 1) / TM);
+    ayk_launch_as(grid.x * grid.y <= AYK_FEW_BLOCKS, gemm_f32_kernel<TM, VEC>, grid, dim3(256), f32_smem(TM), stream, C + (size_t)m * N,
+                  A + (size_t)m * K, W, bias, residual ? residual + (size_t)m * N : nullptr, rows, N, K, act);
+    if (M - m <= MOST) break;
+  }
   return ayk_check_launch("ayk_gemm_simt");
 }
 
@@ -183,7 +190,6 @@ template <bool VEC>
 int launch_f32_rows(float* C, const float* A, const float* W, const float* bias, const float* residual, int M, int N, int K, int act,
                     cudaStream_t stream) {
   switch (f32_rows(M, N, ayk_sm_count())) {
-    case 64: return launch_f32<64, VEC>(C, A, W, bias, residual, M, N, K, act, stream);
     case 32: return launch_f32<32, VEC>(C, A, W, bias, residual, M, N, K, act, stream);
     case 16: return launch_f32<16, VEC>(C, A, W, bias, residual, M, N, K, act, stream);
     default: return launch_f32<8, VEC>(C, A, W, bias, residual, M, N, K, act, stream);

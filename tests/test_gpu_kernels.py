@@ -158,6 +158,21 @@ def test_gemm_simt_float32_tiles(M, N, K):
     assert torch.equal(last, out[M - 1:])
 
 
+@pytest.mark.parametrize("K", [1, 4, 28, 29, 32, 36, 127, 128, 132])
+@pytest.mark.parametrize("M,N", [(8, 2400), (31, 4800), (33, 200), (1200, 576)])          # tiles of 8, 16, 8 and 32 rows
+def test_gemm_simt_float32_warps_of_four_k(M, N, K):
+    """Ends of k within a warp's four and within a slab: a sum is off by at most a rounding per term of its warp (K / 8 of
+    them and its last slab's), three more for the warps' sums, 2^-24 each; two rows have the bits that they have alone."""
+    from ayaka_py_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    a, w = torch.randn(M, K, generator=gen, device="cuda"), torch.randn(N, K, generator=gen, device="cuda")
+    out = ops.gemm_simt(a, w)
+    bound = (K / 8 + 8) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    assert bool(((out.double() - a.double() @ w.double().T).abs() <= bound).all())
+    for i in (0, M - 1):
+        assert torch.equal(ops.gemm_simt(a[i:i + 1].contiguous(), w), out[i:i + 1])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("case", ATTENTION_CASES)
 def test_append_then_attention(dtype, case):
