@@ -68,13 +68,6 @@ __device__ __forceinline__ uint32_t pack(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Most waits find their barrier complete: one poll inline, the rest out of line.  (The code of the softmax warps and of the issuing thread
-// share the instruction caches; every expansion of a wait's loops was fetched anew each time.)
-__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity, int* error, int code) { return mbar_wait(bar, parity, error, code); }
-__device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity, int* error, int code) {
-  return mbar_try(bar, parity) || wait_on(bar, parity, error, code);
-}
-
 template <int KC, bool F16>
 __global__ void __launch_bounds__(THREADS, 1)
 attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q2, const __grid_constant__ CUtensorMap map_k,
@@ -181,7 +174,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     auto arm = [&](uint32_t full, uint32_t empty, int use, uint32_t bytes) -> bool {      // the use-th copy into this place
       bool fine = true;
       if (lane == 0) {
-        if (use > 0) fine = wait_for(empty, (uint32_t)(use - 1) & 1u, args.error, 81);
+        if (use > 0) fine = mbar_wait_short(empty, (uint32_t)(use - 1) & 1u, args.error, 81);
         if (fine) mbar_expect_tx(full, bytes);
       }
       return __shfl_sync(0xffffffffu, fine ? 1 : 0, 0) != 0;
@@ -244,7 +237,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (ok && wipes) {
       // positions behind the last row's are nobody's yet: what their places hold enters P V times zero, so it has to be finite
       const int t = num_tiles - 1, live = last_key - (k_begin + t * KEYS) + 1;
-      if (lane == 0) ok = wait_for(v_full + 8 * (t % ST), (uint32_t)(t / ST) & 1u, args.error, 85);
+      if (lane == 0) ok = mbar_wait_short(v_full + 8 * (t % ST), (uint32_t)(t / ST) & 1u, args.error, 85);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       uint8_t* at = smem_raw + (v_tile - base) + (uint32_t)(t % ST) * 2 * K_CHUNK;
       for (int i = lane; ok && i < 2 * (KEYS - live) * 8; i += 32) {
@@ -256,9 +249,9 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       if (ok && lane == 0) mbar_arrive(wiped);
     }
     if (!ok && lane == 0) {                            // nobody may be consuming any more: wait for the copies in flight
-      for (int x = 0; x < q_tiles; ++x) wait_for(q_full + 8 * x, 0u, args.error, 82);
-      for (int t = max(0, k_issued - ST); t < k_issued; ++t) wait_for(k_full + 8 * (t % ST), (uint32_t)(t / ST) & 1u, args.error, 82);
-      for (int t = max(0, v_issued - ST); t < v_issued; ++t) wait_for(v_full + 8 * (t % ST), (uint32_t)(t / ST) & 1u, args.error, 82);
+      for (int x = 0; x < q_tiles; ++x) mbar_wait_short(q_full + 8 * x, 0u, args.error, 82);
+      for (int t = max(0, k_issued - ST); t < k_issued; ++t) mbar_wait_short(k_full + 8 * (t % ST), (uint32_t)(t / ST) & 1u, args.error, 82);
+      for (int t = max(0, v_issued - ST); t < v_issued; ++t) mbar_wait_short(v_full + 8 * (t % ST), (uint32_t)(t / ST) & 1u, args.error, 82);
     }
     __syncwarp();
   } else if (warp > SOFT_WARPS) {
@@ -275,7 +268,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (elect_one()) {
       bool ok = true;
       auto wait = [&](uint32_t bar, int use, int code) {
-        if (ok) ok = wait_for(bar, (uint32_t)use & 1u, args.error, code);
+        if (ok) ok = mbar_wait_short(bar, (uint32_t)use & 1u, args.error, code);
       };
       const uint64_t da = make_desc(q_tile + x * KC * CHUNK);
       int k_st = 0, k_use = 0, v_st = 0, v_use = 0;    // the next tile's places, and how often they have been used
@@ -347,7 +340,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     for (int t = start; t < end; ++t) {
       const int local = t - start, k0 = k_begin + t * KEYS, buffer = 2 * x + (local & 1);
       const uint32_t s_at = s_first + 64u * (local & 1);
-      if (lane == 0) ok = wait_for(s_full + 8 * buffer, (uint32_t)(local >> 1) & 1u, args.error, 89);
+      if (lane == 0) ok = mbar_wait_short(s_full + 8 * buffer, (uint32_t)(local >> 1) & 1u, args.error, 89);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       tc_fence_after();
@@ -383,7 +376,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       // the barrier is waited for, also where no maximum has grown: a wait two phases ahead would be answered at once.  Four more warps
       // that scale O for the softmax warps were no faster: P V, the scaling and the next P V follow one another either way.)
       if (local > 0) {
-        if (lane == 0) ok = wait_for(pv_done + 8 * x, (uint32_t)(local - 1) & 1u, args.error, 91);
+        if (lane == 0) ok = mbar_wait_short(pv_done + 8 * x, (uint32_t)(local - 1) & 1u, args.error, 91);
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         if (!ok) break;
         if (grown) {
@@ -405,7 +398,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       if (lane == 0) mbar_arrive(p_full + 8 * buffer);
     }
     if (ok && end > start) {
-      if (lane == 0) ok = wait_for(pv_done + 8 * x, (uint32_t)(end - start - 1) & 1u, args.error, 90);
+      if (lane == 0) ok = mbar_wait_short(pv_done + 8 * x, (uint32_t)(end - start - 1) & 1u, args.error, 90);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (ok) {
         tc_fence_after();

@@ -442,49 +442,54 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       }
       bool ok = true;
       int issued = pre;
-      int s = pre == STAGES ? 0 : pre;              // the stage of iteration `pre`
+      const uint32_t bars_end = full_bar(STAGES);
+      uint32_t bar = full_bar(pre == STAGES ? 0 : pre), dst = tiles + (pre == STAGES ? 0u : pre * STAGE_BYTES);      // the stage of iteration `pre`
       uint32_t wait_parity = 0;                     // the first refill of a stage waits for its first release
       for (int it = pre; it < total_it; ++it) {
-        ok = mbar_wait(empty_bar(s), wait_parity, args.error, 21);
+        ok = mbar_wait_short(bar + (empty_bar(0) - full_bar(0)), wait_parity, args.error, 21);
         if (!ok) break;
-        mbar_expect_tx(full_bar(s), TX_BYTES);
-        const uint32_t dst = tiles + s * STAGE_BYTES;
-        bring_weights(dst + A_BYTES, cx.kx, cx.n0, full_bar(s));
-        tma_load_2d(dst, &map_x, cx.kx, cx.m0, full_bar(s));
+        mbar_expect_tx(bar, TX_BYTES);
+        bring_weights(dst + A_BYTES, cx.kx, cx.n0, bar);
+        tma_load_2d(dst, &map_x, cx.kx, cx.m0, bar);
         advance(cx);
         issued = it + 1;
-        if (++s == STAGES) { s = 0; wait_parity ^= 1u; }
+        bar += 8u;
+        dst += STAGE_BYTES;
+        if (bar == bars_end) { bar = full_bar(0); dst = tiles; wait_parity ^= 1u; }
       }
       if (!ok) {
         for (int j = max(0, issued - STAGES); j < issued; ++j)
-          mbar_wait(full_bar(j % STAGES), (uint32_t)(j / STAGES) & 1u, args.error, 22);
+          mbar_wait_short(full_bar(j % STAGES), (uint32_t)(j / STAGES) & 1u, args.error, 22);
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     if (elect_one()) {
       bool ok = true;
-      int s = 0;
+      const uint32_t bars_end = full_bar(STAGES);
+      const uint64_t da_first = make_desc(tiles), db_first = make_desc(tiles + A_BYTES);
+      uint32_t bar = full_bar(0), at = 0;           // this K block's stage: its barrier, and its 16-byte units from the first stage's on
       uint32_t full_parity = 0;
       for (int t = 0; t < my_tiles && ok; ++t) {
         const int b = t & 1;
         if (t >= 2) {
-          ok = mbar_wait(tmem_empty(b), (uint32_t)((t >> 1) & 1) ^ 1u, args.error, 23);
+          ok = mbar_wait_short(tmem_empty(b), (uint32_t)((t >> 1) & 1) ^ 1u, args.error, 23);
           if (!ok) break;
           tc_fence_after();
         }
         const uint32_t acc = tmem_base + (uint32_t)b * 256u;
         for (int kb = 0; kb < my_kb && ok; ++kb) {
-          ok = mbar_wait(full_bar(s), full_parity, args.error, 24);
+          ok = mbar_wait_short(bar, full_parity, args.error, 24);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a_src = tiles + s * STAGE_BYTES;
-          const uint64_t da0 = make_desc(a_src), db0 = make_desc(a_src + A_BYTES);
+          const uint64_t da0 = da_first + at, db0 = db_first + at;
 #pragma unroll
           for (int k = 0; k < BLOCK_K / 16; ++k)     // 32 bytes further along K: two 16-byte units of the address field
             umma(acc, da0 + (uint64_t)(2 * k), db0 + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit(empty_bar(s));
-          if (++s == STAGES) { s = 0; full_parity ^= 1u; }
+          umma_commit(bar + (empty_bar(0) - full_bar(0)));
+          bar += 8u;
+          at += STAGE_BYTES >> 4;
+          if (bar == bars_end) { bar = full_bar(0); at = 0; full_parity ^= 1u; }
         }
         umma_commit(tmem_full(b));
       }
@@ -505,7 +510,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       const int b = t & 1;
       const int tile = blockIdx.x + t * gridDim.x;
       const int m0 = (tile / args.n_tiles) * BM + quarter * 32, nh = (tile % args.n_tiles) * BN + half * half_cols;
-      if (lane == 0) ok = mbar_wait(tmem_full(b), (uint32_t)(t >> 1) & 1u, args.error, 25);
+      if (lane == 0) ok = mbar_wait_short(tmem_full(b), (uint32_t)(t >> 1) & 1u, args.error, 25);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       tc_fence_after();
@@ -573,7 +578,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
           tma_load_2d(stage0 + c * STAGED_CHUNK, &map_r, nh + 32 * c, m0, res_full(half, c));
         }
       }
-      if (lane == 0) ok = mbar_wait(tmem_full(b), (uint32_t)(t >> 1) & 1u, args.error, 25);
+      if (lane == 0) ok = mbar_wait_short(tmem_full(b), (uint32_t)(t >> 1) & 1u, args.error, 25);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       tc_fence_after();
@@ -582,7 +587,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         const int buf = nbuf == 2 ? (c & 1) : 0;
         uint32_t r[32];
         tmem_ld32(taddr + 32 * c, r);
-        if (lane == 0) ok = mbar_wait(res_full(half, buf), fills[buf] & 1u, args.error, 27);
+        if (lane == 0) ok = mbar_wait_short(res_full(half, buf), fills[buf] & 1u, args.error, 27);
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         ++fills[buf];
         tmem_ld_wait();
@@ -633,7 +638,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       const int m0 = (tile / args.n_tiles) * BM, n0 = (tile % args.n_tiles) * BN;
       const long long place = cache_place(args, m0 + quarter * 32 + lane);   // three dependent loads: under the main loop
       // One lane per warp watches the barrier; 256 threads polling it slow the producer and MMA warps down.
-      if (lane == 0) ok = mbar_wait(tmem_full(b), (uint32_t)(t >> 1) & 1u, args.error, 25);
+      if (lane == 0) ok = mbar_wait_short(tmem_full(b), (uint32_t)(t >> 1) & 1u, args.error, 25);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       tc_fence_after();
@@ -661,7 +666,7 @@ gemm_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     const int row_in_tile = quarter * 32 + lane;
     bool ok = my_tiles == 1;
     if (warp >= 2 && ok) {
-      if (lane == 0) ok = mbar_wait(tmem_full(0), 0u, args.error, 25);
+      if (lane == 0) ok = mbar_wait_short(tmem_full(0), 0u, args.error, 25);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       tc_fence_after();
     }
@@ -979,7 +984,8 @@ bool split_fits(int tiles, int num_kb, int splits, int sms, int bn) {
 }
 
 double kblock_us(int a_rows, int bn, int active);              // the model of the product's time, below
-double whole_tiles_us(int M, int N, int K, int bn, int sms, bool wide_rows);
+double whole_tiles_us(int M, int N, int K, int bn, int sms, int wide_rows);
+double wide_kblock_us(int a_rows, int bn, int active, double stream);
 
 // Does splitting K beat whole tiles going round the CTAs, and with which tile width and how many parts?
 // Times from the model above; the two cluster barriers, the exchange of the sums through shared memory and
@@ -988,7 +994,7 @@ double whole_tiles_us(int M, int N, int K, int bn, int sms, bool wide_rows);
 // rows, residual 0.7 us rms; with a split taken where it is modelled 10 % ahead, the choice is within 1.4 % of the
 // best measured form in 46 of 48 cases and 4.3 % behind at worst).
 constexpr double SPLIT_FIX_US = 0.0, SPLIT_FIX_PER_COL = 0.016, SPLIT_FIX_PER_CTA = 0.35, SPLIT_MARGIN = 0.90;
-bool split_pays(int M, int N, int K, int sms, int tile_n, bool wide_rows, int* bn_out, int* splits_out) {
+bool split_pays(int M, int N, int K, int sms, int tile_n, int wide_rows, int* bn_out, int* splits_out) {
   const int m_tiles = (M + BM - 1) / BM, num_kb = (K + BLOCK_K - 1) / BLOCK_K;
   if (N % 8 != 0) return false;
   double best_whole = -1.0;
@@ -1003,12 +1009,14 @@ bool split_pays(int M, int N, int K, int sms, int tile_n, bool wide_rows, int* b
     const long tiles = (long)m_tiles * ((N + bn - 1) / bn);
     for (int sp = 2; sp <= 8; sp *= 2) {
       if (!split_fits((int)tiles, num_kb, sp, sms, bn)) continue;
-      const double us = 3.4 + (double)((num_kb + sp - 1) / sp) * kblock_us(M >= BM ? BM : (M + 7) / 8 * 8, bn, (int)tiles * sp) +
-                        SPLIT_FIX_US + SPLIT_FIX_PER_COL * bn + SPLIT_FIX_PER_CTA * sp;
+      const int a_rows = M >= BM ? BM : (M + 7) / 8 * 8, part = (num_kb + sp - 1) / sp;
+      const double us = wide_rows ? 4.55 + (double)part * wide_kblock_us(a_rows, bn, (int)tiles * sp, 20.4) + 0.0287 * bn
+                                  : 3.4 + (double)part * kblock_us(a_rows, bn, (int)tiles * sp) + SPLIT_FIX_US + SPLIT_FIX_PER_COL * bn +
+                                        SPLIT_FIX_PER_CTA * sp;
       if (best_split < 0 || us < best_split) { best_split = us; *bn_out = bn; *splits_out = sp; }
     }
   }
-  return best_split > 0 && best_split < SPLIT_MARGIN * best_whole;
+  return best_split > 0 && best_split < (wide_rows ? 1.0 : SPLIT_MARGIN) * best_whole;
 }
 
 // rows x n float32, row-major; box of 128 rows x 32 columns (128 bytes), 128-byte swizzle: a chunk of the
@@ -1065,28 +1073,45 @@ double kblock_us(int a_rows, int bn, int active) {
   const double stream_us = (double)(a_rows + bn) * 128.0 * active / 18.0e6;
   return floor_us > stream_us ? floor_us : stream_us;
 }
-double whole_tiles_us(int M, int N, int K, int bn, int sms, bool wide_rows) {
+// The same for products with 32-bit rows out, fitted apart (1: over a residual, 2: without): 140 products of 1,024 ... 8,224 features,
+// K 512 ... 8,192, 130 ... 2,048 rows, each at every width, whole and split by 2, 4 and 8 where that fits.  A K block takes the larger
+// of 0.188 us (1.9 ns a column less 0.083 us from 143 columns on) and its operand bytes over 17.6 TB/s, 20.4 where K is split; a launch 2.7 us, and 4.6 us with
+// 28.7 ns a column where the sums of a split meet; the last epilogue 19.4 ns a column staged, 42.3 ns over a residual that is not, 26.5 ns
+// without one.  The choice is 0.4 % behind the best measured one on average (14 % at worst: 1,400 rows, K 8,192); with the constants of the
+// 16-bit rows, which see too little in the staged form and too little cost in a split, it was 9.3 % behind (49 % at worst): 576 rows, N 1280,
+// K 1280 10.3 us split in two, 7.9 whole; 1,024 rows, N 1600, K 1600 16.1, 10.7; 1,801 rows, N 1024, K 4096 25.5, 19.0.
+double wide_kblock_us(int a_rows, int bn, int active, double stream) {
+  double us = (double)(a_rows + bn) * 128.0 * active / (stream * 1.0e6);
+  if (us < 0.188) us = 0.188;
+  const double by_columns = 0.0019 * bn - 0.083;
+  return us > by_columns ? us : by_columns;
+}
+double whole_tiles_us(int M, int N, int K, int bn, int sms, int wide_rows) {
   const int m_tiles = (M + BM - 1) / BM, num_kb = (K + BLOCK_K - 1) / BLOCK_K;
   const int a_rows = M >= BM ? BM : (M + 7) / 8 * 8;
   const long tiles = (long)m_tiles * ((N + bn - 1) / bn);
   const long full = tiles / sms, rest = tiles % sms;
-  // 32-bit rows cost the epilogue 26 ns more per column unless they go through the staged form (widths 64, 128, 192)
-  const bool staged = wide_rows && bn % 64 == 0 && bn <= 192 && M >= BM;
-  double t = 3.4 + (double)full * num_kb * kblock_us(a_rows, bn, sms) + (wide_rows && !staged ? 0.0418 : 0.0158) * bn;
+  if (wide_rows) {
+    const bool staged = wide_rows == 1 && bn % 64 == 0 && M >= BM;
+    double t = 2.72 + (double)full * num_kb * wide_kblock_us(a_rows, bn, sms, 17.6) + (staged ? 0.0194 : (wide_rows == 1 ? 0.0423 : 0.0265)) * bn;
+    if (rest) t += (double)num_kb * wide_kblock_us(a_rows, bn, (int)rest, 17.6);
+    return t;
+  }
+  double t = 3.4 + (double)full * num_kb * kblock_us(a_rows, bn, sms) + 0.0158 * bn;
   if (rest) t += (double)num_kb * kblock_us(a_rows, bn, (int)rest);
   return t;
 }
 }  // namespace
 
 // The tile width (out features per tile) with the shortest modelled time on `sms` SMs.
-// wide_rows: the epilogue reads or writes 32-bit rows (a residual sum, float32 out).
+// wide_rows: the epilogue reads and writes 32-bit rows (1: a residual sum) or writes them (2: float32 out); 0: 16-bit rows.
 AYK_EXPORT int ayk_gemm_tc_prefill_tile_k(int M, int N, int K, int sms, int wide_rows);
 AYK_EXPORT int ayk_gemm_tc_prefill_tile(int M, int N, int sms) { return ayk_gemm_tc_prefill_tile_k(M, N, 1600, sms, 0); }
 AYK_EXPORT int ayk_gemm_tc_prefill_tile_k(int M, int N, int K, int sms, int wide_rows) {
   int best = 256;
   double best_us = -1.0;
   for (int bn = 32; bn <= 256; bn += 32) {
-    const double us = whole_tiles_us(M, N, K, bn, sms, wide_rows != 0);
+    const double us = whole_tiles_us(M, N, K, bn, sms, wide_rows);
     if (best_us < 0 || us < best_us) { best_us = us; best = bn; }
   }
   return best;
@@ -1096,7 +1121,7 @@ AYK_EXPORT int ayk_gemm_tc_prefill_tile_k(int M, int N, int K, int sms, int wide
 // would split the K blocks of a tile (1: whole tiles).  Host arithmetic only; needs no device.
 AYK_EXPORT void ayk_gemm_tc_prefill_plan(int M, int N, int K, int sms, int wide_rows, int* tile, int* parts) {
   int bn = ayk_gemm_tc_prefill_tile_k(M, N, K, sms, wide_rows), sp = 1, sbn = 0, ssp = 0;
-  if (split_pays(M, N, K, sms, 0, wide_rows != 0, &sbn, &ssp)) { bn = sbn; sp = ssp; }
+  if (split_pays(M, N, K, sms, 0, wide_rows, &sbn, &ssp)) { bn = sbn; sp = ssp; }
   if (tile) *tile = bn;
   if (parts) *parts = sp;
 }
@@ -1229,8 +1254,8 @@ int prefill_product(void* C, const void* X, const void* W, const float* bias, co
     cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel, mx, mw, args);
     return ayk_check_launch("ayk_gemm_tc_prefill (pairs)");
   }
-  const bool wide_rows = residual != nullptr || out_dtype == AYK_DTYPE_F32;
-  int BN = tile_n > 0 ? tile_n : ayk_gemm_tc_prefill_tile_k(M, N, K, sms, wide_rows ? 1 : 0);
+  const int wide_rows = residual != nullptr ? 1 : (out_dtype == AYK_DTYPE_F32 ? 2 : 0);
+  int BN = tile_n > 0 ? tile_n : ayk_gemm_tc_prefill_tile_k(M, N, K, sms, wide_rows);
   int splits = 1;
   if (g_split < 0) {
     int sbn = 0, ssp = 0;
@@ -1345,7 +1370,7 @@ AYK_EXPORT int ayk_gemm_tc_prefill_grouped(void* C, const void* X, const void* W
   AYK_REQUIRE(!glu || (N % 8 == 0 && act == AYK_ACT_NONE && out_dtype == AYK_DTYPE_BF16), "ayk_gemm_tc_prefill_grouped: the gated form makes bfloat16 rows of whole 16-byte pieces");
   if (sms <= 0) sms = ayk_sm_count();
   const int cols = glu ? 2 * N : N;
-  int BN = ayk_gemm_tc_prefill_tile_k(expected > 0 ? expected : M, cols, K, sms, out_dtype == AYK_DTYPE_F32);
+  int BN = ayk_gemm_tc_prefill_tile_k(expected > 0 ? expected : M, cols, K, sms, out_dtype == AYK_DTYPE_F32 ? 2 : 0);
   if (glu) BN = (BN + 32) / 64 * 64;               // a quarter of the columns is a thread's whole 16s
   AYK_REQUIRE(BN >= 32 && BN <= 256 && BN % 32 == 0, "ayk_gemm_tc_prefill_grouped: tile width %d", BN);
   {

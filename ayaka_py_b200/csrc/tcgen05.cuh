@@ -77,6 +77,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* er
   return false;
 }
 
+// The same by the suspending poll alone: a few instructions, for the loops whose pace the waiting thread sets.  (Inline: a
+// kernel's warps share the instruction caches, and no call is made from one lane of a warp.)
+__device__ __forceinline__ bool mbar_wait_short(uint32_t bar, uint32_t parity, int* error, int code) {
+  if (__builtin_expect(mbar_try(bar, parity), 1)) return true;
+#pragma unroll 1
+  for (uint32_t i = 1; i < WAIT_LIMIT; ++i) {
+    if (mbar_try(bar, parity)) return true;
+  }
+  atomicExch(error, code);
+  return false;
+}
+
 // ---------------------------------------------------------------------- TMA --
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
