@@ -1004,7 +1004,10 @@ def grouped_part(max_len: int, blocks: int = 0) -> int:
     A block of one 64-key tile has nothing to load while it computes, and the merge reads 520 bytes per head and partition.
     Measured, 16 heads over 4 key heads of 128, a cache of 2,048 keys (us; 64, 128, 256 keys): 32 requests of 1,948 keys 74.7, 59.3, 54.2;
     of 250 19.1, 13.7, 15.4; 128 requests of 100 48.6, 29.7, 22.4; but 8 requests of 250 8.6, 10.8, 14.7, of 1,948 26.3, 20.1, 17.1.
-    Keys of 512 numbers (tiles of 32): 30 requests of 250 38.0, 29.3, 25.1, of 1,948 178, 156, 148."""
+    Keys of 512 numbers (tiles of 32): 30 requests of 250 38.0, 29.3, 25.1, of 1,948 178, 156, 148.
+    With warps that stream tiles of their own (heads of 64 and 128, up to 8 to a group; a whole layer of width 2,048): 32 requests of 1,948
+    keys 59.8, 51.2, 48.0; of 250 22.6, 22.8, 24.5; 128 requests of 100 40.1, 35.2, 32.8; 8 requests of 250 20.3, 18.7, 20.5, of 1,948
+    28.7, 25.9, 24.6: the larger partitions cost less there, the line stays where the other kernels need it."""
     part = 64
     while part * 64 < max_len:
         part *= 2

@@ -25,7 +25,8 @@ class PreNormBlock(Block):
     def _program(self, x, ctx, caches):
         """The block as one call into the library (``engine/program.py``), where its parts can be lowered: nine launches from Python took 13 us
         each and bounded every step of up to a few hundred rows (a layer of the small GPT-2 shape, 8 single rows beside 60 rows: 126 ->
-        42 us; of the XL shape, 2 beside 8 rows 132 -> 41)."""
+        42 us; of the XL shape, 2 beside 8 rows 132 -> 41).  Made at the second call with a cache: it takes about 70 us, which a caller
+        that comes once would not get back."""
         if x.dtype != torch.float32 or not x.is_contiguous():
             return None
         from ..engine.program import BlockProgram, native_allowed
@@ -34,7 +35,10 @@ class PreNormBlock(Block):
         binding = caches.get("mixer")
         programs = self._programs.setdefault(ctx.cache, {})
         key = None if binding is None else (binding.group, binding.layer, binding.writes)
-        program = programs.get(key, False)
+        if key not in programs:
+            programs[key] = False
+            return None
+        program = programs[key]
         if program is False or (program is not None and not program.current()):
             try:
                 program = BlockProgram(self, caches, ctx.cache, ctx.dtype)
