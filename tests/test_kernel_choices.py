@@ -70,3 +70,12 @@ def test_wide_rows_keep_to_the_staged_widths_when_it_pays():
     # 32-bit rows in and out: 192 columns go through the staged epilogue, 256 do not
     assert ops.prefill_plan(2048, 1600, 6400, wide_rows=True)[0] == 192
     assert ops.prefill_plan(2048, 1600, 1600, wide_rows=True)[0] == 192
+
+
+@pytest.mark.parametrize("M,N,K,plan", [
+    (130, 768, 3072, (64, 4)), (200, 1600, 6400, (128, 4)), (300, 2048, 2048, (64, 1)), (576, 1280, 1280, (64, 1)), (576, 1280, 5120, (96, 2)),
+    (700, 1280, 5120, (128, 2)), (1024, 768, 768, (64, 1)), (1024, 1600, 1600, (128, 1)), (1801, 1024, 4096, (128, 1)), (2048, 768, 3072, (128, 1)),
+])
+def test_plan_over_a_residual_is_the_measured_best(M, N, K, plan):
+    # the best of 8 widths, whole and split by 2, 4 and 8, each measured with a float32 residual
+    assert ops.prefill_plan(M, N, K, wide_rows=True) == plan
