@@ -9,8 +9,9 @@
 // scales its rows' O where one of their maxima has grown.
 //
 // Keys have KC chunks of 64 numbers.  Two sources: a paged cache (pages found through the block table; positions on no page are read
-// behind the pages' end as zeros, positions behind the last row's are wiped from the values), or rows side by side (latent_expand.cu),
-// whose third chunk, a part that all heads share, comes from pages.  F16: queries, keys, weights and values are float16
+// behind the pages' end as zeros), or rows side by side (latent_expand.cu), request after request, whose third chunk, a part that all
+// heads share, comes from pages.  From both, the values of positions behind the block's last row are wiped: they may be anything, another
+// request's not-a-numbers too.  F16: queries, keys, weights and values are float16
 // (the shared third chunk bfloat16 on both sides), with a factor per row and head on the scores (q_scale); else bfloat16.
 //
 // Warps 0-3: rows of tile A, 4-7: of tile B; 8: TMA; 9 and 10: MMA issue of A and of B (9: tensor memory).  One block to a multiprocessor (192 or 224 KB).  Every wait
@@ -122,7 +123,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   const int end_a = (pos_a + rows_a - 1 - k_begin) / KEYS + 1;
   const int start_b = rows_b > 0 ? (first_key(pos_b) - k_begin) / KEYS : 0;
   const int end_b = rows_b > 0 ? (pos_b + rows_b - 1 - k_begin) / KEYS + 1 : 0;
-  const bool wipes = !args.side_by_side && (last_key - k_begin + 1) % KEYS != 0;      // the last tile holds positions behind the last row's
+  const bool wipes = (last_key - k_begin + 1) % KEYS != 0;      // the last tile holds positions behind the last row's (side by side: the next request's too)
   const int num_tiles = max(end_a, end_b);             // no tile is read by neither: B's first key is at most the one behind A's last
 
   if (threadIdx.x == 0) {
@@ -235,7 +236,8 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       if (ok) v_issued = t + 1;
     }
     if (ok && wipes) {
-      // positions behind the last row's are nobody's yet: what their places hold enters P V times zero, so it has to be finite
+      // positions behind the last row's are nobody's yet, or (side by side) another request's: what their places hold enters P V times
+      // zero, so it has to be finite
       const int t = num_tiles - 1, live = last_key - (k_begin + t * KEYS) + 1;
       if (lane == 0) ok = mbar_wait_short(v_full + 8 * (t % ST), (uint32_t)(t / ST) & 1u, args.error, 85);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;

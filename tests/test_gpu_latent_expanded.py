@@ -89,3 +89,49 @@ def test_expanded_keys_and_values(monkeypatch, H, page, window, gate, layout, di
     assert errors[1] < (8e-3 if gain == 1.0 else 0.2), errors
     assert errors[1] < 1.2 * errors[0] + 1e-3, errors
     cache.rollback(res)
+
+
+def a_layer(H, before, brings, window=None, page=16, scales=None):
+    """(part, weights, context, packed rows, place of every request's rows) of a step that brings ``brings`` tokens behind ``before``; ``scales``:
+    factors on the weights by name."""
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts.latent_attention import LatentAttention
+    torch.manual_seed(H + sum(brings))
+    width = 256
+    part = LatentAttention(width, H, DIM, ROT, DIM, RANK, (DIM + ROT) ** -0.5, 1e-6, {"base": 50000.0, "dims": ROT, "layout": "halves"}, gate="head",
+                           window=window, dtype=torch.bfloat16)
+    w = {name: (torch.randn(d.shape, device="cuda") / d.shape[-1] ** 0.5).to(torch.bfloat16) if len(d.shape) == 2 else 1 + 0.1 * torch.randn(d.shape, device="cuda")
+         for name, d in part.tensors().items()}
+    for name, factor in (scales or {}).items():
+        w[name] = w[name] * factor
+    part.bind(w)
+    cache, runner = context_for([CacheGroupSpec("g", part.cache_need(), 1)], "bfloat16", max_requests=4, page_size=page,
+                                pages=sum(-(-(a + b) // page) for a, b in zip(before, brings)) + 2)
+    for pages in cache.kv_layer(0, 0):
+        pages.copy_(torch.randn(pages.shape, device="cuda"))
+    for i, n in enumerate(before):
+        slot = cache.open(i)
+        if n:
+            cache.commit(cache.reserve([(slot, 0, n)]))
+    ctx, _ = step_of(cache, runner, dict(enumerate(brings)))
+    order = [int(i) for i in ctx.host["order"]]
+    at = {i: slice(int(ctx.host["q_start"][k]), int(ctx.host["q_start"][k + 1])) for k, i in enumerate(order)}
+    return part, w, ctx, torch.randn(ctx.num_rows, width, device="cuda").to(torch.bfloat16), at
+
+
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("before,brings,bad", [([0, 0], [65, 70], 1), ([0, 0], [64, 64], 1), ([63, 10], [130, 257], 1), ([3, 300], [2, 5], 1),
+                                               ([0, 0, 0], [700, 257, 33], 1), ([500, 40], [300, 2], 0)])
+def test_a_request_that_is_no_number_keeps_to_itself(monkeypatch, before, brings, bad, window):
+    """Keys and values lie request after request, and a tile of 64 of them holds the next request's first ones."""
+    from ayaka_py_b200 import ops
+    monkeypatch.setattr(ops, "latent_expanded_pays", lambda *a: True)
+    part, _, ctx, x, at = a_layer(2, before, brings, window)
+    binding = SimpleNamespace(group=0, layer=0, writes=True)
+    want = part.forward(x, None, ctx, binding).clone()
+    x[at[bad]] = math.inf
+    got = part.forward(x, None, ctx, binding)
+    assert ops.tc_error() == 0 and not torch.isfinite(got[at[bad]]).any()
+    for i in range(len(brings)):
+        if i != bad:
+            assert torch.isfinite(want[at[i]]).all() and torch.equal(got[at[i]], want[at[i]]), i
