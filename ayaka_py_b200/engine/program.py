@@ -232,24 +232,38 @@ class BlockProgram:
         self.ops = (_Op * self.n_ops)(*builder.ops)
         self.buffers = (_Buffer * max(1, len(builder.buffers)))(*[_Buffer(k, b) for k, b in builder.buffers])
         self.keep, self.floats = builder.keep, builder.decode_floats_per_request
+        widths = {op.i[0] for op in builder.ops if STREAM in (op.src, op.src2, op.out)}        # a norm's rows, a product's out features
+        if len(widths) != 1:
+            raise NotLowered("the block does not read and write its stream at one width")
+        self.width, self.device = widths.pop(), builder.keep[0].device
+        self.groups = sorted({op.i[6] for op in builder.ops if op.kind == OP_ATTENTION})       # whose tables the operations read
         # the tensors that the operations were recorded with, as the parts hold them: a part that is given others needs a new program
         self.bound = [(part, name.replace(".", "_"), getattr(part, name.replace(".", "_"))) for part in block.parts.values() for name in part.tensors()]
 
     def current(self) -> bool:
         return all(getattr(part, name) is tensor for part, name, tensor in self.bound)
 
+    def takes(self, x: torch.Tensor, ctx) -> bool:
+        """Whether the stream is this block's rows of this step, and the step's arrays are as the kernels read them.  The parts' own
+        calls check the same tensor by tensor and refuse what does not fit."""
+        if x.shape != (ctx.num_rows, self.width) or x.device != self.device or x.dtype != torch.float32 or not x.is_contiguous():
+            return False
+        if ctx.req_pos0.numel() != ctx.num_requests:
+            return False
+        arrays = (ctx.positions, ctx.row_req, ctx.req_q_start, ctx.req_pos0, *(ctx.tables[g] for g in self.groups))
+        return all(t is not None and t.dtype == torch.int32 and t.device == self.device and t.is_contiguous() for t in arrays)
+
     def run(self, x: torch.Tensor, ctx) -> torch.Tensor:
+        """The block over a stream that it ``takes``, in place."""
         T, cache, step = ctx.num_rows, ctx.cache, _Step()
-        if x.shape[0] != T:
-            raise ops.KernelError(f"a stream of {x.shape[0]} rows in a step of {T}")
         workspace = torch.empty(sum((T * b + 255) // 256 * 256 for b in self.row_bytes) or 256, dtype=torch.uint8, device=x.device)
         step.T, step.R, step.num_single, step.max_q_len = T, ctx.num_requests, ctx.num_single, ctx.max_q_len
         step.max_context, step.settled = cache.max_len, 1 if ctx.earlier_rows_settled else 0
         step.positions, step.row_req = ctx.positions.data_ptr(), ctx.row_req.data_ptr()
         step.req_q_start, step.req_pos0 = ctx.req_q_start.data_ptr(), ctx.req_pos0.data_ptr()
-        for g, table in enumerate(ctx.tables[:MAX_GROUPS]):
-            if table is not None:
-                step.tables[g], step.table_stride[g] = table.data_ptr(), table.stride(0)
+        for g in self.groups:
+            table = ctx.tables[g]
+            step.tables[g], step.table_stride[g] = table.data_ptr(), table.stride(0)
         step.workspace, step.workspace_bytes, step.stream = workspace.data_ptr(), workspace.numel(), x.data_ptr()
         if self.floats:
             scratch = ops._decode_buffer(x.device, ctx.num_requests * self.floats * -(-cache.max_len // ops.DECODE_PART))

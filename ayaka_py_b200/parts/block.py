@@ -4,8 +4,6 @@ from __future__ import annotations
 
 import weakref
 
-import torch
-
 from .. import ops
 from .base import Block, NotLowered, register_block
 
@@ -27,8 +25,6 @@ class PreNormBlock(Block):
         each and bounded every step of up to a few hundred rows (a layer of the small GPT-2 shape, 8 single rows beside 60 rows: 126 ->
         42 us; of the XL shape, 2 beside 8 rows 132 -> 41).  Made at the second call with a cache: it takes about 70 us, which a caller
         that comes once would not get back."""
-        if x.dtype != torch.float32 or not x.is_contiguous():
-            return None
         from ..engine.program import BlockProgram, native_allowed
         if not native_allowed(x.device):
             return None
@@ -45,7 +41,7 @@ class PreNormBlock(Block):
             except NotLowered:
                 program = None
             programs[key] = program
-        return program
+        return program if program is not None and program.takes(x, ctx) else None
 
     def forward(self, x, ctx, caches):
         program = self._program(x, ctx, caches)

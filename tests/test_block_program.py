@@ -1,0 +1,75 @@
+"""A block's program by itself, without a GPU: which calls it takes and what it holds.  The library's calls are stubs."""
+
+from types import SimpleNamespace
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from ayaka_py_b200 import ops                                     # noqa: E402
+from ayaka_py_b200.cache import CacheGroupSpec                    # noqa: E402
+from ayaka_py_b200.cache.manager import CacheManager              # noqa: E402
+from ayaka_py_b200.cache.spec import CacheBinding                 # noqa: E402
+from ayaka_py_b200.engine import program                          # noqa: E402
+from ayaka_py_b200.engine.step import StepEntry, StepRunner       # noqa: E402
+from ayaka_py_b200.parts.attention import Attention               # noqa: E402
+from ayaka_py_b200.parts.block import PreNormBlock                # noqa: E402
+from ayaka_py_b200.parts.mlp import MLP                           # noqa: E402
+from ayaka_py_b200.parts.norm import LayerNorm                    # noqa: E402
+
+WIDTH = 128
+
+
+@pytest.fixture
+def steps(monkeypatch):
+    """The steps that the library was given."""
+    given = []
+
+    class Library:
+        def ayk_program_run(self, recorded, n_ops, buffers, n_buffers, step, launched, stream):
+            given.append(step._obj)
+            return 0
+
+    monkeypatch.setattr(ops, "_ready", Library)
+    monkeypatch.setattr(ops, "_stream", lambda: None)
+    monkeypatch.setattr(program, "native_allowed", lambda device: True)
+    return given
+
+
+def a_block():
+    parts = {"norm1": LayerNorm(WIDTH, 1e-5), "mixer": Attention(WIDTH, 2, 64, 0.125), "norm2": LayerNorm(WIDTH, 1e-5),
+             "ffn": MLP(WIDTH, 4 * WIDTH, "gelu_tanh")}
+    for part in parts.values():
+        part.bind({name: torch.zeros(d.shape) for name, d in part.tensors().items()})
+    return PreNormBlock(parts)
+
+
+def a_cache(block):
+    return CacheManager([CacheGroupSpec("g", block.mixer.cache_need(), 1)], kv_pages=16, page_size=16, max_requests=4, max_len=64,
+                        dtype=torch.float32, device="cpu")
+
+
+def a_step(cache, counts=(3, 1)):
+    runner = StepRunner(SimpleNamespace(device="cpu", dtype=torch.float32, max_positions=64, vocab_size=10), cache, max_tokens=64)
+    slots = [cache.open(i) for i in range(len(counts))]
+    cache.reserve([(s, 0, n) for s, n in zip(slots, counts)])
+    return runner.prepare([StepEntry(s, 0, [0] * n) for s, n in zip(slots, counts)])
+
+
+BINDING = {"mixer": CacheBinding(0, "g", 0)}
+
+
+def test_a_stream_that_does_not_fit_is_refused_at_every_call(steps):
+    block = a_block()
+    ctx = a_step(a_cache(block))
+    x = torch.zeros(4, WIDTH)
+    assert block._program(x, ctx, BINDING) is None                # the first call with a cache is the parts' own
+    assert block.forward(x, ctx, BINDING) is x and len(steps) == 1
+    with pytest.raises(ops.KernelError, match="row width"):
+        block.forward(torch.zeros(4, 100), ctx, BINDING)
+    # what does not fit goes to the parts' own calls, whose checks are the same at every call
+    for wrong in (torch.zeros(4, 100), torch.zeros(5, WIDTH), torch.zeros(4), torch.zeros(4, WIDTH, dtype=torch.float64),
+                  torch.zeros(4, 2 * WIDTH)[:, ::2]):
+        assert block._program(wrong, ctx, BINDING) is None
+    ctx.req_pos0 = ctx.req_pos0.long()
+    assert block._program(x, ctx, BINDING) is None and len(steps) == 1
