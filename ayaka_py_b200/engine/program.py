@@ -220,8 +220,9 @@ def native_allowed(device) -> bool:
 
 
 class BlockProgram:
-    """The operations of one block over the caller's residual stream, for a caller that runs a layer by itself.  Nothing of a call is
-    kept: the workspace is the call's own, so calls on several streams and threads do not meet."""
+    """The operations of one block over the caller's residual stream, for a caller that runs a layer by itself (a ``StepRunner`` runs
+    whole models, through ``StepProgram``).  Nothing of a call is kept: its buffers and the partial sums of its single rows are its
+    own, allocated on the stream that it runs on, so calls on several streams and threads share no memory but the caller's."""
 
     def __init__(self, block, caches: dict, cache, dtype: torch.dtype):
         builder = ProgramBuilder(cache, dtype)
@@ -256,7 +257,10 @@ class BlockProgram:
     def run(self, x: torch.Tensor, ctx) -> torch.Tensor:
         """The block over a stream that it ``takes``, in place."""
         T, cache, step = ctx.num_rows, ctx.cache, _Step()
-        workspace = torch.empty(sum((T * b + 255) // 256 * 256 for b in self.row_bytes) or 256, dtype=torch.uint8, device=x.device)
+        size = sum((T * b + 255) // 256 * 256 for b in self.row_bytes)
+        single = ctx.num_requests if ctx.max_q_len == 1 else ctx.num_single             # rows that take the decode kernels
+        floats = single * self.floats * -(-cache.max_len // ops.DECODE_PART)
+        workspace = torch.empty(size + 4 * floats or 256, dtype=torch.uint8, device=x.device)
         step.T, step.R, step.num_single, step.max_q_len = T, ctx.num_requests, ctx.num_single, ctx.max_q_len
         step.max_context, step.settled = cache.max_len, 1 if ctx.earlier_rows_settled else 0
         step.positions, step.row_req = ctx.positions.data_ptr(), ctx.row_req.data_ptr()
@@ -264,10 +268,9 @@ class BlockProgram:
         for g in self.groups:
             table = ctx.tables[g]
             step.tables[g], step.table_stride[g] = table.data_ptr(), table.stride(0)
-        step.workspace, step.workspace_bytes, step.stream = workspace.data_ptr(), workspace.numel(), x.data_ptr()
-        if self.floats:
-            scratch = ops._decode_buffer(x.device, ctx.num_requests * self.floats * -(-cache.max_len // ops.DECODE_PART))
-            step.decode_scratch, step.decode_scratch_floats = scratch.data_ptr(), scratch.numel()
+        step.workspace, step.workspace_bytes, step.stream = workspace.data_ptr(), size, x.data_ptr()
+        if floats:
+            step.decode_scratch, step.decode_scratch_floats = workspace.data_ptr() + size, floats
         launched = ctypes.c_int(0)
         code = self.lib.ayk_program_run(self.ops, self.n_ops, self.buffers, len(self.row_bytes), ctypes.byref(step), ctypes.byref(launched),
                                         ops._stream())

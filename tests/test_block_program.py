@@ -73,3 +73,24 @@ def test_a_stream_that_does_not_fit_is_refused_at_every_call(steps):
         assert block._program(wrong, ctx, BINDING) is None
     ctx.req_pos0 = ctx.req_pos0.long()
     assert block._program(x, ctx, BINDING) is None and len(steps) == 1
+
+
+@pytest.mark.parametrize("counts,single", [((3, 5), 0), ((1, 5, 1), 2), ((1, 1), 2)])
+def test_the_partial_sums_of_single_rows_are_the_calls_own(steps, monkeypatch, counts, single):
+    """Calls on two streams would meet in a buffer kept per device."""
+    monkeypatch.setattr(ops, "_decode_buffer", None)
+    block = a_block()
+    cache = a_cache(block)
+    ctx = a_step(cache, counts)
+    x = torch.zeros(sum(counts), WIDTH)
+    kept, empty = [], torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: kept.append(empty(*a, **k)) or kept[-1])
+    assert block._program(x, ctx, BINDING) is None
+    block.forward(x, ctx, BINDING), block.forward(x, ctx, BINDING)
+    assert len(steps) == 2
+    for step, own in zip(steps, kept[-2:]):
+        assert own.data_ptr() == step.workspace and step.decode_scratch_floats == single * 2 * (64 + 2) * -(-cache.max_len // ops.DECODE_PART)
+        if single:
+            assert step.workspace + step.workspace_bytes <= step.decode_scratch
+            assert step.decode_scratch + 4 * step.decode_scratch_floats <= step.workspace + own.numel()
+    assert steps[0].workspace != steps[1].workspace
