@@ -21,6 +21,7 @@ same for every model.
 from __future__ import annotations
 
 import ctypes
+import operator
 import os
 
 import torch
@@ -225,6 +226,12 @@ class BlockProgram:
     own, allocated on the stream that it runs on, so calls on several streams and threads share no memory but the caller's."""
 
     def __init__(self, block, caches: dict, cache, dtype: torch.dtype):
+        self.parts = {name: getattr(block, name) for name in block.parts}
+        for part in self.parts.values():
+            # a ``forward`` of the object's own, or of a class below the one that says how the part is lowered, is not what is recorded
+            says = [c for c in (part, *type(part).__mro__) if "lower" in vars(c) or "forward" in vars(c)]
+            if not says or "lower" not in vars(says[0]):
+                raise NotLowered(f"{type(part).__name__} has a forward of its own")
         builder = ProgramBuilder(cache, dtype)
         if block.lower(builder, STREAM, caches) != STREAM:
             raise NotLowered("the block does not keep its stream in place")
@@ -232,17 +239,36 @@ class BlockProgram:
         self.n_ops, self.row_bytes = len(builder.ops), [b for _, b in builder.buffers]
         self.ops = (_Op * self.n_ops)(*builder.ops)
         self.buffers = (_Buffer * max(1, len(builder.buffers)))(*[_Buffer(k, b) for k, b in builder.buffers])
-        self.keep, self.floats = builder.keep, builder.decode_floats_per_request
+        self.floats = builder.decode_floats_per_request
         widths = {op.i[0] for op in builder.ops if STREAM in (op.src, op.src2, op.out)}        # a norm's rows, a product's out features
         if len(widths) != 1:
             raise NotLowered("the block does not read and write its stream at one width")
         self.width, self.device = widths.pop(), builder.keep[0].device
         self.groups = sorted({op.i[6] for op in builder.ops if op.kind == OP_ATTENTION})       # whose tables the operations read
-        # the tensors that the operations were recorded with, as the parts hold them: a part that is given others needs a new program
-        self.bound = [(part, name.replace(".", "_"), getattr(part, name.replace(".", "_"))) for part in block.parts.values() for name in part.tensors()]
+        # what the operations were recorded from: the block's parts, all that the parts hold, and where every tensor lay
+        self.held = [(part, list(vars(part)), list(vars(part).values())) for part in self.parts.values()]
+        groups = {b.group for b in caches.values() if b is not None}
+        self.pages = [(g, cache.kv[g]) for g in groups]
+        kept = [*builder.keep, *(t for _, pair in self.pages for t in pair)]
+        self.places = [(t, t.data_ptr()) for t in {id(t): t for t in kept}.values()]
 
-    def current(self) -> bool:
-        return all(getattr(part, name) is tensor for part, name, tensor in self.bound)
+    def current(self, block, cache) -> bool:
+        """Whether the parts and the cache still hold what the operations were recorded from: other parts, weights, constants or pages, in
+        the place of the old ones or laid out anew under their names, need a new program."""
+        for name, part in self.parts.items():
+            if getattr(block, name) is not part:
+                return False
+        for part, names, values in self.held:
+            have = vars(part)
+            if list(have) != names or not all(map(operator.is_, have.values(), values)):
+                return False
+        for g, pair in self.pages:
+            if cache.kv[g] is not pair:
+                return False
+        for tensor, place in self.places:
+            if tensor.data_ptr() != place:
+                return False
+        return True
 
     def takes(self, x: torch.Tensor, ctx) -> bool:
         """Whether the stream is this block's rows of this step, and the step's arrays are as the kernels read them.  The parts' own

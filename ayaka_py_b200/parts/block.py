@@ -30,12 +30,12 @@ class PreNormBlock(Block):
             return None
         binding = caches.get("mixer")
         programs = self._programs.setdefault(ctx.cache, {})
-        key = None if binding is None else (binding.group, binding.layer, binding.writes)
+        key = (ctx.dtype, None if binding is None else (binding.group, binding.layer, binding.writes))
         if key not in programs:
             programs[key] = False
             return None
         program = programs[key]
-        if program is False or (program is not None and not program.current()):
+        if program is False or (program is not None and not program.current(self, ctx.cache)):
             try:
                 program = BlockProgram(self, caches, ctx.cache, ctx.dtype)
             except NotLowered:

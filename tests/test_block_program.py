@@ -94,3 +94,50 @@ def test_the_partial_sums_of_single_rows_are_the_calls_own(steps, monkeypatch, c
             assert step.workspace + step.workspace_bytes <= step.decode_scratch
             assert step.decode_scratch + 4 * step.decode_scratch_floats <= step.workspace + own.numel()
     assert steps[0].workspace != steps[1].workspace
+
+
+def another_forward(self, h, residual, ctx):
+    return residual
+
+
+CHANGES = {
+    "a weight": lambda block, cache: block.ffn.bind({"up_weight": torch.ones(4 * WIDTH, WIDTH)}),
+    "a weight's storage": lambda block, cache: setattr(block.norm1.weight, "data", torch.ones(WIDTH)),
+    "a constant": lambda block, cache: setattr(block.norm2, "eps", 1e-6),
+    "a part": lambda block, cache: setattr(block, "norm1", a_block().norm1),
+    "the pages": lambda block, cache: cache.kv.__setitem__(0, tuple(t.clone() for t in cache.kv[0])),
+}
+
+
+@pytest.mark.parametrize("what", CHANGES)
+def test_a_program_of_something_else_is_made_anew(steps, what):
+    block = a_block()
+    cache = a_cache(block)
+    ctx = a_step(cache)
+    x = torch.zeros(4, WIDTH)
+    block._program(x, ctx, BINDING)
+    first = block._program(x, ctx, BINDING)
+    assert first is not None and block._program(x, ctx, BINDING) is first
+    CHANGES[what](block, cache)
+    second = block._program(x, ctx, BINDING)
+    assert second is not first and block._program(x, ctx, BINDING) is second
+
+
+def test_a_part_with_a_forward_of_its_own_is_not_lowered(steps):
+    class Mine(MLP):
+        forward = another_forward
+
+    for change in (lambda block: setattr(block.ffn, "__class__", Mine), lambda block: setattr(block.ffn, "forward", another_forward),
+                   lambda block: setattr(block, "ffn", SimpleNamespace(forward=another_forward))):
+        block = a_block()
+        ctx = a_step(a_cache(block))
+        change(block)
+        x = torch.zeros(4, WIDTH)
+        assert [block._program(x, ctx, BINDING) for _ in range(3)] == [None] * 3
+    # ... nor one that is given such a forward later
+    block = a_block()
+    ctx = a_step(a_cache(block))
+    block._program(x, ctx, BINDING)
+    assert block._program(x, ctx, BINDING) is not None
+    block.ffn.forward = another_forward
+    assert block._program(x, ctx, BINDING) is None
