@@ -20,6 +20,12 @@ class PreNormBlock(Block):
         super().__init__(parts)
         self._programs = weakref.WeakKeyDictionary()       # cache manager -> {cache binding: the block as a program, or None}
 
+    def __getstate__(self):
+        return {name: value for name, value in vars(self).items() if name != "_programs"}         # a copy records programs of its own
+
+    def __setstate__(self, state):
+        vars(self).update(state, _programs=weakref.WeakKeyDictionary())
+
     def _program(self, x, ctx, caches):
         """The block as one call into the library (``engine/program.py``), where its parts can be lowered: nine launches from Python took 13 us
         each and bounded every step of up to a few hundred rows (a layer of the small GPT-2 shape, 8 single rows beside 60 rows: 126 ->

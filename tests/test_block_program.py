@@ -1,5 +1,7 @@
 """A block's program by itself, without a GPU: which calls it takes and what it holds.  The library's calls are stubs."""
 
+import copy
+import pickle
 from types import SimpleNamespace
 
 import pytest
@@ -141,3 +143,15 @@ def test_a_part_with_a_forward_of_its_own_is_not_lowered(steps):
     assert block._program(x, ctx, BINDING) is not None
     block.ffn.forward = another_forward
     assert block._program(x, ctx, BINDING) is None
+
+
+def test_a_block_with_programs_can_be_copied(steps):
+    block = a_block()
+    ctx = a_step(a_cache(block))
+    x = torch.zeros(4, WIDTH)
+    block._program(x, ctx, BINDING)
+    assert block._program(x, ctx, BINDING) is not None
+    for other in (copy.deepcopy(block), pickle.loads(pickle.dumps(block))):
+        assert other.norm1 is not block.norm1 and other.norm1 is other.parts["norm1"]
+        assert other._program(x, ctx, BINDING) is None            # its own first call
+        assert other._program(x, ctx, BINDING) is not None
