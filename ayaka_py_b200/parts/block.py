@@ -35,7 +35,10 @@ class PreNormBlock(Block):
         if not native_allowed(x.device):
             return None
         binding = caches.get("mixer")
-        programs = self._programs.setdefault(ctx.cache, {})
+        try:
+            programs = self._programs.setdefault(ctx.cache, {})
+        except TypeError:                                  # a cache that cannot be a weak key
+            return None
         key = (ctx.dtype, None if binding is None else (binding.group, binding.layer, binding.writes))
         if key not in programs:
             programs[key] = False

@@ -155,3 +155,10 @@ def test_a_block_with_programs_can_be_copied(steps):
         assert other.norm1 is not block.norm1 and other.norm1 is other.parts["norm1"]
         assert other._program(x, ctx, BINDING) is None            # its own first call
         assert other._program(x, ctx, BINDING) is not None
+
+
+def test_a_cache_that_cannot_be_a_weak_key_leaves_the_block_to_its_parts(steps):
+    block = a_block()
+    ctx = a_step(a_cache(block))
+    ctx.cache = SimpleNamespace(**vars(ctx.cache))
+    assert [block._program(torch.zeros(4, WIDTH), ctx, BINDING) for _ in range(3)] == [None] * 3
