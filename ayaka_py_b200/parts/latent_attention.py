@@ -89,6 +89,7 @@ class LatentAttention(Mixer):
             at += rows
         self.in_weight = fused
         self.uk_heads = self.uk_weight.view(H, self.dim, self.rank).transpose(1, 2).contiguous()      # [H, rank, dim]
+        self.up_weight = None                              # of weights bound before
         if self.dtype == torch.bfloat16 and self.own_latent and (self.dim, self.rot_dim, self.vdim) == (128, 64, 128) and self.rank % 8 == 0 \
                 and self.scale > 0:
             # keys over values for ``ops.latent_expanded``, whose keys and values are float16: a latent is at most sqrt(rank) times its
