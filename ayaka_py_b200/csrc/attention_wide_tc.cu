@@ -12,7 +12,8 @@
 // behind the pages' end as zeros), or rows side by side (latent_expand.cu), request after request, whose third chunk, a part that all
 // heads share, comes from pages.  From both, the values of positions behind the block's last row are wiped: they may be anything, another
 // request's not-a-numbers too.  F16: queries, keys, weights and values are float16
-// (the shared third chunk bfloat16 on both sides), with a factor per row and head on the scores (q_scale); else bfloat16.
+// (the shared third chunk bfloat16 on both sides), with a factor per row and head on the scores (q_scale), one per head on the values
+// (v_scale), and weights 2^14 times as large, which leaves 28 powers of two of full precision below the largest; else bfloat16.
 //
 // Warps 0-3: rows of tile A, 4-7: of tile B; 8: TMA; 9 and 10: MMA issue of A and of B (9: tensor memory).  One block to a multiprocessor (192 or 224 KB).  Every wait
 // is bounded; one that runs out records its code, and the block ends when its copies have landed.
@@ -50,6 +51,7 @@ struct WideArgs {
   const float* sinks;            // [H] or null: the score of one more key without a value
   const float* gate;             // float32 rows or null: the output is multiplied by sigmoid of the row's number at h * gate_head + d * gate_col
   const float* q_scale;          // [T, H] or null: the factor of a row's scores
+  const float* v_scale;          // F16: [H], the factor that a head's values carry
   int* error;
   long long gate_stride;
   int gate_head, gate_col;
@@ -331,12 +333,14 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int qpos = (x == 0 ? pos_a : pos_b) + r;
     const int qlow = first_key(qpos);
     const uint32_t s_first = tmem + 128u * x + ((uint32_t)((warp & 3) * 32) << 16), o_at = s_first + 256u;
+    const float v_scale = F16 ? args.v_scale[h] : 1.f;
     pdl_wait();
     const float scale = args.scale_log2 * (args.q_scale && live ? args.q_scale[(size_t)row * args.H + h] : 1.f);
+    constexpr float UP = F16 ? 14.f : 0.f;             // the weights and their sum are 2^UP times what they are
     float m_run = -INFINITY, l = 0.f;
     if (args.sinks) {
       m_run = args.sinks[h] * 1.4426950408889634f;
-      l = 1.f;
+      l = F16 ? 16384.f : 1.f;
     }
     bool ok = true;
     for (int t = start; t < end; ++t) {
@@ -364,7 +368,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       const bool grown = __any_sync(0xffffffffu, m_new > m_run);
       const float alpha = m_new > -INFINITY ? fast_exp2(m_run - m_new) : 1.f;        // 2^(-inf) = 0 before the first visible key
       m_run = m_new;
-      const float m = m_run > -INFINITY ? m_run : 0.f;  // nothing seen yet: every weight is 2^(-inf) = 0
+      const float m = m_run > -INFINITY ? m_run - UP : 0.f;  // nothing seen yet: every weight is 2^(-inf) = 0
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int j = 0; j < KEYS; j += 2) {
@@ -404,7 +408,7 @@ attention_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (ok) {
         tc_fence_after();
-        const float inv = l > 0.f ? 1.f / l : 0.f;
+        const float inv = l > 0.f ? 1.f / (l * v_scale) : 0.f;
         // through this tile's place of the queries (its products are done), so that a warp stores whole rows of 256 bytes: a
         // piece of 16 bytes lies at its number XOR the low bits of its row
         uint8_t* stage = smem_raw + (uint32_t)x * KC * CHUNK + (uint32_t)(warp & 3) * 32 * 256;
@@ -537,7 +541,7 @@ AYK_EXPORT int ayk_attention_wide_tc(void* out, const void* q, const void* kcach
   CUtensorMap mq, mk, mv;
   if (encode_rows(&mq, q, total_rows, H * 128, false) || encode(&mk, kcache, cells, G, 128, box, false) || encode(&mv, vcache, cells, G, 128, box, false)) return -1;
   const int pair = (H / G) % 2 == 0 ? 1 : 0, span = pair ? ROWS : 2 * ROWS;
-  WideArgs args{(__nv_bfloat16*)out, table, req_q_start, req_pos0, sinks, gate, nullptr, g_error_dev, gate_stride, 128, 1, 0,
+  WideArgs args{(__nv_bfloat16*)out, table, req_q_start, req_pos0, sinks, gate, nullptr, nullptr, g_error_dev, gate_stride, 128, 1, 0,
                 table_stride, num_req, H, H / G, 0, shift, (int)cells, window, chunk, pair, scale * 1.4426950408889634f};
   AYK_REQUIRE(total_rows / span + num_req <= 65535, "ayk_attention_wide_tc: too many row tiles (%d rows, %d requests)", total_rows, num_req);
   ayk_launch(attention_wide_tc_kernel<2, false>, dim3(pair ? H / 2 : H, total_rows / span + num_req), dim3(THREADS), smem_bytes(2), stream, mq, mq, mk, mv, mk, args);
@@ -545,9 +549,9 @@ AYK_EXPORT int ayk_attention_wide_tc(void* out, const void* q, const void* kcach
 }
 
 // The expanded latent attention: out [T, H * 128] bfloat16; q16, q_rot, q_scale as latent_expand.cu makes them; kv [kv_rows, 2 H, 128] float16, keys of
-// every head and then values; rope_pages [pages, page_size, 64] bfloat16, shared by the heads.  gate: float32 rows of gate_stride, the number at
+// every head and then values, which carry the factor v_scale [H]; rope_pages [pages, page_size, 64] bfloat16, shared by the heads.  gate: float32 rows of gate_stride, the number at
 // h * gate_head + d * gate_col, or null.
-AYK_EXPORT int ayk_attention_expanded_tc(void* out, const void* q16, const void* q_rot, const float* q_scale, const void* kv, int kv_rows, const void* rope_pages,
+AYK_EXPORT int ayk_attention_expanded_tc(void* out, const void* q16, const void* q_rot, const float* q_scale, const float* v_scale, const void* kv, int kv_rows, const void* rope_pages,
                                          int pages, const int* table, int table_stride, const int* req_q_start, const int* req_pos0, int num_req,
                                          int total_rows, int H, int page_size, float scale, int window, const float* gate, long long gate_stride,
                                          int gate_head, int gate_col, cudaStream_t stream) {
@@ -564,7 +568,7 @@ AYK_EXPORT int ayk_attention_expanded_tc(void* out, const void* q16, const void*
   CUtensorMap mq, mr, mkv, ms;
   if (encode_rows(&mq, q16, total_rows, H * 128, true) || encode_rows(&mr, q_rot, total_rows, H * 64, false) ||
       encode(&mkv, kv, kv_rows, 2 * H, 128, KEYS, true) || encode(&ms, rope_pages, cells, 1, 64, box, false)) return -1;
-  WideArgs args{(__nv_bfloat16*)out, table, req_q_start, req_pos0, nullptr, gate, q_scale, g_error_dev, gate_stride, gate_head, gate_col, 1,
+  WideArgs args{(__nv_bfloat16*)out, table, req_q_start, req_pos0, nullptr, gate, q_scale, v_scale, g_error_dev, gate_stride, gate_head, gate_col, 1,
                 table_stride, num_req, H, 1, H, shift, (int)cells, window, 0, 0, scale * 1.4426950408889634f};
   AYK_REQUIRE(total_rows / (2 * ROWS) + num_req <= 65535, "ayk_attention_expanded_tc: too many row tiles (%d rows, %d requests)", total_rows, num_req);
   ayk_launch(attention_wide_tc_kernel<3, true>, dim3(H, total_rows / (2 * ROWS) + num_req), dim3(THREADS), smem_bytes(3), stream, mq, mr, mkv, mkv, ms, args);

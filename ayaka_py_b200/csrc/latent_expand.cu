@@ -12,8 +12,10 @@
 //             turn(rotated part) bfloat16; the factor that undoes it goes to the scores (q_scale)
 // For a token that earlier steps cached: its latent from its page to its place.
 // float16 keeps three more bits than bfloat16: with queries, keys, weights and values in bfloat16 the layer's error against 64 bits was 15 %
-// larger than with U_k^T applied to 32-bit queries.  The power of two keeps any query inside float16's range; keys and values are
-// bounded by the norms of U_k, U_v and the latent's norm weight, which the caller checks once, when the weights are laid out.
+// larger than with U_k^T applied to 32-bit queries.  It has three bits of exponent less, so everything comes into its range by powers of
+// two: queries as above; a head's keys and its values by `up_scale` (LatentAttention.bind), which brings the largest number that they
+// can hold to [2^14, 2^15), 28 powers of two above float16's smallest of full precision.  The keys' factor is also on the rotated
+// query parts, whose keys have none, and q_scale takes both out; the values' is taken out with the softmax's sum.
 // Bound by the projection's 32-bit rows (14.6 KB a row at 16 heads): 11 us for 1,801 rows, 41 MB.
 // Measured, the layer of width 2,048 (16 heads, latent 512 + 64), 1,024 + 777 rows: 280 -> 105 us (absorbed attention 176, its two products per
 // head 52, preparation 19; now preparation 11, keys and values 13, attention 28); error against 64 bits 3.2e-3 -> 2.8e-3, and over 23
@@ -32,8 +34,8 @@ __device__ __forceinline__ int first_token(int pos0, int window) { return window
 
 __global__ void __launch_bounds__(THREADS)
 latent_expand_prepare_kernel(__nv_bfloat16* latent_pages, __nv_bfloat16* __restrict__ rope_pages, __half* q16, __nv_bfloat16* q_rot, float* q_scale,
-                             __nv_bfloat16* side, const float* proj, long long proj_stride, const float* __restrict__ norm_w, const float* __restrict__ freq,
-                             float gain, int rot_dims, int halves, const int* __restrict__ row_req, const int* __restrict__ positions,
+                             __nv_bfloat16* side, const float* proj, long long proj_stride, const float* __restrict__ norm_w, const float* __restrict__ up_scale,
+                             const float* __restrict__ freq, float gain, int rot_dims, int halves, const int* __restrict__ row_req, const int* __restrict__ positions,
                              const int* __restrict__ table, int table_stride, int page_size, const int* __restrict__ req_q_start,
                              const int* __restrict__ req_pos0, int num_req, int T, int H, int rank, float eps, int window) {
   __shared__ float turn[ROT];                              // cos [rot_dims / 2], sin [rot_dims / 2]
@@ -90,6 +92,7 @@ latent_expand_prepare_kernel(__nv_bfloat16* latent_pages, __nv_bfloat16* __restr
   for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
   base += p - first_token(req_pos0[my_req], window);
   __syncthreads();
+  float up_next = up_scale[min(warp, H - 1)];              // asked for a head ahead
   pdl_wait();
   const float* row = proj + (size_t)t * proj_stride;
   const float* down = row + (size_t)H * (DIM + ROT);
@@ -103,19 +106,22 @@ latent_expand_prepare_kernel(__nv_bfloat16* latent_pages, __nv_bfloat16* __restr
   };
   for (int h = warp; h < H; h += WARPS) {
     const float* src = row + (size_t)h * (DIM + ROT);
+    const int up = ((int)__float_as_uint(up_next) >> 23) - 127;          // the keys' factor is 2^up, 0 <= up <= 40
+    up_next = up_scale[min(h + WARPS, H - 1)];
     const float4 v = *reinterpret_cast<const float4*>(src + lane * 4);
     const float2 w = *reinterpret_cast<const float2*>(src + DIM + lane * 2);
     const float r0 = turned(src + DIM, lane * 2, w.x), r1 = turned(src + DIM, lane * 2 + 1, w.y);
     const float top = warp_max(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-    // 2^k with top 2^k in [128, 256); 1 for zeros, infinities and not-a-numbers
-    const int e = ((int)__float_as_uint(top) >> 23) & 0xff;      // of 2^(e - 127) <= top
-    const int k = e > 0 && e < 255 ? min(max(134 - e, -120), 120) : 0;
-    const float by = __uint_as_float((uint32_t)(k + 127) << 23);
+    // 2^k with top 2^k in [128, 256); 1 for zeros, infinities and not-a-numbers.  At most 2^(60 - up): queries that would need more are so
+    // small that, with keys of at most 2^(15 - up), what they lose moves a score by less than 2^-40.
+    const int e = ((int)__float_as_uint(top) >> 23) & 0xff;              // of 2^(e - 127) <= top
+    const int k = e > 0 && e < 255 ? min(max(134 - e, -120), 60 - up) : 0;
+    const float by = __uint_as_float((uint32_t)(k + 127) << 23), by_rot = __uint_as_float((uint32_t)(k + up + 127) << 23);
     const size_t at = (size_t)t * H + h;
     const __half2 a = __floats2half2_rn(v.x * by, v.y * by), b = __floats2half2_rn(v.z * by, v.w * by);
     *reinterpret_cast<uint2*>(q16 + at * DIM + lane * 4) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-    *reinterpret_cast<__nv_bfloat162*>(q_rot + at * ROT + lane * 2) = __floats2bfloat162_rn(r0 * by, r1 * by);
-    if (lane == 0) q_scale[at] = __uint_as_float((uint32_t)(127 - k) << 23);
+    *reinterpret_cast<__nv_bfloat162*>(q_rot + at * ROT + lane * 2) = __floats2bfloat162_rn(r0 * by_rot, r1 * by_rot);
+    if (lane == 0) q_scale[at] = __uint_as_float((uint32_t)(127 - k - up) << 23);
   }
   const size_t cell = (size_t)max(page, 0) * page_size + p % page_size;
   if (page > 0 && tid < ROT) rope_pages[cell * ROT + tid] = __float2bfloat16_rn(turned(down + rank, tid, down[rank + tid]));
@@ -140,9 +146,9 @@ latent_expand_prepare_kernel(__nv_bfloat16* latent_pages, __nv_bfloat16* __restr
 }  // namespace
 
 // See above.  q16 [T, H, 128] float16, q_rot [T, H, 64] bfloat16, q_scale [T, H] float32, side [rows, rank] bfloat16: T rows and `cached` tokens
-// of earlier steps, request after request.  rank a multiple of 8, proj_stride of 4, all tensors 16-byte aligned.
+// of earlier steps, request after request.  up_scale [H or more]: the heads' factors on the keys.  rank a multiple of 8, proj_stride of 4, all tensors 16-byte aligned.
 AYK_EXPORT int ayk_latent_expand_prepare(void* latent_pages, void* rope_pages, void* q16, void* q_rot, float* q_scale, void* side, const float* proj,
-                                         long long proj_stride, const float* norm_w, const float* freq, float gain, int rot_dims, int halves,
+                                         long long proj_stride, const float* norm_w, const float* up_scale, const float* freq, float gain, int rot_dims, int halves,
                                          const int* row_req, const int* positions, const int* table, int table_stride, int page_size,
                                          const int* req_q_start, const int* req_pos0, int num_req, int T, int cached, int H, int rank, float eps,
                                          int window, cudaStream_t stream) {
@@ -152,7 +158,7 @@ AYK_EXPORT int ayk_latent_expand_prepare(void* latent_pages, void* rope_pages, v
   AYK_REQUIRE((((uintptr_t)latent_pages | (uintptr_t)q16 | (uintptr_t)q_rot | (uintptr_t)side | (uintptr_t)proj | (uintptr_t)norm_w) & 15) == 0,
               "ayk_latent_expand_prepare: operands must be 16-byte aligned");
   ayk_launch(latent_expand_prepare_kernel, dim3((unsigned)(T + cached)), dim3(THREADS), 0, stream, (__nv_bfloat16*)latent_pages, (__nv_bfloat16*)rope_pages,
-             (__half*)q16, (__nv_bfloat16*)q_rot, q_scale, (__nv_bfloat16*)side, proj, proj_stride, norm_w, freq, gain, rot_dims, halves, row_req,
+             (__half*)q16, (__nv_bfloat16*)q_rot, q_scale, (__nv_bfloat16*)side, proj, proj_stride, norm_w, up_scale, freq, gain, rot_dims, halves, row_req,
              positions, table, table_stride, page_size, req_q_start, req_pos0, num_req, T, H, rank, eps, window);
   return ayk_check_launch("ayk_latent_expand_prepare");
 }

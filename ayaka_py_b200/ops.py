@@ -663,18 +663,20 @@ def latent_expanded_pays(ctx, heads: int, rank: int, window: int | None, pages: 
     return ctx.host[key]
 
 
-def latent_expanded(proj: torch.Tensor, latent_pages: torch.Tensor, rope_pages: torch.Tensor, up_weight: torch.Tensor, norm_weight: torch.Tensor,
-                    freq: torch.Tensor, gain: float, rot_dims: int, ctx, table: torch.Tensor, heads: int, eps: float, halves: bool, scale: float,
-                    window: int | None, gate: torch.Tensor | None) -> torch.Tensor:
+def latent_expanded(proj: torch.Tensor, latent_pages: torch.Tensor, rope_pages: torch.Tensor, up_weight: torch.Tensor, up_scale: torch.Tensor,
+                    norm_weight: torch.Tensor, freq: torch.Tensor, gain: float, rot_dims: int, ctx, table: torch.Tensor, heads: int, eps: float,
+                    halves: bool, scale: float, window: int | None, gate: torch.Tensor | None) -> torch.Tensor:
     """The latent attention of a step's rows with keys and values expanded (``csrc/latent_expand.cu``): float32 projection rows
     [q (heads x (128 + 64)) | down (rank + 64) | ...], the normed latents and rotated key parts go into their pages, ``up_weight``
-    [2 heads * 128, rank] makes keys (the first half) and values of every token that the rows see, in float16; returns the
+    [2 heads * 128, rank] makes keys (the first half) and values of every token that the rows see, in float16.  Each head's rows carry the
+    factor that ``up_scale`` gives (float32 [2 heads], powers of two from 1 to 2^40, taken out again); no product may leave float16.  Returns the
     heads' outputs [T, heads * 128] in the pages' dtype, times sigmoid(gate) (float32 [T, heads] or [T, heads * 128])."""
     lib = _ready()
-    _f32(proj, "proj"); _f32(freq, "freq"); _f32(norm_weight, "norm_weight")
+    _f32(proj, "proj"); _f32(freq, "freq"); _f32(norm_weight, "norm_weight"); _f32(up_scale, "up_scale")
     T, rank, P, pages = proj.shape[0], latent_pages.shape[-1], latent_pages.shape[1], latent_pages.shape[0]
     if (latent_pages.dtype != torch.bfloat16 or rope_pages.dtype != torch.bfloat16 or up_weight.dtype != torch.bfloat16 or not up_weight.is_contiguous()
-            or up_weight.shape != (2 * heads * 128, rank) or rope_pages.shape[-1] != 64 or proj.shape[1] < heads * 192 + rank + 64 or proj.stride(1) != 1):
+            or up_weight.shape != (2 * heads * 128, rank) or up_scale.shape != (2 * heads,) or rope_pages.shape[-1] != 64
+            or proj.shape[1] < heads * 192 + rank + 64 or proj.stride(1) != 1):
         raise KernelError("latent_expanded: projection rows, weights or pages do not fit")
     if gate is not None and (gate.dtype != torch.float32 or gate.shape not in ((T, heads), (T, heads * 128)) or gate.stride(1) != 1):
         raise KernelError("latent_expanded: gate must be float32 [T, heads] or [T, heads * 128]")
@@ -689,7 +691,7 @@ def latent_expanded(proj: torch.Tensor, latent_pages: torch.Tensor, rope_pages: 
     table_ptr, stride, window_ = _ptr(_i32(table, "table")), ctypes.c_int(table.stride(0)), ctypes.c_int(window or 0)
     starts, pos0, requests = _ptr(ctx.req_q_start), _ptr(ctx.req_pos0), ctypes.c_int(ctx.num_requests)
     _launch(lib.ayk_latent_expand_prepare(_ptr(latent_pages), _ptr(rope_pages), _ptr(q16), _ptr(q_rot), _ptr(q_scale), _ptr(side), _ptr(proj),
-                                          ctypes.c_longlong(proj.stride(0)), _ptr(norm_weight), _ptr(freq), ctypes.c_float(gain),
+                                          ctypes.c_longlong(proj.stride(0)), _ptr(norm_weight), _ptr(up_scale), _ptr(freq), ctypes.c_float(gain),
                                           ctypes.c_int(rot_dims), ctypes.c_int(1 if halves else 0), _ptr(ctx.row_req), _ptr(ctx.positions),
                                           table_ptr, stride, ctypes.c_int(P), starts, pos0, requests, ctypes.c_int(T), ctypes.c_int(held - T),
                                           ctypes.c_int(heads), ctypes.c_int(rank), ctypes.c_float(eps), window_, _stream()))
@@ -697,8 +699,8 @@ def latent_expanded(proj: torch.Tensor, latent_pages: torch.Tensor, rope_pages: 
                                     ctypes.c_int(rank), ctypes.c_int(ACTIVATIONS["none"]), ctypes.c_int(F16), ctypes.c_int(0),
                                     ctypes.c_int(sm_count()), ctypes.c_int(-1), _stream()))
     gate_head, gate_col = (0, 0) if gate is None else (1, 0) if gate.shape[1] == heads else (128, 1)
-    _launch(lib.ayk_attention_expanded_tc(_ptr(out), _ptr(q16), _ptr(q_rot), _ptr(q_scale), _ptr(kv), ctypes.c_int(held), _ptr(rope_pages),
-                                          ctypes.c_int(pages), table_ptr, stride, starts, pos0, requests, ctypes.c_int(T), ctypes.c_int(heads),
+    _launch(lib.ayk_attention_expanded_tc(_ptr(out), _ptr(q16), _ptr(q_rot), _ptr(q_scale), _ptr(up_scale[heads:]), _ptr(kv), ctypes.c_int(held),
+                                          _ptr(rope_pages), ctypes.c_int(pages), table_ptr, stride, starts, pos0, requests, ctypes.c_int(T), ctypes.c_int(heads),
                                           ctypes.c_int(P), ctypes.c_float(scale), window_, _ptr(gate),
                                           ctypes.c_longlong(gate.stride(0) if gate is not None else 0), ctypes.c_int(gate_head),
                                           ctypes.c_int(gate_col), _stream()))

@@ -36,6 +36,18 @@ def _padded(n: int) -> int:
     return -(-n // 8) * 8
 
 
+def _float16_scale(up: torch.Tensor, norm: torch.Tensor, rows: int) -> torch.Tensor | None:
+    """The power of two for every ``rows`` rows of ``up`` that brings the largest product of one of them with a normed latent to
+    [2^14, 2^15).  (A latent is at most sqrt(rank) times its norm's largest weight long, so no product can be larger than that times the
+    longest row.)  None where a product could leave float16 without a factor, or where some rows are so small that they need more than
+    2^40; rows of zeros need none."""
+    longest = up.double().norm(dim=1).view(-1, rows).amax(dim=1) * (norm.abs().max() * up.shape[1] ** 0.5)
+    if not bool((longest < 30000.0).all()):
+        return None
+    power = torch.where(longest > 0, 15 - torch.frexp(longest).exponent, 0)
+    return None if int(power.max()) > 40 else torch.ldexp(torch.ones_like(longest), power).float()
+
+
 class LatentAttention(Mixer):
     KIND = "latent_attention"
 
@@ -57,7 +69,7 @@ class LatentAttention(Mixer):
         self.rotary = None if rot is None else make_part(
             PartSpec("rotary", {"dims": rot["dims"], "base": rot["base"], "scaling": rot.get("scaling"),
                                 "layout": rot.get("layout", "interleaved")}), dtype, device)
-        self.no_freq = self.up_weight = None
+        self.no_freq = self.up_weight = self.up_scale = None
         self.q_width = heads * (dim + rot_dim)
         self.down_width = kv_rank + rot_dim if own_latent else 0
         self.in_weight = self.down_norm = None
@@ -89,15 +101,15 @@ class LatentAttention(Mixer):
             at += rows
         self.in_weight = fused
         self.uk_heads = self.uk_weight.view(H, self.dim, self.rank).transpose(1, 2).contiguous()      # [H, rank, dim]
-        self.up_weight = None                              # of weights bound before
+        self.up_weight = self.up_scale = None              # of weights bound before
         if self.dtype == torch.bfloat16 and self.own_latent and (self.dim, self.rot_dim, self.vdim) == (128, 64, 128) and self.rank % 8 == 0 \
                 and self.scale > 0:
-            # keys over values for ``ops.latent_expanded``, whose keys and values are float16: a latent is at most sqrt(rank) times its
-            # norm's largest weight long, so no number of theirs can be larger than that times the longest row
+            # keys over values for ``ops.latent_expanded``, whose keys and values are float16: each head times its power of two (exact), a
+            # copy beside the matrices of the other form
             up = torch.cat([self.uk_weight, self.uv_weight])
-            longest = float(up.float().norm(dim=1).max()) * float(self.down_norm.abs().max()) * self.rank ** 0.5
-            if longest < 30000.0:
-                self.up_weight, self.uk_weight, self.uv_weight = up, up[:H * self.dim], up[H * self.dim:]
+            self.up_scale = _float16_scale(up, self.down_norm, 128)
+            if self.up_scale is not None:
+                self.up_weight = up.mul_(self.up_scale.repeat_interleave(128)[:, None].to(up.dtype))
         self.uv_heads = self.uv_weight.view(H, self.vdim, self.rank)                                   # [H, vdim, rank]
 
     def cache_need(self):
@@ -120,8 +132,8 @@ class LatentAttention(Mixer):
         first = self.q_width + self.down_width
         gate = proj[:, first:first + self.gate_width] if self.gate_width else None
         if self.up_weight is not None and ops.latent_expanded_pays(ctx, H, self.rank, self.window, latent_pages, ops.sm_count()):
-            o = ops.latent_expanded(proj, latent_pages, rope_pages, self.up_weight, self.down_norm, freq, gain, rot_dims, ctx, table, H, self.eps,
-                                    halves, self.scale, self.window, gate)
+            o = ops.latent_expanded(proj, latent_pages, rope_pages, self.up_weight, self.up_scale, self.down_norm, freq, gain, rot_dims, ctx, table, H,
+                                    self.eps, halves, self.scale, self.window, gate)
             return ops.linear(o, self.out_weight, None, residual=residual, out_dtype=torch.float32, out=residual)
         query = ops.latent_prepare(proj, latent_pages, rope_pages, self.down_norm, freq, gain, rot_dims, ctx, table, H,
                                    self.dim, self.rot_dim, self.rank, self.eps, cache.writes, halves)

@@ -135,3 +135,78 @@ def test_a_request_that_is_no_number_keeps_to_itself(monkeypatch, before, brings
     for i in range(len(brings)):
         if i != bad:
             assert torch.isfinite(want[at[i]]).all() and torch.equal(got[at[i]], want[at[i]]), i
+
+
+def heads_of(monkeypatch, part, x, ctx):
+    """The heads' outputs [T, H, 128] of the expanded form."""
+    from ayaka_py_b200 import ops
+    made, expanded = [], ops.latent_expanded
+    monkeypatch.setattr(ops, "latent_expanded_pays", lambda *a: True)
+    with monkeypatch.context() as m:
+        m.setattr(ops, "latent_expanded", lambda *a: made.append(expanded(*a)) or made[-1])
+        part.forward(x, None, ctx, SimpleNamespace(group=0, layer=0, writes=True))
+    assert ops.tc_error() == 0
+    return made[0].view(x.shape[0], part.heads, DIM).double()
+
+
+@pytest.mark.parametrize("before,brings", [([0], [257]), ([70, 300], [129, 3])])
+@pytest.mark.parametrize("power", [-24, -28, 9])
+def test_a_heads_scale_is_not_its_precision(monkeypatch, before, brings, power):
+    """U_v of one head times a power of two is its output times that, bit for bit; U_k times it and the queries divided by it change nothing."""
+    H, head = 3, 1
+    part, w, ctx, x, _ = a_layer(H, before, brings)
+    want = heads_of(monkeypatch, part, x, ctx)
+    values = {k: v.clone() for k, v in w.items()}
+    values["uv_weight"].view(H, DIM, RANK)[head] *= 2.0 ** power
+    part.bind(values)
+    got = heads_of(monkeypatch, part, x, ctx)
+    got[:, head] *= 2.0 ** -power
+    assert part.up_weight is not None and torch.equal(got, want)
+    keys = {k: v.clone() for k, v in w.items()}
+    keys["uk_weight"].view(H, DIM, RANK)[head] *= 2.0 ** power
+    keys["q_weight"].view(H, DIM + ROT, -1)[head, :DIM] *= 2.0 ** -power
+    part.bind(keys)
+    assert part.up_weight is not None and torch.equal(heads_of(monkeypatch, part, x, ctx), want)
+
+
+def test_small_values_keep_their_bits(monkeypatch):
+    """Values of 1e-7 lose 17 % in float16 without a factor; bounds as for ordinary ones."""
+    part, w, ctx, x, _ = a_layer(2, [0], [300], scales={"uv_weight": 1e-7})
+    from ayaka_py_b200 import ops
+    monkeypatch.setattr(ops, "latent_expanded_pays", lambda *a: True)
+    got = part.forward(x, None, ctx, SimpleNamespace(group=0, layer=0, writes=True)).double()
+    want = reference(x, w, 2, {"base": 50000.0, "dims": ROT, "layout": "halves"}, None, "head", 0)
+    assert part.up_weight is not None and float((got - want).norm() / want.norm()) < 8e-3
+
+
+def test_small_weights_keep_their_bits():
+    """One key takes all but 2e-9 of the weight and has a value of zero: what the others leave is the whole output.  Their weights
+    are rounded to float16 (2^-11 of each), their values too, the output to bfloat16: 2^-8 of the whole."""
+    from ayaka_py_b200 import ops
+    from ayaka_py_b200.cache import CacheGroupSpec
+    from ayaka_py_b200.parts.base import KVNeed
+    torch.manual_seed(1)
+    T = 200
+    need = KVNeed(kv_heads=1, head_dim=ROT, value_heads=1, value_dim=RANK)
+    cache, runner = context_for([CacheGroupSpec("g", need, 1)], "bfloat16", page_size=16, pages=20)
+    ctx, _ = step_of(cache, runner, {0: T})
+    rope, latent = cache.kv_layer(0, 0)
+    proj = torch.zeros(T, DIM + ROT + RANK + ROT, device="cuda")
+    proj[:, 0] = 1.25                                    # 20 with the first key
+    down = proj[:, DIM + ROT:]
+    down[0, 0] = 1.0                                     # the first latent: 16 in its first place
+    down[1:, RANK // 2:RANK] = torch.randn(T - 1, RANK // 2, device="cuda")
+    up = torch.zeros(2 * DIM, RANK, device="cuda")
+    up[0, 0] = 1.0
+    up[DIM:, RANK // 2:] = torch.randn(DIM, RANK // 2, device="cuda") / 16
+    up = up.to(torch.bfloat16)
+    factor = torch.tensor([512.0, 256.0], device="cuda")
+    scaled = (up.view(2, DIM, RANK) * factor[:, None, None]).to(torch.bfloat16).view(2 * DIM, RANK)
+    got = ops.latent_expanded(proj, latent, rope, scaled, factor, torch.ones(RANK, device="cuda"),
+                              torch.zeros(1, device="cuda"), 1.0, 0, ctx, ctx.tables[0], 1, 1e-12, False, 1.0, None, None).double()
+    c = down[:, :RANK].double()
+    c = c / torch.sqrt((c * c).mean(-1, keepdim=True) + 1e-12)
+    scores = (proj[:, :1].double() @ c[:, :1].T).masked_fill(torch.ones(T, T, device="cuda").triu(1).bool(), -math.inf)
+    want = torch.softmax(scores, dim=1) @ (c @ up[DIM:].double().T)
+    assert ops.tc_error() == 0 and float(want[1:].abs().max()) < 1e-6
+    assert float((got[1:] - want[1:]).norm() / want[1:].norm()) < 2.0 ** -8
