@@ -34,10 +34,11 @@ __device__ __forceinline__ int first_token(int pos0, int window) { return window
 
 __global__ void __launch_bounds__(THREADS)
 latent_expand_prepare_kernel(__nv_bfloat16* latent_pages, __nv_bfloat16* __restrict__ rope_pages, __half* q16, __nv_bfloat16* q_rot, float* q_scale,
-                             __nv_bfloat16* side, const float* proj, long long proj_stride, const float* __restrict__ norm_w, const float* __restrict__ up_scale,
-                             const float* __restrict__ freq, float gain, int rot_dims, int halves, const int* __restrict__ row_req, const int* __restrict__ positions,
-                             const int* __restrict__ table, int table_stride, int page_size, const int* __restrict__ req_q_start,
-                             const int* __restrict__ req_pos0, int num_req, int T, int H, int rank, float eps, int window) {
+                             __nv_bfloat16* side, const float* proj, long long proj_stride, const float* __restrict__ norm_w, const float* up_scale,
+                             const float* __restrict__ freq, float gain, int rot_dims, int halves, const int* __restrict__ row_req,
+                             const int* __restrict__ positions, const int* __restrict__ table, int table_stride, int page_size,
+                             const int* __restrict__ req_q_start, const int* __restrict__ req_pos0, int num_req, int T, int H, int rank, float eps,
+                             int window) {
   __shared__ float turn[ROT];                              // cos [rot_dims / 2], sin [rot_dims / 2]
   __shared__ float red[WARPS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
