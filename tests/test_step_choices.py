@@ -79,3 +79,18 @@ def test_latent_attention_expands_keys_and_values_where_that_is_the_faster_form(
     pages = SimpleNamespace(shape=(4000, 16, 1, 512))
     assert ops.latent_expanded_pays(step(plan), heads, 512, window, pages, SMS) is expanded
     assert not ops.latent_expanded_pays(step(plan), heads, 512, window, SimpleNamespace(shape=(4000, 12, 1, 512)), SMS)
+
+
+@pytest.mark.parametrize("requests", [1, 2, 23, 24, 25, 60])
+@pytest.mark.parametrize("rows,past,most,within", [(256, 128.0, np.inf, True), (16, 8.0, 100, True), (8, 16.0, 320.0, False), (1, 0.5, np.inf, False)])
+def test_sums_over_a_steps_requests_are_the_same_for_few_and_for_many(requests, rows, past, most, within):
+    """Few requests are summed in a loop, many by NumPy."""
+    rng = np.random.default_rng(requests)
+    plan = [(int(p), int(n)) for p, n in zip(rng.integers(0, 2000, requests), rng.integers(1, 600, requests))]
+    tiles = [-(-n // rows) for _, n in plan]
+    keys = [min(p + n / 2 + past, most, p + n if within else np.inf) for p, n in plan]
+    got = ops._portions(step(plan), rows, past, most, within)
+    assert got[0] == sum(tiles) and got[1] == sum(t * k for t, k in zip(tiles, keys))
+    for window in (None, 1, 70, 4096):
+        held = sum(p + n - (0 if window is None else max(p - window + 1, 0) // 64 * 64) for p, n in plan)
+        assert ops._latent_expanded_rows(step(plan), window) == held
