@@ -663,6 +663,7 @@ def _latent_expanded_rows(ctx, window: int | None) -> int:
     return ctx.host[key]
 
 
+GRID_TILES = 65535        # row tiles of the tcgen05 attention of wide heads: the second dimension of its grid
 LATENT_EXPANDED_BYTES = 256 << 20         # at most this much for a step's expanded keys and values
 
 
@@ -676,6 +677,8 @@ def latent_expanded_pays(ctx, heads: int, rank: int, window: int | None, pages: 
     24 x 8 behind 500 95, 118; 64 x 2 behind 500 97, 150."""
     P = pages.shape[1]
     if ctx.max_q_len == 1 or "counts" not in ctx.host or P < 8 or P & (P - 1) or pages.shape[0] * P >= 1 << 31:
+        return False
+    if ctx.num_rows // 256 + ctx.num_requests > GRID_TILES:
         return False
     key = ("latent_expanded", heads, rank, window)
     if key not in ctx.host:
@@ -1094,6 +1097,8 @@ def _grouped_wide_pays(ctx, heads: int, groups: int, window: int | None, chunk: 
     over 2 to 8 key heads; 1 to 32 requests of 2 to 1,024 rows, contexts of 2 to 1,924 keys): the choice is on average
     0.3 % behind the faster form, more than 6 % in 6 of them.  Measured, mma.sync and tcgen05, 16 heads over 4: one prompt of 32 rows 7.5, 7.9, of
     128 12.0, 9.8, of 1,024 63, 28; 8 of 512 78, 27; 2 rows behind 500 keys 25, 19; 32 requests of 2 rows behind 500 26, 38."""
+    if heads % groups or ctx.num_rows // 128 + ctx.num_requests > GRID_TILES:
+        return False                       # the other form takes these, or says what is wrong
     if "counts" not in ctx.host:
         return True
     key = ("grouped_wide", heads, groups, window, chunk)

@@ -94,3 +94,11 @@ def test_sums_over_a_steps_requests_are_the_same_for_few_and_for_many(requests, 
     for window in (None, 1, 70, 4096):
         held = sum(p + n - (0 if window is None else max(p - window + 1, 0) // 64 * 64) for p, n in plan)
         assert ops._latent_expanded_rows(step(plan), window) == held
+
+
+def test_steps_beyond_the_grid_and_heads_that_do_not_divide_stay_with_the_other_forms():
+    many = step([(0, 2)] * 65500)                          # 1,023 + 65,500 tiles of 128 rows at most
+    assert not ops._grouped_wide_pays(many, 16, 4, None, None, SMS)
+    assert not ops.latent_expanded_pays(step([(0, 1024)] * 65500), 16, 512, None, SimpleNamespace(shape=(4000, 16, 1, 512)), SMS)
+    assert not ops._grouped_wide_pays(step([(0, 512)]), 2, 4, None, None, SMS)            # refused by the kernel's own checks
+    assert not ops._grouped_wide_pays(step([(0, 512)]), 6, 4, None, None, SMS)
