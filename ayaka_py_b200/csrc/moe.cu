@@ -1030,7 +1030,7 @@ namespace {
 template <typename O, bool GLU>
 int gemv(O* out, const __nv_bfloat16* a, long long a_stride, const __nv_bfloat16* w, const int* ids, int pairs, int top, int gather, int N,
          int N_w, int Kd, float limit, float slope, float plus, int act, const float* early, cudaStream_t stream) {
-  if ((long long)pairs * N * Kd < GV_LINE) {
+  if ((long long)pairs * N * Kd < GV_LINE || top > GV_MOST) {       // a launch below holds whole tokens
     ayk_launch(moe_pair_gemv_kernel<O, GLU>, dim3(pairs, (N + pv_cols(GLU) - 1) / pv_cols(GLU)), dim3(256), (size_t)Kd * sizeof(float), stream,
                out, a, a_stride, w, ids, top, gather, N, N_w, Kd, limit, slope, plus, act, early);
     return ayk_check_launch("ayk_moe_gemv");
@@ -1061,7 +1061,7 @@ AYK_EXPORT int ayk_moe_gemv(void* out, const void* a, long long a_stride, const 
                             cudaStream_t stream) {
   if (pairs == 0 || N == 0) return 0;
   AYK_REQUIRE(ayk_moe_gemv_takes(Kd, a_stride), "ayk_moe_gemv: rows of %d elements (stride %lld)", Kd, a_stride);
-  AYK_REQUIRE(top >= 1 && top <= GV_MOST, "ayk_moe_gemv: %d choices a row", top);
+  AYK_REQUIRE(top >= 1, "ayk_moe_gemv: %d choices a row", top);
   const __nv_bfloat16 *rows = (const __nv_bfloat16*)a, *weights = (const __nv_bfloat16*)w;
   if (glu)
     return gemv<__nv_bfloat16, true>((__nv_bfloat16*)out, rows, a_stride, weights, ids, pairs, top, gather, N, N_w, Kd, limit, slope, plus, act, early, stream);

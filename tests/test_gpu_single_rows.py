@@ -75,3 +75,18 @@ def test_single_rows_of_heads_that_share_their_keys(H, G, D, page, window, keep,
         # the weights enter the second product as bfloat16 (2^-9 of each), the result is rounded to bfloat16 twice
         assert float((got - want).abs().max()) < 1.5e-2 * float(want.abs().max())
     cache.rollback(res)
+
+
+def test_more_choices_a_row_than_a_grouped_launch_holds():
+    """Routes that a caller made: 130 experts a row."""
+    from ayaka_py_b200 import ops
+    T, top, N, K = 2, 130, 256, 512
+    assert T * top * N * K >= 20 << 20
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    a = torch.randn(T, K, generator=gen, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(top, N, K, generator=gen, device="cuda") / K ** 0.5).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(top, generator=gen, device="cuda") for _ in range(T)]).to(torch.int32)
+    route = ops.MoeRoute(ids, torch.ones(T, top, device="cuda"), None, None, 0, top)
+    got = ops.moe_gemv(a, w, route, glu=None, activation="relu2").double().view(T, top, N)
+    want = torch.einsum("tk,tenk->ten", a.double(), w.double()[ids.long()]).clamp(min=0.0) ** 2
+    assert bool(((got - want).abs() <= want * 2.0 ** -8 + 1e-5).all())
