@@ -87,13 +87,13 @@ def set_staged(on: bool) -> None:
     _ready().ayk_gemm_tc_prefill_staged(ctypes.c_int(1 if on else 0))
 
 
-def prefill_plan(M: int, N: int, K: int, sms: int = 148, wide_rows: bool = False) -> tuple[int, int]:
+def prefill_plan(M: int, N: int, K: int, sms: int = 148, wide_rows: bool = False, residual: bool = True) -> tuple[int, int]:
     """(tile width, parts of K per tile) that ``gemm_tc_prefill`` picks for an [M, K] x [N, K]^T product
-    on ``sms`` SMs; ``wide_rows``: the epilogue reads or writes 32-bit rows.  Host arithmetic from the
-    kernel's fitted time model: works without a GPU."""
+    on ``sms`` SMs; ``wide_rows``: float32 rows out, over a float32 residual or (``residual`` False) without one.  Host arithmetic from the
+    kernel's fitted time models, one for each of the three: works without a GPU."""
     tile, parts = ctypes.c_int(0), ctypes.c_int(0)
     library().ayk_gemm_tc_prefill_plan(ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K), ctypes.c_int(sms),
-                                       ctypes.c_int(1 if wide_rows else 0), ctypes.byref(tile), ctypes.byref(parts))
+                                       ctypes.c_int(0 if not wide_rows else 1 if residual else 2), ctypes.byref(tile), ctypes.byref(parts))
     return tile.value, parts.value
 
 

@@ -67,7 +67,7 @@ def test_a_split_fits_the_sms_and_the_tile():
 
 
 def test_wide_rows_keep_to_the_staged_widths_when_it_pays():
-    # 32-bit rows in and out: 192 columns go through the staged epilogue, 256 do not
+    # 32-bit rows in and out, both widths through the staged epilogue: at 256 columns it has room for one buffer beside three stages
     assert ops.prefill_plan(2048, 1600, 6400, wide_rows=True)[0] == 192
     assert ops.prefill_plan(2048, 1600, 1600, wide_rows=True)[0] == 192
 
@@ -79,3 +79,12 @@ def test_wide_rows_keep_to_the_staged_widths_when_it_pays():
 def test_plan_over_a_residual_is_the_measured_best(M, N, K, plan):
     # the best of 8 widths, whole and split by 2, 4 and 8, each measured with a float32 residual
     assert ops.prefill_plan(M, N, K, wide_rows=True) == plan
+
+
+@pytest.mark.parametrize("M,N,K,plan", [
+    (130, 2048, 2048, (64, 2)), (300, 3664, 2048, (96, 1)), (300, 1024, 2048, (64, 2)), (576, 3088, 2048, (128, 1)), (700, 2048, 1408, (96, 1)),
+    (1024, 3664, 2048, (224, 1)), (1024, 2048, 2048, (128, 1)), (1801, 1600, 1024, (96, 1)), (2048, 3088, 2048, (192, 1)), (2048, 4096, 1024, (160, 1)),
+    (2048, 2048, 4096, (256, 1)), (512, 1280, 5120, (96, 2)), (1400, 1024, 8192, (192, 2))])
+def test_plan_of_float32_rows_without_a_residual_is_the_measured_best(M, N, K, plan):
+    """The best of 8 widths, whole and split by 2, 4 and 8, each measured.  (Of a fourteenth shape, 1801 x 3664 x 2048, the plan is 6 % behind.)"""
+    assert ops.prefill_plan(M, N, K, wide_rows=True, residual=False) == plan
