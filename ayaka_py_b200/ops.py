@@ -1467,15 +1467,16 @@ def moe_gemm(a: torch.Tensor, w: torch.Tensor, route: MoeRoute, glu: tuple | Non
 
 
 def moe_gemv_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether the pair-by-pair product takes these operands (bfloat16, rows in whole 16-byte pieces)."""
+    """Whether the product of a few pairs takes these operands (bfloat16, rows in whole 16-byte pieces)."""
     return (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
             and bool(_ready().ayk_moe_gemv_takes(ctypes.c_int(w.shape[2]), ctypes.c_longlong(a.stride(0)))))
 
 
 def moe_gemv(a: torch.Tensor, w: torch.Tensor, route: MoeRoute, glu: tuple | None, activation: str | None = None,
              weigh_input: bool = False) -> torch.Tensor:
-    """The experts' product for a handful of pairs, each pair streaming its expert's matrix on its own: no
-    sorting, rows lie pair by pair (token-major).  ``glu`` = (limit, slope): a [T, K] tokens' rows, w
+    """The experts' product for a handful of pairs, bound by the stream of their experts' matrices: small ones pair by pair, each streaming
+    its expert's on its own, larger ones with the pairs of one expert (up to eight) sharing a stream.  No sorting, rows lie pair by
+    pair (token-major).  ``glu`` = (limit, slope): a [T, K] tokens' rows, w
     [experts, 2 N, K], bfloat16 activations [T * top, N]; ``activation``: a [T, K], w [experts, N, K], bfloat16
     activations of the product; neither: a [T * top, K], w [experts, N, K], float32 out.  ``weigh_input``: as in
     ``moe_gemm``."""

@@ -24,7 +24,7 @@ The experts' matrices are kept stacked ([experts, 2 inner, width] with gate over
 [experts, width, inner]); a step sorts its (token, choice) pairs by expert on the device and runs
 two grouped products over the sorted rows, so nothing about the routing comes back to the host
 (``csrc/moe.cu``): on tcgen05 for bfloat16 steps of many pairs (every expert's rows padded to whole
-128-row tiles), pair by pair as matrix-vector products for a handful of pairs, on mma.sync or the
+128-row tiles), streaming the chosen experts' matrices for a handful of pairs, on mma.sync or the
 FP32 pipes otherwise.  The router and the shared expert's gate, up and mixing row are one dense product."""
 
 from __future__ import annotations
@@ -144,7 +144,7 @@ class MoE(FeedForward):
             return picked, rows, route, logits
         glu = glu if act is None else None
         if few:
-            # a handful of pairs (a step of single tokens): every pair streams its expert's matrices on its own
+            # a handful of pairs (a step of single tokens): the experts' matrices are streamed, by pairs or by groups of one expert's pairs
             hidden = ops.moe_gemv(h, self.in_weight, route, glu=glu, activation=act, weigh_input=early)
             return ops.moe_gemv(hidden, self.down_weight, route, glu=None), None, route, logits            # [T * K, d]
         hidden = ops.moe_gemm(h, self.in_weight, route, glu=glu, out_dtype=self.dtype, activation=act, weigh_input=early)

@@ -827,12 +827,12 @@ def run_luporax(width: int, layers: int, batch: int, steps: int, warmup: int, pk
                 kernel("experts on tcgen05: plan, gather, gate | up, activation, down (prefill)", ms,
                        gflop=2.0 * 2 * rows * 3 * width * d / 1e9, like="linear + gelu")
             else:
-                touched = 2 * rows * 2 * width * d * 2 / 1e9          # every pair streams its expert's rows
+                touched = int(route.ids.unique().numel()) * 2 * width * d * 2 / 1e9          # the chosen experts' matrices, once each
                 ms = timed(lambda: ops.moe_gemv(h, ff.in_weight, route, glu=(7.0, 1.702)))
-                kernel("experts' gate | up product + activation, pair by pair (decode)", ms, gbytes=touched, like="linear (decode)")
+                kernel("experts' gate | up product + activation, few pairs (decode)", ms, gbytes=touched, like="linear (decode)")
                 hidden = ops.moe_gemv(h, ff.in_weight, route, glu=(7.0, 1.702))
                 ms = timed(lambda: ops.moe_gemv(hidden, ff.down_weight, route, glu=None))
-                kernel("experts' down product, pair by pair (decode)", ms, gbytes=touched / 2, like="linear (decode)")
+                kernel("experts' down product, few pairs (decode)", ms, gbytes=touched / 2, like="linear (decode)")
                 ms = timed(lambda: ops.moe_gemm(h, ff.in_weight, route, glu=(7.0, 1.702), out_dtype=bf))
                 kernel("grouped gate | up product + activation on mma.sync (decode; not the path taken)", ms,
                        gbytes=min(16, 2 * rows) * 2 * width * d * 2 / 1e9, like="linear (decode)")
@@ -1348,8 +1348,9 @@ def run_tesozen(width: int, layers: int, batch: int, steps: int, warmup: int, pk
                     kernel("experts on tcgen05: plan, gather, gate | up, silu gating, down (prefill)", name, ms,
                            gflop=2.0 * 2 * rows * 3 * width * d / 1e9, like="experts on tcgen05")
                 else:
+                    chosen = int(route.ids.unique().numel())              # their matrices are read once each
                     ms = timed(lambda: ops.moe_gemv(h, ff.in_weight, route, glu=(inf, 1.0, 0.0)))
-                    kernel("experts' gate | up product + silu gating, pair by pair (decode)", name, ms, gbytes=2 * rows * 2 * width * d * 2 / 1e9,
+                    kernel("experts' gate | up product + silu gating, few pairs (decode)", name, ms, gbytes=chosen * 2 * width * d * 2 / 1e9,
                            like="experts' gate | up product")
                 dn = model.blocks[3].ffn if len(model.blocks) > 3 else None
                 if dn is not None:
@@ -1399,8 +1400,9 @@ def run_tesozen(width: int, layers: int, batch: int, steps: int, warmup: int, pk
                     kernel("experts on tcgen05: plan, gather, gate | up, activation, down (prefill)", name, ms,
                            gflop=2.0 * 2 * rows * 3 * width * d / 1e9)
                 else:
+                    chosen = int(route.ids.unique().numel())              # their matrices are read once each
                     ms = timed(lambda: ops.moe_gemv(h, ff.in_weight, route, glu=(7.0, 1.702)))
-                    kernel("experts' gate | up product + activation, pair by pair (decode)", name, ms, gbytes=2 * rows * 2 * width * d * 2 / 1e9)
+                    kernel("experts' gate | up product + activation, few pairs (decode)", name, ms, gbytes=chosen * 2 * width * d * 2 / 1e9)
             cache.rollback(res)
             for sl in slots:
                 cache.close(sl)
@@ -1534,8 +1536,9 @@ def run_murutar(width: int, layers: int, batch: int, steps: int, warmup: int, pk
                     ms = timed(lambda: ops.stream_update(xr, picked, rec.gate2.scale, gate=gate, post="copy", out_dtype=bf))
                     kernel("experts' weighted sum + gated update + copy (prefill)", name, ms, gbytes=rows * d * 22 / 1e9, like="experts' weighted sum")
                 else:
+                    chosen = int(route.ids.unique().numel())              # their matrices are read once each
                     ms = timed(lambda: ops.moe_gemv(h, ff.in_weight, route, glu=None, activation="relu2"))
-                    kernel("experts' up product + squared ReLU, pair by pair (decode)", name, ms, gbytes=2 * rows * ff.inner * d * 2 / 1e9,
+                    kernel("experts' up product + squared ReLU, few pairs (decode)", name, ms, gbytes=chosen * ff.inner * d * 2 / 1e9,
                            like="experts' gate | up product")
                 if dn is not None:
                     n = dn.stack.weight.shape[0]
@@ -1591,8 +1594,9 @@ def run_murutar(width: int, layers: int, batch: int, steps: int, warmup: int, pk
                     ms = timed(lambda: ops.moe_combine(picked, route, shared, None, where))
                     kernel("experts' weighted sum (prefill)", name, ms, gbytes=rows * d * 16 / 1e9)
                 else:
+                    chosen = int(route.ids.unique().numel())              # their matrices are read once each
                     ms = timed(lambda: ops.moe_gemv(h, ff.in_weight, route, glu=(float("inf"), 1.0, 0.0)))
-                    kernel("experts' gate | up product + silu gating, pair by pair (decode)", name, ms, gbytes=2 * rows * 2 * width * d * 2 / 1e9)
+                    kernel("experts' gate | up product + silu gating, few pairs (decode)", name, ms, gbytes=chosen * 2 * width * d * 2 / 1e9)
                 if dn is not None:
                     ms = timed(lambda: ops.linear(h, dn.up_weight, None, activation="relu2", out_dtype=bf))
                     kernel(f"linear {rows}x{dn.inner}x{d} + squared ReLU ({label})", name, ms, gflop=2.0 * rows * dn.inner * d / 1e9)
@@ -1758,12 +1762,13 @@ def run_tomodra(width: int, layers: int, batch: int, steps: int, warmup: int, pk
                        like=like("experts on tcgen05"))
                 picked, where = ops.moe_experts_tc(h, ff.in_weight, ff.down_weight, route, inf, 1.0, 0.0)
             else:
+                chosen = int(route.ids.unique().numel())              # their matrices are read once each
                 ms = timed(lambda: ops.moe_gemv(h, ff.in_weight, route, glu=(inf, 1.0, 0.0), weigh_input=mine))
-                kernel("experts' gate | up product + silu gating, pair by pair (decode)", name, ms, gbytes=2 * rows * 2 * width * d * 2 / 1e9,
+                kernel("experts' gate | up product + silu gating, few pairs (decode)", name, ms, gbytes=chosen * 2 * width * d * 2 / 1e9,
                        like=like("experts' gate | up product"))
                 hidden = ops.moe_gemv(h, ff.in_weight, route, glu=(inf, 1.0, 0.0))
                 ms = timed(lambda: ops.moe_gemv(hidden, ff.down_weight, route, glu=None))
-                kernel("experts' down product, pair by pair (decode)", name, ms, gbytes=2 * rows * width * d * 2 / 1e9, like=like("experts' down product"))
+                kernel("experts' down product, few pairs (decode)", name, ms, gbytes=chosen * width * d * 2 / 1e9, like=like("experts' down product"))
                 picked, where = ops.moe_gemv(hidden, ff.down_weight, route, glu=None), None
             shared = torch.randn(rows, d, device="cuda")
             if mine:
