@@ -26,6 +26,8 @@ product makes the step's keys and values from the latents, and the rows attend t
 
 from __future__ import annotations
 
+import math
+
 import torch
 
 from .. import ops
@@ -41,11 +43,12 @@ def _float16_scale(up: torch.Tensor, norm: torch.Tensor, rows: int) -> torch.Ten
     [2^14, 2^15).  (A latent is at most sqrt(rank) times its norm's largest weight long, so no product can be larger than that times the
     longest row.)  None where a product could leave float16 without a factor, or where some rows are so small that they need more than
     2^40; rows of zeros need none."""
-    longest = up.double().norm(dim=1).view(-1, rows).amax(dim=1) * (norm.abs().max() * up.shape[1] ** 0.5)
-    if not bool((longest < 30000.0).all()):
+    longest = torch.linalg.vector_norm(up, dim=1, dtype=torch.float64).view(-1, rows).amax(dim=1) * (norm.abs().max() * up.shape[1] ** 0.5)
+    longest = longest.tolist()                             # the only wait for the device
+    powers = [15 - math.frexp(n)[1] if n > 0 else 0 for n in longest if n < 30000.0]
+    if len(powers) < len(longest) or max(powers) > 40:
         return None
-    power = torch.where(longest > 0, 15 - torch.frexp(longest).exponent, 0)
-    return None if int(power.max()) > 40 else torch.ldexp(torch.ones_like(longest), power).float()
+    return torch.tensor([2.0 ** k for k in powers], dtype=torch.float32, device=up.device)
 
 
 class LatentAttention(Mixer):
@@ -109,7 +112,8 @@ class LatentAttention(Mixer):
             up = torch.cat([self.uk_weight, self.uv_weight])
             self.up_scale = _float16_scale(up, self.down_norm, 128)
             if self.up_scale is not None:
-                self.up_weight = up.mul_(self.up_scale.repeat_interleave(128)[:, None].to(up.dtype))
+                up.view(2 * H, 128, self.rank).mul_(self.up_scale[:, None, None])
+                self.up_weight = up
         self.uv_heads = self.uv_weight.view(H, self.vdim, self.rank)                                   # [H, vdim, rank]
 
     def cache_need(self):
