@@ -407,7 +407,7 @@ int launch(const GroupedArgs& a, int page_shift, int tq, int DKP, int qrows, siz
 // and registers of O += P V.  A piece of 16 bytes lies at its number XOR the low bits of its key, which leaves ldmatrix without bank
 // conflicts.  Three blocks to a multiprocessor (64 KB each for heads of 128).
 // Measured, the rotary layer of width 2,048, 16 heads over 4 key heads of 128, against the form of the kernel above in which the
-// block's warps share each tile of 64 keys behind a barrier (us): 32 requests of 1,900 keys 64.0 -> 46.7 (this kernel 47 -> 26, 4.2 TB/s),
+// block's warps share each tile of 64 keys behind a barrier (us): 32 requests of 1,900 keys 64.0 -> 46.7 (this kernel 47 -> 26, 4.3 TB/s),
 // 17 of 1,900 56.9 -> 40.9, 8 of 1,900 39.0 -> 28.7, 32 of 250 29.1 -> 24.0, 1 of 30 18.5 -> 16.4; none of 80 steps slower.  A warp to an
 // item, with no sums to meet, was slower for short parts (8 of 250: 22.6 against 19.9) and no faster for long ones (47.2).
 constexpr int GD_WARPS = 4, GD_STAGES = 2, GD_KEYS = 16, GD_HEADS = 8;

@@ -24,7 +24,7 @@
 // end (queries and keys of all blocks at once) and 3,700 behind the last one.  The instructions are fetched by far more code than the
 // first-level caches hold, so every loop is as short as it can be: unrolled copies of the waits and products alone had made it 25 us.
 // Measured, 16 heads over 4 key heads of 128: 2 prompts of 1,024 tokens in chunks of 512 53 -> 19.4 us (mma.sync form, this), the layer of width 2,048
-// 120.5 -> 86.6; 1 prompt of 1,024 63 -> 28; 128 rows 12.0 -> 9.8.
+// 120.5 -> 85.8; 1 prompt of 1,024 63 -> 28; 128 rows 12.0 -> 9.8.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <math.h>

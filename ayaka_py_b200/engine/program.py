@@ -246,11 +246,12 @@ class BlockProgram:
         self.width, self.device = widths.pop(), builder.keep[0].device
         self.groups = sorted({op.i[6] for op in builder.ops if op.kind == OP_ATTENTION})       # whose tables the operations read
         # what the operations were recorded from: the block's parts, all that the parts hold, and where every tensor lay
-        self.held = [(part, list(vars(part)), list(vars(part).values())) for part in self.parts.values()]
+        self.held = [(part, list(vars(part).values())) for part in self.parts.values()]
         groups = {b.group for b in caches.values() if b is not None}
         self.pages = [(g, cache.kv[g]) for g in groups]
         kept = [*builder.keep, *(t for _, pair in self.pages for t in pair)]
-        self.places = [(t, t.data_ptr()) for t in {id(t): t for t in kept}.values()]
+        self.tensors = list({id(t): t for t in kept}.values())
+        self.places = [t.data_ptr() for t in self.tensors]
 
     def current(self, block, cache) -> bool:
         """Whether the parts and the cache still hold what the operations were recorded from: other parts, weights, constants or pages, in
@@ -258,17 +259,14 @@ class BlockProgram:
         for name, part in self.parts.items():
             if getattr(block, name) is not part:
                 return False
-        for part, names, values in self.held:
-            have = vars(part)
-            if list(have) != names or not all(map(operator.is_, have.values(), values)):
+        for part, values in self.held:
+            have = vars(part).values()
+            if len(have) != len(values) or not all(map(operator.is_, have, values)):
                 return False
         for g, pair in self.pages:
             if cache.kv[g] is not pair:
                 return False
-        for tensor, place in self.places:
-            if tensor.data_ptr() != place:
-                return False
-        return True
+        return [t.data_ptr() for t in self.tensors] == self.places
 
     def takes(self, x: torch.Tensor, ctx) -> bool:
         """Whether the stream is this block's rows of this step, and the step's arrays are as the kernels read them.  The parts' own
@@ -277,26 +275,28 @@ class BlockProgram:
             return False
         if ctx.req_pos0.numel() != ctx.num_requests:
             return False
-        arrays = (ctx.positions, ctx.row_req, ctx.req_q_start, ctx.req_pos0, *(ctx.tables[g] for g in self.groups))
-        return all(t is not None and t.dtype == torch.int32 and t.device == self.device and t.is_contiguous() for t in arrays)
+        where = x.get_device()
+        for t in (ctx.positions, ctx.row_req, ctx.req_q_start, ctx.req_pos0, *[ctx.tables[g] for g in self.groups]):
+            if t is None or t.dtype != torch.int32 or t.get_device() != where or not t.is_contiguous():
+                return False
+        return True
 
     def run(self, x: torch.Tensor, ctx) -> torch.Tensor:
         """The block over a stream that it ``takes``, in place."""
-        T, cache, step = ctx.num_rows, ctx.cache, _Step()
-        size = sum((T * b + 255) // 256 * 256 for b in self.row_bytes)
+        T, cache = ctx.num_rows, ctx.cache
+        size = sum([(T * b + 255) // 256 * 256 for b in self.row_bytes])
         single = ctx.num_requests if ctx.max_q_len == 1 else ctx.num_single             # rows that take the decode kernels
         floats = single * self.floats * -(-cache.max_len // ops.DECODE_PART)
         workspace = torch.empty(size + 4 * floats or 256, dtype=torch.uint8, device=x.device)
-        step.T, step.R, step.num_single, step.max_q_len = T, ctx.num_requests, ctx.num_single, ctx.max_q_len
-        step.max_context, step.settled = cache.max_len, 1 if ctx.earlier_rows_settled else 0
-        step.positions, step.row_req = ctx.positions.data_ptr(), ctx.row_req.data_ptr()
-        step.req_q_start, step.req_pos0 = ctx.req_q_start.data_ptr(), ctx.req_pos0.data_ptr()
+        at = workspace.data_ptr()
+        step = _Step(T, ctx.num_requests, 0, ctx.num_single, ctx.max_q_len, cache.max_len, 1 if ctx.earlier_rows_settled else 0, 0,
+                     None, ctx.positions.data_ptr(), ctx.row_req.data_ptr(), None, ctx.req_q_start.data_ptr(), ctx.req_pos0.data_ptr())
         for g in self.groups:
             table = ctx.tables[g]
             step.tables[g], step.table_stride[g] = table.data_ptr(), table.stride(0)
-        step.workspace, step.workspace_bytes, step.stream = workspace.data_ptr(), size, x.data_ptr()
+        step.workspace, step.workspace_bytes, step.stream = at, size, x.data_ptr()
         if floats:
-            step.decode_scratch, step.decode_scratch_floats = workspace.data_ptr() + size, floats
+            step.decode_scratch, step.decode_scratch_floats = at + size, floats
         launched = ctypes.c_int(0)
         code = self.lib.ayk_program_run(self.ops, self.n_ops, self.buffers, len(self.row_bytes), ctypes.byref(step), ctypes.byref(launched),
                                         ops._stream())

@@ -28,15 +28,18 @@ class PreNormBlock(Block):
 
     def _program(self, x, ctx, caches):
         """The block as one call into the library (``engine/program.py``), where its parts can be lowered: nine launches from Python took 13 us
-        each and bounded every step of up to a few hundred rows (a layer of the small GPT-2 shape, 8 single rows beside 60 rows: 126 ->
-        42 us; of the XL shape, 2 beside 8 rows 132 -> 41).  Made at the second call with a cache: it takes about 70 us, which a caller
-        that comes once would not get back."""
+        each and bounded every step of up to a few hundred rows (a layer of the small GPT-2 shape, 8 single rows beside 60 rows: 128 ->
+        49 us; of the XL shape, 2 beside 8 rows 138 -> 47; 4 of these are the comparison with what the program was recorded from).  For callers
+        of a block: an engine's steps run whole models as one program.  Made at the second call with a cache: it takes about 70 us, which a
+        caller that comes once would not get back."""
         from ..engine.program import BlockProgram, native_allowed
         if not native_allowed(x.device):
             return None
         binding = caches.get("mixer")
         try:
-            programs = self._programs.setdefault(ctx.cache, {})
+            programs = self._programs.get(ctx.cache)
+            if programs is None:
+                programs = self._programs.setdefault(ctx.cache, {})
         except TypeError:                                  # a cache that cannot be a weak key
             return None
         key = (ctx.dtype, None if binding is None else (binding.group, binding.layer, binding.writes))
