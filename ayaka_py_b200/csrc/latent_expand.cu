@@ -17,7 +17,7 @@
 // can hold to [2^14, 2^15), 28 powers of two above float16's smallest of full precision.  The keys' factor is also on the rotated
 // query parts, whose keys have none, and q_scale takes both out; the values' is taken out with the softmax's sum.
 // Bound by the projection's 32-bit rows (14.6 KB a row at 16 heads): 11 us for 1,801 rows, 41 MB.
-// Measured, the layer of width 2,048 (16 heads, latent 512 + 64), 1,024 + 777 rows: 280 -> 105 us (absorbed attention 176, its two products per
+// Measured, the layer of width 2,048 (16 heads, latent 512 + 64), 1,024 + 777 rows: 280 -> 104 us (absorbed attention 176, its two products per
 // head 52, preparation 19; now preparation 11, keys and values 13, attention 28); error against 64 bits 3.2e-3 -> 2.8e-3, and over 23
 // drawn steps 0.69 to 1.00 of what it was.
 #include <cuda_fp16.h>
